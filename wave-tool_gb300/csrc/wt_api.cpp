@@ -168,12 +168,8 @@ wt_status run_displace(const wt_patch* patches, uint32_t n_patches, const wt_wav
         return fail(WT_ERR_INVALID_ARG, "nrm_out misaligned for its layout");
     }
     if (n_patches == 0) return WT_OK;
-    cudaError_t e = wt::launch_prep(patches, n_patches, waves, n_waves, P.hm, cap, 32u * cfg.s, ws, P.L, s);
-    if (e != cudaSuccess) return cuda_fail(e, "prep launch");
-    if (flags & WT_PHASE_FP32_NAIVE)
-        e = wt::launch_forward_naive(patches, n_patches, waves, P.hm, pos, nrm, flags, ws, P.L, cap, s);
-    else
-        e = wt::launch_forward(cfg, patches, n_patches, P.hm, pos, nrm, flags, ws, P.L, extra, s);
+    const cudaError_t e = wt::launch_displace(cfg, patches, n_patches, waves, n_waves, P.hm, pos, nrm, cap, flags, ws,
+                                              P.L, extra, s);
     if (e != cudaSuccess) return cuda_fail(e, "forward launch");
     return WT_OK;
 }

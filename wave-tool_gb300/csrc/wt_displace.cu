@@ -29,6 +29,8 @@
 #include <cstdint>
 
 #include "wt_device.cuh"
+#include "wt_forward.cuh"
+#include "wt_prep.cuh"
 #include "wt_internal.h"
 
 namespace wt {
@@ -36,7 +38,6 @@ namespace {
 
 using namespace wt::dev;
 
-constexpr uint32_t kNoPatch = 0xffffffffu;
 constexpr int kSortBins = 1024;         // wave counts >= 1023 share the last bin
 constexpr uint32_t kWaveMaskWords = 512;  // waves validated into a shared bitmask up to 16384
 constexpr uint32_t kRankSortMax = 64;
@@ -47,105 +48,7 @@ __device__ __forceinline__ void flag_error(WsHeader* h, uint32_t code, uint32_t 
     atomicMin(&h->bad_patch, patch);
 }
 
-__device__ __forceinline__ bool finitef(float x) { return isfinite(x); }
-
-__device__ bool wave_ok(const wt_wave& w) {
-    bool lam_ok = (w.wavelength > 0.0f) && !isnan(w.wavelength);  // +inf allowed (k = 0)
-    return lam_ok && finitef(w.amplitude) && finitef(w.dir_x) && finitef(w.dir_z) &&
-           finitef(w.steepness_q) && finitef(w.speed) && finitef(w.phase);
-}
-
-__device__ __forceinline__ unsigned long long to_fixed_turns(double turns) {
-    double f = turns - floor(turns);                 // [0, 1)
-    double hi = floor(f * 4294967296.0);             // < 2^32
-    double lo = floor((f * 4294967296.0 - hi) * 4294967296.0);
-    return ((unsigned long long)hi << 32) | (unsigned long long)lo;
-}
-
-// positive remainder of x by m (FP64)
-__device__ __forceinline__ double pmod(double x, double m) {
-    double r = x - m * floor(x / m);
-    return r >= m ? r - m : (r < 0.0 ? r + m : r);
-}
-
-// FP64 constants of wave w on patch Pt (the phase on the patch's bilinear grid
-// as 64-bit fixed-point turns, and the FP32 coefficients of the eight sums).
-__device__ PairCoef make_pair_coef(const wt_patch& Pt, const wt_wave w) {
-    double lam = w.wavelength;
-    double inv_lam = isinf(lam) ? 0.0 : 1.0 / lam;     // k / 2pi
-    double k = kTwoPi * inv_lam;
-    double Dx = w.dir_x, Dz = w.dir_z, A = w.amplitude, Q = w.steepness_q;
-    double blx = Pt.bl[0], blz = Pt.bl[1];
-    double e1x = (double)Pt.br[0] - blx, e1z = (double)Pt.br[1] - blz;
-    double e2x = (double)Pt.tl[0] - blx, e2z = (double)Pt.tl[1] - blz;
-    double e3x = (double)Pt.tr[0] - Pt.tl[0] - Pt.br[0] + blx;
-    double e3z = (double)Pt.tr[1] - Pt.tl[1] - Pt.br[1] + blz;
-    const double inv_cm1 = 1.0 / (double)(Pt.cols - 1), inv_rm1 = 1.0 / (double)(Pt.rows - 1);
-    // theta / 2pi at (col, row) = t00 + col*ta + row*tb + col*row*tg
-    double t00 = (Dx * blx + Dz * blz) * inv_lam + (double)w.speed * Pt.time_s * inv_lam +
-                 (double)w.phase * (1.0 / kTwoPi);
-    double ta = (Dx * e1x + Dz * e1z) * inv_lam * inv_cm1;
-    double tb = (Dx * e2x + Dz * e2z) * inv_lam * inv_rm1;
-    double tg = (Dx * e3x + Dz * e3z) * inv_lam * (inv_cm1 * inv_rm1);
-    PairCoef c;
-    c.t00 = to_fixed_turns(t00);
-    c.ta = to_fixed_turns(ta);
-    c.tb = to_fixed_turns(tb);
-    c.tg = to_fixed_turns(tg);
-    c.qadx = (float)(Q * A * Dx);
-    c.a = (float)A;
-    c.qadz = (float)(Q * A * Dz);
-    c.akdx = (float)(A * k * Dx);
-    c.akdz = (float)(A * k * Dz);
-    c.qakxx = (float)(Q * A * k * Dx * Dx);
-    c.qakxz = (float)(Q * A * k * Dx * Dz);
-    c.qakzz = (float)(Q * A * k * Dz * Dz);
-    return c;
-}
-
-// Per-patch constants: local frame, steps, texel origin reduced by the wrap
-// period in FP64, bounce, first coefficient slot.
-__device__ PatchAux make_patch_aux(const wt_patch& Pt, const HmDev& hm, uint32_t pair_offset) {
-    double blx = Pt.bl[0], blz = Pt.bl[1];
-    PatchAux a;
-    a.e1x = (float)((double)Pt.br[0] - blx);
-    a.e1z = (float)((double)Pt.br[1] - blz);
-    a.e2x = (float)((double)Pt.tl[0] - blx);
-    a.e2z = (float)((double)Pt.tl[1] - blz);
-    a.e3x = (float)((double)Pt.tr[0] - Pt.tl[0] - Pt.br[0] + blx);
-    a.e3z = (float)((double)Pt.tr[1] - Pt.tl[1] - Pt.br[1] + blz);
-    a.blx = Pt.bl[0];
-    a.blz = Pt.bl[1];
-    a.inv_cm1 = Pt.cols > 1 ? 1.0f / (float)(Pt.cols - 1) : 0.0f;
-    a.inv_rm1 = Pt.rows > 1 ? 1.0f / (float)(Pt.rows - 1) : 0.0f;
-    if (hm.present) {
-        double W = hm.width, H = hm.height;
-        double pu = hm.wrap == WT_WRAP_MIRRORED_REPEAT ? 2.0 * W : W;
-        double pv = hm.wrap == WT_WRAP_MIRRORED_REPEAT ? 2.0 * H : H;
-        // texel coordinate of the world point X: sample_scale*W*X - 0.5;
-        // the BL part is reduced by the wrap period in FP64
-        a.hu0 = (float)(pmod((double)hm.sample_scale * W * blx, pu) - 0.5);
-        a.hv0 = (float)(pmod(-(double)hm.sample_scale * H * blz, pv) - 0.5);
-        a.su = (float)((double)hm.sample_scale * W);
-        a.sv = (float)(-(double)hm.sample_scale * H);
-    } else {
-        a.hu0 = a.hv0 = a.su = a.sv = 0.0f;
-    }
-    a.y_offset = Pt.y_offset;
-    a.pair_offset = pair_offset;
-    return a;
-}
-
 // ---- stage 1: validation, prefix sums, LPT order ---------------------------
-__device__ __forceinline__ bool patch_ok(const wt_patch& P, uint32_t n_waves, uint64_t out_capacity) {
-    const uint64_t verts = (uint64_t)P.cols * P.rows;
-    return P.cols >= 2 && P.rows >= 2 && P.cols <= (1u << 20) && P.rows <= (1u << 20) && verts < (1ull << 31) &&
-           P.flags == 0 && (uint64_t)P.wave_offset + P.wave_count <= n_waves && P.out_offset <= out_capacity &&
-           verts <= out_capacity - P.out_offset && finitef(P.bl[0]) && finitef(P.bl[1]) && finitef(P.br[0]) &&
-           finitef(P.br[1]) && finitef(P.tl[0]) && finitef(P.tl[1]) && finitef(P.tr[0]) && finitef(P.tr[1]) &&
-           isfinite(P.time_s) && finitef(P.y_offset);
-}
-
 // Tables of at most kSmallPrep patches whose constants are formed here too
 // (k_prep_scan with fuse_coef): the whole prep through shared memory, with
 // two dependent global loads (the patches, then each pair's wave) instead of
@@ -526,27 +429,7 @@ __global__ void __launch_bounds__(256) k_prep_coef(const wt_patch* __restrict__ 
 #endif
 }
 
-// ---- stage 3: the persistent forward kernel --------------------------------
-// EPI = 0: epilogue unrolled over the lane's vertices straight from the
-// accumulator registers; EPI = 1: the sums are parked in shared memory and a
-// single rolled copy of the epilogue runs (smaller code, larger smem carve-out).
-// MODE (FwdMode): kModeSave also stores each vertex's eight wave sums to `sums`,
-// kModeStage the vertex-stage outputs of `view` (a compile-time switch: a
-// run-time null test of the sums pointer in the epilogue cost 4 % of the
-// kernel).
-// A patch in the forward's shared-memory tile table (queue order).
-struct QInfo {
-    uint32_t cols, nwaves, pair_offset, p;
-    uint64_t out0;
-};
-constexpr uint32_t kTabPatches = 1024;
-// Per warp in the forward's shared memory (float4 units): the wave staging
-// and, for the shared-memory epilogue, the parked sums.
-__host__ __device__ constexpr int fwd_warp_f4(int epi, int smax) { return 32 * kStage + epi * smax * 2 * 32; }
-__host__ __device__ constexpr size_t tab_bytes(uint32_t n) {
-    return n <= kTabPatches ? sizeof(QInfo) * n + 4 * (n + 1) : 0;
-}
-
+// ---- stage 3: the persistent forward kernel (its tile: wt_forward.cuh) ------
 template <int THREADS, int MINB, int SMAX, int EPI, int MODE>
 __global__ void __launch_bounds__(THREADS, MINB)
 k_forward(const wt_patch* __restrict__ patches, HmDev hm, float* __restrict__ pos,
@@ -572,8 +455,6 @@ k_forward(const wt_patch* __restrict__ patches, HmDev hm, float* __restrict__ po
     const PatchAux* aux = reinterpret_cast<const PatchAux*>(ws + L.aux);
     const PairCoef* coef = reinterpret_cast<const PairCoef*>(ws + L.coef);
     const int lane = threadIdx.x & 31;
-    float4* wst = wbase;
-    float4* ebuf = wbase + 32 * kStage;
     const uint32_t n = hdr->n_patches;
     const uint32_t total = hdr->total_tiles;
     const bool pow2 = hm.present && (hm.width & (hm.width - 1)) == 0 && (hm.height & (hm.height - 1)) == 0;
@@ -622,11 +503,6 @@ k_forward(const wt_patch* __restrict__ patches, HmDev hm, float* __restrict__ po
         }
         uint32_t p, cols, nwaves, pair_offset;
         uint64_t out0;
-        // the rest of the patch's constants are loaded after the wave loop
-        // (held across it they would take 15 registers), except for the
-        // saving forward, which spills less with them loaded here
-        constexpr bool kLateAux = MODE != kModeSave;
-        PatchAux a;
         if (ts) {
             const QInfo e = tab[q];
             p = e.p;
@@ -634,106 +510,19 @@ k_forward(const wt_patch* __restrict__ patches, HmDev hm, float* __restrict__ po
             nwaves = e.nwaves;
             pair_offset = e.pair_offset;
             out0 = e.out0;
-            if (!kLateAux) a = aux[p];
         } else {
             p = sorted[q];
             cols = patches[p].cols;
             nwaves = patches[p].wave_count;
             out0 = patches[p].out_offset;
-            if (!kLateAux) a = aux[p];
-            pair_offset = kLateAux ? aux[p].pair_offset : a.pair_offset;
+            pair_offset = aux[p].pair_offset;
         }
         const uint32_t lt = t - tpre[q];
         const uint32_t tpr = tiles_per_row(cols, SMAX);
         const uint32_t row = lt / tpr;
         const uint32_t c0 = (lt - row * tpr) * 32u * SMAX;
-        const uint32_t S = min((uint32_t)SMAX, (cols - c0 + 31u) / 32u);  // the row's last tile is narrower
-
-        float2 acc[SMAX][4];
-#pragma unroll
-        for (int j = 0; j < SMAX; ++j)
-#pragma unroll
-            for (int m = 0; m < 4; ++m) acc[j][m] = make_float2(0.0f, 0.0f);
-
-        for (uint32_t w0 = 0; w0 < nwaves; w0 += chunk) {
-            const uint32_t nw = min(chunk, nwaves - w0);
-            __syncwarp();
-            if ((uint32_t)lane < nw) {
-                stage_wave(coef[pair_offset + w0 + lane], c0, row, wst + kStage * lane);
-            }
-            __syncwarp();
-            wave_loop_dispatch<SMAX>(S, acc, wst, nw, lane);
-        }
-        if (kLateAux) a = aux[p];
-
-        // grid position along the row: x(col) = col * du * (e1 + v e3) + v e2
-        const float v = (float)row * a.inv_rm1;
-        const float gx = (a.e1x + v * a.e3x) * a.inv_cm1, gz = (a.e1z + v * a.e3z) * a.inv_cm1;
-        const float colf = (float)(c0 + lane);
-        const float xb = fmaf(colf, gx, v * a.e2x), zb = fmaf(colf, gz, v * a.e2z);
-        const uint64_t rowbase = out0 + (uint64_t)row * cols;
-        if (EPI == 1) {
-            // park the sums, then one rolled copy of the per-vertex epilogue
-            // (each lane reads back only its own slots)
-#pragma unroll
-            for (int j = 0; j < SMAX; ++j) {
-                if ((uint32_t)j < S) {
-                    ebuf[(2 * j) * 32 + lane] = make_float4(acc[j][0].x, acc[j][0].y, acc[j][1].x, acc[j][1].y);
-                    ebuf[(2 * j + 1) * 32 + lane] = make_float4(acc[j][2].x, acc[j][2].y, acc[j][3].x, acc[j][3].y);
-                }
-            }
-#pragma unroll 1
-            for (uint32_t j = 0; j < S; ++j) {
-                const uint32_t col = c0 + lane + 32 * j;
-                if (col < cols) {
-                    const float4 s0 = ebuf[(2 * j) * 32 + lane], s1 = ebuf[(2 * j + 1) * 32 + lane];
-                    const float xl = fmaf(32.0f * (float)j, gx, xb);
-                    const float zl = fmaf(32.0f * (float)j, gz, zb);
-                    const float2 pr[4] = {make_float2(s0.x, s0.y), make_float2(s0.z, s0.w), make_float2(s1.x, s1.y),
-                                          make_float2(s1.z, s1.w)};
-                    if (MODE == kModePlain && fast)
-                        finish_vertex<MODE, true>(sums_of(pr), xl, zl, a, hm, pow2, rowbase + col, pos, nrm, flags,
-                                                  sums, su, so);
-                    else
-                        finish_vertex<MODE>(sums_of(pr), xl, zl, a, hm, pow2, rowbase + col, pos, nrm, flags, sums,
-                                            su, so);
-                }
-            }
-        } else {
-            // kB vertices at a time: their texel loads are all issued before
-            // the first of them is used (half the lane's vertices: 1.079 ->
-            // 1.059 ms on 256 uneven patches at 8 per lane, 4 and 1 measured
-            // the same; the saving and staging epilogues, with more outputs
-            // live, take one at a time: more would spill)
-            constexpr int kB = MODE == kModePlain ? SMAX / 2 : 1;
-#pragma unroll
-            for (int jb = 0; jb < SMAX; jb += kB) {
-                HmTexels T[kB];
-#pragma unroll
-                for (int u = 0; u < kB; ++u) {
-                    const int j = jb + u;
-                    const uint32_t col = c0 + lane + 32 * j;
-                    T[u] = HmTexels{};
-                    if ((uint32_t)j < S && col < cols && hm.present) {
-                        const float xd = fmaf(32.0f * j, gx, xb) + acc[j][0].x;
-                        const float zd = fmaf(32.0f * j, gz, zb) + acc[j][1].x;
-                        if (MODE == kModePlain && fast) T[u] = hm_fetch<true>(hm, a, xd, zd, pow2);
-                        else T[u] = hm_fetch<false>(hm, a, xd, zd, pow2);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < kB; ++u) {
-                    const int j = jb + u;
-                    const uint32_t col = c0 + lane + 32 * j;
-                    if ((uint32_t)j < S && col < cols) {
-                        const float xl = fmaf(32.0f * j, gx, xb);
-                        const float zl = fmaf(32.0f * j, gz, zb);
-                        finish_vertex_t<MODE>(sums_of(acc[j]), xl, zl, a, hm, T[u], rowbase + col, pos, nrm, flags,
-                                              sums, su, so);
-                    }
-                }
-            }
-        }
+        forward_tile<SMAX, EPI, MODE>(coef + pair_offset, nwaves, cols, out0, row, c0, aux + p, hm, pow2, fast, pos,
+                                      nrm, flags, chunk, sums, wbase, su, so);
         t = __shfl_sync(0xffffffffu, t_a, 0);
     }
 }
@@ -911,6 +700,21 @@ cudaError_t launch_forward(const FwdConfig& cfg, const wt_patch* patches, uint32
         if (cfg.warps == 16) return launch_fwd_t<512, 1, 8, 1, kModePlain>(cfg, patches, n_patches, hm, pos, nrm, flags, ws, L, x, s);
     }
     return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_displace(const FwdConfig& cfg, const wt_patch* patches, uint32_t n_patches, const wt_wave* waves,
+                            uint32_t n_waves, const HmDev& hm, float* pos, float* nrm, uint64_t out_capacity,
+                            uint32_t flags, void* ws, const WsLayout& L, const FwdExtra& x, cudaStream_t s) {
+    const bool naive = (flags & WT_PHASE_FP32_NAIVE) != 0;
+    // one patch at the built-in launch shape (another shape, set or autotuned,
+    // is run as asked for)
+    if (!naive && n_patches == 1 && n_waves <= kSingleWaves && cfg.s == 8 && cfg.warps == 16 && cfg.epi == 1 &&
+        cfg.blocks_per_sm == 0)
+        return launch_single(cfg, patches, waves, n_waves, hm, pos, nrm, out_capacity, flags, ws, L, x, s);
+    cudaError_t e = launch_prep(patches, n_patches, waves, n_waves, hm, out_capacity, 32u * cfg.s, ws, L, s);
+    if (e != cudaSuccess) return e;
+    if (naive) return launch_forward_naive(patches, n_patches, waves, hm, pos, nrm, flags, ws, L, out_capacity, s);
+    return launch_forward(cfg, patches, n_patches, hm, pos, nrm, flags, ws, L, x, s);
 }
 
 cudaError_t launch_forward_naive(const wt_patch* patches, uint32_t n_patches, const wt_wave* waves,

@@ -167,6 +167,18 @@ cudaError_t launch_forward_naive(const wt_patch* patches, uint32_t n_patches, co
                                  void* ws, const WsLayout& L, uint64_t total_vertices,
                                  cudaStream_t s);
 bool forward_config_supported(const FwdConfig& cfg);
+// The whole forward, after the arguments are checked: the one-patch kernel
+// where it applies, else the prep and the recurrence kernel (or, with
+// WT_PHASE_FP32_NAIVE, the precision-study kernel).
+cudaError_t launch_displace(const FwdConfig& cfg, const wt_patch* patches, uint32_t n_patches, const wt_wave* waves,
+                            uint32_t n_waves, const HmDev& hm, float* pos, float* nrm, uint64_t out_capacity,
+                            uint32_t flags, void* ws, const WsLayout& L, const FwdExtra& x, cudaStream_t s);
+// (wt_single.cu) a one-patch table of at most kSingleWaves waves, 8 vertices
+// per lane
+constexpr uint32_t kSingleWaves = 128;
+cudaError_t launch_single(const FwdConfig& cfg, const wt_patch* patches, const wt_wave* waves, uint32_t n_waves,
+                          const HmDev& hm, float* pos, float* nrm, uint64_t out_capacity, uint32_t flags, void* ws,
+                          const WsLayout& L, const FwdExtra& x, cudaStream_t s);
 
 // ---- adjoint (wt_adjoint.cu) ----------------------------------------------
 // Records (tile chunks x waves) of one patch, as the adjoint lays them out.
