@@ -408,20 +408,34 @@ __global__ void __launch_bounds__(256) k_prep_coef(const wt_patch* __restrict__ 
         total = pair_off_g[n];  // 0 when the workspace is short
     }
     const uint32_t* pair_off = own ? off_s : pair_off_g;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t P = blockIdx.x * blockDim.x + threadIdx.x; P < total; P += stride) {
+    // One kind of constant of 32 pairs per warp task (the four phase constants,
+    // the sum coefficients), and the constants of 32 patches: neighbouring tasks
+    // on different SMs, so that the FP64 chains (a warp-wide operation holds the
+    // pipe for about 64 cycles) run side by side.  One thread per pair doing all
+    // of it in consecutive warps: 14.0 us for 48 patches of 0-40 waves, 6.5 us
+    // this way.
+    const uint32_t groups = (total + 31u) / 32u, tasks = 5u * groups + (n + 31u) / 32u;
+    const uint32_t lane = threadIdx.x & 31u, warps = gridDim.x * (blockDim.x >> 5);
+    for (uint32_t t = blockIdx.x + gridDim.x * (threadIdx.x >> 5); t < tasks; t += warps) {
+        if (t >= 5u * groups) {
+            const uint32_t p = 32u * (t - 5u * groups) + lane;
+            if (p < n) aux[p] = make_patch_aux(patches[p], hm, pair_off[p]);
+            continue;
+        }
+        const uint32_t kind = t % 5u, P = 32u * (t / 5u) + lane;
+        if (P >= total) continue;
         // owning patch: last p with pair_off[p] <= P
         uint32_t lo = 0, hi = n + 1;
         while (lo < hi) {
             uint32_t mid = (lo + hi) >> 1;
             if (pair_off[mid] <= P) lo = mid + 1; else hi = mid;
         }
-        uint32_t p = lo - 1;
+        const uint32_t p = lo - 1;
         const wt_patch& Pt = patches[p];
-        coef[P] = make_pair_coef(Pt, waves[Pt.wave_offset + (P - pair_off[p])]);
+        const wt_wave w = waves[Pt.wave_offset + (P - pair_off[p])];
+        if (kind < 4u) (&coef[P].t00)[kind] = phase_turns((int)kind, Pt, w);
+        else sum_coefs(w, coef[P]);
     }
-    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += stride)
-        aux[p] = make_patch_aux(patches[p], hm, pair_off[p]);
 #if __CUDA_ARCH__ >= 900
     // complete only after the scan kernel: whatever waits for this grid then
     // sees both (a no-op when already waited for above)
