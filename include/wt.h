@@ -38,8 +38,10 @@ typedef enum wt_status {
     WT_OK = 0,
     WT_ERR_INVALID_ARG = 1,  /* bad pointer, size, alignment or parameter */
     WT_ERR_CUDA = 2,         /* a CUDA runtime call failed (see wt_last_error) */
-    WT_ERR_TIMEOUT = 3,      /* reserved: no kernel of this library spins on a flag or on
-                                another kernel, so no call returns it */
+    WT_ERR_TIMEOUT = 3,      /* read back by wt_workspace_status: a wait inside a kernel (for its
+                                own matrix products, within one thread block) ran past its limit
+                                of two seconds; the outputs are incomplete.  No kernel waits on
+                                another kernel */
     WT_ERR_NOMEM = 4,        /* workspace smaller than the size query asked for */
     WT_ERR_UNSUPPORTED = 5   /* a parameter combination this build does not handle */
 } wt_status;
@@ -530,8 +532,10 @@ wt_status wt_wave_from_reference(float amplitude_A, float frequency_w,
  * lane with 8 or 16 warps and either epilogue, or 20 warps and the register
  * epilogue (the saving and vertex-stage forwards run it as 16); 4 vertices per
  * lane with 8 warps and the register epilogue).  Process-wide; applies to
- * launches issued after it is set.  No reference counterpart (the reference
- * has one fixed draw call). */
+ * launches issued after it is set.  Patches that run as matrix products (exact
+ * parallelograms of 8 to 128 waves) do not depend on it, and the built-in shape
+ * runs a one-patch table in a kernel of its own.  No reference counterpart
+ * (the reference has one fixed draw call). */
 typedef struct wt_tuning {
     uint32_t warps_per_block; /* 8, 16 or 20 (0 = 16) */
     uint32_t blocks_per_sm;   /* 0 = as many as fit */

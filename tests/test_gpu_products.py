@@ -1,0 +1,98 @@
+"""The forward's matrix-product path (parallelogram patches of 8 to 128 waves)
+at the edges of its tiles (128 columns by 32 or 16 rows, 32 waves a step, two
+accumulators above 48 waves), against the FP64 oracle at the path's bounds, and
+one patch alone against the same patch in a table, bit for bit."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from helpers import angle_deg, rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+def patch_table(sizes, seed, wrap, tex):
+    """Parallelogram patches (cols, rows, waves), a skewed one and one of four waves."""
+    from wave_tool_gb300 import workloads
+    rng = workloads.SplitMix64(seed)
+    base = workloads.small_random(seed, n_patches=1, side_range=(40, 40), n_waves_range=(9, 9), heightmap=True, wrap=wrap)
+    rows, waves, out = [], [], 0
+    for cols, rws, n in [*sizes, (40, 40, 9), (50, 21, 4)]:
+        if (cols, rws, n) == (40, 40, 9):
+            p = base.patches.copy()
+        else:
+            hx, hz = 0.185 * (cols - 1), 0.185 * (rws - 1)
+            cx, cz = rng.uniform(-2000, 2000), rng.uniform(-2000, 2000)
+            s = 0.25 * hx  # a sheared parallelogram: exact in FP32 when the shear is one float
+            p = base.patches.copy()
+            f = np.float32
+            bl, e1, e2 = np.array([f(cx - hx), f(cz + hz)]), np.array([f(2 * hx), f(0)]), np.array([f(s), f(-2 * hz)])
+            for k, v in (("bl", bl), ("br", bl + e1), ("tl", bl + e2)):
+                p[k] = v
+            p["tr"] = p["br"].astype(np.float64) + p["tl"] - p["bl"]
+            exact = np.all(p["tr"].astype(np.float64) - p["tl"] - p["br"] + p["bl"] == 0)
+            if not exact:  # fall back to an axis-aligned one, exact by construction
+                p["bl"], p["br"], p["tl"], p["tr"] = (cx - hx, cz + hz), (cx + hx, cz + hz), (cx - hx, cz - hz), (cx + hx, cz - hz)
+            p["cols"], p["rows"] = cols, rws
+            p["time_s"] = rng.uniform(0.0, 5.0e3)
+        p["wave_offset"], p["wave_count"], p["out_offset"] = len(waves), n, out
+        rows.append(p)
+        waves.extend(workloads.waves_wide(rng, n))
+        out += cols * rws
+    hm = workloads.Heightmap(*tex, 0.05, 0.3, wrap, workloads.noise_terms(rng, n=8, kmax=3)) if tex else None
+    return np.concatenate(rows), np.array(waves, dtype=base.waves.dtype), hm
+
+
+SIZES = [[(32, 2, 8), (33, 15, 9), (127, 16, 31), (128, 17, 32)],
+         [(129, 31, 33), (257, 32, 48), (300, 33, 49), (64, 65, 64)],
+         [(160, 97, 65), (385, 18, 127), (96, 130, 128), (1030, 5, 24)]]
+
+
+@pytest.mark.parametrize("sizes", SIZES)
+@pytest.mark.parametrize("wrap,tex,flags", [(0, None, 1), (0, (32, 16), 3), (1, (37, 21), 1), (1, (32, 32), 0)])
+def test_products_against_oracle(wt, oracle, gpu, sizes, wrap, tex, flags):
+    import torch
+    patches, waves, hmw = patch_table(sizes, 31 + len(sizes) + wrap, wrap, tex)
+    hm = wt.heightmap_from(hmw)
+    surf = wt.Surface(patches, waves, hm)
+    pos, nrm = surf.displace(flags=flags)
+    torch.cuda.synchronize()
+    assert surf.status()[0] == 0
+    texels = hm.texels.cpu().numpy() if hm is not None else None
+    pos64, disp64, nrm64, edge = oracle.displace_f64(patches, waves, texels, hmw)
+    want = disp64 if flags & 1 else pos64
+    got = pos[:, :3].double().cpu().numpy()
+    assert rel_err(got, want) <= 1e-5
+    ok = edge > 1e-3
+    assert angle_deg(nrm[:, :3].double().cpu().numpy()[ok], nrm64[ok]).max() < 1e-2
+    # each patch alone: the same bits
+    for p in patches:
+        one = p.reshape(1).copy()
+        o, n = int(one["out_offset"][0]), int(one["cols"][0]) * int(one["rows"][0])
+        one["out_offset"] = 0
+        a = wt.Surface(one, waves[int(p["wave_offset"]):int(p["wave_offset"]) + int(p["wave_count"])].copy(), hm)
+        a.host_patches["wave_offset"] = 0
+        a.patches.copy_(wt.to_device(a.host_patches))
+        p1, n1 = a.displace(flags=flags)
+        assert torch.equal(p1, pos[o:o + n]) and torch.equal(n1, nrm[o:o + n])
+
+
+def test_waves_out_of_the_products_range(wt, oracle, gpu):
+    """Waves whose coefficients leave the products' common scale no room, and
+    patches of no amplitude, give finite results as before."""
+    import torch
+    patches, waves, _ = patch_table([(130, 20, 10), (64, 40, 12)], 5, 0, None)
+    waves["amplitude"][3] = 2e12
+    waves["steepness_q"][3] = 0.0
+    waves["amplitude"][10:22] = 0.0
+    for table in (patches, patches[1:2].copy()):
+        table = table.copy()
+        table["out_offset"] -= table["out_offset"][0]
+        surf = wt.Surface(table, waves)
+        pos, nrm = surf.displace(flags=1)
+        torch.cuda.synchronize()
+        assert surf.status()[0] == 0
+        _, disp64, _, _ = oracle.displace_f64(table, waves, None, None)
+        assert rel_err(pos[:, :3].double().cpu().numpy(), disp64) <= 1e-5 or np.abs(disp64).max() == 0
+        assert bool(torch.isfinite(pos).all()) and bool(torch.isfinite(nrm).all())

@@ -239,6 +239,7 @@ wt_status wt_workspace_status(const void* workspace, wt_stream stream, uint32_t*
     if (bad_patch) *bad_patch = h[1];
     if (h[0] == WT_OK) return WT_OK;
     if (h[0] == WT_ERR_NOMEM) return fail(WT_ERR_NOMEM, "workspace too small for the patches' wave slots");
+    if (h[0] == WT_ERR_TIMEOUT) return fail(WT_ERR_TIMEOUT, "a bounded wait of a matrix-product kernel ran out");
     return fail((wt_status)h[0], "device-side validation failed at patch %u", h[1]);
 }
 
@@ -325,7 +326,7 @@ static wt_status run_adjoint(const wt_patch* host_patches, const wt_patch* patch
     wt::AdjScanArgs args;
     cudaError_t e = wt::adjoint_scan_args(sums != nullptr, L, &args);
     if (e != cudaSuccess) return cuda_fail(e, "adjoint set-up");
-    e = wt::launch_prep(patches, n_patches, waves, n_waves, P.hm, out_capacity, 256u, workspace, L.f, s, &args);
+    e = wt::launch_prep(patches, n_patches, waves, n_waves, P.hm, out_capacity, 256u, workspace, L.f, s, false, &args);
     if (e != cudaSuccess) return cuda_fail(e, "prep launch");
     uint32_t maxw = 0;
     for (uint32_t i = 0; i < n_patches; ++i) maxw = host_patches[i].wave_count > maxw ? host_patches[i].wave_count : maxw;

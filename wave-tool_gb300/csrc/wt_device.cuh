@@ -98,6 +98,49 @@ __host__ __device__ __forceinline__ uint32_t tiles_per_row(uint32_t cols, uint32
     return (cols + 32 * smax - 1) / (32 * smax);
 }
 
+// a + b == c + d exactly: both sums as rounded sum and remainder (Knuth's
+// two-sum).  In FP32, since this is asked by every thread of a kernel's start
+// and a warp-wide FP64 operation holds the pipe for about 64 cycles (2.4 us
+// of a small call).
+__device__ __forceinline__ bool same_sum(float a, float b, float c, float d) {
+    const float s = a + b, bb = s - a, e = (a - (s - bb)) + (b - bb);
+    const float t = c + d, dd = t - c, f = (c - (t - dd)) + (d - dd);
+    return s == t && e == f;
+}
+
+// Whether a valid patch's forward runs as matrix products (wt_mma.cuh): its
+// corners span a parallelogram exactly (the phase is then a sum of a column
+// and a row part), it has waves enough (at 8 the two paths cost about the same)
+// and not more than the operands' shared memory holds, and a full warp of
+// columns.  A rule on the patch alone, so that a patch gives the same bits in
+// every table.  Measured, products / recurrence: 256 patches of 64-1024 side
+// 383 / 956 us, of 64-128 side 61 / 89 us, one patch of 1024^2 with 8 waves
+// 12.5 / 13.1 us, with 32 13.9 / 22.9; what it costs is on small one-patch calls
+// of few waves (128^2: 8 waves 8.0 / 6.8 us, 32 9.0 / 8.4, 64 12.1 / 12.5).
+// A lower limit on the patch's size would split a batch over two kernels: with
+// one at 2^18 terms 256 patches of 64-128 side took 77 us.
+__device__ __forceinline__ bool mma_patch(const wt_patch& P) {
+    return P.wave_count >= kMmaMinWaves && P.wave_count <= kMmaMaxWaves && P.cols >= 32 &&
+           same_sum(P.tr[0], P.bl[0], P.tl[0], P.br[0]) && same_sum(P.tr[1], P.bl[1], P.tl[1], P.br[1]);
+}
+
+// A wave whose sum coefficients leave room for the products' common scale
+// (finite, and far from FP32's limits).
+__device__ __forceinline__ bool mma_wave(const wt_wave& w) {
+    const float k = 6.2831855f / w.wavelength, a = fabsf(w.amplitude), q = fabsf(w.steepness_q) * a;
+    return a <= 1e12f && q <= 1e12f && a * k <= 1e12f && q * k <= 1e12f && fabsf(w.dir_x) <= 2.0f &&
+           fabsf(w.dir_z) <= 2.0f;
+}
+
+// Rows per item of the matrix-product kernel for `rowct` rows (summed over
+// the patches' 128-column blocks): one item per SM while that is at most 128
+// rows, else a whole number of items per SM of at most about 128 (operand A,
+// formed once per item, is then a tenth of its work).
+__device__ __forceinline__ uint32_t mma_item_rows(uint64_t rowct, uint32_t sms) {
+    const uint64_t w = (rowct + 128ull * sms - 1u) / (128ull * sms);
+    return max((uint32_t)((rowct + sms * w - 1u) / (sms * w)), 4u);
+}
+
 // ---- shared epilogue -------------------------------------------------------
 
 // Texel coordinate -> the two texel indices of the GL_LINEAR footprint and

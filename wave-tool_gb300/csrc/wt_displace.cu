@@ -38,10 +38,17 @@ namespace {
 
 using namespace wt::dev;
 
-constexpr int kSortBins = 1024;         // wave counts >= 1023 share the last bin
+constexpr uint32_t kWaveBins = 1024;     // wave counts >= 1023 share the last bin
+constexpr uint32_t kSortBins = 2 * kWaveBins;  // matrix-product patches (mma_patch) above the others
+constexpr uint32_t kMmaFlag = 0x80000000u;     // in the tile counts: the patch qualifies
 constexpr uint32_t kWaveMaskWords = 512;  // waves validated into a shared bitmask up to 16384
 constexpr uint32_t kRankSortMax = 64;
 
+
+// Sort key of a patch: larger keys run first.
+__device__ __forceinline__ uint32_t sort_key(uint32_t wave_count, bool mma) {
+    return min(wave_count, kWaveBins - 1u) + (mma ? kWaveBins : 0u);
+}
 
 __device__ __forceinline__ void flag_error(WsHeader* h, uint32_t code, uint32_t patch) {
     atomicCAS(&h->status, 0u, code);
@@ -59,13 +66,14 @@ constexpr uint32_t kSmallPrep = 32;
 
 __device__ void prep_small(const wt_patch* __restrict__ patches, uint32_t n, const wt_wave* __restrict__ waves,
                            uint32_t n_waves, uint64_t out_capacity, uint64_t coef_capacity, uint32_t tile_cols,
-                           char* ws, const WsLayout& L, const HmDev& hm, int do_adj, const AdjLayout& AL,
-                           uint32_t adj_chunk_max, uint32_t adj_min_tiles) {
+                           char* ws, const WsLayout& L, const HmDev& hm, uint32_t mma_sms, int do_adj,
+                           const AdjLayout& AL, uint32_t adj_chunk_max, uint32_t adj_min_tiles) {
     __shared__ wt_patch sp[kSmallPrep];
     __shared__ uint32_t s_sorted[kSmallPrep];      // patch at each sorted rank
     __shared__ uint32_t s_off[kSmallPrep + 1];     // pair prefix over the structurally valid patches
     __shared__ uint32_t s_rank_tiles[kSmallPrep];  // tiles of the patch at each sorted rank
     __shared__ uint32_t s_struct_bad, s_wave_bad;  // bit p: patch p fails that check
+    __shared__ uint32_t s_wave_wild;               // bit p: a wave of patch p is no mma_wave
     WsHeader* hdr = reinterpret_cast<WsHeader*>(ws);
     uint32_t* sorted = reinterpret_cast<uint32_t*>(ws + L.sorted);
     uint32_t* tile_pre = reinterpret_cast<uint32_t*>(ws + L.tile_pre);
@@ -77,9 +85,10 @@ __device__ void prep_small(const wt_patch* __restrict__ patches, uint32_t n, con
     constexpr unsigned kAll = 0xffffffffu;
 
     if (tid < n) sp[tid] = patches[tid];
-    if (tid == 0) s_wave_bad = 0;
+    if (tid == 0) s_wave_bad = s_wave_wild = 0;
     __syncthreads();
     uint32_t tiles_p = 0;  // warp 0: lane p's patch
+    bool mma_p = false;
     if (tid < 32) {
         bool ok = false;
         uint32_t wc = 0;
@@ -88,6 +97,7 @@ __device__ void prep_small(const wt_patch* __restrict__ patches, uint32_t n, con
             ok = patch_ok(P, n_waves, out_capacity);
             wc = ok ? P.wave_count : 0u;
             tiles_p = ok ? P.rows * tiles_per_row(P.cols, tile_cols / 32) : 0u;
+            mma_p = mma_sms > 0 && ok && mma_patch(P);
         }
         uint32_t x = wc;  // inclusive prefix of the pair counts
         for (int o = 1; o < 32; o <<= 1) {
@@ -109,6 +119,7 @@ __device__ void prep_small(const wt_patch* __restrict__ patches, uint32_t n, con
         const wt_patch& Pt = sp[p];
         const wt_wave w = waves[Pt.wave_offset + (tid - s_off[p])];
         if (!wave_ok(w)) atomicOr(&s_wave_bad, 1u << p);
+        if (!mma_wave(w)) atomicOr(&s_wave_wild, 1u << p);
         if (!nomem) coef[tid] = make_pair_coef(Pt, w);
     }
     if (tid < n && !nomem) aux[tid] = make_patch_aux(sp[tid], hm, s_off[tid]);
@@ -116,6 +127,18 @@ __device__ void prep_small(const wt_patch* __restrict__ patches, uint32_t n, con
     if (tid >= 32) return;
     const unsigned bad = s_struct_bad | s_wave_bad;
     if (tid < n && ((s_wave_bad >> tid) & 1u)) tiles_p = 0;
+    mma_p = mma_p && tiles_p > 0 && !((s_wave_wild >> tid) & 1u);
+    uint32_t mma_rows = 0, mma_items = 0;
+    const unsigned mma_set = __ballot_sync(kAll, mma_p);
+    if (mma_set) {
+        const uint32_t ct = mma_p ? (sp[tid].cols + 127u) / 128u : 0u;
+        const uint32_t rows = mma_p ? sp[tid].rows : 0u;
+        unsigned long long rowct = (unsigned long long)rows * ct;
+        for (int o = 16; o > 0; o >>= 1) rowct += __shfl_xor_sync(kAll, rowct, o);
+        mma_rows = mma_item_rows(rowct, mma_sms);
+        if (mma_p) tiles_p = ct * ((rows + mma_rows - 1u) / mma_rows);
+        mma_items = __reduce_add_sync(kAll, mma_p ? tiles_p : 0u);
+    }
     if (tid < n) {
         pair_off[tid] = s_off[tid];
         tiles_g[tid] = tiles_p;
@@ -131,7 +154,7 @@ __device__ void prep_small(const wt_patch* __restrict__ patches, uint32_t n, con
         }
     } else {
         // descending wave count, ties by index (as the general path's rank sort)
-        const uint32_t key = tid < n ? min(sp[tid].wave_count, (uint32_t)kSortBins - 1) : 0u;
+        const uint32_t key = tid < n ? sort_key(sp[tid].wave_count, mma_p) : 0u;
         uint32_t rank = 0;
         for (uint32_t q = 0; q < n; ++q) {
             const uint32_t kq = __shfl_sync(kAll, key, q);
@@ -199,9 +222,12 @@ __device__ void prep_small(const wt_patch* __restrict__ patches, uint32_t n, con
     if (tid == 0) {
         hdr->status = bad ? (uint32_t)WT_ERR_INVALID_ARG : (nomem || adj_nomem ? (uint32_t)WT_ERR_NOMEM : 0u);
         hdr->bad_patch = bad ? (uint32_t)(__ffs(bad) - 1) : kNoPatch;
-        hdr->tile_counter = 0;
+        hdr->tile_counter = nomem ? 0u : mma_items;  // the recurrence kernel's tiles follow the items
         hdr->n_patches = n;
         hdr->tile_cols = tile_cols;
+        hdr->mma_items = nomem ? 0u : mma_items;
+        hdr->mma_rows = mma_rows;
+        hdr->mma_counter = 0;
         if (nomem) hdr->total_tiles = 0;
     }
 }
@@ -213,7 +239,7 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
                                                     const wt_wave* __restrict__ waves, uint32_t n_waves,
                                                     uint64_t out_capacity, uint64_t coef_capacity,
                                                     uint32_t tile_cols, char* ws, WsLayout L, HmDev hm,
-                                                    int fuse_coef, int do_adj, AdjLayout AL,
+                                                    int fuse_coef, uint32_t mma_sms, int do_adj, AdjLayout AL,
                                                     uint32_t adj_chunk_max, uint32_t adj_min_tiles) {
 #if __CUDA_ARCH__ >= 900
     // the coefficient kernel does not read what this one writes (it forms its
@@ -223,7 +249,7 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
     if (!fuse_coef) cudaTriggerProgrammaticLaunchCompletion();
 #endif
     if (n <= kSmallPrep && fuse_coef) {
-        prep_small(patches, n, waves, n_waves, out_capacity, coef_capacity, tile_cols, ws, L, hm, do_adj, AL,
+        prep_small(patches, n, waves, n_waves, out_capacity, coef_capacity, tile_cols, ws, L, hm, mma_sms, do_adj, AL,
                    adj_chunk_max, adj_min_tiles);
         return;
     }
@@ -236,6 +262,9 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
     constexpr uint32_t kScanSmemOffsets = 4096;
     __shared__ uint32_t off_s[kScanSmemOffsets];
     __shared__ uint32_t good_wave[kWaveMaskWords];  // bit w: wave w passes wave_ok
+    __shared__ uint32_t tame_wave[kWaveMaskWords];  // bit w: wave w is an mma_wave
+    __shared__ unsigned long long s_rowct;          // rows x 128-column blocks of the matrix-product patches
+    __shared__ uint32_t s_mma_items;
 
     if (threadIdx.x == 0) {
         hdr->status = 0;
@@ -243,12 +272,16 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
         hdr->tile_counter = 0;
         hdr->n_patches = n;
         hdr->tile_cols = tile_cols;
+        hdr->mma_items = 0;
+        hdr->mma_counter = 0;
+        s_rowct = 0;
+        s_mma_items = 0;
     }
     // up to kRankSortMax patches are ordered by rank (their keys in bins[]),
     // more by a counting sort over the bins
     const bool rank_sort = n <= kRankSortMax;
     if (!rank_sort)
-        for (int i = threadIdx.x; i < kSortBins; i += blockDim.x) bins[i] = 0;
+        for (uint32_t i = threadIdx.x; i < kSortBins; i += blockDim.x) bins[i] = 0;
     __syncthreads();
 
     // structural validation; pair_off <- wave counts of the patches that pass
@@ -257,10 +290,7 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
         const bool ok = patch_ok(P, n_waves, out_capacity);
         if (!ok) flag_error(hdr, WT_ERR_INVALID_ARG, p);
         pair_off[p] = ok ? P.wave_count : 0u;
-        tiles[p] = ok ? P.rows * tiles_per_row(P.cols, tile_cols / 32) : 0u;
-        const uint32_t key = P.wave_count < kSortBins ? P.wave_count : kSortBins - 1;
-        if (rank_sort) bins[p] = key;
-        else atomicAdd(&bins[kSortBins - 1 - key], 1u);  // descending wave count
+        tiles[p] = ok ? P.rows * tiles_per_row(P.cols, tile_cols / 32) | (mma_sms > 0 && mma_patch(P) ? kMmaFlag : 0u) : 0u;
     }
     __syncthreads();
     const uint32_t total_pairs = block_exclusive_scan(pair_off, n);
@@ -279,24 +309,35 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
         const uint32_t nw_round = (n_waves + 31u) & ~31u;
 #pragma unroll 4
         for (uint32_t w = threadIdx.x; w < nw_round; w += blockDim.x) {
-            const bool good = w < n_waves && wave_ok(waves[w]);
-            const uint32_t word = __ballot_sync(0xffffffffu, good);
-            if ((threadIdx.x & 31) == 0) good_wave[w >> 5] = word;
+            bool good = false, tame = false;
+            if (w < n_waves) {
+                const wt_wave v = waves[w];
+                good = wave_ok(v);
+                tame = mma_wave(v);
+            }
+            const uint32_t word = __ballot_sync(0xffffffffu, good), tword = __ballot_sync(0xffffffffu, tame);
+            if ((threadIdx.x & 31) == 0) {
+                good_wave[w >> 5] = word;
+                tame_wave[w >> 5] = tword;
+            }
         }
         __syncthreads();
         for (uint32_t p = threadIdx.x; p < n; p += blockDim.x) {
             if (off[p + 1] == off[p]) continue;  // invalid patch (or no waves)
             const uint32_t w0 = patches[p].wave_offset, w1 = w0 + (off[p + 1] - off[p]);
-            bool bad = false;
+            bool bad = false, wild = false;
             for (uint32_t w = w0; w < w1 && !bad;) {
                 const uint32_t bit = w & 31u, take = min(32u - bit, w1 - w);
                 const uint32_t want = (take == 32u ? 0xffffffffu : ((1u << take) - 1u)) << bit;
                 bad = (good_wave[w >> 5] & want) != want;
+                wild |= (tame_wave[w >> 5] & want) != want;
                 w += take;
             }
             if (bad) {
                 flag_error(hdr, WT_ERR_INVALID_ARG, p);
                 tiles[p] = 0;
+            } else if (wild) {
+                tiles[p] &= ~kMmaFlag;
             }
         }
     } else {
@@ -308,9 +349,12 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
                 if (off[mid] <= P) lo = mid + 1; else hi = mid;
             }
             const uint32_t p = lo - 1;
-            if (!wave_ok(waves[patches[p].wave_offset + (P - off[p])])) {
+            const wt_wave w = waves[patches[p].wave_offset + (P - off[p])];
+            if (!wave_ok(w)) {
                 flag_error(hdr, WT_ERR_INVALID_ARG, p);
-                tiles[p] = 0;
+                atomicAnd(&tiles[p], 0u);
+            } else if (!mma_wave(w)) {
+                atomicAnd(&tiles[p], ~kMmaFlag);
             }
         }
     }
@@ -328,8 +372,36 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
         for (uint32_t p = threadIdx.x; p <= n; p += blockDim.x) tile_pre[p] = 0;
         return;
     }
-    // sort by descending wave count, ties in any order: the order only
-    // schedules tiles, results do not depend on it
+    // the matrix-product patches' items, then the sort keys
+    if (mma_sms > 0) {
+        for (uint32_t p = threadIdx.x; p < n; p += blockDim.x)
+            if (tiles[p] & kMmaFlag)
+                atomicAdd(&s_rowct, (unsigned long long)patches[p].rows * ((patches[p].cols + 127u) / 128u));
+        __syncthreads();
+        if (s_rowct > 0) {
+            const uint32_t h = mma_item_rows(s_rowct, mma_sms);
+            for (uint32_t p = threadIdx.x; p < n; p += blockDim.x) {
+                if (!(tiles[p] & kMmaFlag)) continue;
+                const uint32_t items = (patches[p].cols + 127u) / 128u * ((patches[p].rows + h - 1u) / h);
+                tiles[p] = items | kMmaFlag;
+                atomicAdd(&s_mma_items, items);
+            }
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                hdr->mma_items = s_mma_items;
+                hdr->mma_rows = h;
+                hdr->tile_counter = s_mma_items;  // the recurrence kernel's tiles follow the items
+            }
+        }
+    }
+    for (uint32_t p = threadIdx.x; p < n; p += blockDim.x) {
+        const uint32_t key = sort_key(patches[p].wave_count, tiles[p] & kMmaFlag);
+        if (rank_sort) bins[p] = key;
+        else atomicAdd(&bins[kSortBins - 1 - key], 1u);  // descending
+    }
+    __syncthreads();
+    // sort by descending key, ties in any order: the order only schedules
+    // tiles, results do not depend on it
     if (rank_sort) {
         for (uint32_t p = threadIdx.x; p < n; p += blockDim.x) {
             const uint32_t key = bins[p];
@@ -341,13 +413,12 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
         block_exclusive_scan(bins, kSortBins);
         __syncthreads();
         for (uint32_t p = threadIdx.x; p < n; p += blockDim.x) {
-            const uint32_t wc = patches[p].wave_count;
-            const uint32_t key = wc < kSortBins ? wc : kSortBins - 1;
+            const uint32_t key = sort_key(patches[p].wave_count, tiles[p] & kMmaFlag);
             sorted[atomicAdd(&bins[kSortBins - 1 - key], 1u)] = p;
         }
     }
     __syncthreads();
-    for (uint32_t q = threadIdx.x; q < n; q += blockDim.x) tile_pre[q] = tiles[sorted[q]];
+    for (uint32_t q = threadIdx.x; q < n; q += blockDim.x) tile_pre[q] = tiles[sorted[q]] & ~kMmaFlag;
     __syncthreads();
     const uint32_t total_tiles = block_exclusive_scan(tile_pre, n);
     if (threadIdx.x == 0) {
@@ -483,8 +554,10 @@ k_forward(const wt_patch* __restrict__ patches, HmDev hm, float* __restrict__ po
     // uneven patches at 8 vertices per lane, 1.0777 -> 1.0680 at 4).
     QInfo* const tab = reinterpret_cast<QInfo*>(su + (MODE == kModeStage ? 36 : 0));
     uint32_t* const tab_pre = reinterpret_cast<uint32_t*>(tab + (tab_in_smem ? n : 0));
-    // (a table the prep refused, total 0, has no order to copy: skipped)
-    if (tab_in_smem && total > 0) {
+    // nothing to run: a table the prep refused (no order to copy), or one whose
+    // patches all ran as matrix products
+    if (total <= hdr->mma_items) return;
+    if (tab_in_smem) {
         for (uint32_t qq = threadIdx.x; qq < n; qq += THREADS) {
             const uint32_t pp = sorted[qq];
             tab[qq] = QInfo{patches[pp].cols, patches[pp].wave_count, aux[pp].pair_offset, pp,
@@ -493,7 +566,7 @@ k_forward(const wt_patch* __restrict__ patches, HmDev hm, float* __restrict__ po
         for (uint32_t qq = threadIdx.x; qq <= n; qq += THREADS) tab_pre[qq] = tile_pre[qq];
         __syncthreads();
     }
-    const bool ts = tab_in_smem && total > 0;
+    const bool ts = tab_in_smem != 0;
     const uint32_t* const tpre = ts ? tab_pre : tile_pre;
 
     // The queue index of the next tile is fetched while the current one runs;
@@ -639,7 +712,7 @@ cudaError_t launch_fwd_t(const FwdConfig& cfg, const wt_patch* patches, uint32_t
 
 cudaError_t launch_prep(const wt_patch* patches, uint32_t n_patches, const wt_wave* waves, uint32_t n_waves,
                         const HmDev& hm, uint64_t out_capacity, uint32_t tile_cols, void* ws,
-                        const WsLayout& L, cudaStream_t s, const AdjScanArgs* adj) {
+                        const WsLayout& L, cudaStream_t s, bool use_mma, const AdjScanArgs* adj) {
     char* w = static_cast<char*>(ws);
     // coefficient capacity = what the caller's workspace holds past the fixed part
     // (the header records the real total; the scan refuses to overflow it)
@@ -648,13 +721,13 @@ cudaError_t launch_prep(const wt_patch* patches, uint32_t n_patches, const wt_wa
     const int fuse = (uint64_t)n_patches * n_waves <= 1024u;
     const AdjScanArgs none{};
     const AdjScanArgs& A = adj ? *adj : none;
+    const int sms = sm_count();
+    if (sms <= 0) return cudaErrorInvalidDevice;
     k_prep_scan<<<1, 1024, 0, s>>>(patches, n_patches, waves, n_waves, out_capacity, coef_cap, tile_cols, w, L,
-                                   hm, fuse, adj ? 1 : 0, A.L, A.chunk_max, A.min_tiles);
+                                   hm, fuse, use_mma ? (uint32_t)sms : 0u, adj ? 1 : 0, A.L, A.chunk_max, A.min_tiles);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (fuse) return cudaSuccess;
-    const int sms = sm_count();
-    if (sms <= 0) return cudaErrorInvalidDevice;
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((unsigned)sms);
     lc.blockDim = dim3(256);
@@ -725,9 +798,15 @@ cudaError_t launch_displace(const FwdConfig& cfg, const wt_patch* patches, uint3
     if (!naive && n_patches == 1 && n_waves <= kSingleWaves && cfg.s == 8 && cfg.warps == 16 && cfg.epi == 1 &&
         cfg.blocks_per_sm == 0)
         return launch_single(cfg, patches, waves, n_waves, hm, pos, nrm, out_capacity, flags, ws, L, x, s);
-    cudaError_t e = launch_prep(patches, n_patches, waves, n_waves, hm, out_capacity, 32u * cfg.s, ws, L, s);
+    // with fewer waves than mma_patch asks for, no patch can qualify
+    const bool mma = !naive && n_waves >= kMmaMinWaves;
+    cudaError_t e = launch_prep(patches, n_patches, waves, n_waves, hm, out_capacity, 32u * cfg.s, ws, L, s, mma);
     if (e != cudaSuccess) return e;
     if (naive) return launch_forward_naive(patches, n_patches, waves, hm, pos, nrm, flags, ws, L, out_capacity, s);
+    if (mma) {
+        e = launch_forward_mma(patches, hm, pos, nrm, flags, ws, L, x, s);
+        if (e != cudaSuccess) return e;
+    }
     return launch_forward(cfg, patches, n_patches, hm, pos, nrm, flags, ws, L, x, s);
 }
 

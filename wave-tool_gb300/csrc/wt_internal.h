@@ -12,8 +12,10 @@ namespace wt {
 
 // ---- workspace layout ------------------------------------------------------
 // [0, 256)                 WsHeader
-// sorted   u32[n_patches]  patch indices, descending wave count (LPT order)
-// tile_pre u32[n+1]        exclusive prefix of tiles over the sorted order
+// sorted   u32[n_patches]  patch indices, first the patches that run as matrix products
+//                          (mma_patch), then the others, each by descending wave count (LPT order)
+// tile_pre u32[n+1]        exclusive prefix of work items over the sorted order (matrix-product
+//                          items, then tiles of the recurrence kernel)
 // pair_off u32[n+1]        exclusive prefix of wave_count (original order)
 // tiles    u32[n]          tile count per patch (original order, 0 = invalid)
 // aux      PatchAux[n]
@@ -27,7 +29,10 @@ struct WsHeader {
     uint32_t tile_cols;    // vertices per tile row (32 * S)
     uint32_t total_chunks; // adjoint: tile chunks in its queue (0 = do not run)
     uint32_t adj_chunk;    // adjoint: tiles per chunk
-    uint32_t pad[56];
+    uint32_t mma_items;    // items of the matrix-product kernel: [0, mma_items) of the prefix
+    uint32_t mma_rows;     // its rows per item (a patch's rows are split evenly into items of at most this)
+    uint32_t mma_counter;  // its queue head, past the first item of each block
+    uint32_t pad[53];
 };
 static_assert(sizeof(WsHeader) == 256, "header size");
 
@@ -144,6 +149,16 @@ struct HmDev {
     int present;
 };
 
+// How the layer is sampled: 0 absent, 1 by the mask-only wrap (REPEAT,
+// power-of-two sides), 2 by the general one.
+inline int hm_kind(const HmDev& hm) {
+    const bool pow2 = (hm.width & (hm.width - 1)) == 0 && (hm.height & (hm.height - 1)) == 0;
+    return !hm.present ? 0 : (pow2 && hm.wrap == WT_WRAP_REPEAT ? 1 : 2);
+}
+
+// Waves of a patch that runs as matrix products (mma_patch).
+constexpr uint32_t kMmaMinWaves = 8, kMmaMaxWaves = 128;
+
 // The adjoint's queue set-up (ranks, chunk and record prefixes), formed by the
 // prep's scan kernel when the prep runs for an adjoint.
 struct AdjScanArgs {
@@ -153,11 +168,12 @@ struct AdjScanArgs {
 };
 
 // ---- launchers (wt_displace.cu) -------------------------------------------
-// tile_cols: tile width (each row's last tile narrower, see tiles_per_row)
+// tile_cols: tile width (each row's last tile narrower, see tiles_per_row);
+// use_mma: the patches that qualify (mma_patch) are queued for launch_forward_mma
 cudaError_t launch_prep(const wt_patch* patches, uint32_t n_patches, const wt_wave* waves,
                         uint32_t n_waves, const HmDev& hm, uint64_t out_capacity,
                         uint32_t tile_cols, void* ws, const WsLayout& L, cudaStream_t s,
-                        const AdjScanArgs* adj = nullptr);
+                        bool use_mma, const AdjScanArgs* adj = nullptr);
 // pos may be NULL only with x.view set
 cudaError_t launch_forward(const FwdConfig& cfg, const wt_patch* patches, uint32_t n_patches,
                            const HmDev& hm, float* pos, float* nrm, uint32_t flags, void* ws,
@@ -168,11 +184,15 @@ cudaError_t launch_forward_naive(const wt_patch* patches, uint32_t n_patches, co
                                  cudaStream_t s);
 bool forward_config_supported(const FwdConfig& cfg);
 // The whole forward, after the arguments are checked: the one-patch kernel
-// where it applies, else the prep and the recurrence kernel (or, with
-// WT_PHASE_FP32_NAIVE, the precision-study kernel).
+// where it applies, else the prep, the matrix-product kernel where a patch can
+// qualify and the recurrence kernel (or, with WT_PHASE_FP32_NAIVE, the
+// precision-study kernel).
 cudaError_t launch_displace(const FwdConfig& cfg, const wt_patch* patches, uint32_t n_patches, const wt_wave* waves,
                             uint32_t n_waves, const HmDev& hm, float* pos, float* nrm, uint64_t out_capacity,
                             uint32_t flags, void* ws, const WsLayout& L, const FwdExtra& x, cudaStream_t s);
+// (wt_mma.cu) the patches the prep queued for it; exits at once when there are none
+cudaError_t launch_forward_mma(const wt_patch* patches, const HmDev& hm, float* pos, float* nrm, uint32_t flags,
+                               void* ws, const WsLayout& L, const FwdExtra& x, cudaStream_t s);
 // (wt_single.cu) a one-patch table of at most kSingleWaves waves, 8 vertices
 // per lane
 constexpr uint32_t kSingleWaves = 128;

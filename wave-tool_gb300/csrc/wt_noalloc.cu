@@ -116,6 +116,7 @@ extern "C" wt_status wt_noalloc_status(wt_stream stream, uint32_t* bad_patch) {
     if (bad_patch) *bad_patch = h[1];
     if (h[0] == WT_OK) return WT_OK;
     if (h[0] == WT_ERR_NOMEM) return fail(WT_ERR_NOMEM, "no-alloc scratch too small for the patches' wave slots");
+    if (h[0] == WT_ERR_TIMEOUT) return fail(WT_ERR_TIMEOUT, "a bounded wait of a matrix-product kernel ran out");
     char buf[96];
     snprintf(buf, sizeof(buf), "device-side validation failed at patch %u", h[1]);
     return fail((wt_status)h[0], buf);

@@ -26,7 +26,7 @@ __device__ __forceinline__ bool patch_ok(const wt_patch& P, uint32_t n_waves, ui
            P.flags == 0 && (uint64_t)P.wave_offset + P.wave_count <= n_waves && P.out_offset <= out_capacity &&
            verts <= out_capacity - P.out_offset && finitef(P.bl[0]) && finitef(P.bl[1]) && finitef(P.br[0]) &&
            finitef(P.br[1]) && finitef(P.tl[0]) && finitef(P.tl[1]) && finitef(P.tr[0]) && finitef(P.tr[1]) &&
-           isfinite(P.time_s) && finitef(P.y_offset);
+           (__double2hiint(P.time_s) & 0x7ff00000) != 0x7ff00000 && finitef(P.y_offset);
 }
 
 // turns mod 1 as 64-bit fixed point
