@@ -224,3 +224,26 @@ def test_png_heightmap_end_to_end(wt, oracle, gpu, tmp_path):
                                                           wt.WT_WRAP_MIRRORED_REPEAT)).displace()[0]
     torch.cuda.synchronize()
     assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("w,h,n,k", [(1, 1, 1, 1), (1, 70, 3, 2), (33, 31, 64, 8), (65, 32, 65, 16), (1000, 700, 5, 32),
+                                     (1030, 611, 130, 32), (2048, 33, 1, 3)])
+def test_noise_tile_and_chunk_edges(wt, oracle, gpu, w, h, n, k):
+    """Partial tiles, several tiles per block, one term past a chunk; the
+    extremes map to exactly 0 and 1 (a constant layer to 0)."""
+    from wave_tool_gb300 import workloads
+    terms = workloads.noise_terms(workloads.SplitMix64(w + n), n=n, kmax=k)
+    rates = np.linspace(-3.0, 3.0, n).astype(np.float32)
+    got = wt.noise_synth(terms, w, h, rates=rates, time_s=77.25).cpu().numpy()
+    if w * h == 1:
+        assert got[0, 0] == 0.0
+        return
+    assert got.min() == 0.0 and got.max() == 1.0
+    assert np.abs(got - oracle.noise_f64(terms, w, h, rates=rates, time_s=77.25)).max() < 2e-6 * n ** 0.5 + 2e-6
+
+
+def test_noise_without_terms_is_zero(wt, gpu):
+    import torch
+    out = torch.full((300, 500), 7.0, device="cuda")
+    wt.noise_synth(wt.empty_bytes(16)[:0], 500, 300, out=out)
+    assert bool((out == 0).all())

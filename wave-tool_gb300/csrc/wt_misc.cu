@@ -2,6 +2,7 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 
+#include "wt_device.cuh"
 #include "wt_internal.h"
 
 namespace wt {
@@ -46,7 +47,7 @@ __global__ void __launch_bounds__(256) k_unorm8(const uint8_t* __restrict__ px, 
 }
 
 // ---- noise heightmap -------------------------------------------------------
-constexpr size_t kNoiseHeader = 256;  // workspace: min / max, then the factor tables
+constexpr size_t kNoiseHeader = 256;
 __device__ __forceinline__ uint32_t ordered(float f) {
     uint32_t b = __float_as_uint(f);
     return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
@@ -55,104 +56,143 @@ __device__ __forceinline__ float unordered(uint32_t k) {
     return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
 
-__global__ void k_noise_init(uint32_t* mm) {
-    mm[0] = 0xffffffffu;  // min (ordered)
-    mm[1] = 0u;           // max (ordered)
-}
-
 // h(i, j) = sum_m a_m sin(x_m(i) + y_m(j)),
 //   x_m(i) = 2 pi (kx_m i mod W) / W,  y_m(j) = 2 pi (ky_m j mod H) / H + psi_m + rate_m t,
-// is separable: sin(x + y) = sin x cos y + cos x sin y.  k_noise_tables forms,
-// once per term, the column factors (sin x, cos x) for every column and the
-// row factors a (cos y, sin y) for every row (integer products reduced
-// exactly, the time-shifted row turn reduced in FP64, sines by FP32
-// sincospi); k_noise_tiles then spends two FMAs per texel and term.
-constexpr uint32_t kNoiseTile = 32;     // texels per block side (16 x 16 threads, 2 x 2 each)
-constexpr uint32_t kNoiseChunk = 32;    // terms staged in shared memory at a time
+// is separable: sin(x + y) = sin x cos y + cos x sin y.  A block forms, per tile
+// of texels and chunk of terms, the factors (sin x, cos x) of its columns and
+// a (cos y, sin y) of its rows in shared memory (phases as 32-bit fixed-point
+// turns, so that the wrap-around is the reduction; the time-shifted phase reduced
+// in FP64 once per term), then spends one paired FMA per texel and term.  Each block leaves its
+// minimum and maximum in the workspace, and k_noise_norm reduces those and
+// normalises.  Two dependent launches: the layer of 512^2 texels and 64 terms
+// took 23.4 us as four (min / max reset, factor tables through global memory,
+// tiles, normalise), 10.0 us this way; what is left is launches and latency
+// (33 MFMA, 2 MB).
+// A tile is 16 x 16 threads of M x M texels: M = 2 for layers that fill the GPU
+// only so, 4 where there are tiles enough (a quarter of the factors and half
+// the shared-memory reads per texel: 1024^2 x 64 terms 22.6 against 26.2 us,
+// 2048^2 x 128 105 against 143 us).
+constexpr uint32_t kNoiseBlocks = 608; // resident blocks at most (4 per SM)
+__host__ __device__ constexpr uint32_t noise_tile(int m) { return 16u * (uint32_t)m; }
 
-__global__ void __launch_bounds__(256) k_noise_tables(const wt_noise_term* __restrict__ terms, uint32_t n_terms,
-                                                      const float* __restrict__ rates, double t, uint32_t W,
-                                                      uint32_t H, float2* __restrict__ col, float2* __restrict__ row) {
-    const uint64_t per = (uint64_t)W + H, n = per * n_terms;
-    for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t m = (uint32_t)(k / per);
-        const uint32_t r = (uint32_t)(k - (uint64_t)m * per);
-        const wt_noise_term tm = terms[m];
-        float sn, cs;
-        if (r < W) {
-            long long ni = ((long long)tm.kx * r) % (long long)W;
-            ni += ni < 0 ? W : 0;
-            sincospif(2.0f * (float)((double)ni / W), &sn, &cs);
-            col[(size_t)m * W + r] = make_float2(sn, cs);
-        } else {
-            const uint32_t j = r - W;
-            long long nj = ((long long)tm.ky * j) % (long long)H;
-            nj += nj < 0 ? H : 0;
-            // the row's turn: exact fraction plus (psi + rate t) / 2 pi,
-            // reduced mod 1 in FP64 (t may be large), then an FP32 sincospi
-            double turns = (double)nj / H + ((double)tm.phase + (rates ? (double)rates[m] * t : 0.0)) *
-                                                (0.5 / 3.14159265358979323846);
-            turns -= floor(turns);
-            sincospif(2.0f * (float)turns, &sn, &cs);
-            row[(size_t)m * H + j] = make_float2(tm.amplitude * cs, tm.amplitude * sn);
-        }
-    }
-}
-
-__global__ void __launch_bounds__(256) k_noise_tiles(const float2* __restrict__ col, const float2* __restrict__ row,
-                                                     uint32_t n_terms, uint32_t W, uint32_t H,
-                                                     float* __restrict__ out, uint32_t* mm) {
-    __shared__ float2 sc[kNoiseChunk][kNoiseTile], sr[kNoiseChunk][kNoiseTile];
+template <int M>
+__global__ void __launch_bounds__(256) k_noise_tiles(const wt_noise_term* __restrict__ terms, uint32_t n_terms,
+                                                     const float* __restrict__ rates, double t, uint32_t W, uint32_t H,
+                                                     unsigned long long inv_w, unsigned long long inv_h,
+                                                     float* __restrict__ out, uint2* __restrict__ mm) {
+    cudaTriggerProgrammaticLaunchCompletion();  // the normalising pass waits for this grid's end
+    constexpr uint32_t kNoiseTile = noise_tile(M), kNoiseChunk = 128u / M;  // terms at a time
+    __shared__ __align__(16) float2 sc[kNoiseChunk][kNoiseTile], sr[kNoiseChunk][kNoiseTile];
+    __shared__ uint4 term[kNoiseChunk];  // kx mod W, ky mod H, phase (turns * 2^32), amplitude
+    __shared__ uint32_t s_lo, s_hi;
     const uint32_t tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const uint32_t i0 = blockIdx.x * kNoiseTile, j0 = blockIdx.y * kNoiseTile;
-    float h[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};
-    for (uint32_t m0 = 0; m0 < n_terms; m0 += kNoiseChunk) {
-        const uint32_t nm = min(kNoiseChunk, n_terms - m0);
-        __syncthreads();
-        for (uint32_t e = threadIdx.x; e < kNoiseChunk * kNoiseTile; e += blockDim.x) {
-            const uint32_t m = e / kNoiseTile, q = e - m * kNoiseTile;
-            const bool tm = m < nm;
-            sc[m][q] = tm && i0 + q < W ? col[(size_t)(m0 + m) * W + i0 + q] : make_float2(0.0f, 0.0f);
-            sr[m][q] = tm && j0 + q < H ? row[(size_t)(m0 + m) * H + j0 + q] : make_float2(0.0f, 0.0f);
-        }
-        __syncthreads();
-        for (uint32_t m = 0; m < nm; ++m) {
+    const uint32_t tiles_x = (W + kNoiseTile - 1) / kNoiseTile, tiles = tiles_x * ((H + kNoiseTile - 1) / kNoiseTile);
+    if (threadIdx.x == 0) {
+        s_lo = 0xffffffffu;
+        s_hi = 0u;
+    }
+    float lo = INFINITY, hi = -INFINITY;
+    cudaGridDependencySynchronize();
+    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const uint32_t j0 = tile / tiles_x * kNoiseTile, i0 = (tile % tiles_x) * kNoiseTile;
+        float2 h[M][M];  // (sine, cosine) parts
 #pragma unroll
-            for (int b = 0; b < 2; ++b) {
-                const float2 y = sr[m][2 * ty + b];
+        for (int b = 0; b < M; ++b)
 #pragma unroll
-                for (int a = 0; a < 2; ++a) {
-                    const float2 x = sc[m][2 * tx + a];
-                    h[b][a] = fmaf(x.x, y.x, fmaf(x.y, y.y, h[b][a]));
+            for (int a = 0; a < M; ++a) h[b][a] = make_float2(0.0f, 0.0f);
+        for (uint32_t m0 = 0; m0 < n_terms; m0 += kNoiseChunk) {
+            const uint32_t nm = min(kNoiseChunk, n_terms - m0);
+            __syncthreads();
+            if (threadIdx.x < nm) {
+                const wt_noise_term tm = terms[m0 + threadIdx.x];
+                const int32_t x = (int32_t)((int64_t)tm.kx % (int64_t)W), y = (int32_t)((int64_t)tm.ky % (int64_t)H);
+                // (psi + rate t) / 2 pi, reduced mod 1 in FP64 (t may be large)
+                double turns = ((double)tm.phase + (rates ? (double)rates[m0 + threadIdx.x] * t : 0.0)) *
+                               (0.5 / 3.14159265358979323846);
+                turns -= floor(turns);
+                term[threadIdx.x] = make_uint4((uint32_t)(x < 0 ? x + (int32_t)W : x), (uint32_t)(y < 0 ? y + (int32_t)H : y),
+                                               (uint32_t)__double2ull_rn(turns * 4294967296.0),
+                                               __float_as_uint(isfinite(turns) ? tm.amplitude : NAN));
+            }
+            __syncthreads();
+            for (uint32_t e = threadIdx.x; e < nm * 2u * kNoiseTile; e += blockDim.x) {
+                const uint32_t m = e / (2u * kNoiseTile), q = e % kNoiseTile;
+                const uint4 tm = term[m];
+                float sn, cs;
+                if ((e & kNoiseTile) == 0u) {
+                    dev::sincos_turns((uint32_t)((tm.x * (unsigned long long)(i0 + q) * inv_w) >> 32), sn, cs);
+                    sc[m][q] = make_float2(sn, cs);
+                } else {
+                    dev::sincos_turns((uint32_t)((tm.y * (unsigned long long)(j0 + q) * inv_h) >> 32) + tm.z, sn, cs);
+                    const float a = __uint_as_float(tm.w);
+                    sr[m][q] = make_float2(a * cs, a * sn);
                 }
             }
-        }
-    }
-    // block min / max, then one atomic each
-    float lo = INFINITY, hi = -INFINITY;
+            __syncthreads();
+#pragma unroll 4
+            for (uint32_t m = 0; m < nm; ++m) {
+                float2 x[M], y[M];
 #pragma unroll
-    for (int b = 0; b < 2; ++b)
+                for (int a = 0; a < M; a += 2) {
+                    const float4 v = *reinterpret_cast<const float4*>(&sc[m][M * tx + a]);
+                    const float4 w = *reinterpret_cast<const float4*>(&sr[m][M * ty + a]);
+                    x[a] = make_float2(v.x, v.y);
+                    x[a + 1] = make_float2(v.z, v.w);
+                    y[a] = make_float2(w.x, w.y);
+                    y[a + 1] = make_float2(w.z, w.w);
+                }
 #pragma unroll
-        for (int a = 0; a < 2; ++a) {
-            const uint32_t i = i0 + 2 * tx + a, j = j0 + 2 * ty + b;
-            if (i < W && j < H) {
-                lo = fminf(lo, h[b][a]);
-                hi = fmaxf(hi, h[b][a]);
-                out[(size_t)j * W + i] = h[b][a];
+                for (int b = 0; b < M; ++b)
+#pragma unroll
+                    for (int a = 0; a < M; ++a) h[b][a] = __ffma2_rn(x[a], y[b], h[b][a]);
             }
         }
-    for (int o = 16; o > 0; o >>= 1) {
-        lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-        hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+#pragma unroll
+        for (int b = 0; b < M; ++b)
+#pragma unroll
+            for (int a = 0; a < M; ++a) {
+                const uint32_t i = i0 + M * tx + a, j = j0 + M * ty + b;
+                if (i < W && j < H) {
+                    const float v = h[b][a].x + h[b][a].y;
+                    lo = fminf(lo, v);
+                    hi = fmaxf(hi, v);
+                    out[(size_t)j * W + i] = v;
+                }
+            }
     }
-    if ((threadIdx.x & 31) == 0 && lo <= hi) {
-        atomicMin(mm, ordered(lo));
-        atomicMax(mm + 1, ordered(hi));
+    const uint32_t wlo = __reduce_min_sync(0xffffffffu, ordered(lo)), whi = __reduce_max_sync(0xffffffffu, ordered(hi));
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) {
+        atomicMin(&s_lo, wlo);
+        atomicMax(&s_hi, whi);
     }
+    __syncthreads();
+    if (threadIdx.x == 0) mm[blockIdx.x] = make_uint2(s_lo, s_hi);
 }
 
-__global__ void __launch_bounds__(256) k_noise_norm(float* __restrict__ out, size_t n, const uint32_t* mm) {
-    const float lo = unordered(mm[0]), hi = unordered(mm[1]);
+__global__ void __launch_bounds__(256) k_noise_norm(float* __restrict__ out, size_t n, const uint2* __restrict__ mm,
+                                                    uint32_t blocks) {
+    __shared__ uint32_t s_lo, s_hi;
+    if (threadIdx.x == 0) {
+        s_lo = 0xffffffffu;
+        s_hi = 0u;
+    }
+    cudaGridDependencySynchronize();
+    __syncthreads();
+    uint32_t a = 0xffffffffu, b = 0u;
+    for (uint32_t i = threadIdx.x; i < blocks; i += blockDim.x) {
+        const uint2 v = mm[i];
+        a = min(a, v.x);
+        b = max(b, v.y);
+    }
+    a = __reduce_min_sync(0xffffffffu, a);
+    b = __reduce_max_sync(0xffffffffu, b);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMin(&s_lo, a);
+        atomicMax(&s_hi, b);
+    }
+    __syncthreads();
+    const float lo = unordered(s_lo), hi = unordered(s_hi);
     const float span = hi - lo;
     // a correctly rounded division maps the extremes to exactly 0 and 1
     for (size_t v = blockIdx.x * (size_t)blockDim.x + threadIdx.x; v < n; v += (size_t)gridDim.x * blockDim.x)
@@ -214,21 +254,32 @@ cudaError_t launch_unorm8(const uint8_t* px, uint32_t w, uint32_t h, uint32_t ch
 
 cudaError_t launch_noise(const wt_noise_term* terms, uint32_t n_terms, const float* rates, double t, uint32_t w,
                          uint32_t h, float* out, void* ws, cudaStream_t s) {
-    uint32_t* mm = static_cast<uint32_t*>(ws);
-    float2* col = reinterpret_cast<float2*>(static_cast<char*>(ws) + kNoiseHeader);
-    float2* row = col + (size_t)n_terms * w;
-    k_noise_init<<<1, 1, 0, s>>>(mm);
-    const uint64_t entries = (uint64_t)n_terms * ((uint64_t)w + h);
-    if (entries > 0) {
-        const uint64_t tb = (entries + 255) / 256;
-        k_noise_tables<<<(unsigned)(tb < 65536 ? tb : 65536), 256, 0, s>>>(terms, n_terms, rates, t, w, h, col, row);
-    }
-    dim3 grid((w + kNoiseTile - 1) / kNoiseTile, (h + kNoiseTile - 1) / kNoiseTile);
-    k_noise_tiles<<<grid, 256, 0, s>>>(col, row, n_terms, w, h, out, mm);
-    size_t n = (size_t)w * h;
-    unsigned blocks = (unsigned)((n + 255) / 256 < 4096 ? (n + 255) / 256 : 4096);
-    k_noise_norm<<<blocks, 256, 0, s>>>(out, n, mm);
-    return cudaGetLastError();
+    // a block's minimum and maximum: the workspace holds 8 (256 + terms * (w + h))
+    // bytes or more of them, never fewer than min(tiles, kNoiseBlocks) with a
+    // term, and 32 without any (all texels are then zero)
+    const auto tiles_of = [&](uint32_t side) { return (uint64_t)((w + side - 1) / side) * ((h + side - 1) / side); };
+    const bool wide = tiles_of(noise_tile(4)) >= 256;
+    const uint64_t tiles = tiles_of(noise_tile(wide ? 4 : 2));
+    const uint32_t cap = n_terms > 0 ? kNoiseBlocks : (uint32_t)(kNoiseHeader / sizeof(uint2));
+    const uint32_t blocks = (uint32_t)(tiles < cap ? tiles : cap);
+    uint2* mm = static_cast<uint2*>(ws);
+    cudaLaunchConfig_t lc = {};
+    lc.blockDim = dim3(256);
+    lc.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = attr;
+    lc.numAttrs = 1;
+    lc.gridDim = dim3(blocks);
+    // 2^64 / size, rounded down: a product with k j < 2^30 is off by less than
+    // 2^-34 turns
+    const auto inverse = [](uint32_t n) { return n > 1u ? ~0ull / n : 0ull; };
+    cudaError_t e = cudaLaunchKernelEx(&lc, wide ? k_noise_tiles<4> : k_noise_tiles<2>, terms, n_terms, rates, t, w, h, inverse(w), inverse(h), out, mm);
+    if (e != cudaSuccess) return e;
+    const size_t n = (size_t)w * h;
+    lc.gridDim = dim3((unsigned)((n + 255) / 256 < 4096 ? (n + 255) / 256 : 4096));
+    return cudaLaunchKernelEx(&lc, k_noise_norm, out, n, static_cast<const uint2*>(mm), blocks);
 }
 
 size_t noise_workspace_bytes(uint32_t n_terms, uint32_t w, uint32_t h) {

@@ -137,24 +137,6 @@ __device__ __forceinline__ void tmem_wait(float (&a)[8], float (&b)[8]) {
                  : "+f"(b[0]), "+f"(b[1]), "+f"(b[2]), "+f"(b[3]), "+f"(b[4]), "+f"(b[5]), "+f"(b[6]), "+f"(b[7])::"memory");
 }
 
-// sin and cos of 2 pi t / 2^32: the nearest quarter turn taken off exactly,
-// then y P(y^2) and Q(y^2) on |y| <= 1/8 turn (least maximum error over that
-// range, degrees 7 and 8, fitted here), 1e-7 with their FP32 rounding.
-__device__ __forceinline__ void sincos_turns(uint32_t t, float& s, float& c) {
-    const uint32_t q = (t + 0x20000000u) >> 30;
-    const float y = (float)(int)(t - (q << 30)) * 2.3283064365386963e-10f;
-    const float w = y * y;
-    const float2 w2 = make_float2(w, w);
-    float2 pq = make_float2(-75.40206909179688f, fmaf(59.22040557861328f, w, -85.44285583496094f));
-    pq = __ffma2_rn(pq, w2, make_float2(81.5925521850586f, 64.93931579589844f));
-    pq = __ffma2_rn(pq, w2, make_float2(-41.3416633605957f, -19.739208221435547f));
-    pq = __ffma2_rn(pq, w2, make_float2(6.2831854820251465f, 1.0f));
-    const float s0 = y * pq.x, c0 = pq.y;
-    const bool odd = q & 1u;
-    s = __uint_as_float(__float_as_uint(odd ? c0 : s0) ^ ((q & 2u) << 30));
-    c = __uint_as_float(__float_as_uint(odd ? s0 : c0) ^ (((q + 1u) & 2u) << 30));
-}
-
 __device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
 
 // p as fp16 pairs hi + lo
