@@ -367,7 +367,7 @@ typedef struct wt_view {
  * degrees, the clamp the reference applies to every pitch. */
 wt_status wt_projected_grid(const wt_camera* camera, wt_patch* patch, wt_view* view, uint32_t* status);
 
-/* The same computation as one single-thread kernel on `stream`, reading the
+/* The same computation as one small kernel on `stream`, reading the
  * camera from device memory and writing the corners of the device patch and
  * the device wt_view, so a camera -> vertices frame (this, then
  * wt_gerstner_displace, then wt_vertex_stage) can be captured and replayed as

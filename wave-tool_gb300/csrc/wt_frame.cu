@@ -2,9 +2,9 @@
 // outputs that follow the displacement.
 //
 // The projected grid restates src/render-engine.cpp:797-1042 in FP64 as a
-// set of __host__ __device__ steps: wt_projected_grid runs them one after
-// another on the host, wt_projected_grid_async spreads them over one warp of
-// a kernel that reads the camera from device memory, so that camera ->
+// set of steps: wt_projected_grid runs them one after another on the host,
+// wt_projected_grid_async spreads them over the lanes of two warps of a kernel
+// that reads the camera from device memory, so that camera ->
 // corners -> displaced vertices is one stream of kernels a CUDA graph can
 // replay with a new camera every frame.
 //
@@ -42,8 +42,6 @@ WT_HD D3 operator+(D3 a, D3 b) { return {a.x + b.x, a.y + b.y, a.z + b.z}; }
 WT_HD D3 operator-(D3 a, D3 b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
 WT_HD D3 operator*(double s, D3 a) { return {s * a.x, s * a.y, s * a.z}; }
 WT_HD double dot(D3 a, D3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-WT_HD D3 cross(D3 a, D3 b) { return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x}; }
-WT_HD D3 unit(D3 a) { return (1.0 / sqrt(dot(a, a))) * a; }
 
 // 4x4 matrix in OpenGL (column-major) order: m[c][r] is row r of column c.
 struct M4 {
@@ -69,9 +67,9 @@ WT_HD M4 mul(const M4& a, const M4& b) {
 }
 
 // The camera's basis (Camera::updateBasisVectors, src/camera.cpp:130-137)
-// for a yaw given by its cosine and sine: pitch clamped, world up +y.  The
-// right vector normalize(cross(forward, +y)) is (-sin yaw, 0, cos yaw) for
-// every pitch.
+// for a yaw and a clamped pitch given by their sines and cosines, world up +y:
+// with those, normalize(cross(forward, +y)) is (-sin yaw, 0, cos yaw) and
+// cross(right, forward) is unit as it stands.
 struct Basis {
     D3 pos, fwd, right, up;
 };
@@ -85,16 +83,12 @@ WT_HD void sincos_pi(double x, double* s, double* c) {
 #endif
 }
 
-// cos(89 degrees), the smallest cosine of a clamped pitch
+// cosine and sine of 89 degrees, the clamp of a pitch
 WT_HD double cos89() { return 0.017452406437283512819; }
+WT_HD double sin89() { return 0.99984769515639123916; }
 
 WT_HD Basis camera_basis(D3 pos, double cy, double sy, double sp, double cp) {
-    Basis b;
-    b.pos = pos;
-    b.fwd = unit(D3{cy * cp, sp, sy * cp});
-    b.right = D3{-sy, 0.0, cy};
-    b.up = unit(cross(b.right, b.fwd));
-    return b;
+    return Basis{pos, D3{cy * cp, sp, sy * cp}, D3{-sy, 0.0, cy}, D3{-cy * sp, cp, -sy * sp}};
 }
 
 // Right-handed look-at along the basis' forward vector (glm::lookAt, whose
@@ -122,11 +116,19 @@ WT_HD M4 perspective(double tan_half_fov, double aspect, double zn, double zf) {
     return p;
 }
 
+WT_HD bool finite_bits(double x) {
+#ifdef __CUDA_ARCH__
+    return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000;  // (no FP64 comparison)
+#else
+    return std::isfinite(x);
+#endif
+}
+
 WT_HD bool camera_ok(const wt_camera& c) {
     const double v[10] = {c.position[0], c.position[1], c.position[2], c.yaw_deg, c.pitch_deg,
                           c.fov_deg, c.aspect, c.z_near, c.z_far, c.displaceable_amplitude};
     for (double x : v)
-        if (!isfinite(x)) return false;
+        if (!finite_bits(x)) return false;
     return c.fov_deg > 0.0 && c.fov_deg < 180.0 && c.aspect > 0.0 && c.z_near > 0.0 && c.z_far > c.z_near &&
            c.displaceable_amplitude >= 0.0;
 }
@@ -181,7 +183,10 @@ WT_HD void frame_setup(const wt_camera& c, double sy, double cy, double sp, doub
     // its sine and cosine come straight from d
     const double hz = sqrt(d.x * d.x + d.z * d.z), r = sqrt(hz * hz + d.y * d.y);
     double psp = -fabs(d.y) / r, pcp = hz / r;
-    if (!(pcp >= cos89())) sincos_pi(-kPitchLimit / 180.0, &psp, &pcp);
+    if (!(pcp >= cos89())) {
+        psp = -sin89();
+        pcp = cos89();
+    }
     f->pj = camera_basis(ppos, cy, sy, psp, pcp);
 }
 
@@ -303,86 +308,141 @@ WT_HD void store_result(const wt_camera& c, const Grid& g, wt_patch* patch, wt_v
     }
 }
 
-__device__ __forceinline__ D3 shfl_d3(D3 v, int src) {
-    return D3{__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src),
-              __shfl_sync(0xffffffffu, v.z, src)};
+__device__ __forceinline__ double shfl(double v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+__device__ __forceinline__ D3 shfl_d3(D3 v, int src) { return D3{shfl(v.x, src), shfl(v.y, src), shfl(v.z, src)}; }
+
+// Doubles as signed integers in the same order, and their extremes over a warp
+// by integer comparisons (an FP64 one costs as much as an addition).
+__device__ __forceinline__ long long order_key(double x) {
+    const long long b = __double_as_longlong(x);
+    return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+__device__ __forceinline__ double key_value(long long k) {
+    return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
 }
 
-// The same steps spread over one warp: three lanes take the trigonometry,
-// eight the frustum corners, twelve the edges and eight the corners inside
-// the slab, the NDC bounds are reduced across lanes, four lanes cast the grid
-// corners and sixteen write the matrices.  A single thread on GB300's FP64
-// pipe spends most of its time in dependent-instruction latency.
-__global__ void __launch_bounds__(32) k_projected_grid(const wt_camera* __restrict__ camera, wt_patch* patch,
+// The same steps in one block of two warps on different schedulers: warp 0
+// finds the corners, warp 1 the matrices.  Everything is FP64 latency: a
+// warp-wide FP64 operation takes about 64 cycles on GB300 and a division or
+// square root about 550, whatever the number of lanes, so divisions that do
+// not depend on one another are taken together, one per lane (the three camera
+// angles; four quotients of the angles and the aim; 24 edge-plane crossings and
+// 8 corners, one point per lane).  One warp going through the steps of
+// projected_grid took 19.0 us; a frame's vertices (513^2 grid, 4 waves) went
+// from 32.8 to 24.6 us.
+__global__ void __launch_bounds__(64) k_projected_grid(const wt_camera* __restrict__ camera, wt_patch* patch,
                                                        wt_view* view) {
-    const int lane = threadIdx.x;
+    const int lane = threadIdx.x & 31;
     const wt_camera c = *camera;
     if (!camera_ok(c)) {
-        if (lane == 0) view->status = WT_VIEW_INVALID_CAMERA;
+        if (threadIdx.x == 0) view->status = WT_VIEW_INVALID_CAMERA;
         return;
     }
-    // lanes 0-2: camera_trig(c, lane) with one shared instruction stream (a
-    // warp-wide FP64 operation costs ~64 cycles and a division ~550 on
-    // GB300; three divergent branches ran three sines and cosines one after
-    // another): each lane selects its own numerator and denominator
-    double ts = 0.0, tc = 1.0;
-    if (lane < 3) {
-        const double yaw = c.yaw_deg - 360.0 * floor(c.yaw_deg / 360.0);
+    // lanes 0-2: yaw, clamped pitch, half the field of view
+    double ts, tc;
+    {
+        const double yaw = c.yaw_deg - 360.0 * floor(c.yaw_deg * (1.0 / 360.0));
         const double pitch = fmin(fmax(c.pitch_deg, -kPitchLimit), kPitchLimit);
-        const double num = lane == 0 ? yaw : (lane == 1 ? pitch : c.fov_deg);
-        sincos_pi(num / (lane == 2 ? 360.0 : 180.0), &ts, &tc);
+        const double angle = lane == 0 ? yaw : (lane == 1 ? pitch : c.fov_deg);
+        sincos_pi(angle * (lane < 2 ? 1.0 / 180.0 : 1.0 / 360.0), &ts, &tc);
     }
-    const double sy = __shfl_sync(0xffffffffu, ts, 0), cy = __shfl_sync(0xffffffffu, tc, 0);
-    const double sp = __shfl_sync(0xffffffffu, ts, 1), cp = __shfl_sync(0xffffffffu, tc, 1);
-    const double sf = __shfl_sync(0xffffffffu, ts, 2), cf = __shfl_sync(0xffffffffu, tc, 2);
-    Frame f;
-    frame_setup(c, sy, cy, sp, cp, sf, cf, &f);
+    const double sy = shfl(ts, 0), cy = shfl(tc, 0), sp = shfl(ts, 1), cp = shfl(tc, 1), sf = shfl(ts, 2), cf = shfl(tc, 2);
+    const D3 eye{c.position[0], c.position[1], c.position[2]};
+    const Basis cam = camera_basis(eye, cy, sy, sp, cp);
 
-    const D3 mine = frustum_corner(f, lane & 7);
-    const int e = lane < 12 ? lane : 0;
-    const D3 ea = shfl_d3(mine, edge_end(e, 0)), eb = shfl_d3(mine, edge_end(e, 1));
-    const D3 corner = shfl_d3(mine, (lane >= 12 && lane < 20) ? lane - 12 : 0);
-    double px[2], pz[2];
-    int n = 0;
-    if (lane < 12) {
-        n = edge_points(f, ea, eb, px, pz);
-    } else if (lane < 20 && -f.amp <= corner.y && corner.y <= f.amp) {
-        px[0] = corner.x;
-        pz[0] = corner.z;
-        n = 1;
+    if (threadIdx.x >= 32) {
+        // the four entries of the perspective matrix, one division per lane
+        const double num = lane < 2 ? cf : (lane == 2 ? -(c.z_far + c.z_near) : -2.0 * c.z_far * c.z_near);
+        const double den = lane == 0 ? sf * c.aspect : (lane == 1 ? sf : c.z_far - c.z_near);
+        const double quot = num / den;
+        const double p22 = shfl(quot, 2), p32 = shfl(quot, 3);
+        // element (row, column) of perspective * view and of the yaw-only view:
+        // row r of a view matrix is (b, -b . eye) with b = right, up or -forward,
+        // and the perspective's rows scale rows 0, 1, 2, and repeat row 2 negated
+        const int col = (lane >> 2) & 3, row = lane & 3;
+        const D3 b = row == 0 ? cam.right : (row == 1 ? cam.up : -1.0 * cam.fwd);
+        const D3 y = row == 0 ? cam.right : (row == 1 ? D3{0.0, 1.0, 0.0} : D3{-cy, 0.0, -sy});
+        const double bd = -dot(b, eye), yd = -dot(y, eye);
+        const double be = col == 0 ? b.x : (col == 1 ? b.y : (col == 2 ? b.z : bd));
+        const double ye = col == 0 ? y.x : (col == 1 ? y.y : (col == 2 ? y.z : yd));
+        const double scale = row == 3 ? -1.0 : (row == 2 ? p22 : (row == 1 ? shfl(quot, 1) : shfl(quot, 0)));
+        const double element = scale * be + (row == 2 && col == 3 ? p32 : 0.0);
+        if (lane < 16) {
+            view->view_projection[lane] = (float)element;
+            view->view_only_yaw[lane] = row == 3 ? (col == 3 ? 1.0f : 0.0f) : (float)ye;
+        }
+        if (lane < 3) view->camera_position[lane] = (float)c.position[lane];
+        return;
     }
-    double x0 = INFINITY, x1 = -INFINITY, y0 = INFINITY, y1 = -INFINITY;
-    for (int k = 0; k < n; ++k) {
-        double X, Y;
-        projector_ndc(f, px[k], pz[k], &X, &Y);
-        x0 = fmin(x0, X);
-        x1 = fmax(x1, X);
-        y0 = fmin(y0, Y);
-        y1 = fmax(y1, Y);
+
+    // the aim ray (frame_setup's steps), and tan(fov / 2), its inverses and the
+    // ray's length to the base plane in one division
+    const double amp = c.displaceable_amplitude, min_height = amp + kProjectorElevation;
+    const bool underwater = eye.y < 0.0;
+    D3 fs = cam.fwd;
+    if (fabs(fs.y) < kHorizonEpsilon) fs.y = (fs.y >= 0.0) ? kHorizonEpsilon : -kHorizonEpsilon;
+    const D3 ray = ((fs.y < 0.0) != underwater) ? fs : D3{fs.x, -fs.y, fs.z};
+    double quot;
+    {
+        const double num = lane == 0 ? sf : (lane < 3 ? cf : -eye.y);
+        const double den = lane == 0 ? cf : (lane == 1 ? sf : (lane == 2 ? sf * c.aspect : ray.y));
+        quot = num / den;
     }
-    const bool any = __ballot_sync(0xffffffffu, n > 0) != 0;
+    const double ty = shfl(quot, 0), ity = shfl(quot, 1), itx = shfl(quot, 2), reach = shfl(quot, 3), tx = ty * c.aspect;
+    D3 ppos = eye;
+    if (eye.y < min_height) ppos.y = underwater ? min_height - eye.y : min_height;
+    const double a = fabs(fs.y), a1 = 1.0 - a;
+    const D3 d = {a1 * (eye.x + cam.fwd.x) + a * (eye.x + reach * ray.x) - ppos.x,
+                  a * (eye.y + reach * ray.y) - ppos.y,
+                  a1 * (eye.z + cam.fwd.z) + a * (eye.z + reach * ray.z) - ppos.z};
+    const double h2 = d.x * d.x + d.z * d.z;
+    const double root = sqrt(lane == 0 ? h2 : h2 + d.y * d.y);
+    const double r = shfl(root, 1), ratio = (lane == 0 ? root : -fabs(d.y)) / r;
+    double pcp = shfl(ratio, 0), psp = shfl(ratio, 1);
+    if (!(pcp >= cos89())) {
+        psp = -sin89();
+        pcp = cos89();
+    }
+    const Basis pj = camera_basis(ppos, cy, sy, psp, pcp);
+
+    // lane 2 e + k: where edge e crosses y = +-amp; lane 24 + i: corner i, if it
+    // lies in the slab
+    const double depth = (lane & 1) ? c.z_far : c.z_near;
+    const double X = ((lane & 4) ? kFrustumPad : -kFrustumPad) * tx * depth;
+    const double Y = ((lane & 2) ? kFrustumPad : -kFrustumPad) * ty * depth;
+    const D3 corner = eye + X * cam.right + Y * cam.up + depth * cam.fwd;  // of index lane & 7
+    const int e = lane < 24 ? lane >> 1 : 0;
+    const D3 e0 = shfl_d3(corner, edge_end(e, 0)), e1 = shfl_d3(corner, edge_end(e, 1));
+    const double h = (lane & 1) ? -amp : amp;
+    const double t = (h - e0.y) / (e1.y - e0.y);
+    double px = e0.x + t * (e1.x - e0.x), pz = e0.z + t * (e1.z - e0.z);
+    bool found = e0.y != e1.y && fmin(e0.y, e1.y) <= h && h <= fmax(e0.y, e1.y);
+    if (lane >= 24) {
+        px = corner.x;
+        pz = corner.z;
+        found = -amp <= corner.y && corner.y <= amp;
+    }
+    const D3 q = D3{px, 0.0, pz} - pj.pos;
+    const double iw = 1.0 / dot(pj.fwd, q);
+    const double nx = dot(pj.right, q) * itx * iw, ny = dot(pj.up, q) * ity * iw;
+    // (a point whose NDC is not a number bounds nothing, as with fmin and fmax)
+    const bool any = __ballot_sync(0xffffffffu, found) != 0;
+    const long long top = 0x7ff0000000000000ll;  // order_key(inf); of -inf: its complement
+    long long x0 = found && nx == nx ? order_key(nx) : top, x1 = found && nx == nx ? x0 : ~top;
+    long long y0 = found && ny == ny ? order_key(ny) : top, y1 = found && ny == ny ? y0 : ~top;
     for (int o = 16; o > 0; o >>= 1) {
-        x0 = fmin(x0, __shfl_xor_sync(0xffffffffu, x0, o));
-        x1 = fmax(x1, __shfl_xor_sync(0xffffffffu, x1, o));
-        y0 = fmin(y0, __shfl_xor_sync(0xffffffffu, y0, o));
-        y1 = fmax(y1, __shfl_xor_sync(0xffffffffu, y1, o));
+        x0 = min(x0, __shfl_xor_sync(0xffffffffu, x0, o));
+        x1 = max(x1, __shfl_xor_sync(0xffffffffu, x1, o));
+        y0 = min(y0, __shfl_xor_sync(0xffffffffu, y0, o));
+        y1 = max(y1, __shfl_xor_sync(0xffffffffu, y1, o));
     }
-    double gx = 0.0, gz = 0.0;
-    const bool ok = lane < 4 && any && corner_ray(f, (lane & 1) ? x1 : x0, (lane & 2) ? y1 : y0, &gx, &gz);
+    // lanes 0-3: a corner of the bounds cast onto y = 0
+    const double cx = key_value((lane & 1) ? x1 : x0), cyy = key_value((lane & 2) ? y1 : y0);
+    const D3 dir = (cx * tx) * pj.right + (cyy * ty) * pj.up + pj.fwd;
+    const double s = -pj.pos.y / dir.y;
+    const double gx = pj.pos.x + s * dir.x, gz = pj.pos.z + s * dir.z;
+    const bool ok = any && dir.y != 0.0 && finite_bits(gx) && finite_bits(gz);
     const bool visible = (__ballot_sync(0xffffffffu, ok) & 0xfu) == 0xfu;
-    if (lane < 16) {
-        // view_matrices, one element per lane: the two factors of the
-        // view-projection in full (cheap), then this lane's element of
-        // their product in mul's order
-        const M4 P = perspective(f.ty, c.aspect, c.z_near, c.z_far), V = view_matrix(f.cam);
-        const M4 yaw = view_matrix(Basis{f.cam.pos, D3{cy, 0.0, sy}, D3{-sy, 0.0, cy}, D3{0.0, 1.0, 0.0}});
-        const int col = lane >> 2, row = lane & 3;
-        double e = 0.0;
-        for (int j = 0; j < 4; ++j) e += P.m[j][row] * V.m[col][j];
-        view->view_projection[lane] = (float)e;
-        view->view_only_yaw[lane] = (float)yaw.m[col][row];
-    }
-    if (lane < 3) view->camera_position[lane] = (float)c.position[lane];
     if (lane == 0) view->status = visible ? WT_VIEW_VISIBLE : WT_VIEW_EMPTY;
     if (visible && lane < 4) {
         float* dst = lane == 0 ? patch->bl : lane == 1 ? patch->br : lane == 2 ? patch->tl : patch->tr;
@@ -449,7 +509,7 @@ extern "C" wt_status wt_projected_grid_async(const wt_camera* camera, wt_patch* 
     if (!camera || !aligned(camera, 8)) return fail(WT_ERR_INVALID_ARG, "wt_projected_grid_async: camera NULL or misaligned");
     if (!patch || !aligned(patch, 8)) return fail(WT_ERR_INVALID_ARG, "wt_projected_grid_async: patch NULL or misaligned");
     if (!view || !aligned(view, 4)) return fail(WT_ERR_INVALID_ARG, "wt_projected_grid_async: view NULL or misaligned");
-    k_projected_grid<<<1, 32, 0, (cudaStream_t)stream>>>(camera, patch, view);
+    k_projected_grid<<<1, 64, 0, (cudaStream_t)stream>>>(camera, patch, view);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? WT_OK : cuda_fail(e, "wt_projected_grid_async launch");
 }
