@@ -14,6 +14,10 @@
 //       shared memory), regenerate the wave's sin/cos there (MUFU start +
 //       Chebyshev steps) and accumulate 11 per-wave moments; add them into
 //       the chunk's record for that wave (no cross-lane reduction).
+//   k_adjoint_mma  parallelogram patches of 8 to 64 waves instead, before it
+//                (wt_adjoint_mma.cu; in tables with work enough,
+//                adjoint_mma_waves): the moments as matrix products, a record
+//                per item of 128 columns by a run of rows
 //   k_adj_cols   column sums of each patch's records over its chunks (FP32
 //                Kahan, fixed order)
 //   k_adj_pairs  closed-form FP64 gradient per (patch, wave) pair, one per thread
@@ -31,6 +35,7 @@
 
 #include <atomic>
 
+#include "wt_adjoint.cuh"
 #include "wt_device.cuh"
 #include "wt_internal.h"
 
@@ -54,49 +59,6 @@ constexpr uint32_t kAdjChunkSaved = 1;
 constexpr uint32_t kAdjChunkMinTilesPerWarp = 8;
 constexpr int kGbufVerts = 256;              // vertices per tile (32 lanes x S <= 8)
 constexpr int kGbufF4 = 2;                   // float4 per parked vertex
-
-// Adjoints of the eight sums at one vertex.  Order: dx, dy, dz, jx, jz, sxx,
-// sxz, szz.  See oracle/gerstner_f64.c:wto_adjoint_f64 for the same algebra.
-__device__ __forceinline__ void vertex_adjoint(const VertexSums& s, float xl, float zl, const PatchAux& a,
-                                               const HmDev& hm, bool pow2, const float* __restrict__ gpos,
-                                               const float* __restrict__ gnrm, uint64_t vidx, bool vec3,
-                                               float g[8]) {
-    const float a1 = 1.0f - s.sxx, a3 = -s.sxz, b1 = -s.sxz, b3 = 1.0f - s.szz;
-    HmSample h = {0.0f, 0.0f, 0.0f, 0.0f};
-    if (hm.present) h = hm_sample(hm, a, xl + s.dx, zl + s.dz, pow2);
-    const float px0 = a1, px1 = fmaf(h.hx, a1, fmaf(h.hz, a3, s.jx)), px2 = a3;
-    const float pz0 = b1, pz1 = fmaf(h.hx, b1, fmaf(h.hz, b3, s.jz)), pz2 = b3;
-    const float* gp = gpos + (vec3 ? 3 : 4) * vidx;
-    const float gpx_ = gp[0], gpy_ = gp[1], gpz_ = gp[2];
-    float gPx0 = 0.0f, gPx1 = 0.0f, gPx2 = 0.0f, gPz0 = 0.0f, gPz1 = 0.0f, gPz2 = 0.0f;
-    if (gnrm) {
-        const float* gn = gnrm + (vec3 ? 3 : 4) * vidx;
-        const float N0 = pz1 * px2 - pz2 * px1, N1 = pz2 * px0 - pz0 * px2, N2 = pz0 * px1 - pz1 * px0;
-        const float inv = rsqrtf(fmaf(N0, N0, fmaf(N1, N1, N2 * N2)));
-        const float n0 = N0 * inv, n1 = N1 * inv, n2 = N2 * inv;
-        const float d = fmaf(n0, gn[0], fmaf(n1, gn[1], n2 * gn[2]));
-        const float gN0 = (gn[0] - n0 * d) * inv, gN1 = (gn[1] - n1 * d) * inv, gN2 = (gn[2] - n2 * d) * inv;
-        // N = Pz x Px:  g_Pz = Px x gN,  g_Px = gN x Pz
-        gPz0 = px1 * gN2 - px2 * gN1;
-        gPz1 = px2 * gN0 - px0 * gN2;
-        gPz2 = px0 * gN1 - px1 * gN0;
-        gPx0 = gN1 * pz2 - gN2 * pz1;
-        gPx1 = gN2 * pz0 - gN0 * pz2;
-        gPx2 = gN0 * pz1 - gN1 * pz0;
-    }
-    const float g_a1 = fmaf(gPx1, h.hx, gPx0), g_a3 = fmaf(gPx1, h.hz, gPx2);
-    const float g_b1 = fmaf(gPz1, h.hx, gPz0), g_b3 = fmaf(gPz1, h.hz, gPz2);
-    const float g_hx = fmaf(gPx1, a1, gPz1 * b1), g_hz = fmaf(gPx1, a3, gPz1 * b3);
-    const float g_X = fmaf(gpy_, h.hx, g_hz * h.hxz), g_Z = fmaf(gpy_, h.hz, g_hx * h.hxz);
-    g[0] = gpx_ + g_X;        // dx
-    g[1] = gpy_;              // dy
-    g[2] = gpz_ + g_Z;        // dz
-    g[3] = gPx1;              // jx
-    g[4] = gPz1;              // jz
-    g[5] = -g_a1;             // sxx
-    g[6] = -g_a3 - g_b1;      // sxz
-    g[7] = -g_b3;             // szz
-}
 
 // Phase 2: lane = one wave; vertices l + 32 j of the tile (gbuf holds the
 // eight vertex adjoints as two float4 of (cos-sum, sin-sum) pairs, (dx, dy)
@@ -289,7 +251,12 @@ k_adjoint(const wt_patch* __restrict__ patches, HmDev hm, const float* __restric
                         const float4 s0 = d[0], s1 = d[1];
                         const float xl = fmaf((float)vi, gx, xb0), zl = fmaf((float)vi, gz, zb0);
                         VertexSums sm{s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
-                        vertex_adjoint(sm, xl, zl, a, hm, pow2, gpos, gnrm, rowbase + col, vec3, g);
+                        const uint64_t at = (vec3 ? 3 : 4) * (rowbase + col);
+                        const float* gp = gpos + at;
+                        const float* gn = gnrm + at;
+                        vertex_adjoint(sm, xl, zl, a, hm, pow2, make_float3(gp[0], gp[1], gp[2]),
+                                       gnrm ? make_float3(gn[0], gn[1], gn[2]) : make_float3(0.0f, 0.0f, 0.0f),
+                                       gnrm != nullptr, g);
                     }
                     // (cos-sum, sin-sum) pairs: (dx, dy) (dz, sxx) | (jx, sxz) (jz, szz)
                     d[0] = make_float4(g[0], g[1], g[2], g[5]);
@@ -571,8 +538,28 @@ uint64_t adjoint_records(const wt_patch& p) {
     return (uint64_t)p.rows * dev::tiles_per_row(p.cols, 8) * p.wave_count;  // chunks of one tile
 }
 
+// By the terms (vertices x waves) of the patches that qualify, of 64 columns and
+// more: below these counts the kernel's own launch and its start cost more than
+// the products save.  Measured, products / recurrence: one patch of 64^2 with 16
+// waves 31.0 / 26.7 us, 32 31.3 / 30.5, 64 35.5 / 41.6, of 128^2 with 32 32.7 /
+// 37.1, of 512^2 with 8 35.5 / 41.1; from saved sums 64^2 with 64 waves 32.6 /
+// 33.2, 4 of 64^2 with 32 31.7 / 30.6, one of 192^2 with 32 31.7 / 42.3.  Patches
+// of fewer columns leave most of an item's 128 empty (16 of 32^2 with 32 waves
+// 38.1 / 34.2): they run as products only in a table that has them anyway.
+uint32_t adjoint_mma_waves(const wt_patch* host_patches, uint32_t n_patches, uint32_t n_waves, bool saved) {
+    uint64_t left = saved ? 9ull << 16 : 6ull << 16;
+    for (uint32_t i = 0; n_waves >= kMmaMinWaves && i < n_patches; ++i) {
+        const wt_patch& p = host_patches[i];
+        if (p.cols < 64 || !dev::mma_patch(p, kMmaAdjMaxWaves)) continue;
+        const uint64_t terms = (uint64_t)p.cols * p.rows * p.wave_count;
+        if (terms >= left) return kMmaAdjMaxWaves;
+        left -= terms;
+    }
+    return 0;
+}
+
 cudaError_t launch_adjoint(const wt_patch* patches, uint32_t n_patches, const wt_wave* waves, uint32_t n_waves,
-                           uint32_t max_waves_per_patch, const HmDev& hm, const float* gpos, const float* gnrm,
+                           uint32_t max_waves_per_patch, bool mma, const HmDev& hm, const float* gpos, const float* gnrm,
                            uint32_t flags, wt_wave_grad* grad, void* ws, const AdjLayout& L, const float* sums,
                            cudaStream_t s) {
     char* w = static_cast<char*>(ws);
@@ -580,6 +567,10 @@ cudaError_t launch_adjoint(const wt_patch* patches, uint32_t n_patches, const wt
     int occ = 1;
     cudaError_t e = sums ? adj_occupancy<true>(&occ) : adj_occupancy<false>(&occ);
     if (e != cudaSuccess) return e;
+    if (mma) {
+        e = launch_adjoint_mma(patches, hm, gpos, gnrm, flags, ws, L, sums, s);
+        if (e != cudaSuccess) return e;
+    }
     e = sums ? launch_adj_main<true>(sms, occ, s, patches, hm, gpos, gnrm, flags, w, L, sums)
              : launch_adj_main<false>(sms, occ, s, patches, hm, gpos, gnrm, flags, w, L, nullptr);
     if (e != cudaSuccess) return e;

@@ -70,11 +70,12 @@ static __device__ uint32_t block_exclusive_scan(uint32_t* a, uint32_t n) {
 
 // The adjoint's queue set-up, by one block after the prep's scans (needs
 // sorted, tile_pre and pair_off, and the header's total_tiles): each patch's
-// sorted rank, its chunks of tiles (chunk_max tiles per chunk when there are
-// at least min_tiles tiles, else single tiles) and the exclusive prefixes of
-// chunks and of records (chunks x waves) over the sorted order.
+// sorted rank, its chunks of tiles (chunk_max tiles per chunk when the table has
+// at least min_tiles tiles, mma_tiles of them in matrix-product patches, else
+// single tiles; a matrix-product patch's items are its chunks) and the exclusive
+// prefixes of chunks and of records (chunks x waves) over the sorted order.
 __device__ inline void adj_scan_body(char* ws, const AdjLayout& L, uint32_t n, uint32_t chunk_max,
-                                     uint32_t min_tiles) {
+                                     uint32_t min_tiles, uint64_t mma_tiles) {
     WsHeader* hdr = reinterpret_cast<WsHeader*>(ws);
     const uint32_t* sorted = reinterpret_cast<const uint32_t*>(ws + L.f.sorted);
     const uint32_t* tile_pre = reinterpret_cast<const uint32_t*>(ws + L.f.tile_pre);
@@ -82,11 +83,13 @@ __device__ inline void adj_scan_body(char* ws, const AdjLayout& L, uint32_t n, u
     uint32_t* rank = reinterpret_cast<uint32_t*>(ws + L.rank);
     uint32_t* part_off = reinterpret_cast<uint32_t*>(ws + L.part_off);
     uint32_t* chunk_pre = reinterpret_cast<uint32_t*>(ws + L.chunk_pre);
-    const uint32_t chunk = hdr->total_tiles >= min_tiles ? chunk_max : 1u;
+    const uint32_t chunk = hdr->total_tiles - hdr->mma_items + mma_tiles >= min_tiles ? chunk_max : 1u;
+    const uint32_t n_mma = hdr->mma_patches;
     for (uint32_t q = threadIdx.x; q < n; q += blockDim.x) {
         const uint32_t p = sorted[q];
         rank[p] = q;
-        const uint32_t chunks = (tile_pre[q + 1] - tile_pre[q] + chunk - 1) / chunk;
+        const uint32_t each = q < n_mma ? 1u : chunk;
+        const uint32_t chunks = (tile_pre[q + 1] - tile_pre[q] + each - 1) / each;
         chunk_pre[q] = chunks;
         const uint64_t rec = (uint64_t)chunks * (pair_off[p + 1] - pair_off[p]);
         part_off[q] = rec > 0xffffffffull ? 0xffffffffu : (uint32_t)rec;
@@ -105,6 +108,7 @@ __device__ inline void adj_scan_body(char* ws, const AdjLayout& L, uint32_t n, u
             // (or the prep refused them)
             if (hdr->total_tiles != 0) atomicCAS(&hdr->status, 0u, (uint32_t)WT_ERR_NOMEM);
             hdr->total_chunks = 0;
+            hdr->mma_items = 0;
         }
     }
 }
@@ -120,7 +124,7 @@ __host__ __device__ __forceinline__ uint32_t tiles_per_row(uint32_t cols, uint32
 // two-sum).  In FP32, since this is asked by every thread of a kernel's start
 // and a warp-wide FP64 operation holds the pipe for about 64 cycles (2.4 us
 // of a small call).
-__device__ __forceinline__ bool same_sum(float a, float b, float c, float d) {
+__host__ __device__ __forceinline__ bool same_sum(float a, float b, float c, float d) {
     const float s = a + b, bb = s - a, e = (a - (s - bb)) + (b - bb);
     const float t = c + d, dd = t - c, f = (c - (t - dd)) + (d - dd);
     return s == t && e == f;
@@ -137,8 +141,8 @@ __device__ __forceinline__ bool same_sum(float a, float b, float c, float d) {
 // of few waves (128^2: 8 waves 8.0 / 6.8 us, 32 9.0 / 8.4, 64 12.1 / 12.5).
 // A lower limit on the patch's size would split a batch over two kernels: with
 // one at 2^18 terms 256 patches of 64-128 side took 77 us.
-__device__ __forceinline__ bool mma_patch(const wt_patch& P) {
-    return P.wave_count >= kMmaMinWaves && P.wave_count <= kMmaMaxWaves && P.cols >= 32 &&
+__host__ __device__ __forceinline__ bool mma_patch(const wt_patch& P, uint32_t max_waves) {
+    return P.wave_count >= kMmaMinWaves && P.wave_count <= max_waves && P.cols >= 32 &&
            same_sum(P.tr[0], P.bl[0], P.tl[0], P.br[0]) && same_sum(P.tr[1], P.bl[1], P.tl[1], P.br[1]);
 }
 

@@ -66,7 +66,7 @@ constexpr uint32_t kSmallPrep = 32;
 
 __device__ void prep_small(const wt_patch* __restrict__ patches, uint32_t n, const wt_wave* __restrict__ waves,
                            uint32_t n_waves, uint64_t out_capacity, uint64_t coef_capacity, uint32_t tile_cols,
-                           char* ws, const WsLayout& L, const HmDev& hm, uint32_t mma_sms, int do_adj,
+                           char* ws, const WsLayout& L, const HmDev& hm, uint32_t mma_sms, uint32_t mma_max, int do_adj,
                            const AdjLayout& AL, uint32_t adj_chunk_max, uint32_t adj_min_tiles) {
     __shared__ wt_patch sp[kSmallPrep];
     __shared__ uint32_t s_sorted[kSmallPrep];      // patch at each sorted rank
@@ -97,7 +97,7 @@ __device__ void prep_small(const wt_patch* __restrict__ patches, uint32_t n, con
             ok = patch_ok(P, n_waves, out_capacity);
             wc = ok ? P.wave_count : 0u;
             tiles_p = ok ? P.rows * tiles_per_row(P.cols, tile_cols / 32) : 0u;
-            mma_p = mma_sms > 0 && ok && mma_patch(P);
+            mma_p = mma_max > 0 && ok && mma_patch(P, mma_max);
         }
         uint32_t x = wc;  // inclusive prefix of the pair counts
         for (int o = 1; o < 32; o <<= 1) {
@@ -129,11 +129,12 @@ __device__ void prep_small(const wt_patch* __restrict__ patches, uint32_t n, con
     if (tid < n && ((s_wave_bad >> tid) & 1u)) tiles_p = 0;
     mma_p = mma_p && tiles_p > 0 && !((s_wave_wild >> tid) & 1u);
     uint32_t mma_rows = 0, mma_items = 0;
+    unsigned long long rowct = 0;  // rows x 128-column blocks of the matrix-product patches
     const unsigned mma_set = __ballot_sync(kAll, mma_p);
     if (mma_set) {
         const uint32_t ct = mma_p ? (sp[tid].cols + 127u) / 128u : 0u;
         const uint32_t rows = mma_p ? sp[tid].rows : 0u;
-        unsigned long long rowct = (unsigned long long)rows * ct;
+        rowct = (unsigned long long)rows * ct;
         for (int o = 16; o > 0; o >>= 1) rowct += __shfl_xor_sync(kAll, rowct, o);
         mma_rows = mma_item_rows(rowct, mma_sms);
         if (mma_p) tiles_p = ct * ((rows + mma_rows - 1u) / mma_rows);
@@ -187,11 +188,12 @@ __device__ void prep_small(const wt_patch* __restrict__ patches, uint32_t n, con
             uint32_t* chunk_pre = reinterpret_cast<uint32_t*>(ws + AL.chunk_pre);
             if (tid < n) s_sorted[rank] = tid;
             __syncwarp();
-            const uint32_t chunk = total_tiles >= adj_min_tiles ? adj_chunk_max : 1u;
+            const uint32_t chunk = total_tiles - mma_items + rowct / 2u >= adj_min_tiles ? adj_chunk_max : 1u;
+            const uint32_t each = tid < (uint32_t)__popc(mma_set) ? 1u : chunk;  // an item is a chunk
             uint32_t chunks = 0, rec = 0;
             if (tid < n) {
                 const uint32_t pq = s_sorted[tid];
-                chunks = (tq + chunk - 1) / chunk;
+                chunks = (tq + each - 1) / each;
                 const uint64_t r = (uint64_t)chunks * (s_off[pq + 1] - s_off[pq]);
                 rec = r > 0xffffffffull ? 0xffffffffu : (uint32_t)r;
                 rank_g[pq] = tid;
@@ -225,9 +227,10 @@ __device__ void prep_small(const wt_patch* __restrict__ patches, uint32_t n, con
         hdr->tile_counter = nomem ? 0u : mma_items;  // the recurrence kernel's tiles follow the items
         hdr->n_patches = n;
         hdr->tile_cols = tile_cols;
-        hdr->mma_items = nomem ? 0u : mma_items;
+        hdr->mma_items = nomem || adj_nomem ? 0u : mma_items;
         hdr->mma_rows = mma_rows;
         hdr->mma_counter = 0;
+        hdr->mma_patches = (uint32_t)__popc(mma_set);
         if (nomem) hdr->total_tiles = 0;
     }
 }
@@ -239,7 +242,8 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
                                                     const wt_wave* __restrict__ waves, uint32_t n_waves,
                                                     uint64_t out_capacity, uint64_t coef_capacity,
                                                     uint32_t tile_cols, char* ws, WsLayout L, HmDev hm,
-                                                    int fuse_coef, uint32_t mma_sms, int do_adj, AdjLayout AL,
+                                                    int fuse_coef, uint32_t mma_sms, uint32_t mma_max, int do_adj,
+                                                    AdjLayout AL,
                                                     uint32_t adj_chunk_max, uint32_t adj_min_tiles) {
 #if __CUDA_ARCH__ >= 900
     // the coefficient kernel does not read what this one writes (it forms its
@@ -249,7 +253,7 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
     if (!fuse_coef) cudaTriggerProgrammaticLaunchCompletion();
 #endif
     if (n <= kSmallPrep && fuse_coef) {
-        prep_small(patches, n, waves, n_waves, out_capacity, coef_capacity, tile_cols, ws, L, hm, mma_sms, do_adj, AL,
+        prep_small(patches, n, waves, n_waves, out_capacity, coef_capacity, tile_cols, ws, L, hm, mma_sms, mma_max, do_adj, AL,
                    adj_chunk_max, adj_min_tiles);
         return;
     }
@@ -264,7 +268,7 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
     __shared__ uint32_t good_wave[kWaveMaskWords];  // bit w: wave w passes wave_ok
     __shared__ uint32_t tame_wave[kWaveMaskWords];  // bit w: wave w is an mma_wave
     __shared__ unsigned long long s_rowct;          // rows x 128-column blocks of the matrix-product patches
-    __shared__ uint32_t s_mma_items;
+    __shared__ uint32_t s_mma_items, s_mma_n;
 
     if (threadIdx.x == 0) {
         hdr->status = 0;
@@ -274,8 +278,9 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
         hdr->tile_cols = tile_cols;
         hdr->mma_items = 0;
         hdr->mma_counter = 0;
+        hdr->mma_patches = 0;
         s_rowct = 0;
-        s_mma_items = 0;
+        s_mma_items = s_mma_n = 0;
     }
     // up to kRankSortMax patches are ordered by rank (their keys in bins[]),
     // more by a counting sort over the bins
@@ -290,7 +295,7 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
         const bool ok = patch_ok(P, n_waves, out_capacity);
         if (!ok) flag_error(hdr, WT_ERR_INVALID_ARG, p);
         pair_off[p] = ok ? P.wave_count : 0u;
-        tiles[p] = ok ? P.rows * tiles_per_row(P.cols, tile_cols / 32) | (mma_sms > 0 && mma_patch(P) ? kMmaFlag : 0u) : 0u;
+        tiles[p] = ok ? P.rows * tiles_per_row(P.cols, tile_cols / 32) | (mma_max > 0 && mma_patch(P, mma_max) ? kMmaFlag : 0u) : 0u;
     }
     __syncthreads();
     const uint32_t total_pairs = block_exclusive_scan(pair_off, n);
@@ -373,7 +378,7 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
         return;
     }
     // the matrix-product patches' items, then the sort keys
-    if (mma_sms > 0) {
+    if (mma_max > 0) {
         for (uint32_t p = threadIdx.x; p < n; p += blockDim.x)
             if (tiles[p] & kMmaFlag)
                 atomicAdd(&s_rowct, (unsigned long long)patches[p].rows * ((patches[p].cols + 127u) / 128u));
@@ -385,10 +390,12 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
                 const uint32_t items = (patches[p].cols + 127u) / 128u * ((patches[p].rows + h - 1u) / h);
                 tiles[p] = items | kMmaFlag;
                 atomicAdd(&s_mma_items, items);
+                atomicAdd(&s_mma_n, 1u);
             }
             __syncthreads();
             if (threadIdx.x == 0) {
                 hdr->mma_items = s_mma_items;
+                hdr->mma_patches = s_mma_n;
                 hdr->mma_rows = h;
                 hdr->tile_counter = s_mma_items;  // the recurrence kernel's tiles follow the items
             }
@@ -441,7 +448,7 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
     }
     if (do_adj) {
         __syncthreads();  // sorted, tile_pre and the header's total_tiles are complete
-        adj_scan_body(ws, AL, n, adj_chunk_max, adj_min_tiles);
+        adj_scan_body(ws, AL, n, adj_chunk_max, adj_min_tiles, s_rowct / 2u);
     }
 }
 
@@ -712,7 +719,8 @@ cudaError_t launch_fwd_t(const FwdConfig& cfg, const wt_patch* patches, uint32_t
 
 cudaError_t launch_prep(const wt_patch* patches, uint32_t n_patches, const wt_wave* waves, uint32_t n_waves,
                         const HmDev& hm, uint64_t out_capacity, uint32_t tile_cols, void* ws,
-                        const WsLayout& L, cudaStream_t s, bool use_mma, const AdjScanArgs* adj) {
+                        const WsLayout& L, cudaStream_t s, uint32_t mma_max_waves,
+                        const AdjScanArgs* adj) {
     char* w = static_cast<char*>(ws);
     // coefficient capacity = what the caller's workspace holds past the fixed part
     // (the header records the real total; the scan refuses to overflow it)
@@ -724,7 +732,7 @@ cudaError_t launch_prep(const wt_patch* patches, uint32_t n_patches, const wt_wa
     const int sms = sm_count();
     if (sms <= 0) return cudaErrorInvalidDevice;
     k_prep_scan<<<1, 1024, 0, s>>>(patches, n_patches, waves, n_waves, out_capacity, coef_cap, tile_cols, w, L,
-                                   hm, fuse, use_mma ? (uint32_t)sms : 0u, adj ? 1 : 0, A.L, A.chunk_max, A.min_tiles);
+                                   hm, fuse, (uint32_t)sms, mma_max_waves, adj ? 1 : 0, A.L, A.chunk_max, A.min_tiles);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (fuse) return cudaSuccess;
@@ -800,7 +808,8 @@ cudaError_t launch_displace(const FwdConfig& cfg, const wt_patch* patches, uint3
         return launch_single(cfg, patches, waves, n_waves, hm, pos, nrm, out_capacity, flags, ws, L, x, s);
     // with fewer waves than mma_patch asks for, no patch can qualify
     const bool mma = !naive && n_waves >= kMmaMinWaves;
-    cudaError_t e = launch_prep(patches, n_patches, waves, n_waves, hm, out_capacity, 32u * cfg.s, ws, L, s, mma);
+    cudaError_t e = launch_prep(patches, n_patches, waves, n_waves, hm, out_capacity, 32u * cfg.s, ws, L, s,
+                                mma ? kMmaMaxWaves : 0u);
     if (e != cudaSuccess) return e;
     if (naive) return launch_forward_naive(patches, n_patches, waves, hm, pos, nrm, flags, ws, L, out_capacity, s);
     if (mma) {

@@ -32,7 +32,8 @@ struct WsHeader {
     uint32_t mma_items;    // items of the matrix-product kernel: [0, mma_items) of the prefix
     uint32_t mma_rows;     // its rows per item (a patch's rows are split evenly into items of at most this)
     uint32_t mma_counter;  // its queue head, past the first item of each block
-    uint32_t pad[53];
+    uint32_t mma_patches;  // patches it runs: the first of the sorted order
+    uint32_t pad[52];
 };
 static_assert(sizeof(WsHeader) == 256, "header size");
 
@@ -157,7 +158,7 @@ inline int hm_kind(const HmDev& hm) {
 }
 
 // Waves of a patch that runs as matrix products (mma_patch).
-constexpr uint32_t kMmaMinWaves = 8, kMmaMaxWaves = 128;
+constexpr uint32_t kMmaMinWaves = 8, kMmaMaxWaves = 128, kMmaAdjMaxWaves = 64;
 
 // The adjoint's queue set-up (ranks, chunk and record prefixes), formed by the
 // prep's scan kernel when the prep runs for an adjoint.
@@ -169,11 +170,12 @@ struct AdjScanArgs {
 
 // ---- launchers (wt_displace.cu) -------------------------------------------
 // tile_cols: tile width (each row's last tile narrower, see tiles_per_row);
-// use_mma: the patches that qualify (mma_patch) are queued for launch_forward_mma
+// mma_max_waves: the patches that qualify (mma_patch) with at most this many waves
+// are queued for the matrix-product kernel (0: none)
 cudaError_t launch_prep(const wt_patch* patches, uint32_t n_patches, const wt_wave* waves,
                         uint32_t n_waves, const HmDev& hm, uint64_t out_capacity,
                         uint32_t tile_cols, void* ws, const WsLayout& L, cudaStream_t s,
-                        bool use_mma, const AdjScanArgs* adj = nullptr);
+                        uint32_t mma_max_waves, const AdjScanArgs* adj = nullptr);
 // pos may be NULL only with x.view set
 cudaError_t launch_forward(const FwdConfig& cfg, const wt_patch* patches, uint32_t n_patches,
                            const HmDev& hm, float* pos, float* nrm, uint32_t flags, void* ws,
@@ -203,12 +205,19 @@ cudaError_t launch_single(const FwdConfig& cfg, const wt_patch* patches, const w
 // ---- adjoint (wt_adjoint.cu) ----------------------------------------------
 // Records (tile chunks x waves) of one patch, as the adjoint lays them out.
 uint64_t adjoint_records(const wt_patch& p);
+// Most waves per patch of the matrix-product kernel for an adjoint over this
+// table (saved: from saved sums); 0: it does not run.
+uint32_t adjoint_mma_waves(const wt_patch* host_patches, uint32_t n_patches, uint32_t n_waves, bool saved);
 // The scan arguments of an adjoint over layout L (saved: from saved sums).
 cudaError_t adjoint_scan_args(bool saved, const AdjLayout& L, AdjScanArgs* out);
+// The patches the prep queued as matrix products (wt_adjoint_mma.cu); exits at
+// once when there are none.
+cudaError_t launch_adjoint_mma(const wt_patch* patches, const HmDev& hm, const float* gpos, const float* gnrm,
+                               uint32_t flags, void* ws, const AdjLayout& L, const float* sums, cudaStream_t s);
 // sums: NULL (phase 1 recomputes the forward sums) or the forward's saved sums;
-// the prep ran with adjoint_scan_args
+// the prep ran with adjoint_scan_args; mma: and with adjoint_mma_waves > 0
 cudaError_t launch_adjoint(const wt_patch* patches, uint32_t n_patches, const wt_wave* waves, uint32_t n_waves,
-                           uint32_t max_waves_per_patch, const HmDev& hm, const float* gpos, const float* gnrm,
+                           uint32_t max_waves_per_patch, bool mma, const HmDev& hm, const float* gpos, const float* gnrm,
                            uint32_t flags, wt_wave_grad* grad, void* ws, const AdjLayout& L, const float* sums,
                            cudaStream_t s);
 

@@ -96,7 +96,12 @@ __device__ __forceinline__ bool warp_wait(unsigned long long* b, uint32_t parity
     return __all_sync(0xffffffffu, mbar_wait(b, parity, fail));
 }
 
-// K-major operand, 128-byte swizzle: rows of 128 B in groups of eight (1024 B)
+// K-major operand, 128-byte swizzle: rows of 128 B in groups of eight (1024 B).
+// Read the other way (M- or N-major), the 64 elements of a row are the M or N
+// direction, the rows K, and `lead` bytes further lie the next 64.
+__device__ __forceinline__ uint64_t transposed_desc(uint32_t addr, uint32_t lead) {
+    return (uint64_t)((addr & 0x3ffffu) >> 4) | ((uint64_t)(lead >> 4) << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+}
 __device__ __forceinline__ uint64_t operand_desc(uint32_t addr) {
     return (uint64_t)((addr & 0x3ffffu) >> 4) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }

@@ -266,7 +266,7 @@ k_single(const wt_patch* __restrict__ patches, const wt_wave* __restrict__ waves
     const bool pow2 = hm.present && (hm.width & (hm.width - 1)) == 0 && (hm.height & (hm.height - 1)) == 0;
     const bool fast = pow2 && hm.wrap == WT_WRAP_REPEAT;
     const uint64_t out0 = P.out_offset;
-    if (mma && total > 0 && !wild && mma_patch(P)) {
+    if (mma && total > 0 && !wild && mma_patch(P, kMmaMaxWaves)) {
         Products& pr = *reinterpret_cast<Products*>(&sh + 1);
         const mma::Output o{pos, nrm, sums, sh.view, so, flags};
         if (!run_products<MODE, HM>(sh, pr, reinterpret_cast<char*>(smem), nw, hm, pow2, o) && tid == 0)
