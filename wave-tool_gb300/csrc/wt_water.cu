@@ -468,28 +468,36 @@ __device__ __forceinline__ uint32_t clampi(int32_t i, uint32_t n) {
     return (uint32_t)(i < 0 ? 0 : (i >= (int32_t)n ? (int32_t)n - 1 : i));
 }
 
-// UNORM8 -> float (c / 255, correctly rounded), one table per block.
-__shared__ float s_unorm8[256];
+// Bytes K and K + 1 of a texel, UNORM8 -> float, c / 255 correctly rounded: c
+// times 1 / 255 as a sum of two floats, the larger product added exactly by the
+// fused multiply-add; this gives the quotient's rounding for each of the 256
+// values.  A table in shared memory took 48 reads a pixel at 32 unrelated
+// addresses a warp, nearly half of the kernel's traffic there.
+template <int K>
+__device__ __forceinline__ float2 unorm8(uint32_t q) {
+    const float2 c = make_float2((float)(uint8_t)(q >> (8 * K)), (float)(uint8_t)(q >> (8 * K + 8)));
+    return __ffma2_rn(c, make_float2(0x1.010102p-8f, 0x1.010102p-8f),
+                      __fmul2_rn(c, make_float2(-0x1.fdfdfep-33f, -0x1.fdfdfep-33f)));
+}
 
 // GL_LINEAR, CLAMP_TO_EDGE over RGBA8 texels converted to c / 255.
-__device__ float4 bilinear_rgba8(const uint8_t* px, uint32_t w, uint32_t h, float s, float t) {
+__device__ __forceinline__ float4 bilinear_rgba8(const uint8_t* px, uint32_t w, uint32_t h, float s, float t) {
     const float u = s * (float)w - 0.5f, v = t * (float)h - 0.5f;
     const float fi = floorf(u), fj = floorf(v);
     const float a = u - fi, b = v - fj;
     const int32_t ii = (int32_t)fi, jj = (int32_t)fj;
     const uint32_t i0 = clampi(ii, w), i1 = clampi(ii + 1, w);
-    const uint32_t j0 = clampi(jj, h), j1 = clampi(jj + 1, h);
-    const uchar4 q00 = *reinterpret_cast<const uchar4*>(px + 4 * ((size_t)j0 * w + i0));
-    const uchar4 q10 = *reinterpret_cast<const uchar4*>(px + 4 * ((size_t)j0 * w + i1));
-    const uchar4 q01 = *reinterpret_cast<const uchar4*>(px + 4 * ((size_t)j1 * w + i0));
-    const uchar4 q11 = *reinterpret_cast<const uchar4*>(px + 4 * ((size_t)j1 * w + i1));
-    auto f = [&](unsigned char c00, unsigned char c10, unsigned char c01, unsigned char c11) {
-        const float t00 = s_unorm8[c00], t10 = s_unorm8[c10];
-        const float t01 = s_unorm8[c01], t11 = s_unorm8[c11];
-        return (1.0f - b) * ((1.0f - a) * t00 + a * t10) + b * ((1.0f - a) * t01 + a * t11);
+    const uint32_t j0 = clampi(jj, h) * w, j1 = clampi(jj + 1, h) * w;  // w, h <= 16384
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(px);
+    const uint32_t q00 = q[j0 + i0], q10 = q[j0 + i1], q01 = q[j1 + i0], q11 = q[j1 + i1];
+    const float am = 1.0f - a, bm = 1.0f - b;
+    const auto f = [&](float t00, float t10, float t01, float t11) {
+        return bm * (am * t00 + a * t10) + b * (am * t01 + a * t11);
     };
-    return make_float4(f(q00.x, q10.x, q01.x, q11.x), f(q00.y, q10.y, q01.y, q11.y), f(q00.z, q10.z, q01.z, q11.z),
-                       f(q00.w, q10.w, q01.w, q11.w));
+    const float2 a00 = unorm8<0>(q00), a10 = unorm8<0>(q10), a01 = unorm8<0>(q01), a11 = unorm8<0>(q11);
+    const float2 b00 = unorm8<2>(q00), b10 = unorm8<2>(q10), b01 = unorm8<2>(q01), b11 = unorm8<2>(q11);
+    return make_float4(f(a00.x, a10.x, a01.x, a11.x), f(a00.y, a10.y, a01.y, a11.y), f(b00.x, b10.x, b01.x, b11.x),
+                       f(b00.y, b10.y, b01.y, b11.y));
 }
 
 // Cube-map face by the major axis (OpenGL 4.1 table 3.19), then bilinear.
@@ -520,7 +528,13 @@ __device__ float4 sample_cube(const uint8_t* faces, uint32_t size, float rx, flo
 __device__ __forceinline__ float clampf(float x, float lo, float hi) { return fminf(fmaxf(x, lo), hi); }
 __device__ __forceinline__ float mixf(float x, float y, float a) { return x * (1.0f - a) + y * a; }
 
-__global__ void __launch_bounds__(256) k_water_shade(const unsigned long long* __restrict__ frag,
+// Bound by instruction issue (75 % of the slots; about 1000 instructions a water
+// pixel: 13 divisions, powf, 48 texel bytes, 24 gathers), with the gathers at half
+// of the load unit's rate.  40 registers (6 blocks a multiprocessor) hide their
+// latency: 5 blocks take 60 us where 6 take 55.  1920 x 1080, 72 % water: 66 us
+// with a table of bytes in shared memory, warps of 32 x 1 pixels and every
+// division per pixel, now 55.
+__global__ void __launch_bounds__(256, 6) k_water_shade(const unsigned long long* __restrict__ frag,
                                                      const float4* __restrict__ clip, uint64_t n_vertices,
                                                      const uint32_t* __restrict__ idx, uint64_t n_tri,
                                                      const float4* __restrict__ facing,
@@ -528,131 +542,139 @@ __global__ void __launch_bounds__(256) k_water_shade(const unsigned long long* _
                                                      const float2* __restrict__ ndc0, uint32_t W, uint32_t H,
                                                      wt_water_shading sh, ShadeTex tex, float4* colour_out,
                                                      float4* composite) {
-    for (uint32_t c = threadIdx.x; c < 256; c += blockDim.x) s_unorm8[c] = (float)c / 255.0f;
+    // a block shades 32 x 8 pixels, a warp 8 x 4 of them: neighbours in both
+    // directions share triangles and texels
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t px = 32u * blockIdx.x + 8u * (warp & 3u) + (lane & 7u);
+    const uint32_t py = 8u * blockIdx.y + 4u * (warp >> 2) + (lane >> 3);
+    // the block's texture coordinates and the scene's depth where there is no
+    // depth image, one division each
+    __shared__ float s_u[32], s_v[8], s_far;
+    const auto linear_depth = [&](float d) { return (sh.z_near * d) / (sh.z_far - d * (sh.z_far - sh.z_near)); };
+    if (threadIdx.x < 32) s_u[threadIdx.x] = ((float)(32u * blockIdx.x + threadIdx.x) + 0.5f) / (float)W;
+    if (warp == 1 && lane < 8) s_v[lane] = ((float)(8u * blockIdx.y + lane) + 0.5f) / (float)H;
+    if (threadIdx.x == 64) s_far = linear_depth(1.0f);
     __syncthreads();
-    const uint64_t n = (uint64_t)W * H;
-    for (uint64_t p = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; p < n; p += (uint64_t)gridDim.x * blockDim.x) {
-        const unsigned long long key = frag[p];
-        const uint32_t tri1 = (uint32_t)(key & 0xffffffffull);
-        const size_t t = tri1 - 1;
-        uint32_t vi[3] = {0u, 0u, 0u};
-        bool water = tri1 != 0 && t < n_tri;
-        if (water) {
-            vi[0] = idx[3 * t];
-            vi[1] = idx[3 * t + 1];
-            vi[2] = idx[3 * t + 2];
-            water = vi[0] < n_vertices && vi[1] < n_vertices && vi[2] < n_vertices;
-        }
-        if (!water) {
-            if (colour_out) colour_out[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            continue;
-        }
-        const uint32_t py = (uint32_t)(p / W), px = (uint32_t)(p - (uint64_t)py * W);
-        // perspective-correct weights: lambda_k ~ (v_{k+1} x v_{k+2}) . (ndc x, ndc y, 1)
-        const float nx = (2.0f * ((float)px + 0.5f)) / (float)W - 1.0f;
-        const float ny = (2.0f * ((float)py + 0.5f)) / (float)H - 1.0f;
-        float cv[3][3];
+    if (px >= W || py >= H) return;
+    const uint32_t p = py * W + px;  // W, H <= 16384
+    const unsigned long long key = frag[p];
+    const uint32_t tri1 = (uint32_t)(key & 0xffffffffull);
+    const uint64_t t = tri1 - 1u;
+    uint32_t vi[3] = {0u, 0u, 0u};
+    bool water = tri1 != 0 && t < n_tri;
+    if (water) {
+        vi[0] = idx[3 * t];
+        vi[1] = idx[3 * t + 1];
+        vi[2] = idx[3 * t + 2];
+        water = vi[0] < n_vertices && vi[1] < n_vertices && vi[2] < n_vertices;
+    }
+    if (!water) {
+        if (colour_out) colour_out[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        return;
+    }
+    // perspective-correct weights: lambda_k ~ (v_{k+1} x v_{k+2}) . (ndc x, ndc y, 1)
+    // (u and 2 u round alike)
+    const float u0 = s_u[px & 31u], u1 = s_v[py & 7u];
+    const float nx = 2.0f * u0 - 1.0f, ny = 2.0f * u1 - 1.0f;
+    float cv[3][3];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const float4 c = clip[vi[k]];
-            cv[k][0] = c.x;
-            cv[k][1] = c.y;
-            cv[k][2] = c.w;
-        }
-        float c[3];
+    for (int k = 0; k < 3; ++k) {
+        const float4 c = clip[vi[k]];
+        cv[k][0] = c.x;
+        cv[k][1] = c.y;
+        cv[k][2] = c.w;
+    }
+    float c[3];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const float* a = cv[k == 2 ? 0 : k + 1];
-            const float* b = cv[k == 0 ? 2 : (k == 1 ? 0 : 1)];
-            const float cx = a[1] * b[2] - a[2] * b[1];
-            const float cy = a[2] * b[0] - a[0] * b[2];
-            const float cz = a[0] * b[1] - a[1] * b[0];
-            c[k] = cx * nx + cy * ny + cz;
-        }
-        const float sum = c[0] + c[1] + c[2];
-        const float l0 = c[0] / sum, l1 = c[1] / sum, l2 = c[2] / sum;
-        const float4 n0 = facing[vi[0]], n1 = facing[vi[1]], n2 = facing[vi[2]];
-        const float4 y0 = nyaw[vi[0]], y1 = nyaw[vi[1]], y2 = nyaw[vi[2]];
-        const float4 w0 = view[vi[0]], w1 = view[vi[1]], w2 = view[vi[2]];
-        const float2 d0 = ndc0[vi[0]], d1 = ndc0[vi[1]], d2 = ndc0[vi[2]];
-        const float N[3] = {l0 * n0.x + l1 * n1.x + l2 * n2.x, l0 * n0.y + l1 * n1.y + l2 * n2.y,
-                            l0 * n0.z + l1 * n1.z + l2 * n2.z};
-        const float NY[3] = {l0 * y0.x + l1 * y1.x + l2 * y2.x, l0 * y0.y + l1 * y1.y + l2 * y2.y,
-                             l0 * y0.z + l1 * y1.z + l2 * y2.z};
-        const float V[3] = {l0 * w0.x + l1 * w1.x + l2 * w2.x, l0 * w0.y + l1 * w1.y + l2 * w2.y,
-                            l0 * w0.z + l1 * w1.z + l2 * w2.z};
-        const float D0[2] = {l0 * d0.x + l1 * d1.x + l2 * d2.x, l0 * d0.y + l1 * d1.y + l2 * d2.y};
-        const float fz = __uint_as_float((uint32_t)(key >> 32));
+    for (int k = 0; k < 3; ++k) {
+        const float* a = cv[k == 2 ? 0 : k + 1];
+        const float* b = cv[k == 0 ? 2 : (k == 1 ? 0 : 1)];
+        const float cx = a[1] * b[2] - a[2] * b[1];
+        const float cy = a[2] * b[0] - a[0] * b[2];
+        const float cz = a[0] * b[1] - a[1] * b[0];
+        c[k] = cx * nx + cy * ny + cz;
+    }
+    const float sum = c[0] + c[1] + c[2];
+    const float l0 = c[0] / sum, l1 = c[1] / sum, l2 = c[2] / sum;
+    const float4 n0 = facing[vi[0]], n1 = facing[vi[1]], n2 = facing[vi[2]];
+    const float4 y0 = nyaw[vi[0]], y1 = nyaw[vi[1]], y2 = nyaw[vi[2]];
+    const float4 w0 = view[vi[0]], w1 = view[vi[1]], w2 = view[vi[2]];
+    const float2 d0 = ndc0[vi[0]], d1 = ndc0[vi[1]], d2 = ndc0[vi[2]];
+    const float N[3] = {l0 * n0.x + l1 * n1.x + l2 * n2.x, l0 * n0.y + l1 * n1.y + l2 * n2.y,
+                        l0 * n0.z + l1 * n1.z + l2 * n2.z};
+    const float NY[3] = {l0 * y0.x + l1 * y1.x + l2 * y2.x, 0.0f, l0 * y0.z + l1 * y1.z + l2 * y2.z};
+    const float V[3] = {l0 * w0.x + l1 * w1.x + l2 * w2.x, l0 * w0.y + l1 * w1.y + l2 * w2.y,
+                        l0 * w0.z + l1 * w1.z + l2 * w2.z};
+    const float D0[2] = {l0 * d0.x + l1 * d1.x + l2 * d2.x, l0 * d0.y + l1 * d1.y + l2 * d2.y};
+    const float fz = __uint_as_float((uint32_t)(key >> 32));
 
-        // water-grid.frag:65-151
-        const float view_len = sqrtf(V[0] * V[0] + V[1] * V[1] + V[2] * V[2]);
-        const float view_depth = clampf(view_len / sh.z_far, 0.0f, 1.0f);
-        const float vv[3] = {V[0] / view_len, V[1] / view_len, V[2] / view_len};
-        const float u0 = ((float)px + 0.5f) / (float)W, u1 = ((float)py + 0.5f) / (float)H;
-        const float h0 = (D0[0] + 1.0f) / 2.0f, h1 = (D0[1] + 1.0f) / 2.0f;
-        float back_raw = 1.0f;
-        if (tex.depth)
-            back_raw = tex.depth[(size_t)clampi((int32_t)floorf(u1 * (float)H), H) * W +
-                                 clampi((int32_t)floorf(u0 * (float)W), W)];
-        const float back = (sh.z_near * back_raw) / (sh.z_far - back_raw * (sh.z_far - sh.z_near));
-        const float sky_behind = back > 0.999f ? 0.0f : 1.0f;
-        const float here = (sh.z_near * fz) / (sh.z_far - fz * (sh.z_far - sh.z_near));
-        const float delta = clampf(back - here, 0.0f, 1.0f);
-        const float I[3] = {-vv[0], -vv[1], -vv[2]};
-        const float kr = 2.0f * (N[0] * I[0] + N[1] * I[1] + N[2] * I[2]);
-        const float R[3] = {I[0] - kr * N[0], I[1] - kr * N[1], I[2] - kr * N[2]};
-        const float4 sky = sample_cube(tex.sky, tex.sky_size, R[0], R[1], R[2]);
-        const float sun_p = powf(
-            clampf(R[0] * sh.sun_position[0] + R[1] * sh.sun_position[1] + R[2] * sh.sun_position[2], 0.0f, 1.0f),
-            sh.sun_shininess);
-        const float sun = (sh.sun_strength * 1.0f) * sun_p;
-        const float cos_t = N[0] * vv[0] + N[1] * vv[1] + N[2] * vv[2];
-        // pow(1 - cos, 5) as products, as shader compilers expand a constant
-        // integer exponent (within a few ulp of powf)
-        const float om = 1.0f - cos_t, om2 = om * om;
-        const float fres = 0.02f + (1.0f - 0.02f) * (om2 * om2 * om);
-        const float ds = 0.1f * (1.0f - view_depth);  // both distortion strengths are 0.1
-        const float ul0 = clampf(mixf(u0, h0, ds) + ds * NY[0], 0.0f, 1.0f);
-        const float ul1 = clampf(mixf(u1, h1, ds) + ds * -NY[2], 0.0f, 1.0f);
-        const float ur0 = clampf(mixf(u0, h0, ds) + ds * -NY[0], 0.0f, 1.0f);
-        const float ur1 = clampf(mixf(u1, h1, ds) + ds * NY[2], 0.0f, 1.0f);
-        const float4 lrefl = tex.refl ? bilinear_rgba8(tex.refl, W, H, ul0, ul1) : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float4 lrefr = tex.refr ? bilinear_rgba8(tex.refr, W, H, ur0, ur1) : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float tint_f = 0.0f == sh.tint_threshold
-                                 ? 0.0f
-                                 : sky_behind * (1.0f - clampf(delta / sh.tint_threshold, 0.0f, 1.0f));
-        const float day = clampf(sh.sun_position[1], 0.0f, 1.0f);
-        const float clarity = sh.water_clarity * lrefr.w * (1.0f - delta);
-        const float deep[3] = {0.0f, 0.341f, 0.482f}, shallow[3] = {0.3f, 0.941f, 0.903f};
-        const float skyc[3] = {sky.x, sky.y, sky.z}, lrc[3] = {lrefl.x, lrefl.y, lrefl.z};
-        const float ltc[3] = {lrefr.x, lrefr.y, lrefr.z};
-        float out[4];
+    // water-grid.frag:65-151
+    const float view_len = sqrtf(V[0] * V[0] + V[1] * V[1] + V[2] * V[2]);
+    const float view_depth = clampf(view_len / sh.z_far, 0.0f, 1.0f);
+    const float vv[3] = {V[0] / view_len, V[1] / view_len, V[2] / view_len};
+    const float h0 = (D0[0] + 1.0f) / 2.0f, h1 = (D0[1] + 1.0f) / 2.0f;
+    const float back = tex.depth ? linear_depth(tex.depth[clampi((int32_t)floorf(u1 * (float)H), H) * W +
+                                                          clampi((int32_t)floorf(u0 * (float)W), W)])
+                                 : s_far;
+    const float sky_behind = back > 0.999f ? 0.0f : 1.0f;
+    const float here = linear_depth(fz);
+    const float delta = clampf(back - here, 0.0f, 1.0f);
+    const float I[3] = {-vv[0], -vv[1], -vv[2]};
+    const float kr = 2.0f * (N[0] * I[0] + N[1] * I[1] + N[2] * I[2]);
+    const float R[3] = {I[0] - kr * N[0], I[1] - kr * N[1], I[2] - kr * N[2]};
+    const float4 sky = sample_cube(tex.sky, tex.sky_size, R[0], R[1], R[2]);
+    const float sun_p = powf(
+        clampf(R[0] * sh.sun_position[0] + R[1] * sh.sun_position[1] + R[2] * sh.sun_position[2], 0.0f, 1.0f),
+        sh.sun_shininess);
+    const float sun = (sh.sun_strength * 1.0f) * sun_p;
+    const float cos_t = N[0] * vv[0] + N[1] * vv[1] + N[2] * vv[2];
+    // pow(1 - cos, 5) as products, as shader compilers expand a constant
+    // integer exponent (within a few ulp of powf)
+    const float om = 1.0f - cos_t, om2 = om * om;
+    const float fres = 0.02f + (1.0f - 0.02f) * (om2 * om2 * om);
+    const float ds = 0.1f * (1.0f - view_depth);  // both distortion strengths are 0.1
+    const float ul0 = clampf(mixf(u0, h0, ds) + ds * NY[0], 0.0f, 1.0f);
+    const float ul1 = clampf(mixf(u1, h1, ds) + ds * -NY[2], 0.0f, 1.0f);
+    const float ur0 = clampf(mixf(u0, h0, ds) + ds * -NY[0], 0.0f, 1.0f);
+    const float ur1 = clampf(mixf(u1, h1, ds) + ds * NY[2], 0.0f, 1.0f);
+    const float4 lrefl = tex.refl ? bilinear_rgba8(tex.refl, W, H, ul0, ul1) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 lrefr = tex.refr ? bilinear_rgba8(tex.refr, W, H, ur0, ur1) : make_float4(0.f, 0.f, 0.f, 0.f);
+    // before the sky both terms are 0 times a number in [0, 1]
+    float tint_f = 0.0f, edge = 0.0f;
+    if (sky_behind != 0.0f) {
+        if (0.0f != sh.tint_threshold) tint_f = sky_behind * (1.0f - clampf(delta / sh.tint_threshold, 0.0f, 1.0f));
+        if (0.0f != sh.soft_edges_threshold)
+            edge = sky_behind * (1.0f - clampf(delta / sh.soft_edges_threshold, 0.0f, 1.0f));
+    }
+    const float day = clampf(sh.sun_position[1], 0.0f, 1.0f);
+    const float clarity = sh.water_clarity * lrefr.w * (1.0f - delta);
+    const float deep[3] = {0.0f, 0.341f, 0.482f}, shallow[3] = {0.3f, 0.941f, 0.903f};
+    const float skyc[3] = {sky.x, sky.y, sky.z}, lrc[3] = {lrefl.x, lrefl.y, lrefl.z};
+    const float ltc[3] = {lrefr.x, lrefr.y, lrefr.z};
+    float out[4];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const float tint = day * mixf(deep[k], shallow[k], tint_f);
-            const float trans = mixf(tint, ltc[k], clarity);
-            const float refl = mixf(skyc[k] + sun, lrc[k], lrefl.w);
-            out[k] = mixf(trans, refl, fres);
-        }
-        out[3] = 0.0f == sh.soft_edges_threshold
-                     ? 1.0f
-                     : 1.0f - (sky_behind * (1.0f - clampf(delta / sh.soft_edges_threshold, 0.0f, 1.0f)));
-        const float fog_a = view_depth >= sh.fog_radius_far
-                                ? sh.fog_colour[3]
-                                : view_depth <= sh.fog_radius_near
-                                      ? 0.0f
-                                      : sh.fog_colour[3] * ((view_depth - sh.fog_radius_near) /
-                                                            (sh.fog_radius_far - sh.fog_radius_near));
+    for (int k = 0; k < 3; ++k) {
+        const float tint = day * mixf(deep[k], shallow[k], tint_f);
+        const float trans = mixf(tint, ltc[k], clarity);
+        const float refl = mixf(skyc[k] + sun, lrc[k], lrefl.w);
+        out[k] = mixf(trans, refl, fres);
+    }
+    out[3] = 1.0f - edge;
+    const float fog_a = view_depth >= sh.fog_radius_far
+                            ? sh.fog_colour[3]
+                            : view_depth <= sh.fog_radius_near
+                                  ? 0.0f
+                                  : sh.fog_colour[3] * ((view_depth - sh.fog_radius_near) /
+                                                        (sh.fog_radius_far - sh.fog_radius_near));
 #pragma unroll
-        for (int k = 0; k < 3; ++k) out[k] = mixf(out[k], sh.fog_colour[k], fog_a);
-        const float4 col = make_float4(out[0], out[1], out[2], out[3]);
-        if (colour_out) colour_out[p] = col;
-        if (composite) {
-            const float4 d = composite[p];
-            const float a = col.w;
-            composite[p] = make_float4(col.x * a + d.x * (1.0f - a), col.y * a + d.y * (1.0f - a),
-                                       col.z * a + d.z * (1.0f - a), col.w * a + d.w * (1.0f - a));
-        }
+    for (int k = 0; k < 3; ++k) out[k] = mixf(out[k], sh.fog_colour[k], fog_a);
+    const float4 col = make_float4(out[0], out[1], out[2], out[3]);
+    if (colour_out) colour_out[p] = col;
+    if (composite) {
+        const float4 d = composite[p];
+        const float a = col.w;
+        composite[p] = make_float4(col.x * a + d.x * (1.0f - a), col.y * a + d.y * (1.0f - a),
+                                   col.z * a + d.z * (1.0f - a), col.w * a + d.w * (1.0f - a));
     }
 }
 
@@ -689,7 +711,7 @@ unsigned resident_grid(K kernel, std::atomic<int> (&cache)[64], int sms, uint64_
     return (unsigned)(need < cap ? need : cap);
 }
 
-std::atomic<int> g_occ_prepare[64], g_occ_deferred[64], g_occ_shade[64];
+std::atomic<int> g_occ_prepare[64], g_occ_deferred[64];
 
 // 256-thread launch that may begin before the previous kernel on the stream
 // has finished (programmatic dependent launch); the kernel waits for that
@@ -812,13 +834,9 @@ extern "C" wt_status wt_water_shade(const uint64_t* fragments, const float* clip
     if (!colour_out && !composite) return WT_OK;
     if ((colour_out && !aligned(colour_out, 16)) || (composite && !aligned(composite, 16)))
         return fail(WT_ERR_INVALID_ARG, "wt_water_shade: colour outputs must be 16-byte aligned");
-    int sms = 0;
-    wt_status st = sms_of_device(&sms);
-    if (st != WT_OK) return st;
-    const uint64_t npx = (uint64_t)width * height;
     const ShadeTex tx{textures->scene_depth, textures->local_reflections, textures->local_refractions,
                       textures->skybox, textures->skybox_size};
-    k_water_shade<<<resident_grid(k_water_shade, g_occ_shade, sms, npx), 256, 0, (cudaStream_t)stream>>>(
+    k_water_shade<<<dim3((width + 31u) / 32u, (height + 7u) / 8u), 256, 0, (cudaStream_t)stream>>>(
         reinterpret_cast<const unsigned long long*>(fragments), reinterpret_cast<const float4*>(clip), n_vertices,
         indices, n_triangles,
         reinterpret_cast<const float4*>(facing), reinterpret_cast<const float4*>(nrm_yaw),
