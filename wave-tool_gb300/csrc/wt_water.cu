@@ -7,18 +7,18 @@
 // colour terms reproduce a scalar CPU restatement bit for bit.
 //
 // Rasterisation (k_water_raster): one lane per triangle.  Window coordinates
-// are snapped to 1/256 pixel and covered with exact 64-bit integer edge
-// functions at pixel centres (left/top fill rule); the window depth is
+// are snapped to 1/256 pixel and covered with exact integer edge
+// functions (in 32 bits where the triangle is small enough) at pixel centres (left/top fill rule); the window depth is
 // interpolated linearly in screen space and folded with the triangle index
 // into one 64-bit key, (depth bits << 32) | (triangle + 1), kept per pixel by
 // a 64-bit atomic minimum (no return value, so no round trip per fragment):
 // nearest fragment wins, ties go to the lower index, and the
 // result does not depend on launch order.  Triangles with more than
-// kOwnPixels pixels in their box, and triangles that reach behind the near
+// own_pixels pixels in their box, and triangles that reach behind the near
 // plane or past a guard band of 64 viewports (clipped in clip space first),
 // go to a queue; a second pass (k_water_raster_deferred) spreads the queue
-// over every warp of a resident grid, each triangle rasterised by a whole
-// warp, lanes striding over the pixels.
+// over every warp of a resident grid, which deals the rows of middling boxes to
+// its lanes; a large one is rasterised by a whole block.
 //
 // Shading (k_water_shade): one thread per pixel; perspective-correct
 // barycentrics from the triangle's three clip-space vertices (2D homogeneous
@@ -36,18 +36,16 @@ namespace {
 
 constexpr float kSub = 256.0f;   // sub-pixel steps per pixel
 constexpr float kGuard = 64.0f;  // guard band, in NDC units
-// Triangles with at most kOwnPixels pixels in their box are rasterised by
-// their own thread in the first pass; 6 blocks of 256 threads a multiprocessor
-// (40 registers) hide its gather latency.  1080p frame of a 1024^2 grid:
-// 16 / 64 / 128 / 256 pixels -> 94 / 62 / 57 / 64 us for the whole call.
-#ifndef WT_OWN_PIXELS
-#define WT_OWN_PIXELS 128
-#endif
-constexpr int kOwnPixels = WT_OWN_PIXELS;
-#ifndef WT_RASTER_MINB
-#define WT_RASTER_MINB 6
-#endif
-constexpr int64_t kSmallExtent = 1 << 13;  // sub-pixel steps (32 pixels)
+// Largest pixel box that a triangle's own thread walks in the first pass.  Few
+// triangles leave no other work to hide a long walk behind, so theirs go to the
+// second pass early; with two million and more it is the queue that costs.
+// Measured, both passes at 24 / 64 / 128 pixels: 481^2 vertices at 950 x 864
+// 20 / 33 / 38 us, 750^2 at 1920 x 1080 35 / 33 / 37, 1024^2 39 / 37 / 36.
+inline int32_t own_pixels(uint64_t n_tri) {
+    return n_tri >> 21 ? 128 : (int32_t)((n_tri >> 14) < 24 ? 24 : n_tri >> 14);
+}
+constexpr int32_t kSmallExtent = 30000;  // sub-pixel steps (117 pixels): 2 x 30000^2 and a step fit 32 bits
+constexpr int kDealPixels = 2048;  // largest box of a small triangle whose rows a warp deals out
 constexpr unsigned kFull = 0xffffffffu;
 
 struct CV4 {
@@ -126,9 +124,9 @@ __device__ __forceinline__ bool setup_tri(const WinTri& w, uint32_t W, uint32_t 
     px1 = min(px1, (int32_t)W - 1);
     py1 = min(py1, (int32_t)H - 1);
     if (px0 > px1 || py0 > py1) return false;
-    const bool small = xmx - xmn < (int32_t)kSmallExtent && ymx - ymn < (int32_t)kSmallExtent;
+    const bool small = xmx - xmn < kSmallExtent && ymx - ymn < kSmallExtent;
     bool ccw;
-    if (small) {  // |products| < 2^26: exact in 32 bits
+    if (small) {  // |products| < 2^30: exact in 32 bits
         int32_t area = (w.X[1] - w.X[0]) * (w.Y[2] - w.Y[0]) - (w.Y[1] - w.Y[0]) * (w.X[2] - w.X[0]);
         if (area == 0) return false;
         ccw = area > 0;
@@ -172,7 +170,7 @@ __device__ __forceinline__ void raster_pixel(const Setup& s, int32_t px, int32_t
 }
 
 // Triangles less than kSmallExtent sub-pixel steps wide and high: the edge
-// functions, taken relative to vertex 0, stay below 2^28 in magnitude, so they
+// functions stay below 2^31 in magnitude over their box, so they
 // are evaluated exactly in 32-bit integers, stepping from pixel to pixel (the
 // same values the 64-bit form gives).
 __device__ __forceinline__ void raster_small(const Setup& s, uint32_t tri, uint32_t W, unsigned long long* frag) {
@@ -220,46 +218,151 @@ __device__ __forceinline__ void raster_own(const Setup& s, uint32_t tri, uint32_
         for (int32_t px = s.px0; px <= s.px1; ++px) raster_pixel(s, px, py, tri, W, frag);
 }
 
-// raster_pixel for a small-extent triangle: the same edge values in 32 bits.
-__device__ __forceinline__ void raster_pixel32(const Setup& s, int32_t px, int32_t py, uint32_t tri, uint32_t W,
-                                               unsigned long long* frag) {
-    const int32_t cx = px * 256 + 128, cy = py * 256 + 128;
-    int32_t e[3], out = 0;
+// A triangle as the rows of its box are walked: five 16-byte pieces, so that the
+// lanes' reads of neighbouring triangles fall on different banks.
+struct RowTri {
+    int32_t e[3];      // edge functions (with the fill rule, raster_small) at the box's first pixel
+    uint32_t start;    // rows of the warp's triangles before it
+    int32_t dx[3];     // per pixel
+    uint32_t tri;
+    int32_t dy[3];     // per row
+    uint32_t offset;   // of the first pixel
+    float z[3];
+    float area_f;
+    int32_t incl, last;  // Setup's; the box's last column
+    int32_t pad[2];
+};
+static_assert(sizeof(RowTri) == 80, "five 16-byte pieces");
+
+// The small triangles of a warp's lanes (own), row by row: the rows of all of
+// them are dealt to the lanes in turn, so a lane with a large box does not hold
+// the others up for its whole area.
+__device__ __forceinline__ void raster_rows(const Setup& s, bool own, uint32_t tri, uint32_t W, unsigned long long* frag,
+                                            RowTri* rec, uint32_t lane) {
+    const uint32_t rows = own ? (uint32_t)(s.py1 - s.py0 + 1) : 0u;
+    uint32_t end = rows;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const int i = k == 2 ? 0 : k + 1, j = k == 0 ? 2 : (k == 1 ? 0 : 1);
-        e[k] = (s.x[j] - s.x[i]) * (cy - s.y[i]) - (s.y[j] - s.y[i]) * (cx - s.x[i]);
-        out |= e[k] + ((s.incl >> k) & 1) - 1;  // negative: outside edge k (as in raster_small)
+    for (uint32_t o = 1; o < 32; o *= 2) {
+        const uint32_t v = __shfl_up_sync(kFull, end, o);
+        if (lane >= o) end += v;
     }
-    if (out < 0) return;
-    float d = ((float)e[0] * s.z[0] + (float)e[1] * s.z[1] + (float)e[2] * s.z[2]) / s.area_f;
-    if (!(d >= 0.0f && d <= 1.0f)) return;
-    d = d + 0.0f;  // -0 -> +0
-    atomicMin(frag + (size_t)py * W + px,
-              ((unsigned long long)__float_as_uint(d) << 32) | (unsigned long long)(tri + 1u));
+    const uint32_t total = __shfl_sync(kFull, end, 31), start = end - rows;
+    const unsigned owners = __ballot_sync(kFull, own);
+    if (own) {
+        RowTri r;
+        const int32_t cx0 = s.px0 * 256 + 128 - s.x[0], cy0 = s.py0 * 256 + 128 - s.y[0];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const int i = k == 2 ? 0 : k + 1, j = k == 0 ? 2 : (k == 1 ? 0 : 1);
+            const int32_t ex = s.x[j] - s.x[i], ey = s.y[j] - s.y[i];
+            r.e[k] = ex * (cy0 - (s.y[i] - s.y[0])) - ey * (cx0 - (s.x[i] - s.x[0])) + ((s.incl >> k) & 1) - 1;
+            r.dx[k] = -ey * 256;
+            r.dy[k] = ex * 256;
+            r.z[k] = s.z[k];
+        }
+        r.start = start;
+        r.tri = tri;
+        r.offset = (uint32_t)s.py0 * W + (uint32_t)s.px0;
+        r.area_f = s.area_f;
+        r.incl = s.incl;
+        r.last = s.px1 - s.px0;
+        r.pad[0] = r.pad[1] = 0;
+        rec[__popc(owners & ((1u << lane) - 1u))] = r;
+    }
+    __syncwarp();
+    for (uint32_t j0 = 0; j0 < total; j0 += 32) {
+        // the triangles that start in these 32 rows, and how many start before
+        const unsigned starts = __reduce_or_sync(kFull, own && start - j0 < 32u ? 1u << (start - j0) : 0u);
+        const uint32_t before = __popc(__ballot_sync(kFull, own && start < j0));
+        const uint32_t owner = before + __popc(starts & ((2u << lane) - 1u)) - 1u;
+        if (j0 + lane >= total) break;
+        const RowTri r = rec[owner];
+        const int32_t row = (int32_t)(j0 + lane - r.start);
+        int32_t e[3], b[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            e[k] = r.e[k] + row * r.dy[k];
+            b[k] = ((r.incl >> k) & 1) - 1;
+        }
+        unsigned long long* at = frag + (r.offset + (uint32_t)row * W);
+        for (int32_t x = 0; x <= r.last; ++x) {
+            if ((e[0] | e[1] | e[2]) >= 0) {
+                float d = ((float)(e[0] - b[0]) * r.z[0] + (float)(e[1] - b[1]) * r.z[1] +
+                           (float)(e[2] - b[2]) * r.z[2]) / r.area_f;
+                if (d >= 0.0f && d <= 1.0f) {
+                    d = d + 0.0f;  // -0 -> +0
+                    atomicMin(at + x, ((unsigned long long)__float_as_uint(d) << 32) | (unsigned long long)(r.tri + 1u));
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 3; ++k) e[k] += r.dx[k];
+        }
+    }
 }
 
-__device__ __forceinline__ void raster_warp(const Setup& s, uint32_t tri, uint32_t W, unsigned long long* frag,
-                                            int lane) {
-    // box <= 16384^2 pixels: 32-bit indices
+// A triangle by all the warps of a block; I holds its edge functions (Setup::small:
+// 32 bits do).
+template <typename I>
+__device__ __forceinline__ void raster_block(const Setup& s, uint32_t tri, uint32_t W, unsigned long long* frag) {
+    const int32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const uint32_t bw = (uint32_t)(s.px1 - s.px0 + 1);
-    const uint32_t n = bw * (uint32_t)(s.py1 - s.py0 + 1);
-    if (s.small) {
-        // pixel p = r * bw + c walked in steps of 32 = qs * bw + rs (one
-        // division per triangle, none per pixel)
-        const uint32_t qs = 32u / bw, rs = 32u - qs * bw;
-        uint32_t r = (uint32_t)lane / bw, c = (uint32_t)lane - r * bw;
-        for (uint32_t p = (uint32_t)lane; p < n; p += 32) {
-            raster_pixel32(s, s.px0 + (int32_t)c, s.py0 + (int32_t)r, tri, W, frag);
-            c += rs;
-            r += qs;
-            if (c >= bw) { c -= bw; ++r; }
+    if (bw < 32) {
+        // box <= 16384^2 pixels: 32-bit indices
+        const uint32_t n = bw * (uint32_t)(s.py1 - s.py0 + 1);
+        for (uint32_t p = threadIdx.x; p < n; p += blockDim.x) {
+            const uint32_t r = p / bw;
+            raster_pixel(s, s.px0 + (int32_t)(p - r * bw), s.py0 + (int32_t)r, tri, W, frag);
         }
         return;
     }
-    for (uint32_t p = (uint32_t)lane; p < n; p += 32) {
-        const uint32_t r = p / bw;
-        raster_pixel(s, s.px0 + (int32_t)(p - r * bw), s.py0 + (int32_t)r, tri, W, frag);
+    // a row of the box per warp, between the edges' crossings of the row (in FP32, to
+    // less than 0.1 pixel, and a pixel more at each end; the exact test decides).
+    // Edge functions with the fill rule in their sign, as in raster_small, stepped by
+    // rows and pixels.
+    I row[3], dy[3], dx[3];
+    float inv[3];
+    const I cx = (I)s.px0 * 256 + 128, cy = (I)(s.py0 + warp) * 256 + 128;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const int i = k == 2 ? 0 : k + 1, j = k == 0 ? 2 : (k == 1 ? 0 : 1);
+        const int32_t ex = s.x[j] - s.x[i], ey = s.y[j] - s.y[i];
+        row[k] = (I)ex * (cy - s.y[i]) - (I)ey * (cx - s.x[i]) + (((s.incl >> k) & 1) - 1);
+        dy[k] = (I)ex * (256 * warps);
+        dx[k] = (I)ey * -256;
+        inv[k] = ey == 0 ? 0.0f : 1.0f / ((float)ey * 256.0f);
+    }
+    for (int32_t py = s.py0 + warp; py <= s.py1; py += warps) {
+        float lo = 0.0f, hi = (float)(bw - 1u);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float at = (float)row[k] * inv[k];  // row - 256 ey x = 0
+            if (inv[k] < 0.0f) lo = fmaxf(lo, at - 1.0f);
+            if (inv[k] > 0.0f) hi = fminf(hi, at + 1.0f);
+        }
+        if (lo <= hi) {
+            const int32_t x1 = (int32_t)hi;
+            int32_t x = (int32_t)lo + lane;
+            I e[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) e[k] = row[k] + dx[k] * x;
+            for (; x <= x1; x += 32) {
+                if ((e[0] | e[1] | e[2]) >= 0) {
+                    I v[3];
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) v[k] = e[k] - (((s.incl >> k) & 1) - 1);
+                    float d = ((float)v[0] * s.z[0] + (float)v[1] * s.z[1] + (float)v[2] * s.z[2]) / s.area_f;
+                    if (d >= 0.0f && d <= 1.0f) {
+                        d = d + 0.0f;  // -0 -> +0
+                        atomicMin(frag + ((uint32_t)py * W + (uint32_t)(s.px0 + x)),
+                                  ((unsigned long long)__float_as_uint(d) << 32) | (unsigned long long)(tri + 1u));
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < 3; ++k) e[k] += 32 * dx[k];
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) row[k] += dy[k];
     }
 }
 
@@ -299,34 +402,15 @@ __global__ void __launch_bounds__(256) k_water_prepare(const float* __restrict__
     }
 }
 
-__device__ __forceinline__ Setup shfl_setup(const Setup& s, int src) {
-    Setup o;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        o.x[k] = __shfl_sync(kFull, s.x[k], src);
-        o.y[k] = __shfl_sync(kFull, s.y[k], src);
-        o.z[k] = __shfl_sync(kFull, s.z[k], src);
-    }
-    o.area_f = __shfl_sync(kFull, s.area_f, src);
-    o.px0 = __shfl_sync(kFull, s.px0, src);
-    o.px1 = __shfl_sync(kFull, s.px1, src);
-    o.py0 = __shfl_sync(kFull, s.py0, src);
-    o.py1 = __shfl_sync(kFull, s.py1, src);
-    const int flags = __shfl_sync(kFull, s.incl | (s.small ? 8 : 0), src);
-    o.incl = flags & 7;
-    o.small = (flags & 8) != 0;
-    return o;
-}
-
 // First pass: one thread per triangle (the grid covers them all).  Triangles
-// whose pixel box holds at most kOwnPixels pixels are rasterised by their
+// whose pixel box holds at most own_pixels pixels are rasterised by their
 // own thread; the others (larger boxes, and triangles that need clipping) are
 // appended to a queue for the second pass (the triangle and its three vertex
 // indices), with one atomic per warp.  Launched dependent on the preparing
 // pass: the index loads are issued before it waits for that pass's results.
-__global__ void __launch_bounds__(256, WT_RASTER_MINB) k_water_raster(const int4* __restrict__ win,
+__global__ void __launch_bounds__(256, 6) k_water_raster(const int4* __restrict__ win,
                                                          uint64_t n_vertices, const uint32_t* __restrict__ idx,
-                                                         uint64_t n_tri, uint32_t W, uint32_t H,
+                                                         uint64_t n_tri, uint32_t W, uint32_t H, int32_t own_box,
                                                          unsigned long long* frag, uint32_t* __restrict__ queue_count,
                                                          uint4* __restrict__ queue) {
     const int lane = threadIdx.x & 31;
@@ -352,7 +436,7 @@ __global__ void __launch_bounds__(256, WT_RASTER_MINB) k_water_raster(const int4
                 if (setup_tri(w, W, H, s)) {
                     // box <= 16384^2 pixels: 32 bits hold its size
                     const int32_t npix = (s.px1 - s.px0 + 1) * (s.py1 - s.py0 + 1);
-                    own = npix <= kOwnPixels;
+                    own = npix <= own_box;
                     defer = !own;
                 }
             } else {
@@ -376,79 +460,86 @@ __global__ void __launch_bounds__(256, WT_RASTER_MINB) k_water_raster(const int4
 }
 
 // Second pass over the queue (launched dependent on the first, whose
-// completion it waits for): every warp of a resident grid takes `per`
-// consecutive entries a round (loads and triangle set-up in parallel, one
-// lane each), then rasterises them one after another with all 32 lanes
-// striding over the pixels; clipped triangles are cut into a fan first.
-// Spreading the queue over every warp keeps the near-camera rows, whose
-// triangles are the large ones and lie next to one another in the index
-// buffer, off a few warps.
-__global__ void __launch_bounds__(256) k_water_raster_deferred(const float4* __restrict__ clip,
-                                                               const int4* __restrict__ win,
-                                                               uint32_t W, uint32_t H, unsigned long long* frag,
-                                                               const uint32_t* __restrict__ queue_count,
-                                                               const uint4* __restrict__ queue) {
+// completion it waits for): a resident grid; block b of G takes the entries b,
+// b + G, ... and deals them to its warps in turn, since the near-camera rows,
+// whose triangles are the large ones, lie next to one another in the queue.  A
+// warp deals the rows of its small triangles to its lanes (raster_rows); the
+// others, and what is left of clipped ones (cut into a fan), are rasterised one
+// after another by the whole block.
+//
+// Bound by the latency of its chain (entry, window coordinates, set-up, rows) at
+// 6 warps a scheduler (80 registers), and by a last block's large
+// triangles.  With a warp per triangle and its pixels in steps of 32 (half of a
+// box is outside, and a box of 15000 pixels was one warp's) both passes took,
+// grid side at viewport: 161 at 2302 x 1361 352 us, now 81; 160 at 1730 x 342 52,
+// now 16; 481 at 950 x 864 78, now 20; 1024 at 1920 x 1080 36, now 36.
+__global__ void __launch_bounds__(256, 3) k_water_raster_deferred(const float4* __restrict__ clip,
+                                                                  const int4* __restrict__ win,
+                                                                  uint32_t W, uint32_t H, unsigned long long* frag,
+                                                                  const uint32_t* __restrict__ queue_count,
+                                                                  const uint4* __restrict__ queue) {
+    __shared__ __align__(16) RowTri s_rows[8][32];
+    __shared__ uint4 s_large[256];
+    __shared__ uint32_t s_n;
     cudaGridDependencySynchronize();  // the first pass is complete: the queue and its count
     const uint64_t n = *queue_count;
-    const int lane = threadIdx.x & 31;
-    const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-    const uint64_t warp = blockIdx.x * (uint64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
-    const uint64_t want = (n + warps - 1) / warps;
-    const uint32_t per = want < 1 ? 1u : (want > 32 ? 32u : (uint32_t)want);
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const float hw = (float)W * 0.5f, hh = (float)H * 0.5f;
-    for (uint64_t e0 = warp * per; e0 < n; e0 += warps * per) {
-        const uint64_t e = e0 + lane;
-        int kind = 0;  // 0 nothing, 2 window triangle set up, 3 clip first
-        uint32_t t = 0;
-        uint32_t vi[3] = {0u, 0u, 0u};
+    const auto window = [&](const uint4& q, WinTri& w) {
+        // the first pass queued only triangles whose three indices are in range
+        const int4 a = win[q.y], b = win[q.z], c = win[q.w];
+        w.X[0] = a.x; w.Y[0] = a.y; w.Z[0] = __int_as_float(a.z);
+        w.X[1] = b.x; w.Y[1] = b.y; w.Z[1] = __int_as_float(b.z);
+        w.X[2] = c.x; w.Y[2] = c.y; w.Z[2] = __int_as_float(c.z);
+        return (a.w & b.w & c.w) != 0;  // else it is clipped first
+    };
+    for (uint64_t e0 = blockIdx.x; e0 < n; e0 += 256ull * gridDim.x) {
+        if (threadIdx.x == 0) s_n = 0;
+        __syncthreads();
+        const uint64_t e = e0 + (uint64_t)(8u * lane + warp) * gridDim.x;
+        uint4 q = make_uint4(0, 0, 0, 0);
         Setup s;
-        if ((uint32_t)lane < per && e < n) {
-            // the first pass queued only triangles whose three indices are in range
-            const uint4 q = queue[e];
-            t = q.x;
-            vi[0] = q.y;
-            vi[1] = q.z;
-            vi[2] = q.w;
-            const int4 a = win[vi[0]], b = win[vi[1]], c = win[vi[2]];
-            if (a.w & b.w & c.w) {
-                WinTri w;
-                w.X[0] = a.x; w.Y[0] = a.y; w.Z[0] = __int_as_float(a.z);
-                w.X[1] = b.x; w.Y[1] = b.y; w.Z[1] = __int_as_float(b.z);
-                w.X[2] = c.x; w.Y[2] = c.y; w.Z[2] = __int_as_float(c.z);
-                if (setup_tri(w, W, H, s)) kind = 2;
-            } else {
-                kind = 3;
+        bool dealt = false;
+        if (e < n) {
+            q = queue[e];
+            WinTri w;
+            bool large = true;
+            if (window(q, w)) {
+                const bool any = setup_tri(w, W, H, s);
+                dealt = any && s.small && (s.px1 - s.px0 + 1) * (s.py1 - s.py0 + 1) <= kDealPixels;
+                large = any && !dealt;
             }
+            if (large) s_large[atomicAdd(&s_n, 1u)] = q;
         }
-        unsigned todo = __ballot_sync(kFull, kind != 0);
-        while (todo) {
-            const int src = __ffs(todo) - 1;
-            todo &= todo - 1;
-            const int k = __shfl_sync(kFull, kind, src);
-            const uint32_t tri = __shfl_sync(kFull, t, src);
-            if (k == 2) {
-                raster_warp(shfl_setup(s, src), tri, W, frag, lane);
+        __syncwarp();
+        if (__any_sync(kFull, dealt)) raster_rows(s, dealt, q.x, W, frag, s_rows[warp], lane);
+        __syncthreads();
+        for (uint32_t k = 0; k < s_n; ++k) {
+            q = s_large[k];
+            WinTri w;
+            if (window(q, w)) {
+                if (!setup_tri(w, W, H, s)) continue;
+                if (s.small) raster_block<int32_t>(s, q.x, W, frag);
+                else raster_block<int64_t>(s, q.x, W, frag);
                 continue;
             }
             CV4 poly[8];
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                const float4 c = clip[__shfl_sync(kFull, vi[j], src)];
-                poly[j] = CV4{c.x, c.y, c.z, c.w};
-            }
+            const float4 c0 = clip[q.y], c1 = clip[q.z], c2 = clip[q.w];
+            poly[0] = CV4{c0.x, c0.y, c0.z, c0.w};
+            poly[1] = CV4{c1.x, c1.y, c1.z, c1.w};
+            poly[2] = CV4{c2.x, c2.y, c2.z, c2.w};
             const int nv = clip_polygon(poly, 3);
             bool bad = nv < 3;
             for (int j = 0; j < nv; ++j) bad |= !(poly[j].w > 0.0f);
             if (bad) continue;
             for (int j = 1; j + 1 < nv; ++j) {
-                WinTri sw;
-                to_window(poly[0], hw, hh, sw.X[0], sw.Y[0], sw.Z[0]);
-                to_window(poly[j], hw, hh, sw.X[1], sw.Y[1], sw.Z[1]);
-                to_window(poly[j + 1], hw, hh, sw.X[2], sw.Y[2], sw.Z[2]);
-                Setup cs;
-                if (setup_tri(sw, W, H, cs)) raster_warp(cs, tri, W, frag, lane);
+                to_window(poly[0], hw, hh, w.X[0], w.Y[0], w.Z[0]);
+                to_window(poly[j], hw, hh, w.X[1], w.Y[1], w.Z[1]);
+                to_window(poly[j + 1], hw, hh, w.X[2], w.Y[2], w.Z[2]);
+                if (setup_tri(w, W, H, s)) raster_block<int64_t>(s, q.x, W, frag);
             }
         }
+        __syncthreads();
     }
 }
 
@@ -796,7 +887,7 @@ extern "C" wt_status wt_water_raster(const float* clip, uint64_t n_vertices, con
     // one thread per triangle (at most 2^24 blocks): most cost almost nothing
     const uint64_t rb = (n_triangles + 255) / 256;
     e = launch_dependent(k_water_raster, dim3((unsigned)rb), s, static_cast<const int4*>(win), n_vertices, indices,
-                         n_triangles, width, height, frag, queue_count, queue);
+                         n_triangles, width, height, own_pixels(n_triangles), frag, queue_count, queue);
     if (e != cudaSuccess) return cuda_fail(e, "wt_water_raster launch");
     // the queue: a resident grid, at most one warp per triangle
     e = launch_dependent(k_water_raster_deferred,
