@@ -25,6 +25,8 @@
 //                            or the vertex stage).
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include <atomic>
 #include <cstdint>
 
@@ -64,6 +66,54 @@ __device__ __forceinline__ void flag_error(WsHeader* h, uint32_t code, uint32_t 
 // constants and, for the adjoint, its queue (adj_scan_body's arrays).
 constexpr uint32_t kSmallPrep = 32;
 
+// The constants of such a table, by the blocks after the first: one kind of
+// constant for 32 pairs (or the patches' own) is a task, and a block takes four at
+// a time, one warp per scheduler.  An FP64 operation holds a scheduler's pipe for
+// 64 cycles, so the five kinds of a pair one after another on one SM, beside the
+// scans, were most of this kernel: 7 patches of 106 pairs 5.6 us, now 2.9.
+constexpr uint32_t kSmallTasks = 4;  // per block and round
+constexpr uint32_t kSmallPairs = 1u << 17;  // patches x waves (the pairs are mostly far fewer)
+
+__device__ void prep_small_constants(const wt_patch* __restrict__ patches, uint32_t n, const wt_wave* __restrict__ waves,
+                                     uint32_t n_waves, uint64_t out_capacity, uint64_t coef_capacity, char* ws,
+                                     const WsLayout& L, const HmDev& hm) {
+    constexpr unsigned kAll = 0xffffffffu;
+    PatchAux* aux = reinterpret_cast<PatchAux*>(ws + L.aux);
+    PairCoef* coef = reinterpret_cast<PairCoef*>(ws + L.coef);
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    if (warp >= kSmallTasks) return;
+    // the pairs' offsets, as the first block finds them
+    uint32_t end = lane < n && patch_ok(patches[lane], n_waves, out_capacity) ? patches[lane].wave_count : 0u;
+    const uint32_t count = end;
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kAll, end, o);
+        if (lane >= o) end += y;
+    }
+    const uint32_t total = __shfl_sync(kAll, end, 31);
+    if (total > coef_capacity) return;
+    const uint32_t tasks = 5u * ((total + 31u) / 32u) + 1u;
+    for (uint32_t t = (blockIdx.x - 1u) * kSmallTasks + warp; t < tasks; t += (gridDim.x - 1u) * kSmallTasks) {
+        if (t == 0) {
+            if (lane < n) aux[lane] = make_patch_aux(patches[lane], hm, end - count);
+            continue;
+        }
+        const uint32_t kind = (t - 1u) % 5u, P = 32u * ((t - 1u) / 5u) + lane;
+        uint32_t p = 0, before = 0;  // the patch of pair P, and the pairs before it
+        for (uint32_t q = 0; q < n; ++q) {
+            const uint32_t e = __shfl_sync(kAll, end, q);
+            if (e <= P) {
+                p = q + 1u;
+                before = e;
+            }
+        }
+        if (P >= total) continue;
+        const wt_patch& Pt = patches[p];
+        const wt_wave w = waves[Pt.wave_offset + (P - before)];
+        if (kind < 4u) (&coef[P].t00)[kind] = phase_turns((int)kind, Pt, w);
+        else sum_coefs(w, coef[P]);
+    }
+}
+
 __device__ void prep_small(const wt_patch* __restrict__ patches, uint32_t n, const wt_wave* __restrict__ waves,
                            uint32_t n_waves, uint64_t out_capacity, uint64_t coef_capacity, uint32_t tile_cols,
                            char* ws, const WsLayout& L, const HmDev& hm, uint32_t mma_sms, uint32_t mma_max, int do_adj,
@@ -79,8 +129,6 @@ __device__ void prep_small(const wt_patch* __restrict__ patches, uint32_t n, con
     uint32_t* tile_pre = reinterpret_cast<uint32_t*>(ws + L.tile_pre);
     uint32_t* pair_off = reinterpret_cast<uint32_t*>(ws + L.pair_off);
     uint32_t* tiles_g = reinterpret_cast<uint32_t*>(ws + L.tiles);
-    PatchAux* aux = reinterpret_cast<PatchAux*>(ws + L.aux);
-    PairCoef* coef = reinterpret_cast<PairCoef*>(ws + L.coef);
     const uint32_t tid = threadIdx.x, lane = tid & 31u;
     constexpr unsigned kAll = 0xffffffffu;
 
@@ -112,17 +160,12 @@ __device__ void prep_small(const wt_patch* __restrict__ patches, uint32_t n, con
     __syncthreads();
     const uint32_t total_pairs = s_off[n];
     const bool nomem = total_pairs > coef_capacity;
-    // one (patch, wave) pair per thread (at most 1024 with fuse_coef)
-    if (tid < total_pairs) {
-        uint32_t p = 0;
-        while (s_off[p + 1] <= tid) ++p;
-        const wt_patch& Pt = sp[p];
-        const wt_wave w = waves[Pt.wave_offset + (tid - s_off[p])];
+    for (uint32_t i = tid, p = 0; i < total_pairs; i += blockDim.x) {
+        while (s_off[p + 1] <= i) ++p;
+        const wt_wave w = waves[sp[p].wave_offset + (i - s_off[p])];
         if (!wave_ok(w)) atomicOr(&s_wave_bad, 1u << p);
         if (!mma_wave(w)) atomicOr(&s_wave_wild, 1u << p);
-        if (!nomem) coef[tid] = make_pair_coef(Pt, w);
     }
-    if (tid < n && !nomem) aux[tid] = make_patch_aux(sp[tid], hm, s_off[tid]);
     __syncthreads();
     if (tid >= 32) return;
     const unsigned bad = s_struct_bad | s_wave_bad;
@@ -252,6 +295,10 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
     // waits at its start anyway)
     if (!fuse_coef) cudaTriggerProgrammaticLaunchCompletion();
 #endif
+    if (blockIdx.x > 0) {
+        prep_small_constants(patches, n, waves, n_waves, out_capacity, coef_capacity, ws, L, hm);
+        return;
+    }
     if (n <= kSmallPrep && fuse_coef) {
         prep_small(patches, n, waves, n_waves, out_capacity, coef_capacity, tile_cols, ws, L, hm, mma_sms, mma_max, do_adj, AL,
                    adj_chunk_max, adj_min_tiles);
@@ -725,13 +772,18 @@ cudaError_t launch_prep(const wt_patch* patches, uint32_t n_patches, const wt_wa
     // coefficient capacity = what the caller's workspace holds past the fixed part
     // (the header records the real total; the scan refuses to overflow it)
     uint64_t coef_cap = (L.end - L.coef) / sizeof(PairCoef);
-    // at most 1024 (patch, wave) pairs: the scan kernel forms the constants too
-    const int fuse = (uint64_t)n_patches * n_waves <= 1024u;
+    // few (patch, wave) pairs, by the most that the table can have: the scan kernel
+    // forms the constants too
+    const uint64_t pairs = (uint64_t)n_patches * n_waves;
+    const int fuse = pairs <= (n_patches <= kSmallPrep ? kSmallPairs : 1024u);
     const AdjScanArgs none{};
     const AdjScanArgs& A = adj ? *adj : none;
     const int sms = sm_count();
     if (sms <= 0) return cudaErrorInvalidDevice;
-    k_prep_scan<<<1, 1024, 0, s>>>(patches, n_patches, waves, n_waves, out_capacity, coef_cap, tile_cols, w, L,
+    const unsigned more = fuse && n_patches <= kSmallPrep
+                              ? std::min((unsigned)sms - 1u, (unsigned)((5u * ((pairs + 31u) / 32u) + kSmallTasks) / kSmallTasks))
+                              : 0u;
+    k_prep_scan<<<1u + more, 1024, 0, s>>>(patches, n_patches, waves, n_waves, out_capacity, coef_cap, tile_cols, w, L,
                                    hm, fuse, (uint32_t)sms, mma_max_waves, adj ? 1 : 0, A.L, A.chunk_max, A.min_tiles);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
