@@ -278,6 +278,170 @@ __device__ void prep_small(const wt_patch* __restrict__ patches, uint32_t n, con
     }
 }
 
+// Tables of up to kMediumPrep patches and 16384 waves whose constants the next
+// kernel forms: a thread has a patch, in registers, and what the threads share
+// is in shared memory, instead of the general path's round trips to global
+// memory between its steps (256 patches of 64-128 side, the whole call 60 us,
+// now 46).  Writes what the general path writes.
+constexpr uint32_t kMediumPrep = 512;
+
+// Exclusive prefix of v over the block's 1024 threads, and the total.
+__device__ __forceinline__ uint32_t block_prefix(uint32_t v, uint32_t* part, uint32_t& total) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t x = v;
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    __syncthreads();  // the last prefix's readers are done
+    if (lane == 31) part[warp] = x;
+    __syncthreads();
+    uint32_t w = part[lane];
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
+        if (lane >= o) w += y;
+    }
+    total = __shfl_sync(0xffffffffu, w, 31);
+    const uint32_t before = __shfl_sync(0xffffffffu, w, (warp + 31u) & 31u);
+    return (warp > 0 ? before : 0u) + x - v;
+}
+
+__device__ void prep_medium(const wt_patch* __restrict__ patches, uint32_t n, const wt_wave* __restrict__ waves,
+                            uint32_t n_waves, uint64_t out_capacity, uint64_t coef_capacity, uint32_t tile_cols, char* ws,
+                            const WsLayout& L, uint32_t mma_sms, uint32_t mma_max, int do_adj, const AdjLayout& AL,
+                            uint32_t adj_chunk_max, uint32_t adj_min_tiles, uint4* s_keys, uint32_t* s_tiles,
+                            uint32_t* s_rank, uint32_t* good_wave, uint32_t* tame_wave) {
+    __shared__ uint32_t part[32], s_bad, s_items, s_mma;
+    __shared__ unsigned long long part64[32];
+    constexpr unsigned kAll = 0xffffffffu;
+    WsHeader* hdr = reinterpret_cast<WsHeader*>(ws);
+    uint32_t* sorted = reinterpret_cast<uint32_t*>(ws + L.sorted);
+    uint32_t* tile_pre = reinterpret_cast<uint32_t*>(ws + L.tile_pre);
+    uint32_t* pair_off = reinterpret_cast<uint32_t*>(ws + L.pair_off);
+    uint32_t* tiles_g = reinterpret_cast<uint32_t*>(ws + L.tiles);
+    const uint32_t p = threadIdx.x, lane = p & 31u, warp = p >> 5;
+    if (p == 0) {
+        s_bad = kNoPatch;
+        s_items = s_mma = 0;
+    }
+    if (p < n) s_rank[p] = 0;
+    uint32_t count = 0, tl = 0, rows = 0, ct = 0, w0 = 0, waves_p = 0;
+    bool ok = false, mma = false;
+    if (p < n) {
+        const wt_patch P = patches[p];
+        ok = patch_ok(P, n_waves, out_capacity);
+        mma = ok && mma_max > 0 && mma_patch(P, mma_max);
+        count = ok ? P.wave_count : 0u;
+        tl = ok ? P.rows * tiles_per_row(P.cols, tile_cols / 32) : 0u;
+        rows = P.rows;
+        ct = (P.cols + 127u) / 128u;
+        w0 = P.wave_offset;
+        waves_p = P.wave_count;
+    }
+    // each wave once, a warp's 32 waves a word
+    const uint32_t nw_round = (n_waves + 31u) & ~31u;
+#pragma unroll 4
+    for (uint32_t w = p; w < nw_round; w += blockDim.x) {
+        bool good = false, tame = false;
+        if (w < n_waves) {
+            const wt_wave v = waves[w];
+            good = wave_ok(v);
+            tame = mma_wave(v);
+        }
+        const uint32_t word = __ballot_sync(kAll, good), tword = __ballot_sync(kAll, tame);
+        if (lane == 0) {
+            good_wave[w >> 5] = word;
+            tame_wave[w >> 5] = tword;
+        }
+    }
+    uint32_t total_pairs;
+    const uint32_t off = block_prefix(count, part, total_pairs);  // (and the bits are written)
+    const bool nomem = total_pairs > coef_capacity;
+    if (p < n) {
+        pair_off[p] = off;
+        bool bad = false, wild = false;
+        for (uint32_t w = w0, w1 = w0 + count; w < w1 && !bad;) {
+            const uint32_t bit = w & 31u, take = min(32u - bit, w1 - w);
+            const uint32_t want = (take == 32u ? 0xffffffffu : ((1u << take) - 1u)) << bit;
+            bad = (good_wave[w >> 5] & want) != want;
+            wild |= (tame_wave[w >> 5] & want) != want;
+            w += take;
+        }
+        if (bad) tl = 0;
+        mma = mma && !bad && !wild;
+        if (!ok || bad) atomicMin(&s_bad, p);
+    }
+    // the matrix-product patches' items
+    unsigned long long rowct = mma ? (unsigned long long)rows * ct : 0ull;
+    for (int o = 16; o > 0; o >>= 1) rowct += __shfl_xor_sync(kAll, rowct, o);
+    if (lane == 0) part64[warp] = rowct;
+    __syncthreads();
+    rowct = part64[lane];
+    for (int o = 16; o > 0; o >>= 1) rowct += __shfl_xor_sync(kAll, rowct, o);
+    uint32_t item_rows = 0;
+    if (rowct > 0) {
+        item_rows = mma_item_rows(rowct, mma_sms);
+        if (mma) tl = ct * ((rows + item_rows - 1u) / item_rows);
+        const uint32_t items = __reduce_add_sync(kAll, mma ? tl : 0u), some = __popc(__ballot_sync(kAll, mma));
+        if (lane == 0 && some > 0) {
+            atomicAdd(&s_items, items);
+            atomicAdd(&s_mma, some);
+        }
+    }
+    // ranks: keys descending, ties by index; each patch's comparisons shared out
+    // over as many threads as there are
+    const uint32_t n4 = (n + 3u) / 4u, key = p < n ? sort_key(waves_p, mma) : 0u;
+    if (p < 4u * n4) reinterpret_cast<uint32_t*>(s_keys)[p] = key;
+    __syncthreads();
+    const uint32_t shares = blockDim.x / n, share = p / n, mine = p - share * n;
+    if (share < shares) {
+        const uint32_t k = reinterpret_cast<const uint32_t*>(s_keys)[mine];
+        uint32_t rank = 0;
+        for (uint32_t q = share * n4 / shares; q < (share + 1u) * n4 / shares; ++q) {
+            const uint4 v = s_keys[q];
+            rank += v.x > k || (v.x == k && 4u * q < mine);
+            rank += v.y > k || (v.y == k && 4u * q + 1u < mine);
+            rank += v.z > k || (v.z == k && 4u * q + 2u < mine);
+            rank += v.w > k || (v.w == k && 4u * q + 3u < mine);
+        }
+        atomicAdd(&s_rank[mine], rank);
+    }
+    __syncthreads();
+    if (p < n) {
+        tiles_g[p] = tl;
+        const uint32_t rank = s_rank[p];
+        s_tiles[rank] = tl;
+        if (!nomem) sorted[rank] = p;
+    }
+    __syncthreads();
+    const uint32_t tq = p < n && !nomem ? s_tiles[p] : 0u;
+    uint32_t total_tiles;
+    const uint32_t before = block_prefix(tq, part, total_tiles);
+    if (p < n) tile_pre[p] = before;
+    if (p == 0) {
+        const bool any_bad = s_bad != kNoPatch;
+        const uint32_t items = nomem ? 0u : s_items;
+        hdr->status = any_bad ? (uint32_t)WT_ERR_INVALID_ARG : (nomem ? (uint32_t)WT_ERR_NOMEM : 0u);
+        hdr->bad_patch = s_bad;
+        hdr->tile_counter = items;  // the recurrence kernel's tiles follow the items
+        hdr->n_patches = n;
+        hdr->tile_cols = tile_cols;
+        hdr->mma_items = items;
+        hdr->mma_rows = item_rows;
+        hdr->mma_counter = 0;
+        hdr->mma_patches = nomem ? 0u : s_mma;
+        hdr->total_tiles = total_tiles;
+        tile_pre[n] = total_tiles;
+        // bounds every coefficient write of the next kernel
+        pair_off[n] = nomem ? 0u : total_pairs;
+        if (nomem && do_adj) hdr->total_chunks = 0;
+    }
+    if (do_adj && !nomem) {
+        __syncthreads();  // sorted, tile_pre and the header are complete
+        adj_scan_body(ws, AL, n, adj_chunk_max, adj_min_tiles, rowct / 2u);
+    }
+}
+
 // fuse_coef: also form the per-(patch, wave) and per-patch constants here
 // (small tables: the host passes it when n_patches * n_waves <= 1024, one
 // pair per thread), so that no second prep kernel runs.
@@ -309,7 +473,7 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
     uint32_t* tile_pre = reinterpret_cast<uint32_t*>(ws + L.tile_pre);
     uint32_t* pair_off = reinterpret_cast<uint32_t*>(ws + L.pair_off);
     uint32_t* tiles = reinterpret_cast<uint32_t*>(ws + L.tiles);
-    __shared__ uint32_t bins[kSortBins];
+    __shared__ __align__(16) uint32_t bins[kSortBins];
     constexpr uint32_t kScanSmemOffsets = 4096;
     __shared__ uint32_t off_s[kScanSmemOffsets];
     __shared__ uint32_t good_wave[kWaveMaskWords];  // bit w: wave w passes wave_ok
@@ -317,6 +481,12 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
     __shared__ unsigned long long s_rowct;          // rows x 128-column blocks of the matrix-product patches
     __shared__ uint32_t s_mma_items, s_mma_n;
 
+    if (n <= kMediumPrep && !fuse_coef && n_waves <= 32u * kWaveMaskWords) {
+        prep_medium(patches, n, waves, n_waves, out_capacity, coef_capacity, tile_cols, ws, L, mma_sms, mma_max, do_adj, AL,
+                    adj_chunk_max, adj_min_tiles, reinterpret_cast<uint4*>(bins), off_s, off_s + kMediumPrep, good_wave,
+                    tame_wave);
+        return;
+    }
     if (threadIdx.x == 0) {
         hdr->status = 0;
         hdr->bad_patch = kNoPatch;
@@ -426,9 +596,12 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
     }
     // the matrix-product patches' items, then the sort keys
     if (mma_max > 0) {
+        unsigned long long rowct = 0;
         for (uint32_t p = threadIdx.x; p < n; p += blockDim.x)
-            if (tiles[p] & kMmaFlag)
-                atomicAdd(&s_rowct, (unsigned long long)patches[p].rows * ((patches[p].cols + 127u) / 128u));
+            if (tiles[p] & kMmaFlag) rowct += (unsigned long long)patches[p].rows * ((patches[p].cols + 127u) / 128u);
+        for (int o = 16; o > 0; o >>= 1) rowct += __shfl_xor_sync(0xffffffffu, rowct, o);
+        // one a warp: a 64-bit sum in shared memory is a loop of compare-and-swaps
+        if ((threadIdx.x & 31u) == 0 && rowct > 0) atomicAdd(&s_rowct, rowct);
         __syncthreads();
         if (s_rowct > 0) {
             const uint32_t h = mma_item_rows(s_rowct, mma_sms);
