@@ -366,8 +366,12 @@ __global__ void __launch_bounds__(32 * kColLanes) k_adj_cols(uint32_t n, const c
 
 // Closed-form FP64 gradient of every (patch, wave) pair from its eleven
 // column sums, one pair per thread (GB300's FP64 rate is low: a warp per
-// wave with one busy lane spent 16 us here on 64 patches).
-__global__ void __launch_bounds__(256) k_adj_pairs(const wt_patch* __restrict__ patches, uint32_t n,
+// wave with one busy lane spent 16 us here on 64 patches), one warp per
+// scheduler: an operation holds a scheduler's FP64 pipe for 64 cycles, so a
+// second warp there only waits (64 patches, 2300 pairs, with 256 threads a block
+// 10.0 us, with 128 7.3).
+constexpr int kPairThreads = 128;
+__global__ void __launch_bounds__(kPairThreads) k_adj_pairs(const wt_patch* __restrict__ patches, uint32_t n,
                                                    const wt_wave* __restrict__ waves, const char* __restrict__ ws,
                                                    AdjLayout L) {
 #if __CUDA_ARCH__ >= 900
@@ -579,7 +583,7 @@ cudaError_t launch_adjoint(const wt_patch* patches, uint32_t n_patches, const wt
     if (e != cudaSuccess) return e;
     const unsigned wb = (n_waves + 7) / 8 < (unsigned)sms * 16 ? (n_waves + 7) / 8 : (unsigned)sms * 16;
     if (wb == 0) return cudaSuccess;
-    e = launch_pdl(k_adj_pairs, dim3((unsigned)sms), dim3(256), 0, s, patches, n_patches, waves,
+    e = launch_pdl(k_adj_pairs, dim3((unsigned)sms), dim3(kPairThreads), 0, s, patches, n_patches, waves,
                    static_cast<const char*>(ws), L);
     if (e != cudaSuccess) return e;
     return launch_pdl(k_adj_waves, dim3(wb), dim3(256), 0, s, patches, n_patches, n_waves,
