@@ -131,20 +131,25 @@ class ClockSampler:
                 "reasons": reasons, "samples": len(load), "power_w_max": pmax}
 
 
-def traffic_from_profile(tuning, vertices):
-    """DRAM bytes of one forward launch of the tuned shape: the bytes per
-    vertex an ncu capture of that kernel measured (profiles/forward_traffic.json,
-    keyed by the kernel's launch shape) times this launch's vertices; None
-    when no capture of the shape exists."""
+def measured_hbm():
+    """The machine's measured copy bandwidth (GB/s), else an earlier measurement."""
+    try:
+        return float(json.loads((ROOT / "MEASURED_PEAKS.json").read_text())["hbm_gbs"]), "measured copy bandwidth"
+    except (OSError, ValueError, KeyError):
+        return 6800.0, "copy bandwidth measured earlier on a GB300"
+
+
+def traffic_from_profile(vertices):
+    """DRAM bytes of one forward launch: the bytes per vertex an ncu capture of
+    the matrix-product kernel measured on this table (profiles/forward_traffic.json)
+    times this launch's vertices; None without that capture."""
     if not PROFILE_TRAFFIC.exists():
         return None
     try:
         rec = json.loads(PROFILE_TRAFFIC.read_text())
     except ValueError:
         return None
-    key = (f"warps={tuning['warps_per_block']},vpl={tuning['max_vertices_per_lane']},"
-           f"epi={tuning['epilogue_in_shared']}")
-    r = rec.get("shapes", {}).get(key)
+    r = rec.get("shapes", {}).get("products")
     return None if r is None else r["dram_bytes_per_vertex"] * vertices
 
 
@@ -744,6 +749,7 @@ def run_ours(args):
         peak_mufu_terms = sin_s / 2.0   # sin + cos per term on the MUFU pipe
         achieved = value / world
         verts = int(np.sum(w.patches["cols"].astype(np.int64) * w.patches["rows"]))
+        hbm_gbs, hbm_source = measured_hbm()
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms_step, "higher_is_better": True,
@@ -759,15 +765,17 @@ def run_ours(args):
             "roofline": {"bound": "fma+mufu", "achieved": achieved / 1e9,
                          "peak": min(peak_fma_terms, peak_mufu_terms) / 1e9,
                          "unit": "Gterms/s", "frac": achieved / min(peak_fma_terms, peak_mufu_terms),
-                         "traffic": traffic_from_profile(tuning, verts),
+                         "traffic": traffic_from_profile(verts),
                          "peak_source": "term roofline min(P_FMA/10, P_MUFU/2) (10 FMA + 2 sin/cos of algorithmic "
                                         "work per term), P_FMA and P_MUFU measured in this run by wt_measure_peaks",
                          "fma_leg_peak": peak_fma_terms / 1e9, "fma_leg_frac": achieved / peak_fma_terms,
                          "mufu_leg_peak": peak_mufu_terms / 1e9,
-                         "hbm_gbs": 32.0 * verts / (ms_step * 1e-3) / 1e9,
-                         "note": "achieved = terms per step / step time (prep launches included); the kernel "
-                                 "takes sin/cos from an FMA recurrence, not 2 MUFU per term, so its own binding "
-                                 "pipe is FMA issue: fma_leg_frac is its fraction of that leg"},
+                         "hbm_gbs": 32.0 * verts / (ms_step * 1e-3) / 1e9, "hbm_peak_gbs": hbm_gbs,
+                         "hbm_frac": 32.0 * verts / (ms_step * 1e-3) / 1e9 / hbm_gbs, "hbm_peak_source": hbm_source,
+                         "note": "achieved = terms per step / step time (prep launches included); the eight sums of "
+                                 "parallelogram patches are products on the tensor cores with sin/cos per column and "
+                                 "per row, not per term, so the FP32 pipes' term roofline is a yardstick (frac can "
+                                 "exceed 1) and the bound left is the outputs' write: hbm_frac"},
             "cpu_baseline": cpu,
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h),
                     "ms_per_step": e2e_ms, "stream_groups": len(groups),
@@ -778,7 +786,7 @@ def run_ours(args):
                             "the host link's D2H bandwidth measured in this run (1 GiB device -> pinned host "
                             "cudaMemcpyAsync, best of 5); link_bound_ms: the step's copies alone at those rates"},
             "accuracy": accuracy,
-            "gpu_launches": 3 * args.steps,
+            "gpu_launches": 4 * args.steps,  # scan, constants, products, recurrence
             "clocks": clocks,
             "wall_s_timed_region": t_wall,
             "extras": extras,

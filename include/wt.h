@@ -291,9 +291,8 @@ wt_status wt_grid_indices(uint32_t cols, uint32_t rows, uint32_t base_vertex,
  * width x height texel grid, then normalised to [0, 1] (min -> 0, max -> 1)
  * so the reference's 2*(r - 0.5) mapping (water-grid.vert:106-111) holds:
  *   h(i, j) = sum_m a_m sin(2 pi (kx_m i / width + ky_m j / height) + phase_m).
- * terms: device array.  workspace: wt_noise_workspace_size bytes (the
- * separable factor tables, 8 bytes per term and texel row / column, and the
- * min / max).  No reference counterpart: the reference loads a fixed PNG
+ * terms: device array.  workspace: wt_noise_workspace_size bytes (the blocks'
+ * minima and maxima, within 8 bytes per term and texel row / column).  No reference counterpart: the reference loads a fixed PNG
  * (render-engine.cpp:1308-1322). */
 wt_status wt_noise_workspace_size(uint32_t n_terms, uint32_t width, uint32_t height, size_t* bytes);
 wt_status wt_noise_synth(const wt_noise_term* terms, uint32_t n_terms,

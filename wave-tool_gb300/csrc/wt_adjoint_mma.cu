@@ -26,7 +26,7 @@
 //
 // What bounds it: issue slots (61 % busy), two thirds of them the vertex adjoints
 // (about 400 instructions per 32 vertices: the normal's adjoint, the scales, 16
-// values split into hi and lo); the products take about half of the tensor pipe,
+// values split into hi and lo); the products take 30 % of the tensor pipe,
 // DRAM 19 % (dL/dpos and dL/dnrm once).  Measured, 64 patches of 64-1024 side
 // with 8-64 waves, 16 M vertices, the whole call: 432 us against 1054 with the
 // recurrence.  On the way: 8 vertex warps and 6 for operands 587 us; 16 and 2 of

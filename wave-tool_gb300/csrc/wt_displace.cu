@@ -6,10 +6,13 @@
 // upload of src/render-engine.cpp:1057-1110 (steepness already normalised by
 // the caller, :1073).
 //
-// Three launches (two when the table has at most 1024 (patch, wave) pairs),
-// all stream-ordered and graph-capturable:
-//   k_prep_scan  (1 block)   validate patches and waves, prefix sums, LPT sort
-//                            of patches by wave count, tile queue reset
+// Three launches (two when the scan kernel forms the constants: small tables), and
+// before the last one the matrix products of parallelogram patches (wt_mma.cu)
+// when the call has 8 waves or more; one launch for one patch (wt_single.cu).  All
+// stream-ordered and graph-capturable:
+//   k_prep_scan              validate patches and waves, prefix sums, LPT sort
+//                            of patches by wave count, tile queue reset (one
+//                            block; the constants of small tables by others)
 //   k_prep_coef  (grid)      FP64 per-(patch, wave) phase constants in 64-bit
 //                            fixed-point turns + FP32 sum coefficients;
 //                            per-patch local frame; runs alongside the scan
@@ -70,7 +73,8 @@ constexpr uint32_t kSmallPrep = 32;
 // constant for 32 pairs (or the patches' own) is a task, and a block takes four at
 // a time, one warp per scheduler.  An FP64 operation holds a scheduler's pipe for
 // 64 cycles, so the five kinds of a pair one after another on one SM, beside the
-// scans, were most of this kernel: 7 patches of 106 pairs 5.6 us, now 2.9.
+// scans, were most of this kernel (7 patches of 106 pairs, the whole call 19.9 us, now
+// 15.7).
 constexpr uint32_t kSmallTasks = 4;  // per block and round
 constexpr uint32_t kSmallPairs = 1u << 17;  // patches x waves (the pairs are mostly far fewer)
 
@@ -282,7 +286,7 @@ __device__ void prep_small(const wt_patch* __restrict__ patches, uint32_t n, con
 // kernel forms: a thread has a patch, in registers, and what the threads share
 // is in shared memory, instead of the general path's round trips to global
 // memory between its steps (256 patches of 64-128 side, the whole call 60 us,
-// now 46).  Writes what the general path writes.
+// now 49).  Writes what the general path writes.
 constexpr uint32_t kMediumPrep = 512;
 
 // Exclusive prefix of v over the block's 1024 threads, and the total.

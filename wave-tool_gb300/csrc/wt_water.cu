@@ -40,7 +40,7 @@ constexpr float kGuard = 64.0f;  // guard band, in NDC units
 // triangles leave no other work to hide a long walk behind, so theirs go to the
 // second pass early; with two million and more it is the queue that costs.
 // Measured, both passes at 24 / 64 / 128 pixels: 481^2 vertices at 950 x 864
-// 20 / 33 / 38 us, 750^2 at 1920 x 1080 35 / 33 / 37, 1024^2 39 / 37 / 36.
+// 20 us at 24, 38 at 128; at 1920 x 1080 750^2 35 / 33 / 37, 1024^2 39 / 37 / 36.
 inline int32_t own_pixels(uint64_t n_tri) {
     return n_tri >> 21 ? 128 : (int32_t)((n_tri >> 14) < 24 ? 24 : n_tri >> 14);
 }
