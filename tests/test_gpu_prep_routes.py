@@ -12,9 +12,9 @@ from test_gpu_adjoint import _check, _upstream, run_adjoint
 pytestmark = pytest.mark.gpu
 
 
-def _table(n, seed):
+def _table(n, seed, hi=14):
     from wave_tool_gb300 import workloads
-    w = workloads.small_random(seed, n_patches=n, side_range=(2, 40), n_waves_range=(0, 14), heightmap=False)
+    w = workloads.small_random(seed, n_patches=n, side_range=(2, 40), n_waves_range=(hi // 20, hi), heightmap=False)
     p = w.patches
     for i in range(0, n, 2):  # every other patch a rectangle, the rest skewed
         p["br"][i][1], p["tl"][i][0] = p["bl"][i][1], p["bl"][i][0]
@@ -22,10 +22,11 @@ def _table(n, seed):
     return w
 
 
-@pytest.mark.parametrize("n", [3, 31, 32, 33, 64, 511, 512, 513])
-def test_forward_and_refusals(wt, oracle, gpu, n):
+# (32 patches of up to 90 waves: more than 1024 pairs)
+@pytest.mark.parametrize("n,hi", [(3, 14), (31, 14), (32, 14), (32, 90), (33, 14), (64, 14), (511, 14), (512, 14), (513, 14)])
+def test_forward_and_refusals(wt, oracle, gpu, n, hi):
     import torch
-    w = _table(n, 5 + n)
+    w = _table(n, 5 + n, hi)
     surf = wt.Surface(w.patches, w.waves)
     pos, nrm = surf.displace(flags=wt.WT_OUT_DISPLACEMENT)
     torch.cuda.synchronize()
@@ -52,10 +53,10 @@ def test_forward_and_refusals(wt, oracle, gpu, n):
         assert torch.equal(p2[o:o + k], pos[o:o + k]) and torch.equal(n2[o:o + k], nrm[o:o + k])
 
 
-@pytest.mark.parametrize("n", [32, 33, 512, 513])
+@pytest.mark.parametrize("n,hi", [(32, 14), (32, 90), (33, 14), (512, 14), (513, 14)])
 @pytest.mark.parametrize("saved", [False, True])
-def test_gradient(wt, oracle, gpu, n, saved):
-    w = _table(n, 70 + n)
+def test_gradient(wt, oracle, gpu, n, hi, saved):
+    w = _table(n, 70 + n, hi)
     gp, gn = _upstream(w.n_vertices, n)
     g, _ = run_adjoint(wt, w, gp, gn, saved=saved)
     _check(g, oracle.adjoint_f64(w.patches, w.waves, gp.numpy(), gn.numpy()))

@@ -164,11 +164,26 @@ __device__ void prep_small(const wt_patch* __restrict__ patches, uint32_t n, con
     __syncthreads();
     const uint32_t total_pairs = s_off[n];
     const bool nomem = total_pairs > coef_capacity;
-    for (uint32_t i = tid, p = 0; i < total_pairs; i += blockDim.x) {
-        while (s_off[p + 1] <= i) ++p;
-        const wt_wave w = waves[sp[p].wave_offset + (i - s_off[p])];
-        if (!wave_ok(w)) atomicOr(&s_wave_bad, 1u << p);
-        if (!mma_wave(w)) atomicOr(&s_wave_wild, 1u << p);
+    if (total_pairs <= blockDim.x) {
+        if (tid < total_pairs) {
+            uint32_t p = 0;
+            while (s_off[p + 1] <= tid) ++p;
+            const wt_wave w = waves[sp[p].wave_offset + (tid - s_off[p])];
+            if (!wave_ok(w)) atomicOr(&s_wave_bad, 1u << p);
+            if (!mma_wave(w)) atomicOr(&s_wave_wild, 1u << p);
+        }
+    } else {
+        // each wave once (patches may share them); the patches of one that fails
+#pragma unroll 4
+        for (uint32_t i = tid; i < n_waves; i += blockDim.x) {
+            const wt_wave w = waves[i];
+            const bool good = wave_ok(w), tame = mma_wave(w);
+            for (uint32_t p = 0; !(good && tame) && p < n; ++p) {
+                if (i - sp[p].wave_offset >= s_off[p + 1] - s_off[p]) continue;  // (none of an invalid patch's)
+                if (!good) atomicOr(&s_wave_bad, 1u << p);
+                if (!tame) atomicOr(&s_wave_wild, 1u << p);
+            }
+        }
     }
     __syncthreads();
     if (tid >= 32) return;
