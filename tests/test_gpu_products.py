@@ -96,3 +96,28 @@ def test_waves_out_of_the_products_range(wt, oracle, gpu):
         _, disp64, _, _ = oracle.displace_f64(table, waves, None, None)
         assert rel_err(pos[:, :3].double().cpu().numpy(), disp64) <= 1e-5 or np.abs(disp64).max() == 0
         assert bool(torch.isfinite(pos).all()) and bool(torch.isfinite(nrm).all())
+
+
+# Ten waves of 15 to 60 m, as steep when their lengths are `far` times as large: the
+# displacements' coefficients grow with them, the slopes' stay.  A slope sum is
+# off by 2^-22 of each coefficient (two halves of 11 bits), 2 x 1e-7 (sines) and
+# 2^-23 (two truncated steps), 5.6e-7 times the coefficients' sum (at most 10 x
+# 2 pi / 100); the normal's rounding adds 3 x 2^-24: 5.4e-7 rad.
+@pytest.mark.parametrize("far", [2.0**0, 2.0**16, 2.0**20, 2.0**26, 2.0**30])
+@pytest.mark.parametrize("alone", [True, False])
+def test_slopes_beside_large_displacements(wt, oracle, gpu, far, alone):
+    import torch
+    from wave_tool_gb300 import workloads
+    rng = workloads.SplitMix64(77)
+    waves = np.array(workloads.waves_wide(rng, 10, lam=(15.0 * far, 60.0 * far)), dtype=wt.WAVE_DTYPE)
+    h = 60.0 * far
+    one = np.array([((-h, h), (h, h), (-h, -h), (h, -h), 160, 96, 0, 10, 100.0, 0.0, 0, 0)], dtype=wt.PATCH_DTYPE)
+    table = one if alone else np.concatenate([one, one])
+    table["out_offset"][1:] = 160 * 96
+    surf = wt.Surface(table, waves)
+    pos, nrm = surf.displace(flags=1)
+    torch.cuda.synchronize()
+    assert surf.status()[0] == 0
+    _, disp64, nrm64, _ = oracle.displace_f64(table, waves, None, None)
+    assert rel_err(pos[:, :3].double().cpu().numpy(), disp64) <= 1e-5
+    assert np.radians(angle_deg(nrm[:, :3].double().cpu().numpy(), nrm64)).max() <= 5.4e-7

@@ -67,8 +67,7 @@ struct Item {
     uint64_t rec0;  // first record
     uint32_t cols, c0, row0, nrows;
     uint32_t nwaves, first;
-    float inv_scale;
-    uint32_t pad;
+    float4 inv[2];  // the forward sums' inverse scales
 };
 
 struct Shared {
@@ -219,19 +218,18 @@ k_adjoint_mma(const wt_patch* __restrict__ patches, HmDev hm, const float* __res
             const PatchAux& pa = aux[p];
             const uint32_t first = pa.pair_offset;
             if (lane < 16) reinterpret_cast<uint32_t*>(&it.aux)[lane] = reinterpret_cast<const uint32_t*>(&pa)[lane];
-            float m = 0.0f;
+            PerSum m{};
             for (uint32_t i = lane; i < nw; i += 32u) {
-                m = coef_max(m, coef[4ull * (first + i) + 2]);
-                m = coef_max(m, coef[4ull * (first + i) + 3]);
+                max8(m, coef[4ull * (first + i) + 2], coef[4ull * (first + i) + 3]);
             }
-            const int ex = scale_exponent(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
+            const PerSum scales = warp_scales(m);
             const uint32_t pad = (nw + 7u) & ~7u;  // zero waves up to a multiple of 8
             for (uint32_t i = lane; i < pad; i += 32u) {
                 float4 v[4];
 #pragma unroll
                 for (uint32_t e = 0; e < 4; ++e)
                     v[e] = i < nw ? coef[4ull * (first + i) + e] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                table_entry(sh.table[slot], i, v, pow2f(ex));
+                table_entry(sh.table[slot], i, v, scales);
             }
             if (lane == 0) {
                 // rows split evenly over the patch's items of this column block
@@ -245,8 +243,8 @@ k_adjoint_mma(const wt_patch* __restrict__ patches, HmDev hm, const float* __res
                 it.nwaves = nw;
                 it.first = first;
                 it.out0 = out + (uint64_t)r0 * cols;
+                write_inverses(it.inv, scales);
                 it.rec0 = part_off[q] + (uint64_t)lt * nw;
-                it.inv_scale = pow2f(-ex);
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(&sh.item_full[slot]);
@@ -478,7 +476,6 @@ k_adjoint_mma(const wt_patch* __restrict__ patches, HmDev hm, const float* __res
             const uint32_t nrows = it.nrows, cols = it.cols, row0 = it.row0;
             if (nrows == 0) break;
             const PatchAux a = it.aux;
-            const float inv_scale = it.inv_scale;
             const uint32_t col = it.c0 + cl;
             const float u = (float)col * a.inv_cm1;
             const float xc = (float)col * (a.e1x * a.inv_cm1), zc = (float)col * (a.e1z * a.inv_cm1);
@@ -523,6 +520,7 @@ k_adjoint_mma(const wt_patch* __restrict__ patches, HmDev hm, const float* __res
                         for (uint32_t i = 0; i < kEach; ++i) tmem_ld8(acc + 8u * (r1 - r0 + group + kVert / 4u * i), g[i]);
                         tmem_wait(g[0], g[1]);
                     }
+                    const float4 i0 = it.inv[0], i1 = it.inv[1];
 #pragma unroll
                     for (uint32_t i = 0; i < kEach; ++i) {
                         const uint32_t r = r1 + group + kVert / 4u * i;
@@ -530,8 +528,7 @@ k_adjoint_mma(const wt_patch* __restrict__ patches, HmDev hm, const float* __res
                         // (the forward's accumulator order: dx, dz, jx, jz, dy, sxx, sxz, szz)
                         const VertexSums sm =
                             SAVED ? VertexSums{f[0], f[1], f[2], f[3], f[4], f[5], f[6], f[7]}
-                                  : VertexSums{f[0] * inv_scale, f[4] * inv_scale, f[1] * inv_scale, f[2] * inv_scale,
-                                               f[3] * inv_scale, f[5] * inv_scale, f[6] * inv_scale, f[7] * inv_scale};
+                                  : scaled_sums(f, i0, i1);
                         const float vv = (float)(row0 + r) * a.inv_rm1;
                         vertex_adjoint(sm, fmaf(vv, a.e2x, xc), fmaf(vv, a.e2z, zc), a, hm, pow2, gp[i], gn[i], gnrm != nullptr,
                                        g[i]);

@@ -33,7 +33,7 @@ struct Item {
     uint64_t out0;  // output index of (row0, column 0)
     uint32_t cols, c0, row0, nrows;
     uint32_t nwaves;
-    float inv_scale;
+    float4 inv[2];  // the sums' inverse scales
 };
 
 struct Shared {
@@ -122,14 +122,13 @@ k_forward_mma(const wt_patch* __restrict__ patches, HmDev hm, float* __restrict_
             const PatchAux& pa = aux[p];
             const uint32_t first = pa.pair_offset;
             if (lane < 16) reinterpret_cast<uint32_t*>(&it.aux)[lane] = reinterpret_cast<const uint32_t*>(&pa)[lane];
-            float m = 0.0f;
+            PerSum m{};
 #pragma unroll
             for (uint32_t c = 0; c < 4; ++c)
                 if (32u * c + lane < nw) {
-                    m = coef_max(m, coef[4ull * (first + 32u * c + lane) + 2]);
-                    m = coef_max(m, coef[4ull * (first + 32u * c + lane) + 3]);
+                    max8(m, coef[4ull * (first + 32u * c + lane) + 2], coef[4ull * (first + 32u * c + lane) + 3]);
                 }
-            const int ex = scale_exponent(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
+            const PerSum scales = warp_scales(m);
             const uint32_t pad = min((nw + 7u) & ~7u, kMmaMaxWaves);  // zero waves up to a multiple of 8
 #pragma unroll 2
             for (uint32_t i = lane; i < pad; i += 32u) {
@@ -137,7 +136,7 @@ k_forward_mma(const wt_patch* __restrict__ patches, HmDev hm, float* __restrict_
 #pragma unroll
                 for (uint32_t e = 0; e < 4; ++e)
                     v[e] = i < nw ? coef[4ull * (first + i) + e] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                table_entry(sh.table[slot], i, v, pow2f(ex));
+                table_entry(sh.table[slot], i, v, scales);
             }
             if (lane == 0) {
                 // rows split evenly over the patch's items of this column block
@@ -150,7 +149,7 @@ k_forward_mma(const wt_patch* __restrict__ patches, HmDev hm, float* __restrict_
                 it.nrows = r1 - r0;
                 it.nwaves = nw;
                 it.out0 = out + (uint64_t)r0 * cols;
-                it.inv_scale = pow2f(-ex);
+                write_inverses(it.inv, scales);
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(&sh.item_full[slot]);
@@ -233,7 +232,7 @@ k_forward_mma(const wt_patch* __restrict__ patches, HmDev hm, float* __restrict_
             const uint32_t nrows = it.nrows, rb = tile_rows(it.nwaves);
             if (nrows == 0) break;
             const PatchAux a = it.aux;
-            Tile t{0, it.cols, it.c0, it.row0, it.out0, it.inv_scale, it.nwaves > kOneAccWaves};
+            Tile t{0, it.cols, it.c0, it.row0, it.out0, it.inv, it.nwaves > kOneAccWaves};
             for (uint32_t r0 = 0; r0 < nrows; r0 += rb, ++tile) {
                 ok = warp_wait(&sh.acc_full[tile & 1u], (tile >> 1) & 1u, &sh.fail);
                 if (!ok) break;

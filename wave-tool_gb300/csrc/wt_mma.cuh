@@ -14,13 +14,15 @@
 //
 // FP32 products from FP16 operands: every operand is split into hi + lo
 // (11 + 11 bits) and lo*hi + hi*lo + hi*hi is accumulated in FP32; what is
-// dropped is 2^-24 of the product.  B is scaled by a power of two per patch
-// (its largest coefficient to [2^13, 2^14)) and the sums are scaled back,
-// exactly.  Sines and cosines are formed from the 64-bit fixed-point phases to
-// 1e-7 (the recurrence starts from MUFU's 5e-7).  Each product step truncates
-// the accumulator, a bias of about 2^-25 of it towards zero: above 48 waves
-// the cross products (2^-11 of the whole, two thirds of the steps) get an
-// accumulator of their own.  Relative displacement error against 64 bits on
+// dropped is 2^-24 of the product.  B is scaled by a power of two per patch and
+// sum (the sum's largest coefficient to [2^13, 2^14)) and the sums are scaled
+// back, exactly; a scale for all eight would take bits from those whose
+// coefficients are small beside another's (slopes beside displacements 2^26 as
+// large: normals off by 5e-4, now 1e-7).  Sines and cosines are formed from the
+// 64-bit fixed-point phases to 1e-7 (the recurrence starts from MUFU's 5e-7).
+// Each product step truncates the accumulator, a bias of about 2^-25 of it
+// towards zero: above 48 waves the cross products (2^-11 of the whole, two
+// thirds of the steps) get an accumulator of their own.  Relative displacement error against 64 bits on
 // 700 x 600 vertices, recurrence / products: 8 waves 3.0e-7 / 0.9e-7, 32 waves
 // 2.2e-7 / 1.2e-7, 48 waves 4.7e-7 / 2.0e-7, 64 waves 2.8e-7 / 1.9e-7, 128
 // waves 3.8e-7 / 3.2e-7 (7.3e-7 with one accumulator).
@@ -158,26 +160,53 @@ __device__ __forceinline__ uint32_t stage_offset(uint32_t rb, uint32_t stage) {
     return (rb == 32u ? 2u : 4u) * kSlotA + stage * (2u * rb * kRowB);
 }
 
-// Power of two that takes the largest coefficient (bits mb of its magnitude) to
-// [2^13, 2^14): fp16 keeps the low parts of coefficients down to 2^-27 of it
-// normal.
+// Power of two that takes a sum's largest coefficient (bits mb of its magnitude)
+// to [2^13, 2^14): fp16's hi + lo then hold every coefficient of the sum to 2^-22
+// of itself or 2^-38 of the largest, whichever is more.
 __device__ __forceinline__ int scale_exponent(uint32_t mb) {
     return mb == 0u ? 0 : min(max(13 - ((int)(mb >> 23) - 127), -110), 110);
 }
 __device__ __forceinline__ float pow2f(int e) { return __uint_as_float((uint32_t)(127 + e) << 23); }
 
-__device__ __forceinline__ float coef_max(float m, const float4& a) {
-    return fmaxf(fmaxf(m, fmaxf(fabsf(a.x), fabsf(a.y))), fmaxf(fabsf(a.z), fabsf(a.w)));
+// A value for each of the eight sums, in the order of PairCoef's coefficients.
+struct PerSum {
+    float4 a, b;
+};
+__device__ __forceinline__ void max8(PerSum& m, const float4& a, const float4& b) {
+    const auto max4 = [](float4& m, const float4& v) {
+        m = make_float4(fmaxf(m.x, fabsf(v.x)), fmaxf(m.y, fabsf(v.y)), fmaxf(m.z, fabsf(v.z)), fmaxf(m.w, fabsf(v.w)));
+    };
+    max4(m.a, a);
+    max4(m.b, b);
+}
+// A patch's scales from its largest coefficients, by a whole warp whose lanes share them out.
+__device__ __forceinline__ float warp_scale(float v) {
+    return pow2f(scale_exponent(__reduce_max_sync(0xffffffffu, __float_as_uint(v))));
+}
+__device__ __forceinline__ PerSum warp_scales(const PerSum& m) {
+    return PerSum{make_float4(warp_scale(m.a.x), warp_scale(m.a.y), warp_scale(m.a.z), warp_scale(m.a.w)),
+                  make_float4(warp_scale(m.b.x), warp_scale(m.b.y), warp_scale(m.b.z), warp_scale(m.b.w))};
+}
+// Their inverses in the accumulators' order (the cosine sums dx, dz, jx, jz, then
+// dy, sxx, sxz, szz), for scaled_sums.
+__device__ __forceinline__ void write_inverses(float4 (&inv)[2], const PerSum& s) {
+    const auto of = [](float scale) { return __uint_as_float((254u << 23) - __float_as_uint(scale)); };
+    inv[0] = make_float4(of(s.a.x), of(s.a.z), of(s.a.w), of(s.b.x));
+    inv[1] = make_float4(of(s.a.y), of(s.b.y), of(s.b.z), of(s.b.w));
+}
+// A vertex's sums from its accumulators and their inverse scales.
+__device__ __forceinline__ VertexSums scaled_sums(const float (&f)[8], const float4& i0, const float4& i1) {
+    return VertexSums{f[0] * i0.x, f[4] * i1.x, f[1] * i0.y, f[2] * i0.z, f[3] * i0.w, f[5] * i1.y, f[6] * i1.z, f[7] * i1.w};
 }
 
 // Wave i's entry: c = its PairCoef as four float4.
-__device__ __forceinline__ void table_entry(Table& T, uint32_t i, const float4 (&c)[4], float scale) {
+__device__ __forceinline__ void table_entry(Table& T, uint32_t i, const float4 (&c)[4], const PerSum& s) {
     const uint32_t at = (i & ~31u) + ((i & 31u) >> 1) + 16u * (i & 1u);
     const uint4 u0 = *reinterpret_cast<const uint4*>(&c[0]), u1 = *reinterpret_cast<const uint4*>(&c[1]);
     T.y[at] = make_ulonglong2(((unsigned long long)u0.y << 32) | u0.x, ((unsigned long long)u1.y << 32) | u1.x);
     T.x[i] = ((unsigned long long)u0.w << 32) | u0.z;
-    T.k0[at] = make_float4(c[2].x * scale, c[2].z * scale, c[2].w * scale, c[3].x * scale);
-    T.k1[at] = make_float4(c[2].y * scale, c[3].y * scale, c[3].z * scale, c[3].w * scale);
+    T.k0[at] = make_float4(c[2].x * s.a.x, c[2].z * s.a.z, c[2].w * s.a.w, c[3].x * s.b.x);
+    T.k1[at] = make_float4(c[2].y * s.a.y, c[3].y * s.b.y, c[3].z * s.b.z, c[3].w * s.b.w);
 }
 
 // A of the 128 columns from c0, by `warps` warps: a thread forms four waves of
@@ -290,7 +319,7 @@ struct Tile {
     uint32_t acc;                // its accumulators
     uint32_t cols, c0, row0;     // the patch's columns; columns from c0, rows from row0
     uint64_t out0;               // output index of (row0, column 0)
-    float inv_scale;
+    const float4* inv;           // the sums' inverse scales
     bool two_acc;
 };
 struct Output {
@@ -363,7 +392,7 @@ __device__ __forceinline__ void tile_epilogue(const Tile& t, const PatchAux& a, 
     const uint32_t at = t.acc + ((32u * quad) << 16);
     const uint64_t v0 = t.out0 + col;
     const bool in = col < t.cols;
-    const float inv_scale = t.inv_scale;
+    const float4 i0 = t.inv[0], i1 = t.inv[1];
     float rowf = (float)(t.row0 + first);
     // two rows at a time: their texel loads are issued before the first is used
     // (four rows by one wider load: 394 against 386 us on 256 patches, in
@@ -396,8 +425,7 @@ __device__ __forceinline__ void tile_epilogue(const Tile& t, const PatchAux& a, 
             rowf += (float)step;
             xl[u] = fmaf(vv, a.e2x, xc);
             zl[u] = fmaf(vv, a.e2z, zc);
-            v[u] = VertexSums{f[u][0] * inv_scale, f[u][4] * inv_scale, f[u][1] * inv_scale, f[u][2] * inv_scale,
-                              f[u][3] * inv_scale, f[u][5] * inv_scale, f[u][6] * inv_scale, f[u][7] * inv_scale};
+            v[u] = scaled_sums(f[u], i0, i1);
             if (HM != 0) T[u] = hm_fetch<HM == 1>(hm, a, xl[u] + v[u].dx, zl[u] + v[u].dz, pow2);
             else T[u] = HmTexels{};
         }

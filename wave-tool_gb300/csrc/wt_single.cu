@@ -51,6 +51,8 @@ struct Products {
     mma::Table table;
     unsigned long long full[2], done[2];          // a step's operands are written / its products complete
     unsigned long long acc_full[2], acc_free[2];  // a tile's sums are complete / read
+    mma::PerSum scales;
+    float4 inv[2];  // their inverses
     uint32_t tmem;
     int fail;
 };
@@ -93,17 +95,20 @@ __device__ __forceinline__ bool run_products(Single& sh, Products& pr, char* op,
     const uint32_t cols = sh.patch.cols, rows = sh.patch.rows, ct = (cols + 127u) / 128u;
     const uint32_t ni = items_per_block(rows, ct, nw, gridDim.x);
     if (blockIdx.x >= ct * ni) return true;
-    // the wave table; every warp finds the scale itself
+    // the scales, a sum a warp, and the wave table
+    if (warp < 8) {
+        float m = 0.0f;
+        for (uint32_t i = lane; i < nw; i += 32u) m = fmaxf(m, fabsf((&sh.coef[i].qadx)[warp]));
+        const float scale = warp_scale(m);
+        if (lane == 0) (&pr.scales.a.x)[warp] = scale;
+    }
+    __syncthreads();
     const float4* coef = reinterpret_cast<const float4*>(sh.coef);
-    float m = 0.0f;
-    for (uint32_t i = lane; i < nw; i += 32u) m = coef_max(coef_max(m, coef[4u * i + 2u]), coef[4u * i + 3u]);
-    const int ex = scale_exponent(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
-    const float inv_scale = pow2f(-ex);
     if (tid < ((nw + 7u) & ~7u)) {
         float4 v[4];
 #pragma unroll
         for (uint32_t e = 0; e < 4; ++e) v[e] = tid < nw ? coef[4u * tid + e] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        table_entry(pr.table, tid, v, pow2f(ex));
+        table_entry(pr.table, tid, v, pr.scales);
     }
     if (tid == 0) {
         for (uint32_t i = 0; i < 2; ++i) {
@@ -113,6 +118,7 @@ __device__ __forceinline__ bool run_products(Single& sh, Products& pr, char* op,
             mbar_init(&pr.acc_free[i], kEpi);
         }
         pr.fail = 0;
+        write_inverses(pr.inv, pr.scales);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kWarps - 1) tmem_alloc(&pr.tmem);
@@ -187,7 +193,7 @@ __device__ __forceinline__ bool run_products(Single& sh, Products& pr, char* op,
         const uint32_t quad = warp & 3u;
         for (uint32_t item = blockIdx.x; item < items && ok; item += gridDim.x) {
             const uint32_t cb = item / ni, ri = item - cb * ni, i0 = first_row(ri), i1 = first_row(ri + 1u);
-            Tile t{0, cols, 128u * cb, i0, sh.patch.out_offset + (uint64_t)i0 * cols, inv_scale, nw > kOneAccWaves};
+            Tile t{0, cols, 128u * cb, i0, sh.patch.out_offset + (uint64_t)i0 * cols, pr.inv, nw > kOneAccWaves};
             for (uint32_t r0 = i0; r0 < i1; r0 += rb, ++tile) {
                 ok = warp_wait(&pr.acc_full[tile & 1u], (tile >> 1) & 1u, &pr.fail);
                 if (!ok) break;
