@@ -121,3 +121,27 @@ def test_slopes_beside_large_displacements(wt, oracle, gpu, far, alone):
     _, disp64, nrm64, _ = oracle.displace_f64(table, waves, None, None)
     assert rel_err(pos[:, :3].double().cpu().numpy(), disp64) <= 1e-5
     assert np.radians(angle_deg(nrm[:, :3].double().cpu().numpy(), nrm64)).max() <= 5.4e-7
+
+
+# What the accumulators' truncation takes from the sums on average (a part of
+# them), in units of 2^-25: half of the steps' count in any order of the waves is
+# given back, rounded to 2^-23 (so to 2 of these units).  Left are, in no order, that rounding and a quarter of the loss;
+# with the largest waves first the other half of it too (128 waves: 16 steps).
+@pytest.mark.parametrize("n,order,units", [(48, 0, 2 + 6.2 / 4), (64, 0, 2 + 4.5 / 4), (128, 0, 2 + 8.5 / 4),
+                                           (128, -1, 2 + 16 - 8.5), (128, 1, 2 + 8.5)])
+def test_sums_are_not_short(wt, oracle, gpu, n, order, units):
+    import torch
+    from wave_tool_gb300 import workloads
+    bias = []
+    for seed in range(4):
+        rng = workloads.SplitMix64(500 + seed)
+        waves = np.array(workloads.waves_wide(rng, n), dtype=wt.WAVE_DTYPE)
+        if order:
+            waves = waves[np.argsort(order * waves["amplitude"])]
+        table = np.array([((-70.0, 50.0), (70.0, 50.0), (-70.0, -50.0), (70.0, -50.0), 300, 200, 0, n, 100.0, 0.0, 0, 0)],
+                         dtype=wt.PATCH_DTYPE)
+        pos, _ = wt.Surface(table, waves).displace(flags=1)
+        torch.cuda.synchronize()
+        _, disp64, _, _ = oracle.displace_f64(table, waves, None, None)
+        bias.append(float(((pos[:, :3].double().cpu().numpy() - disp64) * disp64).sum() / (disp64 * disp64).sum()))
+    assert abs(np.mean(bias)) <= units * 2.0**-25

@@ -243,7 +243,7 @@ k_adjoint_mma(const wt_patch* __restrict__ patches, HmDev hm, const float* __res
                 it.nwaves = nw;
                 it.first = first;
                 it.out0 = out + (uint64_t)r0 * cols;
-                write_inverses(it.inv, scales);
+                write_inverses(it.inv, scales, mean_loss(nw, false));
                 it.rec0 = part_off[q] + (uint64_t)lt * nw;
             }
             __syncwarp();

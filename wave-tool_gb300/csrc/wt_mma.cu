@@ -149,7 +149,7 @@ k_forward_mma(const wt_patch* __restrict__ patches, HmDev hm, float* __restrict_
                 it.nrows = r1 - r0;
                 it.nwaves = nw;
                 it.out0 = out + (uint64_t)r0 * cols;
-                write_inverses(it.inv, scales);
+                write_inverses(it.inv, scales, mean_loss(nw, nw > kOneAccWaves));
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(&sh.item_full[slot]);

@@ -22,10 +22,13 @@
 // 64-bit fixed-point phases to 1e-7 (the recurrence starts from MUFU's 5e-7).
 // Each product step truncates the accumulator, a bias of about 2^-25 of it
 // towards zero: above 48 waves the cross products (2^-11 of the whole, two
-// thirds of the steps) get an accumulator of their own.  Relative displacement error against 64 bits on
-// 700 x 600 vertices, recurrence / products: 8 waves 3.0e-7 / 0.9e-7, 32 waves
-// 2.2e-7 / 1.2e-7, 48 waves 4.7e-7 / 2.0e-7, 64 waves 2.8e-7 / 1.9e-7, 128
-// waves 3.8e-7 / 3.2e-7 (7.3e-7 with one accumulator).
+// thirds of the steps) get an accumulator of their own, and above 32 the mean of
+// what is lost is given back in the inverse scales (mean_loss; 128 waves were
+// short by 2.6e-7 without it, 4.8e-7 with the largest waves first).  Relative
+// displacement error (2-norm) against 64 bits on 500 x 400 vertices, mean of six
+// tables, recurrence / products: 8 waves 2.9e-7 / 0.9e-7, 32 waves 3.3e-7 /
+// 1.3e-7, 48 waves 3.1e-7 / 1.9e-7, 64 waves 3.1e-7 / 1.4e-7, 128 waves 3.9e-7 /
+// 2.2e-7, and with the largest waves first 4.0e-7 / 3.2e-7.
 //
 // A step is 32 waves (64 fp16: one 128-byte row) of one tile: 128 columns by
 // 32 rows (above 48 waves 16).  A stays in shared memory for a run of rows, B
@@ -187,16 +190,32 @@ __device__ __forceinline__ PerSum warp_scales(const PerSum& m) {
     return PerSum{make_float4(warp_scale(m.a.x), warp_scale(m.a.y), warp_scale(m.a.z), warp_scale(m.a.w)),
                   make_float4(warp_scale(m.b.x), warp_scale(m.b.y), warp_scale(m.b.z), warp_scale(m.b.w))};
 }
-// Their inverses in the accumulators' order (the cosine sums dx, dz, jx, jz, then
-// dy, sxx, sxz, szz), for scaled_sums.
-__device__ __forceinline__ void write_inverses(float4 (&inv)[2], const PerSum& s) {
-    const auto of = [](float scale) { return __uint_as_float((254u << 23) - __float_as_uint(scale)); };
+// The mean of what truncation takes from the sums of nw waves, as a part of them:
+// about 2^-25 of the partial sum at each step that adds to it, which are the
+// leading products (with one accumulator also the second chunk's cross products),
+// and the partial sums of waves in no order are as far as the waves added so far.
+// Up to a chunk it is less than FP32 holds beside 1.
+__device__ __forceinline__ float mean_loss(uint32_t nw, bool two_acc) {
+    if (nw <= kChunk) return 0.0f;
+    const float steps = (float)((nw + 7u) / 8u), first = (float)(kChunk / 8u);
+    return 0x1p-25f * (0.5f * (steps + 1.0f) + (two_acc ? 0.0f : 2.0f * (steps - first) * first / steps));
+}
+// The scales' inverses, with the mean loss given back, in the accumulators' order
+// (the cosine sums dx, dz, jx, jz, then dy, sxx, sxz, szz), for scaled_sums.
+__device__ __forceinline__ void write_inverses(float4 (&inv)[2], const PerSum& s, float loss) {
+    const auto of = [&](float scale) {
+        const float i = __uint_as_float((254u << 23) - __float_as_uint(scale));
+        return fmaf(i, loss, i);
+    };
     inv[0] = make_float4(of(s.a.x), of(s.a.z), of(s.a.w), of(s.b.x));
     inv[1] = make_float4(of(s.a.y), of(s.b.y), of(s.b.z), of(s.b.w));
 }
-// A vertex's sums from its accumulators and their inverse scales.
+// A vertex's sums from its accumulators and their inverse scales (no power of two
+// above 32 waves: rounded here, whatever follows, so that every mode has the same
+// bits).
 __device__ __forceinline__ VertexSums scaled_sums(const float (&f)[8], const float4& i0, const float4& i1) {
-    return VertexSums{f[0] * i0.x, f[4] * i1.x, f[1] * i0.y, f[2] * i0.z, f[3] * i0.w, f[5] * i1.y, f[6] * i1.z, f[7] * i1.w};
+    return VertexSums{__fmul_rn(f[0], i0.x), __fmul_rn(f[4], i1.x), __fmul_rn(f[1], i0.y), __fmul_rn(f[2], i0.z),
+                      __fmul_rn(f[3], i0.w), __fmul_rn(f[5], i1.y), __fmul_rn(f[6], i1.z), __fmul_rn(f[7], i1.w)};
 }
 
 // Wave i's entry: c = its PairCoef as four float4.

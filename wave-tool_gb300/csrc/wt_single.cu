@@ -118,7 +118,7 @@ __device__ __forceinline__ bool run_products(Single& sh, Products& pr, char* op,
             mbar_init(&pr.acc_free[i], kEpi);
         }
         pr.fail = 0;
-        write_inverses(pr.inv, pr.scales);
+        write_inverses(pr.inv, pr.scales, mean_loss(nw, nw > kOneAccWaves));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kWarps - 1) tmem_alloc(&pr.tmem);
