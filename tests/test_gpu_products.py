@@ -145,3 +145,20 @@ def test_sums_are_not_short(wt, oracle, gpu, n, order, units):
         _, disp64, _, _ = oracle.displace_f64(table, waves, None, None)
         bias.append(float(((pos[:, :3].double().cpu().numpy() - disp64) * disp64).sum() / (disp64 * disp64).sum()))
     assert abs(np.mean(bias)) <= units * 2.0**-25
+
+
+@pytest.mark.parametrize("alone", [True, False])
+def test_displacements_of_a_patch_wider_than_float(wt, gpu, alone):
+    """The displacement does not depend on where the grid point is: finite on a
+    patch whose sides overflow FP32, as large as its waves at most."""
+    import torch
+    from wave_tool_gb300 import workloads
+    waves = np.array(workloads.waves_wide(workloads.SplitMix64(3), 9), dtype=wt.WAVE_DTYPE)
+    h = 3.0e38
+    one = np.array([((-h, h), (h, h), (-h, -h), (h, -h), 70, 40, 0, 9, 1.0, 0.0, 0, 0)], dtype=wt.PATCH_DTYPE)
+    table = one if alone else np.concatenate([one, one])
+    table["out_offset"][1:] = 70 * 40
+    pos, _ = wt.Surface(table, waves).displace(flags=1)
+    assert bool(torch.isfinite(pos).all())
+    most = float(np.abs(waves["amplitude"] * np.maximum(1.0, waves["steepness_q"])).sum())
+    assert float(pos[:, :3].abs().max()) <= most

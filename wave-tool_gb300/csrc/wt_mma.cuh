@@ -350,14 +350,14 @@ struct Output {
     uint32_t flags;
 };
 
-// One vertex from its sums and texels (world or displaced position without a
-// branch: keep is 1 or 0, bx / bz the corner or 0).  Roundings spelt out where
+// One vertex from its sums and texels (world: the position in the world, else the
+// displacement alone, whatever the grid point: a patch may span more than FP32's
+// largest number).  Roundings spelt out where
 // a multiply-add could be fused one way in one output mode and another way in
 // the next: every mode writes the same bits.
 template <int MODE, int HM>
-__device__ __forceinline__ void finish(const VertexSums& s, float xl, float zl, float keep, float bx, float bz,
-                                       const PatchAux& a, const HmDev& hm, const HmTexels& T, uint64_t v,
-                                       const Output& o) {
+__device__ __forceinline__ void finish(const VertexSums& s, float xl, float zl, bool world, const PatchAux& a,
+                                       const HmDev& hm, const HmTexels& T, uint64_t v, const Output& o) {
     if (MODE == kModeSave) {
         __stcs(o.sums + 2 * v, make_float4(s.dx, s.dy, s.dz, s.jx));
         __stcs(o.sums + 2 * v + 1, make_float4(s.jz, s.sxx, s.sxz, s.szz));
@@ -371,7 +371,8 @@ __device__ __forceinline__ void finish(const VertexSums& s, float xl, float zl, 
         pz1 = fmaf(g.hx, pz0, fmaf(g.hz, pz2, pz1));
     }
     dy = __fadd_rn(dy, a.y_offset);
-    const float ox = bx + fmaf(keep, xl, s.dx), oz = bz + fmaf(keep, zl, s.dz);
+    const float ox = world ? __fadd_rn(a.blx, __fadd_rn(xl, s.dx)) : s.dx;
+    const float oz = world ? __fadd_rn(a.blz, __fadd_rn(zl, s.dz)) : s.dz;
     float n0 = fmaf(pz1, px2, -__fmul_rn(pz2, px1)), n1 = fmaf(pz2, px0, -__fmul_rn(pz0, px2)),
           n2 = fmaf(pz0, px1, -__fmul_rn(pz1, px0));
     const float inv = rsqrtf(fmaf(n0, n0, fmaf(n1, n1, n2 * n2)));
@@ -388,7 +389,7 @@ __device__ __forceinline__ void finish(const VertexSums& s, float xl, float zl, 
             __stcs(N, n0); __stcs(N + 1, n1); __stcs(N + 2, n2);
         }
     } else {
-        if (MODE != kModeStage || o.pos) __stcs(reinterpret_cast<float4*>(o.pos) + v, make_float4(ox, dy, oz, keep));
+        if (MODE != kModeStage || o.pos) __stcs(reinterpret_cast<float4*>(o.pos) + v, make_float4(ox, dy, oz, world ? 1.0f : 0.0f));
         if (o.nrm) __stcs(reinterpret_cast<float4*>(o.nrm) + v, make_float4(n0, n1, n2, 0.0f));
     }
     if (MODE == kModeStage) stage_vertex<false>(o.view, make_float3(ox, dy, oz), make_float3(n0, n1, n2), v, o.so);
@@ -403,8 +404,7 @@ __device__ __forceinline__ void tile_epilogue(const Tile& t, const PatchAux& a, 
                                               const Output& o, uint32_t quad, uint32_t lane, uint32_t first,
                                               uint32_t step, uint32_t rt) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const float keep = o.flags & WT_OUT_DISPLACEMENT ? 0.0f : 1.0f;
-    const float bx = o.flags & WT_OUT_DISPLACEMENT ? 0.0f : a.blx, bz = o.flags & WT_OUT_DISPLACEMENT ? 0.0f : a.blz;
+    const bool world = !(o.flags & WT_OUT_DISPLACEMENT);
     const float gx = a.e1x * a.inv_cm1, gz = a.e1z * a.inv_cm1;
     const uint32_t col = t.c0 + 32u * quad + lane;
     const float xc = (float)col * gx, zc = (float)col * gz;
@@ -449,8 +449,8 @@ __device__ __forceinline__ void tile_epilogue(const Tile& t, const PatchAux& a, 
             else T[u] = HmTexels{};
         }
         if (in) {
-            finish<MODE, HM>(v[0], xl[0], zl[0], keep, bx, bz, a, hm, T[0], v0 + r * t.cols, o);
-            if (second) finish<MODE, HM>(v[1], xl[1], zl[1], keep, bx, bz, a, hm, T[1], v0 + (r + step) * t.cols, o);
+            finish<MODE, HM>(v[0], xl[0], zl[0], world, a, hm, T[0], v0 + r * t.cols, o);
+            if (second) finish<MODE, HM>(v[1], xl[1], zl[1], world, a, hm, T[1], v0 + (r + step) * t.cols, o);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
