@@ -84,6 +84,7 @@ struct Shared {
     unsigned long long d_full[2], d_free[2];       // D complete / read
     unsigned long long a_full, drained;            // an item's E written / its last product complete
     unsigned long long item_full[kRing], item_free[kRing];
+    unsigned long long last;                       // all products issued are complete
     uint32_t tmem;
     int fail;
 };
@@ -111,7 +112,7 @@ template <bool SAVED>
 __global__ void __launch_bounds__(kThreads, 1)
 k_adjoint_mma(const wt_patch* __restrict__ patches, HmDev hm, const float* __restrict__ gpos,
               const float* __restrict__ gnrm, uint32_t flags, char* __restrict__ ws, AdjLayout L,
-              const float4* __restrict__ sums, uint32_t wide) {
+              const float4* __restrict__ sums, uint32_t wide, unsigned long long limit_ns) {
     cudaTriggerProgrammaticLaunchCompletion();  // the next kernel waits for this one's end
     cudaGridDependencySynchronize();
     WsHeader* hdr = reinterpret_cast<WsHeader*>(ws);
@@ -142,7 +143,8 @@ k_adjoint_mma(const wt_patch* __restrict__ patches, HmDev hm, const float* __res
             mbar_init(&sh.item_free[i], kVert + kSums + kProd + 1);
         }
         for (uint32_t i = 0; i < 8; ++i) (&sh.top[0][0])[i] = make_uint4(0, 0, 0, 0);
-        sh.fail = 0;
+        mbar_init(&sh.last, 1);
+        sh.fail = limit_ns == 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kQueue) tmem_alloc(&sh.tmem);
@@ -151,6 +153,7 @@ k_adjoint_mma(const wt_patch* __restrict__ patches, HmDev hm, const float* __res
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = sh.tmem;          // columns 0-127 and 128-255: the forward's sums; 256-383, 384-511: D
     const uint32_t op_s = smem_u32(op);
+    const Limit limit{&sh.fail, limit_ns};
 
     if (warp == kQueue) {
         // ---- the queue: items and their wave tables; the sines of an item's rows
@@ -167,7 +170,7 @@ k_adjoint_mma(const wt_patch* __restrict__ patches, HmDev hm, const float* __res
             const uint32_t nrows = it.nrows, nw = it.nwaves, row0 = it.row0;
             const uint32_t lanes = nw > 16u ? 32u : (nw > 8u ? 16u : 8u), each = 32u / lanes;  // of a row; rows at a time
             for (uint32_t r0 = from; r0 < min(nrows, to); r0 += kTileRows, ++tile) {
-                if (tile >= 2u && !warp_wait(&sh.trig_free[tile & 1u], ((tile >> 1) - 1u) & 1u, &sh.fail)) return false;
+                if (tile >= 2u && !warp_wait(&sh.trig_free[tile & 1u], ((tile >> 1) - 1u) & 1u, limit)) return false;
                 const uint32_t rt = min(kTileRows, nrows - r0);
                 for (uint32_t w = lane & (lanes - 1u); w < nw; w += lanes) {
                     const ulonglong2 y = T.y[(w & ~31u) + ((w & 31u) >> 1) + 16u * (w & 1u)];
@@ -192,7 +195,7 @@ k_adjoint_mma(const wt_patch* __restrict__ patches, HmDev hm, const float* __res
             // the last item's first two tiles before the next item, which is not needed
             // as early and may have to wait for its place
             if (k > 0 && !sines((k - 1u) % kRing, 0, 2u * kTileRows)) break;
-            if (k >= kRing && !warp_wait(&sh.item_free[slot], (k / kRing - 1u) & 1u, &sh.fail)) break;
+            if (k >= kRing && !warp_wait(&sh.item_free[slot], (k / kRing - 1u) & 1u, limit)) break;
             Item& it = sh.item[slot];
             if (t >= n_items) {
                 if (lane == 0) {
@@ -258,21 +261,21 @@ k_adjoint_mma(const wt_patch* __restrict__ patches, HmDev hm, const float* __res
             bool ok = true;
             for (uint32_t k = 0; ok; ++k) {
                 const uint32_t slot = k % kRing;
-                ok = mbar_wait(&sh.item_full[slot], (k / kRing) & 1u, &sh.fail);
+                ok = mbar_wait(&sh.item_full[slot], (k / kRing) & 1u, limit);
                 if (!ok) break;
                 const Item& it = sh.item[slot];
                 const uint32_t nrows = it.nrows, nw = it.nwaves;
                 if (nrows == 0) break;
-                ok = mbar_wait(&sh.a_full, k & 1u, &sh.fail);
+                ok = mbar_wait(&sh.a_full, k & 1u, limit);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 // the forward's products of one tile (one accumulator: at most 64 waves)
                 const auto forward = [&](uint32_t rt) {
-                    if (tile >= 2u) ok = mbar_wait(&sh.acc_free[tile & 1u], ((tile >> 1) - 1u) & 1u, &sh.fail);
+                    if (tile >= 2u) ok = mbar_wait(&sh.acc_free[tile & 1u], ((tile >> 1) - 1u) & 1u, limit);
                     const uint32_t d = tmem + (tile & 1u) * 128u, rn = (rt + 1u) & ~1u;
                     const uint32_t idesc = (1u << 4) | (rn << 17) | ((128u / 16u) << 24);
                     for (uint32_t ch = 0; ch * kChunk < nw && ok; ++ch, ++s) {
-                        ok = mbar_wait(&sh.full[s & 1u], (s >> 1) & 1u, &sh.fail);
+                        ok = mbar_wait(&sh.full[s & 1u], (s >> 1) & 1u, limit);
                         if (!ok) break;
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         const uint32_t ks = (min(kChunk, nw - ch * kChunk) + 7u) / 8u;
@@ -297,9 +300,9 @@ k_adjoint_mma(const wt_patch* __restrict__ patches, HmDev hm, const float* __res
                 for (uint32_t r0 = 0; r0 < nrows && ok; r0 += kTileRows) {
                     if (!SAVED && r0 + kTileRows < nrows) forward(min(kTileRows, nrows - r0 - kTileRows));
                     for (uint32_t r = r0; r < min(r0 + kTileRows, nrows) && ok; r += kHalf, ++half) {
-                        if (half >= 2u) ok = mbar_wait(&sh.d_free[half & 1u], ((half >> 1) - 1u) & 1u, &sh.fail);
+                        if (half >= 2u) ok = mbar_wait(&sh.d_free[half & 1u], ((half >> 1) - 1u) & 1u, limit);
                         const uint32_t d = tmem + 256u + (half & 1u) * 128u;
-                        if (ok) ok = mbar_wait(&sh.g_full, half & 1u, &sh.fail);
+                        if (ok) ok = mbar_wait(&sh.g_full, half & 1u, limit);
                         if (!ok) break;
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         // 16 columns: 2048 bytes on; cross products first
@@ -312,13 +315,8 @@ k_adjoint_mma(const wt_patch* __restrict__ patches, HmDev hm, const float* __res
                 }
                 commit(&sh.drained);
                 mbar_arrive(&sh.item_free[slot]);
-                // the products in flight complete before the block's memory goes
-                // (a wait of its own: a failure elsewhere does not end it)
-                if (!ok) {
-                    int late = 0;
-                    mbar_wait(&sh.drained, k & 1u, &late);
-                }
             }
+            drain(&sh.last, &sh.fail);
         }
         __syncwarp();
     } else if (warp >= kProd0) {
@@ -328,7 +326,7 @@ k_adjoint_mma(const wt_patch* __restrict__ patches, HmDev hm, const float* __res
         bool ok = true;
         for (uint32_t k = 0; ok; ++k) {
             const uint32_t slot = k % kRing;
-            ok = warp_wait(&sh.item_full[slot], (k / kRing) & 1u, &sh.fail);
+            ok = warp_wait(&sh.item_full[slot], (k / kRing) & 1u, limit);
             if (!ok) break;
             const Item& it = sh.item[slot];
             const Table& T = sh.table[slot];
@@ -337,7 +335,7 @@ k_adjoint_mma(const wt_patch* __restrict__ patches, HmDev hm, const float* __res
             const auto rows_b = [&](uint32_t r0) {
                 for (uint32_t w0 = 0; w0 < nw; w0 += kChunk, ++s) {
                     // the stage: its products of two steps ago are complete
-                    if (s >= 2u) ok = warp_wait(&sh.done[s & 1u], ((s - 2u) >> 1) & 1u, &sh.fail);
+                    if (s >= 2u) ok = warp_wait(&sh.done[s & 1u], ((s - 2u) >> 1) & 1u, limit);
                     if (!ok) return;
                     write_b<kTileRows>(op_s + kOffB + (s & 1u) * kStageB, T, nw, w0, row0 + r0, min(kTileRows, nrows - r0), pw, kProd,
                                        lane, dealt);
@@ -348,7 +346,7 @@ k_adjoint_mma(const wt_patch* __restrict__ patches, HmDev hm, const float* __res
             };
             if (!SAVED) rows_b(0);
             // the previous item's products no longer read E
-            if (ok && k > 0) ok = warp_wait(&sh.drained, (k - 1u) & 1u, &sh.fail);
+            if (ok && k > 0) ok = warp_wait(&sh.drained, (k - 1u) & 1u, limit);
             if (!ok) break;
             write_a(op, T, nw, it.c0, pw, kProd, lane);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -368,7 +366,7 @@ k_adjoint_mma(const wt_patch* __restrict__ patches, HmDev hm, const float* __res
         bool ok = true;
         for (uint32_t k = 0; ok; ++k) {
             const uint32_t slot = k % kRing;
-            ok = warp_wait(&sh.item_full[slot], (k / kRing) & 1u, &sh.fail);
+            ok = warp_wait(&sh.item_full[slot], (k / kRing) & 1u, limit);
             if (!ok) break;
             const Item& it = sh.item[slot];
             const uint32_t nrows = it.nrows, nw = it.nwaves, row0 = it.row0;
@@ -384,9 +382,9 @@ k_adjoint_mma(const wt_patch* __restrict__ patches, HmDev hm, const float* __res
 #pragma unroll
             for (int i = 0; i < 8; ++i) P[i] = V[i] = U[i] = make_float2(0.0f, 0.0f);
             for (uint32_t r0 = 0; r0 < nrows && ok; r0 += kTileRows, ++tile) {
-                ok = warp_wait(&sh.trig_full[tile & 1u], (tile >> 1) & 1u, &sh.fail);
+                ok = warp_wait(&sh.trig_full[tile & 1u], (tile >> 1) & 1u, limit);
                 for (uint32_t r1 = r0; r1 < min(r0 + kTileRows, nrows) && ok; r1 += kHalf, ++half) {
-                    ok = warp_wait(&sh.d_full[half & 1u], (half >> 1) & 1u, &sh.fail);
+                    ok = warp_wait(&sh.d_full[half & 1u], (half >> 1) & 1u, limit);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t at = tmem + 256u + (half & 1u) * 128u + ((32u * quad) << 16);
@@ -470,7 +468,7 @@ k_adjoint_mma(const wt_patch* __restrict__ patches, HmDev hm, const float* __res
         bool ok = true;
         for (uint32_t k = 0; ok; ++k) {
             const uint32_t slot = k % kRing;
-            ok = warp_wait(&sh.item_full[slot], (k / kRing) & 1u, &sh.fail);
+            ok = warp_wait(&sh.item_full[slot], (k / kRing) & 1u, limit);
             if (!ok) break;
             const Item& it = sh.item[slot];
             const uint32_t nrows = it.nrows, cols = it.cols, row0 = it.row0;
@@ -498,7 +496,7 @@ k_adjoint_mma(const wt_patch* __restrict__ patches, HmDev hm, const float* __res
             const bool writes = it.c0 + 32u * quad < ((cols + 15u) & ~15u);  // columns past the last step of 16 are not read
             for (uint32_t r0 = 0; r0 < nrows && ok; r0 += kTileRows, ++tile) {
                 if (!SAVED) {
-                    ok = warp_wait(&sh.acc_full[tile & 1u], (tile >> 1) & 1u, &sh.fail);
+                    ok = warp_wait(&sh.acc_full[tile & 1u], (tile >> 1) & 1u, limit);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 }
@@ -553,10 +551,10 @@ k_adjoint_mma(const wt_patch* __restrict__ patches, HmDev hm, const float* __res
                     if (lane < 8) atomicMax(reinterpret_cast<uint32_t*>(top) + lane, mine);
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&sh.top_full);
-                    ok = warp_wait(&sh.top_full, half & 1u, &sh.fail);
+                    ok = warp_wait(&sh.top_full, half & 1u, limit);
                     if (!ok) break;
                     // G: the previous half tile's products no longer read it
-                    if (half >= 1u) ok = warp_wait(&sh.g_free, (half - 1u) & 1u, &sh.fail);
+                    if (half >= 1u) ok = warp_wait(&sh.g_free, (half - 1u) & 1u, limit);
                     if (!ok) break;
                     const uint4 t0 = top[0], t1 = top[1];
                     const float f[8] = {scale_of(t0.x), scale_of(t0.y), scale_of(t0.z), scale_of(t0.w),
@@ -634,7 +632,7 @@ cudaError_t launch_t(const wt_patch* patches, const HmDev& hm, const float* gpos
     lc.attrs = attr;
     lc.numAttrs = 1;
     return cudaLaunchKernelEx(&lc, k_adjoint_mma<SAVED>, patches, hm, gpos, gnrm, flags, static_cast<char*>(ws), L,
-                              reinterpret_cast<const float4*>(sums), wide);
+                              reinterpret_cast<const float4*>(sums), wide, wait_limit());
 }
 
 }  // namespace

@@ -177,6 +177,8 @@ wt_status run_displace(const wt_patch* patches, uint32_t n_patches, const wt_wav
 }  // namespace
 
 namespace wt {
+static thread_local unsigned long long t_wait_limit = kWaitNs;
+unsigned long long wait_limit() { return t_wait_limit; }
 void set_last_error(const char* msg) { g_last_error = msg; }
 
 int sm_count() {
@@ -193,6 +195,8 @@ FwdConfig forward_config(uint32_t n_patches, uint32_t n_waves) { return cfg_for(
 }  // namespace wt
 
 extern "C" {
+
+void wt_internal_wait_limit(unsigned long long ns) { wt::t_wait_limit = ns; }
 
 const char* wt_version(void) { return "wave-tool-gb300 0.1 (sm_103a)"; }
 

@@ -160,6 +160,13 @@ inline int hm_kind(const HmDev& hm) {
 // Waves of a patch that runs as matrix products (mma_patch).
 constexpr uint32_t kMmaMinWaves = 8, kMmaMaxWaves = 128, kMmaAdjMaxWaves = 64;
 
+// Limit of every wait inside the matrix-product kernels, in nanoseconds, and the
+// one that this thread's launches are given: tests of what a wait that runs out
+// leaves behind shorten it by the library's wt_internal_wait_limit, which is no part
+// of the ABI (0: every wait has run out from the start).
+constexpr unsigned long long kWaitNs = 2000000000ull;
+unsigned long long wait_limit();
+
 // The adjoint's queue set-up (ranks, chunk and record prefixes), formed by the
 // prep's scan kernel when the prep runs for an adjoint.
 struct AdjScanArgs {

@@ -42,6 +42,7 @@ struct Shared {
     unsigned long long full[2], done[2];          // a step's operands are written / its products complete
     unsigned long long acc_full[2], acc_free[2];  // a tile's sums are complete / read
     unsigned long long item_full[kRing], item_free[kRing];
+    unsigned long long last;                       // all products issued are complete
     uint32_t tmem;
     int fail;
     float view[36];
@@ -53,7 +54,7 @@ template <int MODE, int HM>
 __global__ void __launch_bounds__(kThreads, 1)
 k_forward_mma(const wt_patch* __restrict__ patches, HmDev hm, float* __restrict__ pos, float* __restrict__ nrm,
               uint32_t flags, char* __restrict__ ws, WsLayout L, float4* __restrict__ sums,
-              const wt_view* __restrict__ view, StageOut so) {
+              const wt_view* __restrict__ view, StageOut so, unsigned long long limit_ns) {
     cudaTriggerProgrammaticLaunchCompletion();  // the next kernel waits for this one's end
     cudaGridDependencySynchronize();
     WsHeader* hdr = reinterpret_cast<WsHeader*>(ws);
@@ -75,7 +76,8 @@ k_forward_mma(const wt_patch* __restrict__ patches, HmDev hm, float* __restrict_
             mbar_init(&sh.item_full[i], 1);
             mbar_init(&sh.item_free[i], kEpi + kProd + 1);
         }
-        sh.fail = 0;
+        mbar_init(&sh.last, 1);
+        sh.fail = limit_ns == 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kQueue) tmem_alloc(&sh.tmem);
@@ -84,6 +86,7 @@ k_forward_mma(const wt_patch* __restrict__ patches, HmDev hm, float* __restrict_
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = sh.tmem;
     const uint32_t op_s = smem_u32(op);
+    const Limit limit{&sh.fail, limit_ns};
 
     if (warp == kQueue) {
         // ---- the queue: items and their wave tables
@@ -97,7 +100,7 @@ k_forward_mma(const wt_patch* __restrict__ patches, HmDev hm, float* __restrict_
             const uint32_t slot = k % kRing;
             uint32_t t_next = 0;
             if (t < n_items && lane == 0) t_next = atomicAdd(&hdr->mma_counter, 1u) + gridDim.x;
-            if (k >= kRing && !warp_wait(&sh.item_free[slot], (k / kRing - 1u) & 1u, &sh.fail)) break;
+            if (k >= kRing && !warp_wait(&sh.item_free[slot], (k / kRing - 1u) & 1u, limit)) break;
             Item& it = sh.item[slot];
             if (t >= n_items) {
                 if (lane == 0) {
@@ -162,15 +165,15 @@ k_forward_mma(const wt_patch* __restrict__ patches, HmDev hm, float* __restrict_
             bool ok = true;
             for (uint32_t k = 0; ok; ++k) {
                 const uint32_t slot = k % kRing;
-                ok = mbar_wait(&sh.item_full[slot], (k / kRing) & 1u, &sh.fail);
+                ok = mbar_wait(&sh.item_full[slot], (k / kRing) & 1u, limit);
                 if (!ok) break;
                 const Item& it = sh.item[slot];
                 const uint32_t nrows = it.nrows, nw = it.nwaves, rb = tile_rows(nw);
                 if (nrows == 0) break;
                 for (uint32_t r0 = 0; r0 < nrows && ok; r0 += rb, ++tile) {
-                    if (tile >= 2u) ok = mbar_wait(&sh.acc_free[tile & 1u], ((tile >> 1) - 1u) & 1u, &sh.fail);
+                    if (tile >= 2u) ok = mbar_wait(&sh.acc_free[tile & 1u], ((tile >> 1) - 1u) & 1u, limit);
                     for (uint32_t ch = 0; ch * kChunk < nw && ok; ++ch, ++s) {
-                        ok = mbar_wait(&sh.full[s & 1u], (s >> 1) & 1u, &sh.fail);
+                        ok = mbar_wait(&sh.full[s & 1u], (s >> 1) & 1u, limit);
                         if (!ok) break;
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         issue_step(op_s, tmem + (tile & 1u) * 256u, nw, rb, min(rb, nrows - r0), ch, s & 1u);
@@ -180,11 +183,7 @@ k_forward_mma(const wt_patch* __restrict__ patches, HmDev hm, float* __restrict_
                 }
                 mbar_arrive(&sh.item_free[slot]);
             }
-            // the products in flight complete before the block's memory goes
-            // (waits of their own: a failure elsewhere does not end them)
-            int late = 0;
-            for (uint32_t i = s >= 2u ? s - 2u : 0u; i < s; ++i) mbar_wait(&sh.done[i & 1u], (i >> 1) & 1u, &late);
-            if (late) sh.fail = 1;
+            drain(&sh.last, &sh.fail);
         }
         __syncwarp();
     } else if (warp >= kEpi) {
@@ -193,21 +192,21 @@ k_forward_mma(const wt_patch* __restrict__ patches, HmDev hm, float* __restrict_
         bool ok = true;
         for (uint32_t k = 0; ok; ++k) {
             const uint32_t slot = k % kRing;
-            ok = warp_wait(&sh.item_full[slot], (k / kRing) & 1u, &sh.fail);
+            ok = warp_wait(&sh.item_full[slot], (k / kRing) & 1u, limit);
             if (!ok) break;
             const Item& it = sh.item[slot];
             const Table& T = sh.table[slot];
             const uint32_t nrows = it.nrows, nw = it.nwaves, rb = tile_rows(nw), row0 = it.row0;
             if (nrows == 0) break;
             // the previous item's products no longer read the operands
-            if (s > 0) ok = warp_wait(&sh.done[(s - 1u) & 1u], ((s - 1u) >> 1) & 1u, &sh.fail);
+            if (s > 0) ok = warp_wait(&sh.done[(s - 1u) & 1u], ((s - 1u) >> 1) & 1u, limit);
             if (!ok) break;
             const uint32_t s0 = s;
             write_a(op, T, nw, it.c0, warp - kEpi, kProd, lane);
             for (uint32_t r0 = 0; r0 < nrows && ok; r0 += rb) {
                 for (uint32_t w0 = 0; w0 < nw; w0 += kChunk, ++s) {
                     // the stage: its products of two steps ago are complete
-                    if (s >= s0 + 2u) ok = warp_wait(&sh.done[s & 1u], ((s - 2u) >> 1) & 1u, &sh.fail);
+                    if (s >= s0 + 2u) ok = warp_wait(&sh.done[s & 1u], ((s - 2u) >> 1) & 1u, limit);
                     if (!ok) break;
                     write_b(op_s, s & 1u, rb, T, nw, w0, row0 + r0, min(rb, nrows - r0), warp - kEpi, kProd, lane, dealt);
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -226,7 +225,7 @@ k_forward_mma(const wt_patch* __restrict__ patches, HmDev hm, float* __restrict_
         bool ok = true;
         for (uint32_t k = 0; ok; ++k) {
             const uint32_t slot = k % kRing;
-            ok = warp_wait(&sh.item_full[slot], (k / kRing) & 1u, &sh.fail);
+            ok = warp_wait(&sh.item_full[slot], (k / kRing) & 1u, limit);
             if (!ok) break;
             const Item& it = sh.item[slot];
             const uint32_t nrows = it.nrows, rb = tile_rows(it.nwaves);
@@ -234,7 +233,7 @@ k_forward_mma(const wt_patch* __restrict__ patches, HmDev hm, float* __restrict_
             const PatchAux a = it.aux;
             Tile t{0, it.cols, it.c0, it.row0, it.out0, it.inv, it.nwaves > kOneAccWaves};
             for (uint32_t r0 = 0; r0 < nrows; r0 += rb, ++tile) {
-                ok = warp_wait(&sh.acc_full[tile & 1u], (tile >> 1) & 1u, &sh.fail);
+                ok = warp_wait(&sh.acc_full[tile & 1u], (tile >> 1) & 1u, limit);
                 if (!ok) break;
                 t.acc = tmem + (tile & 1u) * 256u;
                 if (t.c0 + 32u * (warp & 3u) < t.cols)
@@ -280,7 +279,7 @@ cudaError_t launch_mma_t(const wt_patch* patches, const HmDev& hm, float* pos, f
     lc.attrs = attr;
     lc.numAttrs = 1;
     return cudaLaunchKernelEx(&lc, k_forward_mma<MODE, HM>, patches, hm, pos, nrm, flags, static_cast<char*>(ws), L,
-                              reinterpret_cast<float4*>(x.sums), x.view, x.stage);
+                              reinterpret_cast<float4*>(x.sums), x.view, x.stage, wait_limit());
 }
 
 template <int MODE>

@@ -58,7 +58,6 @@ constexpr uint32_t kOneAccWaves = 48;      // above: cross products in an accumu
 constexpr uint32_t kSlotA = 32768;         // a chunk of A: 128 rows x 128 B, hi and lo
 constexpr uint32_t kRowB = 1024;           // a row's eight sums in a chunk of B: 8 x 128 B
 constexpr uint32_t kOperands = 6 * kSlotA; // A (2 or 4 chunks) and two stages of B
-constexpr unsigned long long kWaitNs = 2000000000ull;  // limit of every wait
 
 // The waves of a patch, chunk by chunk; even waves of a chunk first, then odd.
 struct Table {
@@ -76,9 +75,15 @@ __device__ __forceinline__ void mbar_init(unsigned long long* b, uint32_t count)
 __device__ __forceinline__ void mbar_arrive(unsigned long long* b) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(b)) : "memory");
 }
+// What a wait needs besides its barrier: the block's flag that one ran out, and the
+// limit (nanoseconds; 0: it has run out from the start).
+struct Limit {
+    int* fail;
+    unsigned long long ns;
+};
 // Bounded wait for the phase of the given parity; false when it ran out here
 // or in another warp (`fail`).
-__device__ __forceinline__ bool mbar_wait(unsigned long long* b, uint32_t parity, int* fail) {
+__device__ __forceinline__ bool mbar_wait(unsigned long long* b, uint32_t parity, const Limit& limit) {
     const uint32_t a = smem_u32(b);
     unsigned long long t0 = 0, t1 = 0;
     do {
@@ -89,16 +94,16 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* b, uint32_t parity
             : "r"(a), "r"(parity)
             : "memory");
         if (ok) return true;
-        if (*(volatile int*)fail) return false;
+        if (*(volatile int*)limit.fail) return false;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
         if (t0 == 0) t0 = t1;
-    } while (t1 - t0 < kWaitNs);
-    *(volatile int*)fail = 1;
+    } while (t1 - t0 < limit.ns);
+    *(volatile int*)limit.fail = 1;
     return false;
 }
 // The same by a whole warp, with one answer.
-__device__ __forceinline__ bool warp_wait(unsigned long long* b, uint32_t parity, int* fail) {
-    return __all_sync(0xffffffffu, mbar_wait(b, parity, fail));
+__device__ __forceinline__ bool warp_wait(unsigned long long* b, uint32_t parity, const Limit& limit) {
+    return __all_sync(0xffffffffu, mbar_wait(b, parity, limit));
 }
 
 // K-major operand, 128-byte swizzle: rows of 128 B in groups of eight (1024 B).
@@ -305,6 +310,15 @@ __device__ __forceinline__ void write_b(uint32_t op, uint32_t stage, uint32_t rb
 __device__ __forceinline__ void commit(unsigned long long* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
+}
+
+// By the issuing thread when it issues no more, on every path: all its products and
+// their arrivals on barriers are complete before the block's memory goes.  A
+// limit of its own: a wait that ran out elsewhere does not end this one.
+__device__ __forceinline__ void drain(unsigned long long* bar, int* fail) {
+    commit(bar);
+    int late = 0;
+    if (!mbar_wait(bar, 0, Limit{&late, kWaitNs})) *(volatile int*)fail = 1;
 }
 
 // The products of chunk ch (ks steps of 8 waves) of a tile of rt rows.  op: the operands' shared address; acc: the tile's

@@ -51,6 +51,7 @@ struct Products {
     mma::Table table;
     unsigned long long full[2], done[2];          // a step's operands are written / its products complete
     unsigned long long acc_full[2], acc_free[2];  // a tile's sums are complete / read
+    unsigned long long last;                      // all products issued are complete
     mma::PerSum scales;
     float4 inv[2];  // their inverses
     uint32_t tmem;
@@ -89,7 +90,7 @@ __device__ __forceinline__ uint32_t items_per_block(uint32_t rows, uint32_t ct, 
 // A block's items of a parallelogram patch.  Returns false when a wait ran out.
 template <int MODE, int HM>
 __device__ __forceinline__ bool run_products(Single& sh, Products& pr, char* op, uint32_t nw, const HmDev& hm, bool pow2,
-                                             const mma::Output& o) {
+                                             const mma::Output& o, unsigned long long limit_ns) {
     using namespace mma;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t cols = sh.patch.cols, rows = sh.patch.rows, ct = (cols + 127u) / 128u;
@@ -117,7 +118,8 @@ __device__ __forceinline__ bool run_products(Single& sh, Products& pr, char* op,
             mbar_init(&pr.acc_full[i], 1);
             mbar_init(&pr.acc_free[i], kEpi);
         }
-        pr.fail = 0;
+        mbar_init(&pr.last, 1);
+        pr.fail = limit_ns == 0;
         write_inverses(pr.inv, pr.scales, mean_loss(nw, nw > kOneAccWaves));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -137,6 +139,7 @@ __device__ __forceinline__ bool run_products(Single& sh, Products& pr, char* op,
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
     }
+    const Limit limit{&pr.fail, limit_ns};
     uint32_t s = 0, tile = 0;  // steps and tiles
     bool ok = true;
     if (warp == kIssuer) {
@@ -144,9 +147,9 @@ __device__ __forceinline__ bool run_products(Single& sh, Products& pr, char* op,
             for (uint32_t item = blockIdx.x; item < items && ok; item += gridDim.x) {
                 const uint32_t ri = item % ni, i0 = first_row(ri), i1 = first_row(ri + 1u);
                 for (uint32_t r0 = i0; r0 < i1 && ok; r0 += rb, ++tile) {
-                    if (tile >= 2u) ok = mbar_wait(&pr.acc_free[tile & 1u], ((tile >> 1) - 1u) & 1u, &pr.fail);
+                    if (tile >= 2u) ok = mbar_wait(&pr.acc_free[tile & 1u], ((tile >> 1) - 1u) & 1u, limit);
                     for (uint32_t ch = 0; ch < chunks && ok; ++ch, ++s) {
-                        ok = mbar_wait(&pr.full[s & 1u], (s >> 1) & 1u, &pr.fail);
+                        ok = mbar_wait(&pr.full[s & 1u], (s >> 1) & 1u, limit);
                         if (!ok) break;
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         issue_step(op_s, tmem + (tile & 1u) * 256u, nw, rb, min(rb, i1 - r0), ch, s & 1u);
@@ -155,11 +158,7 @@ __device__ __forceinline__ bool run_products(Single& sh, Products& pr, char* op,
                     if (ok) commit(&pr.acc_full[tile & 1u]);
                 }
             }
-            // the products in flight complete before the block's memory goes
-            // (waits of their own: a failure elsewhere does not end them)
-            int late = 0;
-            for (uint32_t i = s >= 2u ? s - 2u : 0u; i < s; ++i) mbar_wait(&pr.done[i & 1u], (i >> 1) & 1u, &late);
-            if (late) pr.fail = 1;
+            drain(&pr.last, &pr.fail);
         }
         __syncwarp();
     } else if (warp >= kEpi) {
@@ -169,14 +168,14 @@ __device__ __forceinline__ bool run_products(Single& sh, Products& pr, char* op,
             const uint32_t s0 = s;
             if (s > 0) {
                 // the previous item's products no longer read the operands
-                ok = warp_wait(&pr.done[(s - 1u) & 1u], ((s - 1u) >> 1) & 1u, &pr.fail);
+                ok = warp_wait(&pr.done[(s - 1u) & 1u], ((s - 1u) >> 1) & 1u, limit);
                 if (!ok) break;
                 write_a(op, pr.table, nw, 128u * cb, warp - kEpi, kProd, lane);
             }
             for (uint32_t r0 = i0; r0 < i1 && ok; r0 += rb) {
                 for (uint32_t ch = 0; ch < chunks; ++ch, ++s) {
                     // the stage: its products of two steps ago are complete
-                    if (s >= s0 + 2u) ok = warp_wait(&pr.done[s & 1u], ((s - 2u) >> 1) & 1u, &pr.fail);
+                    if (s >= s0 + 2u) ok = warp_wait(&pr.done[s & 1u], ((s - 2u) >> 1) & 1u, limit);
                     if (!ok) break;
                     if (s > 0) {
                         write_b(op_s, s & 1u, rb, pr.table, nw, ch * kChunk, r0, min(rb, i1 - r0), warp - kEpi, kProd, lane,
@@ -195,7 +194,7 @@ __device__ __forceinline__ bool run_products(Single& sh, Products& pr, char* op,
             const uint32_t cb = item / ni, ri = item - cb * ni, i0 = first_row(ri), i1 = first_row(ri + 1u);
             Tile t{0, cols, 128u * cb, i0, sh.patch.out_offset + (uint64_t)i0 * cols, pr.inv, nw > kOneAccWaves};
             for (uint32_t r0 = i0; r0 < i1; r0 += rb, ++tile) {
-                ok = warp_wait(&pr.acc_full[tile & 1u], (tile >> 1) & 1u, &pr.fail);
+                ok = warp_wait(&pr.acc_full[tile & 1u], (tile >> 1) & 1u, limit);
                 if (!ok) break;
                 t.acc = tmem + (tile & 1u) * 256u;
                 if (t.c0 + 32u * quad < cols)
@@ -218,12 +217,15 @@ __global__ void __launch_bounds__(kThreads, 1)
 k_single(const wt_patch* __restrict__ patches, const wt_wave* __restrict__ waves, uint32_t n_waves, HmDev hm,
          float* __restrict__ pos, float* __restrict__ nrm, uint64_t out_capacity, uint64_t coef_capacity,
          uint32_t flags, char* __restrict__ ws, uint32_t chunk, float4* __restrict__ sums,
-         const wt_view* __restrict__ view, StageOut so, uint32_t mma) {
+         const wt_view* __restrict__ view, StageOut so, uint32_t mma, unsigned long long limit_ns) {
     extern __shared__ float4 raw[];
     float4* const smem = mma ? raw + ((1024u - (mma::smem_u32(raw) & 1023u)) & 1023u) / 16u : raw;
     Single& sh = *reinterpret_cast<Single*>(reinterpret_cast<char*>(smem) + (mma ? mma::kOperands : stage_bytes<EPI>()));
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     cudaGridDependencySynchronize();
+    // (before the constants are formed, so well before a block can report a wait)
+    WsHeader* const hdr = reinterpret_cast<WsHeader*>(ws);
+    if (blockIdx.x == 0 && tid == 0) hdr->status = 0;
     // the patch and every wave (the patch says which) in one round of loads
     if (tid >= kThreads - 32) {
         if (lane < sizeof(wt_patch) / 4)
@@ -263,8 +265,7 @@ k_single(const wt_patch* __restrict__ patches, const wt_wave* __restrict__ waves
     const bool nomem = nw > coef_capacity;  // the workspace is short of wave slots: refused, as in the prep
     const uint32_t cols = P.cols, tpr = bad || nomem ? 0u : tiles_per_row(cols, 8), total = P.rows * tpr;
     if (blockIdx.x == 0 && tid == 0) {
-        WsHeader* hdr = reinterpret_cast<WsHeader*>(ws);
-        hdr->status = bad ? (uint32_t)WT_ERR_INVALID_ARG : (nomem ? (uint32_t)WT_ERR_NOMEM : 0u);
+        if (bad || nomem) hdr->status = bad ? (uint32_t)WT_ERR_INVALID_ARG : (uint32_t)WT_ERR_NOMEM;
         hdr->bad_patch = bad ? 0u : kNoPatch;
         hdr->n_patches = 1;
         hdr->total_tiles = total;
@@ -275,8 +276,8 @@ k_single(const wt_patch* __restrict__ patches, const wt_wave* __restrict__ waves
     if (mma && total > 0 && !wild && mma_patch(P, kMmaMaxWaves)) {
         Products& pr = *reinterpret_cast<Products*>(&sh + 1);
         const mma::Output o{pos, nrm, sums, sh.view, so, flags};
-        if (!run_products<MODE, HM>(sh, pr, reinterpret_cast<char*>(smem), nw, hm, pow2, o) && tid == 0)
-            atomicCAS(&reinterpret_cast<WsHeader*>(ws)->status, 0u, (uint32_t)WT_ERR_TIMEOUT);
+        if (!run_products<MODE, HM>(sh, pr, reinterpret_cast<char*>(smem), nw, hm, pow2, o, limit_ns) && tid == 0)
+            atomicCAS(&hdr->status, 0u, (uint32_t)WT_ERR_TIMEOUT);
         return;
     }
     // a block's warps take tiles gridDim.x apart: few tiles spread over the SMs
@@ -317,7 +318,7 @@ cudaError_t launch_t(const FwdConfig& cfg, const wt_patch* patches, const wt_wav
     const uint64_t coef_cap = (L.end - L.coef) / sizeof(PairCoef);
     return cudaLaunchKernelEx(&lc, k_single<EPI, MODE, HM>, patches, waves, n_waves, hm, pos, nrm, out_capacity, coef_cap,
                               flags, static_cast<char*>(ws), (uint32_t)cfg.chunk, reinterpret_cast<float4*>(x.sums),
-                              x.view, x.stage, mma ? 1u : 0u);
+                              x.view, x.stage, mma ? 1u : 0u, wait_limit());
 }
 
 template <int EPI, int MODE>
