@@ -557,10 +557,13 @@ wt_status wt_get_tuning(wt_tuning* tuning);
  * two passes; each timed launch follows a clear of pos_out and nrm_out, which
  * evicts the previous launch's lines from L2 when the outputs outsize it,
  * so the shapes are ranked as a launch with cold inputs finds them) and
- * caches the fastest for the workload's shape bucket (the bit lengths of
- * n_patches and n_waves): later wt_gerstner_displace calls in that bucket use
- * it.  Returns it in *best (may be NULL).  Arguments as wt_gerstner_displace;
- * the outputs are overwritten. */
+ * caches the fastest, if it beats the shape in effect by 1 % and 1.5 us, else that shape,
+ * for the workload's shape bucket (the bit lengths of n_patches and n_waves, and
+ * of out_capacity with one patch): later wt_gerstner_displace calls in that
+ * bucket use it.  A workload none of whose patches depends on the shape (all
+ * matrix products, see wt_tuning) is not timed and caches nothing.  Returns the
+ * shape in *best (may be NULL).  Arguments as wt_gerstner_displace; the outputs
+ * are overwritten. */
 wt_status wt_autotune_displace(const wt_patch* patches, uint32_t n_patches,
                                const wt_wave* waves, uint32_t n_waves,
                                const wt_heightmap* hm,

@@ -65,3 +65,51 @@ def test_autotune_picks_a_supported_shape(wt, gpu, default_tuning):
     best = surf.autotune(pos, nrm, reps=2)
     assert (best["max_vertices_per_lane"], best["warps_per_block"], best["epilogue_in_shared"]) in SHAPES
     assert best["wave_chunk"] in (16, 32)
+
+
+def _one_launch(wt, surf):
+    """Whether a one-patch call runs in the one-patch kernel: the preparation's
+    arrays behind the workspace's header stay as they are."""
+    import torch
+    surf.workspace.fill_(0xAA)
+    surf.displace()
+    torch.cuda.synchronize()
+    assert surf.status()[0] == 0
+    return bool((surf.workspace[256:272] == 0xAA).all())
+
+
+def test_a_table_of_products_has_no_shape_to_tune(wt, gpu, default_tuning):
+    """Where no patch runs by the recurrence every shape is the same launch: the
+    default stays, for this table and for others of its counts."""
+    from wave_tool_gb300 import workloads
+    default = wt.get_tuning()
+    for n in (16, 1):
+        w = workloads.config3(n_patches=n, seed=4)
+        w.patches["cols"], w.patches["rows"] = 130, 90
+        for i in range(n):
+            w.patches["out_offset"][i] = i * 130 * 90
+        surf = wt.Surface(w.patches, w.waves)
+        pos, nrm = surf.alloc_outputs(0)
+        for _ in range(3):
+            best = surf.autotune(pos, nrm, reps=1)
+            assert {k: best[k] for k in default} == default
+    assert _one_launch(wt, surf)
+
+
+def test_a_large_patch_does_not_tune_a_small_one(wt, gpu, default_tuning):
+    """One-patch tables of as many waves: whatever shape a large skewed patch
+    gets, a small one runs in the one-patch kernel."""
+    import torch
+    from wave_tool_gb300 import workloads
+    small = workloads.small_random(5, n_patches=1, side_range=(60, 60), n_waves_range=(40, 40), heightmap=False)
+    large = small.patches.copy()
+    large["cols"] = large["rows"] = 1500
+    big = wt.Surface(large, small.waves)
+    pos, nrm = big.alloc_outputs(0)
+    cam = wt.camera(position=(0.0, 9.0, 30.0), pitch_deg=-20.0, aspect=1.5, displaceable_amplitude=2.0)
+    view = wt.to_device(wt.projected_grid(cam)[1])
+    best = big.autotune(pos, nrm, reps=2)
+    big.autotune_stage(view, big.displace_stage(view), reps=1)
+    assert (best["max_vertices_per_lane"], best["warps_per_block"], best["epilogue_in_shared"]) in SHAPES
+    torch.cuda.synchronize()
+    assert _one_launch(wt, wt.Surface(small.patches, small.waves))

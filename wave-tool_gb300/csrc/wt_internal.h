@@ -230,7 +230,7 @@ cudaError_t launch_adjoint(const wt_patch* patches, uint32_t n_patches, const wt
 
 // ---- host helpers (wt_api.cpp) ---------------------------------------------
 void set_last_error(const char* msg);  // message returned by wt_last_error() on this thread
-FwdConfig forward_config(uint32_t n_patches, uint32_t n_waves);  // tuning in effect for this shape
+FwdConfig forward_config(uint32_t n_patches, uint32_t n_waves, uint64_t out_capacity);  // tuning in effect for this shape
 // SM count of the current device (cached per device; 0 if it cannot be read)
 int sm_count();
 

@@ -264,16 +264,18 @@ k_single(const wt_patch* __restrict__ patches, const wt_wave* __restrict__ waves
     wild = __syncthreads_or(wild);
     const bool nomem = nw > coef_capacity;  // the workspace is short of wave slots: refused, as in the prep
     const uint32_t cols = P.cols, tpr = bad || nomem ? 0u : tiles_per_row(cols, 8), total = P.rows * tpr;
+    const bool products = mma && total > 0 && !wild && mma_patch(P, kMmaMaxWaves);
     if (blockIdx.x == 0 && tid == 0) {
         if (bad || nomem) hdr->status = bad ? (uint32_t)WT_ERR_INVALID_ARG : (uint32_t)WT_ERR_NOMEM;
         hdr->bad_patch = bad ? 0u : kNoPatch;
         hdr->n_patches = 1;
         hdr->total_tiles = total;
+        hdr->mma_items = products ? total : 0u;  // (the autotuner: no tile runs by the recurrence)
     }
     const bool pow2 = hm.present && (hm.width & (hm.width - 1)) == 0 && (hm.height & (hm.height - 1)) == 0;
     const bool fast = pow2 && hm.wrap == WT_WRAP_REPEAT;
     const uint64_t out0 = P.out_offset;
-    if (mma && total > 0 && !wild && mma_patch(P, kMmaMaxWaves)) {
+    if (products) {
         Products& pr = *reinterpret_cast<Products*>(&sh + 1);
         const mma::Output o{pos, nrm, sums, sh.view, so, flags};
         if (!run_products<MODE, HM>(sh, pr, reinterpret_cast<char*>(smem), nw, hm, pow2, o, limit_ns) && tid == 0)
