@@ -1,0 +1,119 @@
+"""Tables whose patches share waves: the preparation's routes for them against
+the FP64 oracle, the same refusals (a wave that is not valid counts where a patch
+uses it), and no route much slower than the same patches with waves of their
+own."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from helpers import rel_err
+from test_gpu_adjoint import _check, _upstream, run_adjoint
+
+pytestmark = pytest.mark.gpu
+
+
+def _table(n, shared=0, own=0, pool=0, side=(2, 30), seed=1):
+    """n patches, every other one a rectangle: all with the `shared` waves, or `own`
+    each, out of as many waves and `pool` more (behind them, or spread between them)."""
+    from wave_tool_gb300 import workloads
+    w = workloads.small_random(seed + n, n_patches=n, side_range=side, n_waves_range=(1, 1), heightmap=False)
+    p = w.patches
+    rng = workloads.SplitMix64(seed + 7 * n)
+    for i in range(0, n, 2):
+        p["br"][i][1], p["tl"][i][0] = p["bl"][i][1], p["bl"][i][0]
+        p["tr"][i] = p["br"][i][0], p["tl"][i][1]
+    waves = np.array(workloads.waves_wide(rng, (shared or n * own) + pool), dtype=w.waves.dtype)
+    p["wave_count"] = shared or own
+    gap = pool // n if own else 0
+    p["wave_offset"] = 0 if shared else np.arange(n) * (own + gap)
+    w.waves = waves
+    return w
+
+
+ROUTES = [dict(n=33, shared=9), dict(n=64, shared=16), dict(n=256, shared=4), dict(n=512, shared=2, side=(2, 16))]
+
+
+@pytest.mark.parametrize("kw", ROUTES, ids=lambda k: "-".join(f"{a}{b}" for a, b in k.items() if a != "side"))
+def test_forward_and_refusals(wt, oracle, gpu, kw):
+    import torch
+    w = _table(**kw)
+    n = len(w.patches)
+    surf = wt.Surface(w.patches, w.waves)
+    pos, nrm = surf.displace(flags=1)
+    torch.cuda.synchronize()
+    assert surf.status()[0] == 0
+    _, disp64, _, _ = oracle.displace_f64(w.patches, w.waves)
+    assert rel_err(pos[:, :3].double().cpu().numpy(), disp64) <= 1e-5
+    # a wave that no patch uses is not looked at
+    used = np.zeros(len(w.waves), bool)
+    for p in w.patches:
+        used[int(p["wave_offset"]):int(p["wave_offset"]) + int(p["wave_count"])] = True
+    if not used.all():
+        waves = w.waves.copy()
+        waves["wavelength"][np.nonzero(~used)[0][0]] = -1.0
+        s = wt.Surface(w.patches, waves)
+        p1, n1 = s.displace(flags=1)
+        assert s.status()[0] == 0 and torch.equal(p1, pos) and torch.equal(n1, nrm)
+    # one that some use, and one that leaves the products no room
+    waves = w.waves.copy()
+    last = int(w.patches["wave_offset"][n - 1]) + int(w.patches["wave_count"][n - 1]) - 1
+    waves["wavelength"][last] = np.nan
+    waves["amplitude"][int(w.patches["wave_offset"][0])] = 2.0e12
+    waves["steepness_q"][int(w.patches["wave_offset"][0])] = 0.0
+    s = wt.Surface(w.patches, waves)
+    p2, _ = s.displace(torch.full_like(pos, 7.0), torch.full_like(nrm, 7.0), flags=1)
+    hit = [i for i in range(n) if w.patches["wave_offset"][i] <= last < w.patches["wave_offset"][i] + w.patches["wave_count"][i]]
+    st, at = s.status()
+    assert st == wt.abi.WT_ERR_INVALID_ARG and at == hit[0]
+    for i in range(n):
+        o, k = int(w.patches["out_offset"][i]), int(w.patches["cols"][i]) * int(w.patches["rows"][i])
+        if i in hit:
+            assert bool((p2[o:o + k] == 7.0).all())
+        elif w.patches["wave_offset"][i] > w.patches["wave_offset"][0]:
+            assert torch.equal(p2[o:o + k], pos[o:o + k])
+
+
+@pytest.mark.parametrize("kw", [ROUTES[1], ROUTES[3]],
+                         ids=lambda k: "-".join(f"{a}{b}" for a, b in k.items() if a != "side"))
+def test_gradient(wt, oracle, gpu, kw):
+    w = _table(**kw)
+    gp, gn = _upstream(w.n_vertices, 3)
+    g, _ = run_adjoint(wt, w, gp, gn)
+    _check(g, oracle.adjoint_f64(w.patches, w.waves, gp.numpy(), gn.numpy()))
+
+
+def _graph_us(f, n=20):
+    import torch
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        for _ in range(3):
+            f()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        for _ in range(n):
+            f()
+    best = 1e9
+    for _ in range(20):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        g.replay()
+        b.record()
+        b.synchronize()
+        best = min(best, a.elapsed_time(b) / n * 1e3)
+    return best
+
+
+@pytest.mark.parametrize("kw,same", [(dict(n=64, shared=16), dict(n=64, own=16)),
+                                     (dict(n=256, shared=4), dict(n=256, own=4))])
+def test_no_route_is_much_slower(wt, gpu, kw, same):
+    """Shared waves cost at most half as much again as waves of their own (up to
+    three times as much when one block formed all constants)."""
+    us = []
+    for k in (kw, same):
+        w = _table(**k, side=(20, 30))
+        surf = wt.Surface(w.patches, w.waves)
+        pos, nrm = surf.alloc_outputs(0)
+        us.append(_graph_us(lambda: surf.displace(pos, nrm)))
+    assert us[0] <= 1.5 * us[1], us

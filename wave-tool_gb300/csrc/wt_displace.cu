@@ -61,12 +61,12 @@ __device__ __forceinline__ void flag_error(WsHeader* h, uint32_t code, uint32_t 
 }
 
 // ---- stage 1: validation, prefix sums, LPT order ---------------------------
-// Tables of at most kSmallPrep patches whose constants are formed here too
-// (k_prep_scan with fuse_coef): the whole prep through shared memory, with
-// two dependent global loads (the patches, then each pair's wave) instead of
-// the general path's chain of global-memory scans.  Writes what the general
-// path writes: header, pair and tile prefixes, the order, tiles, the
-// constants and, for the adjoint, its queue (adj_scan_body's arrays).
+// Tables of at most kSmallPrep patches, in one launch: the first block does the
+// scans through shared memory, with two dependent global loads (the patches, then
+// each pair's wave) instead of the general path's chain of global-memory scans,
+// and the others form the constants.  Writes what the general path writes:
+// header, pair and tile prefixes, the order, tiles, the constants and, for the
+// adjoint, its queue (adj_scan_body's arrays).
 constexpr uint32_t kSmallPrep = 32;
 
 // The constants of such a table, by the blocks after the first: one kind of
@@ -297,11 +297,12 @@ __device__ void prep_small(const wt_patch* __restrict__ patches, uint32_t n, con
     }
 }
 
-// Tables of up to kMediumPrep patches and 16384 waves whose constants the next
-// kernel forms: a thread has a patch, in registers, and what the threads share
-// is in shared memory, instead of the general path's round trips to global
-// memory between its steps (256 patches of 64-128 side, the whole call 60 us,
-// now 49).  Writes what the general path writes.
+// Tables of 33 to kMediumPrep patches and up to 16384 waves: a thread has a
+// patch, in registers, and what the threads share is in shared memory, instead of
+// the general path's round trips to global memory between its steps (256 patches
+// of 64-128 side, the whole call 60 us, now 49).  Writes what the general path
+// writes.  The next kernel forms the constants: with 1024 pairs or fewer this
+// block did, and for 64 patches sharing 16 waves that was 34 of its 41 us.
 constexpr uint32_t kMediumPrep = 512;
 
 // Exclusive prefix of v over the block's 1024 threads, and the total.
@@ -461,14 +462,14 @@ __device__ void prep_medium(const wt_patch* __restrict__ patches, uint32_t n, co
     }
 }
 
-// fuse_coef: also form the per-(patch, wave) and per-patch constants here
-// (small tables: the host passes it when n_patches * n_waves <= 1024, one
-// pair per thread), so that no second prep kernel runs.
+// small: a table of at most kSmallPrep patches whose constants are formed here too,
+// by the blocks after the first (prep_small_constants), so that no second prep
+// kernel runs.
 __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__ patches, uint32_t n,
                                                     const wt_wave* __restrict__ waves, uint32_t n_waves,
                                                     uint64_t out_capacity, uint64_t coef_capacity,
                                                     uint32_t tile_cols, char* ws, WsLayout L, HmDev hm,
-                                                    int fuse_coef, uint32_t mma_sms, uint32_t mma_max, int do_adj,
+                                                    int small, uint32_t mma_sms, uint32_t mma_max, int do_adj,
                                                     AdjLayout AL,
                                                     uint32_t adj_chunk_max, uint32_t adj_min_tiles) {
 #if __CUDA_ARCH__ >= 900
@@ -476,13 +477,13 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
     // own offsets and waits for this grid before it completes): let it start
     // (with the constants formed here the next kernel is the forward, which
     // waits at its start anyway)
-    if (!fuse_coef) cudaTriggerProgrammaticLaunchCompletion();
+    if (!small) cudaTriggerProgrammaticLaunchCompletion();
 #endif
     if (blockIdx.x > 0) {
         prep_small_constants(patches, n, waves, n_waves, out_capacity, coef_capacity, ws, L, hm);
         return;
     }
-    if (n <= kSmallPrep && fuse_coef) {
+    if (small) {
         prep_small(patches, n, waves, n_waves, out_capacity, coef_capacity, tile_cols, ws, L, hm, mma_sms, mma_max, do_adj, AL,
                    adj_chunk_max, adj_min_tiles);
         return;
@@ -500,7 +501,7 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
     __shared__ unsigned long long s_rowct;          // rows x 128-column blocks of the matrix-product patches
     __shared__ uint32_t s_mma_items, s_mma_n;
 
-    if (n <= kMediumPrep && !fuse_coef && n_waves <= 32u * kWaveMaskWords) {
+    if (n <= kMediumPrep && n_waves <= 32u * kWaveMaskWords) {
         prep_medium(patches, n, waves, n_waves, out_capacity, coef_capacity, tile_cols, ws, L, mma_sms, mma_max, do_adj, AL,
                     adj_chunk_max, adj_min_tiles, reinterpret_cast<uint4*>(bins), off_s, off_s + kMediumPrep, good_wave,
                     tame_wave);
@@ -670,20 +671,6 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
     if (threadIdx.x == 0) {
         tile_pre[n] = total_tiles;
         hdr->total_tiles = total_tiles;
-    }
-    if (fuse_coef) {
-        PatchAux* aux = reinterpret_cast<PatchAux*>(ws + L.aux);
-        PairCoef* coef = reinterpret_cast<PairCoef*>(ws + L.coef);
-        for (uint32_t P = threadIdx.x; P < total_pairs; P += blockDim.x) {
-            uint32_t lo = 0, hi = n + 1;
-            while (lo < hi) {
-                const uint32_t mid = (lo + hi) >> 1;
-                if (off[mid] <= P) lo = mid + 1; else hi = mid;
-            }
-            const wt_patch& Pt = patches[lo - 1];
-            coef[P] = make_pair_coef(Pt, waves[Pt.wave_offset + (P - off[lo - 1])]);
-        }
-        for (uint32_t p = threadIdx.x; p < n; p += blockDim.x) aux[p] = make_patch_aux(patches[p], hm, off[p]);
     }
     if (do_adj) {
         __syncthreads();  // sorted, tile_pre and the header's total_tiles are complete
@@ -964,22 +951,22 @@ cudaError_t launch_prep(const wt_patch* patches, uint32_t n_patches, const wt_wa
     // coefficient capacity = what the caller's workspace holds past the fixed part
     // (the header records the real total; the scan refuses to overflow it)
     uint64_t coef_cap = (L.end - L.coef) / sizeof(PairCoef);
-    // few (patch, wave) pairs, by the most that the table can have: the scan kernel
-    // forms the constants too
+    // few patches, and (patch, wave) pairs by the most that the table can have: the scan
+    // kernel forms the constants too
     const uint64_t pairs = (uint64_t)n_patches * n_waves;
-    const int fuse = pairs <= (n_patches <= kSmallPrep ? kSmallPairs : 1024u);
+    const int small = n_patches <= kSmallPrep && pairs <= kSmallPairs;
     const AdjScanArgs none{};
     const AdjScanArgs& A = adj ? *adj : none;
     const int sms = sm_count();
     if (sms <= 0) return cudaErrorInvalidDevice;
-    const unsigned more = fuse && n_patches <= kSmallPrep
+    const unsigned more = small
                               ? std::min((unsigned)sms - 1u, (unsigned)((5u * ((pairs + 31u) / 32u) + kSmallTasks) / kSmallTasks))
                               : 0u;
     k_prep_scan<<<1u + more, 1024, 0, s>>>(patches, n_patches, waves, n_waves, out_capacity, coef_cap, tile_cols, w, L,
-                                   hm, fuse, (uint32_t)sms, mma_max_waves, adj ? 1 : 0, A.L, A.chunk_max, A.min_tiles);
+                                   hm, small, (uint32_t)sms, mma_max_waves, adj ? 1 : 0, A.L, A.chunk_max, A.min_tiles);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    if (fuse) return cudaSuccess;
+    if (small) return cudaSuccess;
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((unsigned)sms);
     lc.blockDim = dim3(256);
