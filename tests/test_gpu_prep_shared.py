@@ -1,7 +1,8 @@
-"""Tables whose patches share waves: the preparation's routes for them against
-the FP64 oracle, the same refusals (a wave that is not valid counts where a patch
-uses it), and no route much slower than the same patches with waves of their
-own."""
+"""Tables whose patches share waves, or use a part of a pool: the preparation's
+routes for them against the FP64 oracle on either side of their limits, the same
+refusals (a wave that is not valid counts where a patch uses it), waves off a
+16-byte boundary, and no route much slower than the same patches with waves of
+their own."""
 from __future__ import annotations
 
 import numpy as np
@@ -31,7 +32,9 @@ def _table(n, shared=0, own=0, pool=0, side=(2, 30), seed=1):
     return w
 
 
-ROUTES = [dict(n=33, shared=9), dict(n=64, shared=16), dict(n=256, shared=4), dict(n=512, shared=2, side=(2, 16))]
+ROUTES = [dict(n=33, shared=9), dict(n=64, shared=16), dict(n=256, shared=4), dict(n=512, shared=2, side=(2, 16)),
+          dict(n=3, own=10, pool=5000), dict(n=2, shared=600, pool=9000, side=(20, 30)), dict(n=33, own=9, pool=16000),
+          dict(n=300, own=9, pool=9000, side=(2, 20)), dict(n=40, own=30, pool=200), dict(n=65, own=4, pool=2100)]
 
 
 @pytest.mark.parametrize("kw", ROUTES, ids=lambda k: "-".join(f"{a}{b}" for a, b in k.items() if a != "side"))
@@ -45,6 +48,13 @@ def test_forward_and_refusals(wt, oracle, gpu, kw):
     assert surf.status()[0] == 0
     _, disp64, _, _ = oracle.displace_f64(w.patches, w.waves)
     assert rel_err(pos[:, :3].double().cpu().numpy(), disp64) <= 1e-5
+    # the waves off a 16-byte boundary: the same bits
+    raw = torch.zeros(surf.waves.numel() + 16, dtype=torch.uint8, device="cuda")
+    raw[4:4 + surf.waves.numel()].copy_(surf.waves)
+    off = wt.Surface(w.patches, w.waves)
+    off.waves = raw[4:4 + surf.waves.numel()]
+    p1, n1 = off.displace(flags=1)
+    assert torch.equal(p1, pos) and torch.equal(n1, nrm)
     # a wave that no patch uses is not looked at
     used = np.zeros(len(w.waves), bool)
     for p in w.patches:
@@ -74,7 +84,7 @@ def test_forward_and_refusals(wt, oracle, gpu, kw):
             assert torch.equal(p2[o:o + k], pos[o:o + k])
 
 
-@pytest.mark.parametrize("kw", [ROUTES[1], ROUTES[3]],
+@pytest.mark.parametrize("kw", [ROUTES[1], ROUTES[3], ROUTES[6], ROUTES[7]],
                          ids=lambda k: "-".join(f"{a}{b}" for a, b in k.items() if a != "side"))
 def test_gradient(wt, oracle, gpu, kw):
     w = _table(**kw)
@@ -106,10 +116,13 @@ def _graph_us(f, n=20):
 
 
 @pytest.mark.parametrize("kw,same", [(dict(n=64, shared=16), dict(n=64, own=16)),
-                                     (dict(n=256, shared=4), dict(n=256, own=4))])
+                                     (dict(n=256, shared=4), dict(n=256, own=4)),
+                                     (dict(n=33, own=4, pool=16000), dict(n=33, own=4)),
+                                     (dict(n=2, shared=600, pool=60000), dict(n=2, shared=600))])
 def test_no_route_is_much_slower(wt, gpu, kw, same):
-    """Shared waves cost at most half as much again as waves of their own (up to
-    three times as much when one block formed all constants)."""
+    """Shared waves, or a pool around the waves that are used, cost at most half as
+    much again as waves of their own (they took 1.5 to 3 times as long when one
+    block formed all constants, or read the whole pool)."""
     us = []
     for k in (kw, same):
         w = _table(**k, side=(20, 30))

@@ -95,6 +95,7 @@ __device__ void prep_small_constants(const wt_patch* __restrict__ patches, uint3
     }
     const uint32_t total = __shfl_sync(kAll, end, 31);
     if (total > coef_capacity) return;
+    const bool wide = waves_wide(waves);
     const uint32_t tasks = 5u * ((total + 31u) / 32u) + 1u;
     for (uint32_t t = (blockIdx.x - 1u) * kSmallTasks + warp; t < tasks; t += (gridDim.x - 1u) * kSmallTasks) {
         if (t == 0) {
@@ -112,9 +113,38 @@ __device__ void prep_small_constants(const wt_patch* __restrict__ patches, uint3
         }
         if (P >= total) continue;
         const wt_patch& Pt = patches[p];
-        const wt_wave w = waves[Pt.wave_offset + (P - before)];
+        const wt_wave w = load_wave(waves, Pt.wave_offset + (P - before), wide);
         if (kind < 4u) (&coef[P].t00)[kind] = phase_turns((int)kind, Pt, w);
         else sum_coefs(w, coef[P]);
+    }
+}
+
+// Validates the waves pair by pair (where the pairs are fewer than the waves: a
+// pool that the table uses a part of), four at a time: wave_of gives the wave of
+// pair i and its patch, found from the last one's, and fails hears of those that
+// do not pass.
+template <typename WaveOf, typename Fails>
+__device__ __forceinline__ void for_pairs(uint32_t total, bool wide, const wt_wave* __restrict__ waves, WaveOf wave_of,
+                                          Fails fails) {
+    uint32_t p = 0;
+    for (uint32_t i0 = threadIdx.x; i0 < total; i0 += 4u * blockDim.x) {
+        wt_wave w[4];
+        uint32_t at[4];
+#pragma unroll
+        for (uint32_t e = 0; e < 4; ++e) {
+            const uint32_t i = i0 + e * blockDim.x;
+            if (i < total) {
+                const uint32_t k = wave_of(i, p);
+                w[e] = load_wave(waves, k, wide);
+            }
+            at[e] = p;
+        }
+#pragma unroll
+        for (uint32_t e = 0; e < 4; ++e) {
+            if (i0 + e * blockDim.x >= total) continue;
+            const bool good = wave_ok(w[e]), tame = mma_wave(w[e]);
+            if (!(good && tame)) fails(at[e], good, tame);
+        }
     }
 }
 
@@ -164,19 +194,20 @@ __device__ void prep_small(const wt_patch* __restrict__ patches, uint32_t n, con
     __syncthreads();
     const uint32_t total_pairs = s_off[n];
     const bool nomem = total_pairs > coef_capacity;
-    if (total_pairs <= blockDim.x) {
-        if (tid < total_pairs) {
-            uint32_t p = 0;
-            while (s_off[p + 1] <= tid) ++p;
-            const wt_wave w = waves[sp[p].wave_offset + (tid - s_off[p])];
-            if (!wave_ok(w)) atomicOr(&s_wave_bad, 1u << p);
-            if (!mma_wave(w)) atomicOr(&s_wave_wild, 1u << p);
-        }
+    const bool wide = waves_wide(waves);
+    if (total_pairs <= max(blockDim.x, n_waves / 4u)) {
+        for_pairs(total_pairs, wide, waves, [&](uint32_t i, uint32_t& p) {
+            while (s_off[p + 1] <= i) ++p;
+            return sp[p].wave_offset + (i - s_off[p]);
+        }, [&](uint32_t p, bool good, bool tame) {
+            if (!good) atomicOr(&s_wave_bad, 1u << p);
+            if (!tame) atomicOr(&s_wave_wild, 1u << p);
+        });
     } else {
-        // each wave once (patches may share them); the patches of one that fails
+        // each wave once (patches share them); the patches of one that fails
 #pragma unroll 4
         for (uint32_t i = tid; i < n_waves; i += blockDim.x) {
-            const wt_wave w = waves[i];
+            const wt_wave w = load_wave(waves, i, wide);
             const bool good = wave_ok(w), tame = mma_wave(w);
             for (uint32_t p = 0; !(good && tame) && p < n; ++p) {
                 if (i - sp[p].wave_offset >= s_off[p + 1] - s_off[p]) continue;  // (none of an invalid patch's)
@@ -326,6 +357,49 @@ __device__ __forceinline__ uint32_t block_prefix(uint32_t v, uint32_t* part, uin
     return (warp > 0 ? before : 0u) + x - v;
 }
 
+// Each wave once: its bits in good_wave and tame_wave, a warp's 32 waves a word.
+template <bool WIDE>
+__device__ __forceinline__ void each_wave(const wt_wave* __restrict__ waves, uint32_t n_waves, uint32_t* good_wave,
+                                          uint32_t* tame_wave) {
+    const uint32_t round = (n_waves + 31u) & ~31u;
+#pragma unroll 4
+    for (uint32_t w = threadIdx.x; w < round; w += blockDim.x) {
+        bool good = false, tame = false;
+        if (w < n_waves) {
+            const wt_wave v = load_wave(waves, w, WIDE);
+            good = wave_ok(v);
+            tame = mma_wave(v);
+        }
+        const uint32_t word = __ballot_sync(0xffffffffu, good), tword = __ballot_sync(0xffffffffu, tame);
+        if ((threadIdx.x & 31u) == 0) {
+            good_wave[w >> 5] = word;
+            tame_wave[w >> 5] = tword;
+        }
+    }
+}
+
+// What few tables take is out of line: the kernel runs once, from instructions
+// that no earlier launch left in the cache (48 patches: 0.5 us the whole call).
+__device__ __noinline__ void wave_masks(const wt_wave* __restrict__ waves, uint32_t n_waves, uint32_t* good_wave,
+                                          uint32_t* tame_wave) {
+    if (waves_wide(waves)) each_wave<true>(waves, n_waves, good_wave, tame_wave);
+    else each_wave<false>(waves, n_waves, good_wave, tame_wave);
+}
+
+// A pool's pairs: sets a patch's bits in `fails`, 1 for a wave that is not valid, 2
+// for one that is no mma_wave.
+__device__ __noinline__ void medium_pairs(uint32_t total, bool wide, const wt_wave* __restrict__ waves, uint32_t n,
+                                          const uint32_t* off, const uint32_t* w0, uint32_t* fails) {
+    for_pairs(total, wide, waves, [&](uint32_t i, uint32_t& q) {
+        uint32_t hi = n;  // the last q with off[q] <= i
+        while (hi - q > 1u) {
+            const uint32_t mid = (q + hi) >> 1;
+            if (off[mid] <= i) q = mid; else hi = mid;
+        }
+        return w0[q] + (i - off[q]);
+    }, [&](uint32_t q, bool good, bool tame) { atomicOr(&fails[q], (good ? 0u : 1u) | (tame ? 0u : 2u)); });
+}
+
 __device__ void prep_medium(const wt_patch* __restrict__ patches, uint32_t n, const wt_wave* __restrict__ waves,
                             uint32_t n_waves, uint64_t out_capacity, uint64_t coef_capacity, uint32_t tile_cols, char* ws,
                             const WsLayout& L, uint32_t mma_sms, uint32_t mma_max, int do_adj, const AdjLayout& AL,
@@ -358,34 +432,45 @@ __device__ void prep_medium(const wt_patch* __restrict__ patches, uint32_t n, co
         w0 = P.wave_offset;
         waves_p = P.wave_count;
     }
-    // each wave once, a warp's 32 waves a word
-    const uint32_t nw_round = (n_waves + 31u) & ~31u;
-#pragma unroll 4
-    for (uint32_t w = p; w < nw_round; w += blockDim.x) {
-        bool good = false, tame = false;
-        if (w < n_waves) {
-            const wt_wave v = waves[w];
-            good = wave_ok(v);
-            tame = mma_wave(v);
-        }
-        const uint32_t word = __ballot_sync(kAll, good), tword = __ballot_sync(kAll, tame);
-        if (lane == 0) {
-            good_wave[w >> 5] = word;
-            tame_wave[w >> 5] = tword;
-        }
-    }
+    // The waves: each once, a warp's 32 waves a word, beside the patches' loads;
+    // or, where the table has a pool of more than 32 a patch, when the pairs are
+    // known, and pair by pair if they are few (a pool of 16000 waves, 33 patches of
+    // 4 waves: 27 us the whole call with each wave once, 14 pair by pair).
+    const bool wide = waves_wide(waves);
+    const bool pool = n_waves > 32u * n;
+    if (!pool && wide) each_wave<true>(waves, n_waves, good_wave, tame_wave);
     uint32_t total_pairs;
     const uint32_t off = block_prefix(count, part, total_pairs);  // (and the bits are written)
     const bool nomem = total_pairs > coef_capacity;
+    const bool by_pair = pool && total_pairs <= n_waves / 4u;
+    if (by_pair) {
+        uint32_t *const s_w0 = reinterpret_cast<uint32_t*>(s_keys), *const s_off = s_w0 + kMediumPrep;
+        if (p < n) {
+            s_w0[p] = w0;
+            s_off[p] = off;
+            s_tiles[p] = 0;
+        }
+        __syncthreads();
+        medium_pairs(total_pairs, wide, waves, n, s_off, s_w0, s_tiles);
+        __syncthreads();
+    } else if (pool || !wide) {
+        wave_masks(waves, n_waves, good_wave, tame_wave);
+        __syncthreads();
+    }
     if (p < n) {
         pair_off[p] = off;
         bool bad = false, wild = false;
-        for (uint32_t w = w0, w1 = w0 + count; w < w1 && !bad;) {
-            const uint32_t bit = w & 31u, take = min(32u - bit, w1 - w);
-            const uint32_t want = (take == 32u ? 0xffffffffu : ((1u << take) - 1u)) << bit;
-            bad = (good_wave[w >> 5] & want) != want;
-            wild |= (tame_wave[w >> 5] & want) != want;
-            w += take;
+        if (by_pair) {
+            bad = s_tiles[p] & 1u;
+            wild = s_tiles[p] & 2u;
+        } else {
+            for (uint32_t w = w0, w1 = w0 + count; w < w1 && !bad;) {
+                const uint32_t bit = w & 31u, take = min(32u - bit, w1 - w);
+                const uint32_t want = (take == 32u ? 0xffffffffu : ((1u << take) - 1u)) << bit;
+                bad = (good_wave[w >> 5] & want) != want;
+                wild |= (tame_wave[w >> 5] & want) != want;
+                w += take;
+            }
         }
         if (bad) tl = 0;
         mma = mma && !bad && !wild;
@@ -547,22 +632,9 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
     if (off_in_smem)
         for (uint32_t i = threadIdx.x; i <= n; i += blockDim.x) off_s[i] = pair_off[i];
     const uint32_t* off = off_in_smem ? off_s : pair_off;
+    const bool wide = waves_wide(waves);
     if (total_pairs > blockDim.x && n_waves <= 32u * kWaveMaskWords) {
-        const uint32_t nw_round = (n_waves + 31u) & ~31u;
-#pragma unroll 4
-        for (uint32_t w = threadIdx.x; w < nw_round; w += blockDim.x) {
-            bool good = false, tame = false;
-            if (w < n_waves) {
-                const wt_wave v = waves[w];
-                good = wave_ok(v);
-                tame = mma_wave(v);
-            }
-            const uint32_t word = __ballot_sync(0xffffffffu, good), tword = __ballot_sync(0xffffffffu, tame);
-            if ((threadIdx.x & 31) == 0) {
-                good_wave[w >> 5] = word;
-                tame_wave[w >> 5] = tword;
-            }
-        }
+        wave_masks(waves, n_waves, good_wave, tame_wave);
         __syncthreads();
         for (uint32_t p = threadIdx.x; p < n; p += blockDim.x) {
             if (off[p + 1] == off[p]) continue;  // invalid patch (or no waves)
@@ -591,7 +663,7 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
                 if (off[mid] <= P) lo = mid + 1; else hi = mid;
             }
             const uint32_t p = lo - 1;
-            const wt_wave w = waves[patches[p].wave_offset + (P - off[p])];
+            const wt_wave w = load_wave(waves, patches[p].wave_offset + (P - off[p]), wide);
             if (!wave_ok(w)) {
                 flag_error(hdr, WT_ERR_INVALID_ARG, p);
                 atomicAnd(&tiles[p], 0u);
@@ -720,6 +792,7 @@ __global__ void __launch_bounds__(256) k_prep_coef(const wt_patch* __restrict__ 
     // this way.
     const uint32_t groups = (total + 31u) / 32u, tasks = 5u * groups + (n + 31u) / 32u;
     const uint32_t lane = threadIdx.x & 31u, warps = gridDim.x * (blockDim.x >> 5);
+    const bool wide = waves_wide(waves);
     for (uint32_t t = blockIdx.x + gridDim.x * (threadIdx.x >> 5); t < tasks; t += warps) {
         if (t >= 5u * groups) {
             const uint32_t p = 32u * (t - 5u * groups) + lane;
@@ -736,7 +809,7 @@ __global__ void __launch_bounds__(256) k_prep_coef(const wt_patch* __restrict__ 
         }
         const uint32_t p = lo - 1;
         const wt_patch& Pt = patches[p];
-        const wt_wave w = waves[Pt.wave_offset + (P - pair_off[p])];
+        const wt_wave w = load_wave(waves, Pt.wave_offset + (P - pair_off[p]), wide);
         if (kind < 4u) (&coef[P].t00)[kind] = phase_turns((int)kind, Pt, w);
         else sum_coefs(w, coef[P]);
     }
