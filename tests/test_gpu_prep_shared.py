@@ -32,7 +32,8 @@ def _table(n, shared=0, own=0, pool=0, side=(2, 30), seed=1):
     return w
 
 
-ROUTES = [dict(n=33, shared=9), dict(n=64, shared=16), dict(n=256, shared=4), dict(n=512, shared=2, side=(2, 16)),
+ROUTES = [dict(n=33, shared=9), dict(n=64, shared=16), dict(n=256, shared=4), dict(n=1024, shared=12),
+          dict(n=1025, shared=12, side=(2, 9)), dict(n=600, own=17, side=(2, 16)),
           dict(n=3, own=10, pool=5000), dict(n=2, shared=600, pool=9000, side=(20, 30)), dict(n=33, own=9, pool=16000),
           dict(n=300, own=9, pool=9000, side=(2, 20)), dict(n=40, own=30, pool=200), dict(n=65, own=4, pool=2100)]
 
@@ -84,7 +85,7 @@ def test_forward_and_refusals(wt, oracle, gpu, kw):
             assert torch.equal(p2[o:o + k], pos[o:o + k])
 
 
-@pytest.mark.parametrize("kw", [ROUTES[1], ROUTES[3], ROUTES[6], ROUTES[7]],
+@pytest.mark.parametrize("kw", [ROUTES[1], ROUTES[3], ROUTES[8], ROUTES[9]],
                          ids=lambda k: "-".join(f"{a}{b}" for a, b in k.items() if a != "side"))
 def test_gradient(wt, oracle, gpu, kw):
     w = _table(**kw)

@@ -146,12 +146,12 @@ __host__ __device__ __forceinline__ bool mma_patch(const wt_patch& P, uint32_t m
            same_sum(P.tr[0], P.bl[0], P.tl[0], P.br[0]) && same_sum(P.tr[1], P.bl[1], P.tl[1], P.br[1]);
 }
 
-// A wave whose sum coefficients leave room for the products' common scale
-// (finite, and far from FP32's limits).
+// A wave whose sum coefficients leave room for the products' scales (finite, and
+// far from FP32's limits): amplitude, Q times it, and both times the wave number
+// at most 1e12.
 __device__ __forceinline__ bool mma_wave(const wt_wave& w) {
-    const float k = 6.2831855f / w.wavelength, a = fabsf(w.amplitude), q = fabsf(w.steepness_q) * a;
-    return a <= 1e12f && q <= 1e12f && a * k <= 1e12f && q * k <= 1e12f && fabsf(w.dir_x) <= 2.0f &&
-           fabsf(w.dir_z) <= 2.0f;
+    const float a = fabsf(w.amplitude), q = fabsf(w.steepness_q) * a, most = 1e12f * (w.wavelength * 0.15915494f);
+    return a <= fminf(1e12f, most) && q <= fminf(1e12f, most) && fabsf(w.dir_x) <= 2.0f && fabsf(w.dir_z) <= 2.0f;
 }
 
 // Rows per item of the matrix-product kernel for `rowct` rows (summed over

@@ -334,7 +334,8 @@ __device__ void prep_small(const wt_patch* __restrict__ patches, uint32_t n, con
 // of 64-128 side, the whole call 60 us, now 49).  Writes what the general path
 // writes.  The next kernel forms the constants: with 1024 pairs or fewer this
 // block did, and for 64 patches sharing 16 waves that was 34 of its 41 us.
-constexpr uint32_t kMediumPrep = 512;
+constexpr uint32_t kMediumPrep = 1024;
+constexpr uint32_t kRankPrep = 512;  // ordered by ranks up to here (n^2 comparisons), by counting above
 
 // Exclusive prefix of v over the block's 1024 threads, and the total.
 __device__ __forceinline__ uint32_t block_prefix(uint32_t v, uint32_t* part, uint32_t& total) {
@@ -398,6 +399,21 @@ __device__ __noinline__ void medium_pairs(uint32_t total, bool wide, const wt_wa
         }
         return w0[q] + (i - off[q]);
     }, [&](uint32_t q, bool good, bool tame) { atomicOr(&fails[q], (good ? 0u : 1u) | (tame ? 0u : 2u)); });
+}
+
+// Ranks by counting: descending keys, ties in any order (the order only schedules).
+__device__ __noinline__ void medium_count_order(uint32_t n, uint32_t key, uint32_t* bins, uint32_t* part, uint32_t* rank) {
+    const uint32_t p = threadIdx.x, at = kSortBins - 1u - key;
+    bins[p] = bins[p + blockDim.x] = 0;
+    __syncthreads();
+    if (p < n) atomicAdd(&bins[at], 1u);
+    __syncthreads();
+    const uint2 c = reinterpret_cast<const uint2*>(bins)[p];
+    uint32_t all;
+    const uint32_t first = block_prefix(c.x + c.y, part, all);
+    reinterpret_cast<uint2*>(bins)[p] = make_uint2(first, first + c.x);
+    __syncthreads();
+    if (p < n) rank[p] = atomicAdd(&bins[at], 1u);
 }
 
 __device__ void prep_medium(const wt_patch* __restrict__ patches, uint32_t n, const wt_wave* __restrict__ waves,
@@ -493,23 +509,29 @@ __device__ void prep_medium(const wt_patch* __restrict__ patches, uint32_t n, co
             atomicAdd(&s_mma, some);
         }
     }
-    // ranks: keys descending, ties by index; each patch's comparisons shared out
-    // over as many threads as there are
-    const uint32_t n4 = (n + 3u) / 4u, key = p < n ? sort_key(waves_p, mma) : 0u;
-    if (p < 4u * n4) reinterpret_cast<uint32_t*>(s_keys)[p] = key;
-    __syncthreads();
-    const uint32_t shares = blockDim.x / n, share = p / n, mine = p - share * n;
-    if (share < shares) {
-        const uint32_t k = reinterpret_cast<const uint32_t*>(s_keys)[mine];
-        uint32_t rank = 0;
-        for (uint32_t q = share * n4 / shares; q < (share + 1u) * n4 / shares; ++q) {
-            const uint4 v = s_keys[q];
-            rank += v.x > k || (v.x == k && 4u * q < mine);
-            rank += v.y > k || (v.y == k && 4u * q + 1u < mine);
-            rank += v.z > k || (v.z == k && 4u * q + 2u < mine);
-            rank += v.w > k || (v.w == k && 4u * q + 3u < mine);
+    const uint32_t key = p < n ? sort_key(waves_p, mma) : 0u;
+    uint32_t* const bins = reinterpret_cast<uint32_t*>(s_keys);  // kSortBins of them
+    if (n <= kRankPrep) {
+        // ranks: keys descending, ties by index; each patch's comparisons shared out
+        // over as many threads as there are
+        const uint32_t n4 = (n + 3u) / 4u;
+        if (p < 4u * n4) bins[p] = key;
+        __syncthreads();
+        const uint32_t shares = blockDim.x / n, share = p / n, mine = p - share * n;
+        if (share < shares) {
+            const uint32_t k = bins[mine];
+            uint32_t rank = 0;
+            for (uint32_t q = share * n4 / shares; q < (share + 1u) * n4 / shares; ++q) {
+                const uint4 v = s_keys[q];
+                rank += v.x > k || (v.x == k && 4u * q < mine);
+                rank += v.y > k || (v.y == k && 4u * q + 1u < mine);
+                rank += v.z > k || (v.z == k && 4u * q + 2u < mine);
+                rank += v.w > k || (v.w == k && 4u * q + 3u < mine);
+            }
+            atomicAdd(&s_rank[mine], rank);
         }
-        atomicAdd(&s_rank[mine], rank);
+    } else {
+        medium_count_order(n, key, bins, part, s_rank);
     }
     __syncthreads();
     if (p < n) {
@@ -612,14 +634,26 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
     __syncthreads();
 
     // structural validation; pair_off <- wave counts of the patches that pass
-    for (uint32_t p = threadIdx.x; p < n; p += blockDim.x) {
-        const wt_patch P = patches[p];
-        const bool ok = patch_ok(P, n_waves, out_capacity);
-        if (!ok) flag_error(hdr, WT_ERR_INVALID_ARG, p);
-        pair_off[p] = ok ? P.wave_count : 0u;
-        tiles[p] = ok ? P.rows * tiles_per_row(P.cols, tile_cols / 32) | (mma_max > 0 && mma_patch(P, mma_max) ? kMmaFlag : 0u) : 0u;
+    const auto row_blocks = [](const wt_patch& P) { return (unsigned long long)P.rows * ((P.cols + 127u) / 128u); };
+    {
+        unsigned long long rowct = 0;
+        for (uint32_t p = threadIdx.x; p < n; p += blockDim.x) {
+            const wt_patch P = patches[p];
+            const bool ok = patch_ok(P, n_waves, out_capacity), mma = ok && mma_max > 0 && mma_patch(P, mma_max);
+            if (!ok) flag_error(hdr, WT_ERR_INVALID_ARG, p);
+            pair_off[p] = ok ? P.wave_count : 0u;
+            tiles[p] = ok ? P.rows * tiles_per_row(P.cols, tile_cols / 32) | (mma ? kMmaFlag : 0u) : 0u;
+            if (mma) rowct += row_blocks(P);
+        }
+        for (int o = 16; o > 0; o >>= 1) rowct += __shfl_xor_sync(0xffffffffu, rowct, o);
+        // one a warp: a 64-bit sum in shared memory is a loop of compare-and-swaps
+        if ((threadIdx.x & 31u) == 0 && rowct > 0) atomicAdd(&s_rowct, rowct);
     }
     __syncthreads();
+    // a patch that turns out not to qualify (keep: what stays of its tiles)
+    const auto clear_tiles = [&](uint32_t p, uint32_t keep) {
+        if (atomicAnd(&tiles[p], keep) & kMmaFlag) atomicAdd(&s_rowct, 0ull - row_blocks(patches[p]));
+    };
     const uint32_t total_pairs = block_exclusive_scan(pair_off, n);
     if (threadIdx.x == 0) pair_off[n] = total_pairs;
     __syncthreads();
@@ -649,9 +683,9 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
             }
             if (bad) {
                 flag_error(hdr, WT_ERR_INVALID_ARG, p);
-                tiles[p] = 0;
+                clear_tiles(p, 0u);
             } else if (wild) {
-                tiles[p] &= ~kMmaFlag;
+                clear_tiles(p, ~kMmaFlag);
             }
         }
     } else {
@@ -666,9 +700,9 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
             const wt_wave w = load_wave(waves, patches[p].wave_offset + (P - off[p]), wide);
             if (!wave_ok(w)) {
                 flag_error(hdr, WT_ERR_INVALID_ARG, p);
-                atomicAnd(&tiles[p], 0u);
+                clear_tiles(p, 0u);
             } else if (!mma_wave(w)) {
-                atomicAnd(&tiles[p], ~kMmaFlag);
+                clear_tiles(p, ~kMmaFlag);
             }
         }
     }
@@ -687,34 +721,25 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
         return;
     }
     // the matrix-product patches' items, then the sort keys
-    if (mma_max > 0) {
-        unsigned long long rowct = 0;
-        for (uint32_t p = threadIdx.x; p < n; p += blockDim.x)
-            if (tiles[p] & kMmaFlag) rowct += (unsigned long long)patches[p].rows * ((patches[p].cols + 127u) / 128u);
-        for (int o = 16; o > 0; o >>= 1) rowct += __shfl_xor_sync(0xffffffffu, rowct, o);
-        // one a warp: a 64-bit sum in shared memory is a loop of compare-and-swaps
-        if ((threadIdx.x & 31u) == 0 && rowct > 0) atomicAdd(&s_rowct, rowct);
+    if (s_rowct > 0) {
+        const uint32_t h = mma_item_rows(s_rowct, mma_sms);
+        for (uint32_t p = threadIdx.x; p < n; p += blockDim.x) {
+            if (!(tiles[p] & kMmaFlag)) continue;
+            const uint32_t items = (patches[p].cols + 127u) / 128u * ((patches[p].rows + h - 1u) / h);
+            tiles[p] = items | kMmaFlag;
+            atomicAdd(&s_mma_items, items);
+            atomicAdd(&s_mma_n, 1u);
+        }
         __syncthreads();
-        if (s_rowct > 0) {
-            const uint32_t h = mma_item_rows(s_rowct, mma_sms);
-            for (uint32_t p = threadIdx.x; p < n; p += blockDim.x) {
-                if (!(tiles[p] & kMmaFlag)) continue;
-                const uint32_t items = (patches[p].cols + 127u) / 128u * ((patches[p].rows + h - 1u) / h);
-                tiles[p] = items | kMmaFlag;
-                atomicAdd(&s_mma_items, items);
-                atomicAdd(&s_mma_n, 1u);
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                hdr->mma_items = s_mma_items;
-                hdr->mma_patches = s_mma_n;
-                hdr->mma_rows = h;
-                hdr->tile_counter = s_mma_items;  // the recurrence kernel's tiles follow the items
-            }
+        if (threadIdx.x == 0) {
+            hdr->mma_items = s_mma_items;
+            hdr->mma_patches = s_mma_n;
+            hdr->mma_rows = h;
+            hdr->tile_counter = s_mma_items;  // the recurrence kernel's tiles follow the items
         }
     }
     for (uint32_t p = threadIdx.x; p < n; p += blockDim.x) {
-        const uint32_t key = sort_key(patches[p].wave_count, tiles[p] & kMmaFlag);
+        const uint32_t key = sort_key(off[p + 1] - off[p], tiles[p] & kMmaFlag);
         if (rank_sort) bins[p] = key;
         else atomicAdd(&bins[kSortBins - 1 - key], 1u);  // descending
     }
@@ -729,10 +754,11 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
             sorted[rank] = p;
         }
     } else {
-        block_exclusive_scan(bins, kSortBins);
+        const uint32_t used = s_mma_n > 0 ? 0u : kSortBins - kWaveBins;  // (larger keys are matrix products')
+        block_exclusive_scan(bins + used, kSortBins - used);
         __syncthreads();
         for (uint32_t p = threadIdx.x; p < n; p += blockDim.x) {
-            const uint32_t key = sort_key(patches[p].wave_count, tiles[p] & kMmaFlag);
+            const uint32_t key = sort_key(off[p + 1] - off[p], tiles[p] & kMmaFlag);
             sorted[atomicAdd(&bins[kSortBins - 1 - key], 1u)] = p;
         }
     }
@@ -789,17 +815,20 @@ __global__ void __launch_bounds__(256) k_prep_coef(const wt_patch* __restrict__ 
     // on different SMs, so that the FP64 chains (a warp-wide operation holds the
     // pipe for about 64 cycles) run side by side.  One thread per pair doing all
     // of it in consecutive warps: 14.0 us for 48 patches of 0-40 waves, 6.5 us
-    // this way.
-    const uint32_t groups = (total + 31u) / 32u, tasks = 5u * groups + (n + 31u) / 32u;
+    // this way.  All kinds in one task from two rounds of tasks on, since every
+    // kind divides by the wavelength again (16000 pairs:
+    // 13.4 us by kinds, now 10.7; 45000 pairs 25.0, now 17.2).
     const uint32_t lane = threadIdx.x & 31u, warps = gridDim.x * (blockDim.x >> 5);
     const bool wide = waves_wide(waves);
+    const uint32_t groups = (total + 31u) / 32u, kinds = 5u * groups <= 8u * gridDim.x ? 5u : 1u;
+    const uint32_t tasks = kinds * groups + (n + 31u) / 32u;
     for (uint32_t t = blockIdx.x + gridDim.x * (threadIdx.x >> 5); t < tasks; t += warps) {
-        if (t >= 5u * groups) {
-            const uint32_t p = 32u * (t - 5u * groups) + lane;
+        if (t >= kinds * groups) {
+            const uint32_t p = 32u * (t - kinds * groups) + lane;
             if (p < n) aux[p] = make_patch_aux(patches[p], hm, pair_off[p]);
             continue;
         }
-        const uint32_t kind = t % 5u, P = 32u * (t / 5u) + lane;
+        const uint32_t kind = t % kinds, P = 32u * (t / kinds) + lane;
         if (P >= total) continue;
         // owning patch: last p with pair_off[p] <= P
         uint32_t lo = 0, hi = n + 1;
@@ -810,7 +839,8 @@ __global__ void __launch_bounds__(256) k_prep_coef(const wt_patch* __restrict__ 
         const uint32_t p = lo - 1;
         const wt_patch& Pt = patches[p];
         const wt_wave w = load_wave(waves, Pt.wave_offset + (P - pair_off[p]), wide);
-        if (kind < 4u) (&coef[P].t00)[kind] = phase_turns((int)kind, Pt, w);
+        if (kinds == 1u) coef[P] = make_pair_coef(Pt, w);
+        else if (kind < 4u) (&coef[P].t00)[kind] = phase_turns((int)kind, Pt, w);
         else sum_coefs(w, coef[P]);
     }
 #if __CUDA_ARCH__ >= 900
