@@ -335,7 +335,7 @@ static wt_status run_adjoint(const wt_patch* host_patches, const wt_patch* patch
     if (e != cudaSuccess) return cuda_fail(e, "adjoint set-up");
     const uint32_t mma_waves = wt::adjoint_mma_waves(host_patches, n_patches, n_waves, sums != nullptr);
     e = wt::launch_prep(patches, n_patches, waves, n_waves, P.hm, out_capacity, 256u, workspace, L.f, s,
-                        mma_waves, &args);
+                        wt::MmaRule{mma_waves, 1u}, &args);
     if (e != cudaSuccess) return cuda_fail(e, "prep launch");
     uint32_t maxw = 0;
     for (uint32_t i = 0; i < n_patches; ++i) maxw = host_patches[i].wave_count > maxw ? host_patches[i].wave_count : maxw;

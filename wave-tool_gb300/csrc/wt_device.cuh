@@ -154,13 +154,45 @@ __device__ __forceinline__ bool mma_wave(const wt_wave& w) {
     return a <= fminf(1e12f, most) && q <= fminf(1e12f, most) && fabsf(w.dir_x) <= 2.0f && fabsf(w.dir_z) <= 2.0f;
 }
 
-// Rows per item of the matrix-product kernel for `rowct` rows (summed over
-// the patches' 128-column blocks): one item per SM while that is at most 128
-// rows, else a whole number of items per SM of at most about 128 (operand A,
-// formed once per item, is then a tenth of its work).
-__device__ __forceinline__ uint32_t mma_item_rows(uint64_t rowct, uint32_t sms) {
-    const uint64_t w = (rowct + 128ull * sms - 1u) / (128ull * sms);
-    return max((uint32_t)((rowct + sms * w - 1u) / (sms * w)), 4u);
+// Rows per item of the matrix-product kernels for `rowct` rows (summed over the
+// patches' 128-column blocks): a whole number of items per SM, as few as make
+// them at most 128 rows (operand A, formed once per item, is then a tenth of its
+// work), and k more.
+__device__ __forceinline__ uint32_t mma_item_rows(uint64_t rowct, uint32_t sms, uint32_t k) {
+    const uint32_t r = (uint32_t)min(rowct, (uint64_t)0xf0000000u);  // (beyond, 128 rows either way)
+    const uint32_t w = (r + 128u * sms - 1u) / (128u * sms) + k;
+    return max((r + sms * w - 1u) / (sms * w), 4u);
+}
+// A patch's rows are split evenly into items of at most that many, so there may be
+// more items than a whole number per SM, and the last round nearly empty.  Where it
+// leaves a seventh of the SMs' time idle, kItemChoices choices of k are compared:
+// by the adjoint, and by the saving forward from 64 rows an SM on (its stores make
+// an item's rows long); a plain forward's items are short, and more of them cost
+// it what the fuller round gives.  40 patches of 200 rows, 160 items on 152 SMs:
+// adjoint of 129 columns and 16 waves 99.2 -> 94.4 us, of 256 and 8 97.9 -> 94.2,
+// saving forward 52.1 -> 39.3 and 46.8 -> 39.6; 10 of 600 x 256, 8 waves: 78.2 ->
+// 57.3 and 35.5 -> 28.2.  (Saving forward of 64 columns, 53 rows an SM: 20.9 -> 25.4
+// if compared, plain 19.6 -> 23.1.)
+constexpr uint32_t kItemChoices = 4;
+constexpr float kItemRows = 6.0f;  // what an item costs besides its rows, in rows
+__device__ __forceinline__ bool mma_compares(const MmaRule& rule, uint64_t rowct, uint32_t items, uint32_t sms) {
+    return rule.spread > 0 && rowct >= (uint64_t)rule.spread * sms &&
+           (uint64_t)((items + sms - 1u) / sms) * sms * 6u > (uint64_t)items * 7u;
+}
+// The choice with the least work on the fullest SM, for items of average rows
+// (items: their count for each k).
+__device__ __forceinline__ uint32_t mma_item_choice(uint64_t rowct, uint32_t sms, const uint32_t* items) {
+    uint32_t best = 0;
+    float least = INFINITY;
+#pragma unroll 1
+    for (uint32_t k = 0; k < kItemChoices; ++k) {
+        const float n = (float)items[k], cost = (float)((items[k] + sms - 1u) / sms) * fmaf(kItemRows, n, (float)rowct) / n;
+        if (cost < least) {
+            least = cost;
+            best = k;
+        }
+    }
+    return best;
 }
 
 // ---- shared epilogue -------------------------------------------------------

@@ -150,7 +150,7 @@ __device__ __forceinline__ void for_pairs(uint32_t total, bool wide, const wt_wa
 
 __device__ void prep_small(const wt_patch* __restrict__ patches, uint32_t n, const wt_wave* __restrict__ waves,
                            uint32_t n_waves, uint64_t out_capacity, uint64_t coef_capacity, uint32_t tile_cols,
-                           char* ws, const WsLayout& L, const HmDev& hm, uint32_t mma_sms, uint32_t mma_max, int do_adj,
+                           char* ws, const WsLayout& L, const HmDev& hm, uint32_t mma_sms, const MmaRule& rule, int do_adj,
                            const AdjLayout& AL, uint32_t adj_chunk_max, uint32_t adj_min_tiles) {
     __shared__ wt_patch sp[kSmallPrep];
     __shared__ uint32_t s_sorted[kSmallPrep];      // patch at each sorted rank
@@ -158,6 +158,7 @@ __device__ void prep_small(const wt_patch* __restrict__ patches, uint32_t n, con
     __shared__ uint32_t s_rank_tiles[kSmallPrep];  // tiles of the patch at each sorted rank
     __shared__ uint32_t s_struct_bad, s_wave_bad;  // bit p: patch p fails that check
     __shared__ uint32_t s_wave_wild;               // bit p: a wave of patch p is no mma_wave
+    __shared__ uint32_t s_choices[kItemChoices];
     WsHeader* hdr = reinterpret_cast<WsHeader*>(ws);
     uint32_t* sorted = reinterpret_cast<uint32_t*>(ws + L.sorted);
     uint32_t* tile_pre = reinterpret_cast<uint32_t*>(ws + L.tile_pre);
@@ -179,7 +180,7 @@ __device__ void prep_small(const wt_patch* __restrict__ patches, uint32_t n, con
             ok = patch_ok(P, n_waves, out_capacity);
             wc = ok ? P.wave_count : 0u;
             tiles_p = ok ? P.rows * tiles_per_row(P.cols, tile_cols / 32) : 0u;
-            mma_p = mma_max > 0 && ok && mma_patch(P, mma_max);
+            mma_p = ok && mma_patch(P, rule.max_waves);
         }
         uint32_t x = wc;  // inclusive prefix of the pair counts
         for (int o = 1; o < 32; o <<= 1) {
@@ -229,9 +230,20 @@ __device__ void prep_small(const wt_patch* __restrict__ patches, uint32_t n, con
         const uint32_t rows = mma_p ? sp[tid].rows : 0u;
         rowct = (unsigned long long)rows * ct;
         for (int o = 16; o > 0; o >>= 1) rowct += __shfl_xor_sync(kAll, rowct, o);
-        mma_rows = mma_item_rows(rowct, mma_sms);
+        const auto count = [&](uint32_t h) { return __reduce_add_sync(kAll, ct * ((rows + h - 1u) / h)); };
+        mma_rows = mma_item_rows(rowct, mma_sms, 0);
+        mma_items = count(mma_rows);
+        if (mma_compares(rule, rowct, mma_items, mma_sms)) {
+#pragma unroll 1
+            for (uint32_t k = 0; k < kItemChoices; ++k) {
+                const uint32_t items = count(mma_item_rows(rowct, mma_sms, k));
+                if (tid == 0) s_choices[k] = items;
+            }
+            __syncwarp();
+            mma_rows = mma_item_rows(rowct, mma_sms, mma_item_choice(rowct, mma_sms, s_choices));
+            mma_items = count(mma_rows);
+        }
         if (mma_p) tiles_p = ct * ((rows + mma_rows - 1u) / mma_rows);
-        mma_items = __reduce_add_sync(kAll, mma_p ? tiles_p : 0u);
     }
     if (tid < n) {
         pair_off[tid] = s_off[tid];
@@ -401,6 +413,21 @@ __device__ __noinline__ void medium_pairs(uint32_t total, bool wide, const wt_wa
     }, [&](uint32_t q, bool good, bool tame) { atomicOr(&fails[q], (good ? 0u : 1u) | (tame ? 0u : 2u)); });
 }
 
+// Rows per item, compared over the block's patches (of rows rows, 0 where it is not
+// queued, in ct column blocks), and the items' count.
+__device__ __noinline__ uint32_t medium_item_rows(uint64_t rowct, uint32_t sms, uint32_t rows, uint32_t ct, uint32_t* count,
+                                                  uint32_t& items) {
+#pragma unroll 1
+    for (uint32_t k = 0; k < kItemChoices; ++k) {
+        const uint32_t h = mma_item_rows(rowct, sms, k), n = __reduce_add_sync(0xffffffffu, ct * ((rows + h - 1u) / h));
+        if ((threadIdx.x & 31u) == 0 && n > 0) atomicAdd(&count[k], n);
+    }
+    __syncthreads();
+    const uint32_t k = mma_item_choice(rowct, sms, count);
+    items = count[k];
+    return mma_item_rows(rowct, sms, k);
+}
+
 // Ranks by counting: descending keys, ties in any order (the order only schedules).
 __device__ __noinline__ void medium_count_order(uint32_t n, uint32_t key, uint32_t* bins, uint32_t* part, uint32_t* rank) {
     const uint32_t p = threadIdx.x, at = kSortBins - 1u - key;
@@ -418,10 +445,10 @@ __device__ __noinline__ void medium_count_order(uint32_t n, uint32_t key, uint32
 
 __device__ void prep_medium(const wt_patch* __restrict__ patches, uint32_t n, const wt_wave* __restrict__ waves,
                             uint32_t n_waves, uint64_t out_capacity, uint64_t coef_capacity, uint32_t tile_cols, char* ws,
-                            const WsLayout& L, uint32_t mma_sms, uint32_t mma_max, int do_adj, const AdjLayout& AL,
+                            const WsLayout& L, uint32_t mma_sms, const MmaRule& rule, int do_adj, const AdjLayout& AL,
                             uint32_t adj_chunk_max, uint32_t adj_min_tiles, uint4* s_keys, uint32_t* s_tiles,
                             uint32_t* s_rank, uint32_t* good_wave, uint32_t* tame_wave) {
-    __shared__ uint32_t part[32], s_bad, s_items, s_mma;
+    __shared__ uint32_t part[32], s_bad, s_items, s_mma, s_choices[kItemChoices];
     __shared__ unsigned long long part64[32];
     constexpr unsigned kAll = 0xffffffffu;
     WsHeader* hdr = reinterpret_cast<WsHeader*>(ws);
@@ -434,13 +461,14 @@ __device__ void prep_medium(const wt_patch* __restrict__ patches, uint32_t n, co
         s_bad = kNoPatch;
         s_items = s_mma = 0;
     }
+    if (p < kItemChoices) s_choices[p] = 0;
     if (p < n) s_rank[p] = 0;
     uint32_t count = 0, tl = 0, rows = 0, ct = 0, w0 = 0, waves_p = 0;
     bool ok = false, mma = false;
     if (p < n) {
         const wt_patch P = patches[p];
         ok = patch_ok(P, n_waves, out_capacity);
-        mma = ok && mma_max > 0 && mma_patch(P, mma_max);
+        mma = ok && mma_patch(P, rule.max_waves);
         count = ok ? P.wave_count : 0u;
         tl = ok ? P.rows * tiles_per_row(P.cols, tile_cols / 32) : 0u;
         rows = P.rows;
@@ -499,15 +527,20 @@ __device__ void prep_medium(const wt_patch* __restrict__ patches, uint32_t n, co
     __syncthreads();
     rowct = part64[lane];
     for (int o = 16; o > 0; o >>= 1) rowct += __shfl_xor_sync(kAll, rowct, o);
-    uint32_t item_rows = 0;
+    uint32_t item_rows = 0, n_items = 0;
     if (rowct > 0) {
-        item_rows = mma_item_rows(rowct, mma_sms);
-        if (mma) tl = ct * ((rows + item_rows - 1u) / item_rows);
-        const uint32_t items = __reduce_add_sync(kAll, mma ? tl : 0u), some = __popc(__ballot_sync(kAll, mma));
+        item_rows = mma_item_rows(rowct, mma_sms, 0);
+        const uint32_t items = __reduce_add_sync(kAll, mma ? ct * ((rows + item_rows - 1u) / item_rows) : 0u);
+        const uint32_t some = __popc(__ballot_sync(kAll, mma));
         if (lane == 0 && some > 0) {
             atomicAdd(&s_items, items);
             atomicAdd(&s_mma, some);
         }
+        __syncthreads();
+        n_items = s_items;
+        if (mma_compares(rule, rowct, n_items, mma_sms))
+            item_rows = medium_item_rows(rowct, mma_sms, mma ? rows : 0u, ct, s_choices, n_items);
+        if (mma) tl = ct * ((rows + item_rows - 1u) / item_rows);
     }
     const uint32_t key = p < n ? sort_key(waves_p, mma) : 0u;
     uint32_t* const bins = reinterpret_cast<uint32_t*>(s_keys);  // kSortBins of them
@@ -547,7 +580,7 @@ __device__ void prep_medium(const wt_patch* __restrict__ patches, uint32_t n, co
     if (p < n) tile_pre[p] = before;
     if (p == 0) {
         const bool any_bad = s_bad != kNoPatch;
-        const uint32_t items = nomem ? 0u : s_items;
+        const uint32_t items = nomem ? 0u : n_items;
         hdr->status = any_bad ? (uint32_t)WT_ERR_INVALID_ARG : (nomem ? (uint32_t)WT_ERR_NOMEM : 0u);
         hdr->bad_patch = s_bad;
         hdr->tile_counter = items;  // the recurrence kernel's tiles follow the items
@@ -576,7 +609,7 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
                                                     const wt_wave* __restrict__ waves, uint32_t n_waves,
                                                     uint64_t out_capacity, uint64_t coef_capacity,
                                                     uint32_t tile_cols, char* ws, WsLayout L, HmDev hm,
-                                                    int small, uint32_t mma_sms, uint32_t mma_max, int do_adj,
+                                                    int small, uint32_t mma_sms, MmaRule rule, int do_adj,
                                                     AdjLayout AL,
                                                     uint32_t adj_chunk_max, uint32_t adj_min_tiles) {
 #if __CUDA_ARCH__ >= 900
@@ -591,7 +624,7 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
         return;
     }
     if (small) {
-        prep_small(patches, n, waves, n_waves, out_capacity, coef_capacity, tile_cols, ws, L, hm, mma_sms, mma_max, do_adj, AL,
+        prep_small(patches, n, waves, n_waves, out_capacity, coef_capacity, tile_cols, ws, L, hm, mma_sms, rule, do_adj, AL,
                    adj_chunk_max, adj_min_tiles);
         return;
     }
@@ -606,10 +639,10 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
     __shared__ uint32_t good_wave[kWaveMaskWords];  // bit w: wave w passes wave_ok
     __shared__ uint32_t tame_wave[kWaveMaskWords];  // bit w: wave w is an mma_wave
     __shared__ unsigned long long s_rowct;          // rows x 128-column blocks of the matrix-product patches
-    __shared__ uint32_t s_mma_items, s_mma_n;
+    __shared__ uint32_t s_mma_n, s_choices[kItemChoices + 1];
 
     if (n <= kMediumPrep && n_waves <= 32u * kWaveMaskWords) {
-        prep_medium(patches, n, waves, n_waves, out_capacity, coef_capacity, tile_cols, ws, L, mma_sms, mma_max, do_adj, AL,
+        prep_medium(patches, n, waves, n_waves, out_capacity, coef_capacity, tile_cols, ws, L, mma_sms, rule, do_adj, AL,
                     adj_chunk_max, adj_min_tiles, reinterpret_cast<uint4*>(bins), off_s, off_s + kMediumPrep, good_wave,
                     tame_wave);
         return;
@@ -624,8 +657,9 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
         hdr->mma_counter = 0;
         hdr->mma_patches = 0;
         s_rowct = 0;
-        s_mma_items = s_mma_n = 0;
+        s_mma_n = 0;
     }
+    if (threadIdx.x <= kItemChoices) s_choices[threadIdx.x] = 0;
     // up to kRankSortMax patches are ordered by rank (their keys in bins[]),
     // more by a counting sort over the bins
     const bool rank_sort = n <= kRankSortMax;
@@ -639,7 +673,7 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
         unsigned long long rowct = 0;
         for (uint32_t p = threadIdx.x; p < n; p += blockDim.x) {
             const wt_patch P = patches[p];
-            const bool ok = patch_ok(P, n_waves, out_capacity), mma = ok && mma_max > 0 && mma_patch(P, mma_max);
+            const bool ok = patch_ok(P, n_waves, out_capacity), mma = ok && mma_patch(P, rule.max_waves);
             if (!ok) flag_error(hdr, WT_ERR_INVALID_ARG, p);
             pair_off[p] = ok ? P.wave_count : 0u;
             tiles[p] = ok ? P.rows * tiles_per_row(P.cols, tile_cols / 32) | (mma ? kMmaFlag : 0u) : 0u;
@@ -722,20 +756,39 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
     }
     // the matrix-product patches' items, then the sort keys
     if (s_rowct > 0) {
-        const uint32_t h = mma_item_rows(s_rowct, mma_sms);
-        for (uint32_t p = threadIdx.x; p < n; p += blockDim.x) {
-            if (!(tiles[p] & kMmaFlag)) continue;
-            const uint32_t items = (patches[p].cols + 127u) / 128u * ((patches[p].rows + h - 1u) / h);
-            tiles[p] = items | kMmaFlag;
-            atomicAdd(&s_mma_items, items);
-            atomicAdd(&s_mma_n, 1u);
+        // the items with at most h rows, into the patches' tiles and summed
+        const auto count_items = [&](uint32_t h, uint32_t* sum) {
+            uint32_t items = 0, some = 0;
+            for (uint32_t p = threadIdx.x; p < n; p += blockDim.x) {
+                if (!(tiles[p] & kMmaFlag)) continue;
+                const uint32_t it = (patches[p].cols + 127u) / 128u * ((patches[p].rows + h - 1u) / h);
+                tiles[p] = it | kMmaFlag;
+                items += it;
+                ++some;
+            }
+            items = __reduce_add_sync(0xffffffffu, items);
+            some = __reduce_add_sync(0xffffffffu, some);
+            if ((threadIdx.x & 31u) == 0 && some > 0) {
+                atomicAdd(sum, items);
+                atomicAdd(&s_mma_n, some);
+            }
+            __syncthreads();
+        };
+        uint32_t k = 0;
+        count_items(mma_item_rows(s_rowct, mma_sms, 0), &s_choices[0]);
+        const uint32_t n_mma = s_mma_n;
+        if (mma_compares(rule, s_rowct, s_choices[0], mma_sms)) {
+            __syncthreads();  // every thread has read the count
+#pragma unroll 1
+            for (k = 1; k < kItemChoices; ++k) count_items(mma_item_rows(s_rowct, mma_sms, k), &s_choices[k]);
+            k = mma_item_choice(s_rowct, mma_sms, s_choices);
+            count_items(mma_item_rows(s_rowct, mma_sms, k), &s_choices[kItemChoices]);
         }
-        __syncthreads();
         if (threadIdx.x == 0) {
-            hdr->mma_items = s_mma_items;
-            hdr->mma_patches = s_mma_n;
-            hdr->mma_rows = h;
-            hdr->tile_counter = s_mma_items;  // the recurrence kernel's tiles follow the items
+            hdr->mma_items = s_choices[k];
+            hdr->mma_patches = n_mma;
+            hdr->mma_rows = mma_item_rows(s_rowct, mma_sms, k);
+            hdr->tile_counter = s_choices[k];  // the recurrence kernel's tiles follow the items
         }
     }
     for (uint32_t p = threadIdx.x; p < n; p += blockDim.x) {
@@ -1048,7 +1101,7 @@ cudaError_t launch_fwd_t(const FwdConfig& cfg, const wt_patch* patches, uint32_t
 
 cudaError_t launch_prep(const wt_patch* patches, uint32_t n_patches, const wt_wave* waves, uint32_t n_waves,
                         const HmDev& hm, uint64_t out_capacity, uint32_t tile_cols, void* ws,
-                        const WsLayout& L, cudaStream_t s, uint32_t mma_max_waves,
+                        const WsLayout& L, cudaStream_t s, const MmaRule& rule,
                         const AdjScanArgs* adj) {
     char* w = static_cast<char*>(ws);
     // coefficient capacity = what the caller's workspace holds past the fixed part
@@ -1066,7 +1119,7 @@ cudaError_t launch_prep(const wt_patch* patches, uint32_t n_patches, const wt_wa
                               ? std::min((unsigned)sms - 1u, (unsigned)((5u * ((pairs + 31u) / 32u) + kSmallTasks) / kSmallTasks))
                               : 0u;
     k_prep_scan<<<1u + more, 1024, 0, s>>>(patches, n_patches, waves, n_waves, out_capacity, coef_cap, tile_cols, w, L,
-                                   hm, small, (uint32_t)sms, mma_max_waves, adj ? 1 : 0, A.L, A.chunk_max, A.min_tiles);
+                                   hm, small, (uint32_t)sms, rule, adj ? 1 : 0, A.L, A.chunk_max, A.min_tiles);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (small) return cudaSuccess;
@@ -1143,7 +1196,7 @@ cudaError_t launch_displace(const FwdConfig& cfg, const wt_patch* patches, uint3
     // with fewer waves than mma_patch asks for, no patch can qualify
     const bool mma = !naive && n_waves >= kMmaMinWaves;
     cudaError_t e = launch_prep(patches, n_patches, waves, n_waves, hm, out_capacity, 32u * cfg.s, ws, L, s,
-                                mma ? kMmaMaxWaves : 0u);
+                                MmaRule{mma ? kMmaMaxWaves : 0u, x.sums ? 64u : 0u});
     if (e != cudaSuccess) return e;
     if (naive) return launch_forward_naive(patches, n_patches, waves, hm, pos, nrm, flags, ws, L, out_capacity, s);
     if (mma) {

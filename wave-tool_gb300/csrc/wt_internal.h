@@ -160,6 +160,13 @@ inline int hm_kind(const HmDev& hm) {
 // Waves of a patch that runs as matrix products (mma_patch).
 constexpr uint32_t kMmaMinWaves = 8, kMmaMaxWaves = 128, kMmaAdjMaxWaves = 64;
 
+// What the prep queues as matrix products: the patches that mma_patch admits with at
+// most max_waves waves (0: none), in items of rows whose number is compared with
+// others (mma_compares) from `spread` rows an SM on (0: never).
+struct MmaRule {
+    uint32_t max_waves, spread;
+};
+
 // Limit of every wait inside the matrix-product kernels, in nanoseconds, and the
 // one that this thread's launches are given: tests of what a wait that runs out
 // leaves behind shorten it by the library's wt_internal_wait_limit, which is no part
@@ -177,12 +184,11 @@ struct AdjScanArgs {
 
 // ---- launchers (wt_displace.cu) -------------------------------------------
 // tile_cols: tile width (each row's last tile narrower, see tiles_per_row);
-// mma_max_waves: the patches that qualify (mma_patch) with at most this many waves
-// are queued for the matrix-product kernel (0: none)
+// rule: the patches that are queued for the matrix-product kernel
 cudaError_t launch_prep(const wt_patch* patches, uint32_t n_patches, const wt_wave* waves,
                         uint32_t n_waves, const HmDev& hm, uint64_t out_capacity,
                         uint32_t tile_cols, void* ws, const WsLayout& L, cudaStream_t s,
-                        uint32_t mma_max_waves, const AdjScanArgs* adj = nullptr);
+                        const MmaRule& rule, const AdjScanArgs* adj = nullptr);
 // pos may be NULL only with x.view set
 cudaError_t launch_forward(const FwdConfig& cfg, const wt_patch* patches, uint32_t n_patches,
                            const HmDev& hm, float* pos, float* nrm, uint32_t flags, void* ws,
