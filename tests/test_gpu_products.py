@@ -162,3 +162,23 @@ def test_displacements_of_a_patch_wider_than_float(wt, gpu, alone):
     assert bool(torch.isfinite(pos).all())
     most = float(np.abs(waves["amplitude"] * np.maximum(1.0, waves["steepness_q"])).sum())
     assert float(pos[:, :3].abs().max()) <= most
+
+
+@pytest.mark.parametrize("alone", [True, False])
+def test_saved_sums_off_a_sector(wt, gpu, alone):
+    """The saved sums on a 16-byte boundary that is no 32-byte one: the same bits."""
+    import torch
+    patches, waves, _ = patch_table(SIZES[0], 47, 0, None)
+    if alone:
+        patches = patches[3:4].copy()
+        patches["out_offset"] = 0
+    surf = wt.Surface(patches, waves)
+    want = torch.zeros((surf.n_vertices, 8), device="cuda")
+    p0, n0 = surf.displace(flags=1, sums=want)
+    buf = torch.zeros(8 * surf.n_vertices + 8, device="cuda")
+    off = buf[4:4 + 8 * surf.n_vertices].view(-1, 8)
+    assert want.data_ptr() % 32 == 0 and off.data_ptr() % 32 == 16
+    p1, n1 = surf.displace(flags=1, sums=off)
+    assert surf.status()[0] == 0
+    assert torch.equal(off, want) and torch.equal(p1, p0) and torch.equal(n1, n0)
+    assert bool((buf[:4] == 0).all()) and bool((buf[-4:] == 0).all())
