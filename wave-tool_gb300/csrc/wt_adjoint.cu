@@ -16,7 +16,7 @@
 //       the chunk's record for that wave (no cross-lane reduction).
 //   k_adjoint_mma  parallelogram patches of 8 to 64 waves instead, before it
 //                (wt_adjoint_mma.cu; in tables with work enough,
-//                adjoint_mma_waves): the moments as matrix products, a record
+//                adjoint_mma_rule): the moments as matrix products, a record
 //                per item of 128 columns by a run of rows
 //   k_adj_cols   column sums of each patch's records over its chunks (FP32
 //                Kahan, fixed order)
@@ -550,16 +550,42 @@ uint64_t adjoint_records(const wt_patch& p) {
 // 33.2, 4 of 64^2 with 32 31.7 / 30.6, one of 192^2 with 32 31.7 / 42.3.  Patches
 // of fewer columns leave most of an item's 128 empty (16 of 32^2 with 32 waves
 // 38.1 / 34.2): they run as products only in a table that has them anyway.
-uint32_t adjoint_mma_waves(const wt_patch* host_patches, uint32_t n_patches, uint32_t n_waves, bool saved) {
-    uint64_t left = saved ? 9ull << 16 : 6ull << 16;
-    for (uint32_t i = 0; n_waves >= kMmaMinWaves && i < n_patches; ++i) {
+// The products take about as long for a row of a column block of one column and 8
+// waves as for one of 128 and 64 (2.6 ns, 3 to 4 where few items share the SMs), the
+// recurrence 8.4 + 1.57 waves ps a vertex (from saved sums 10.8 + 1.06 waves), so
+// patches of few waves, and in small tables those of part-filled column blocks,
+// stay with it, if they are tiles enough to keep its warps at work.  Measured,
+// recurrence / products, us: 40 of 129 x 200, 8 waves 57 / 91, 32 105 / 102; of 256 x
+// 200, 12 waves 78 / 95, 24 115 / 101; of 520 x 200 (80000 vertices more than fill
+// the SMs once), 8 waves 115 / 132, 12 145 / 134; 10 of 1000 x 600, 8 waves 149 /
+// 163, 12 181 / 168; from saved sums 40 of 520 x 200, 16 waves 135 / 151, 24 177 /
+// 153, of 129 x 200, 32 waves 84 / 93, 48 111 / 100.  (64 patches of 64-1024 side
+// with 8-64 waves with their poor patches left out 442, with them 427, so only from
+// kFewTiles tiles on; one of 3000 x 2000, 8 waves, 224 / 137: mma_fills.)
+MmaRule adjoint_mma_rule(const wt_patch* host_patches, uint32_t n_patches, uint32_t n_waves, bool saved) {
+    constexpr uint64_t kFewTiles = 6000, kManyBlocks = 20000;  // (blocks: rows times column blocks)
+    const MmaRule any{kMmaMinWaves, kMmaAdjMaxWaves, 1u, 0u, 0u};
+    if (n_waves < kMmaMinWaves) return MmaRule{};
+    const auto qualifies = [&](const wt_patch& p, const MmaRule& rule) { return p.cols >= 64 && dev::mma_patch(p, rule); };
+    uint64_t blocks = 0, poor = 0;
+    for (uint32_t i = 0; i < n_patches; ++i)
+        if (qualifies(host_patches[i], any)) blocks += (uint64_t)host_patches[i].rows * ((host_patches[i].cols + 127u) / 128u);
+    MmaRule rule = blocks >= kManyBlocks ? MmaRule{saved ? 20u : 11u, kMmaAdjMaxWaves, 1u, 0u, 0u}
+                                         : MmaRule{kMmaMinWaves, kMmaAdjMaxWaves, 1u, saved ? 10u : 5u, saved ? 3400u : 2450u};
+    for (uint32_t i = 0; i < n_patches; ++i) {
         const wt_patch& p = host_patches[i];
-        if (p.cols < 64 || !dev::mma_patch(p, kMmaAdjMaxWaves)) continue;
+        if (qualifies(p, any) && !dev::mma_fills(p, rule)) poor += (uint64_t)p.rows * dev::tiles_per_row(p.cols, 8);
+    }
+    if (poor < kFewTiles) rule = any;
+    uint64_t left = saved ? 9ull << 16 : 6ull << 16;
+    for (uint32_t i = 0; i < n_patches; ++i) {
+        const wt_patch& p = host_patches[i];
+        if (!qualifies(p, rule)) continue;
         const uint64_t terms = (uint64_t)p.cols * p.rows * p.wave_count;
-        if (terms >= left) return kMmaAdjMaxWaves;
+        if (terms >= left) return rule;
         left -= terms;
     }
-    return 0;
+    return MmaRule{};
 }
 
 cudaError_t launch_adjoint(const wt_patch* patches, uint32_t n_patches, const wt_wave* waves, uint32_t n_waves,

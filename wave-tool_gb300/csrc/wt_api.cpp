@@ -333,13 +333,13 @@ static wt_status run_adjoint(const wt_patch* host_patches, const wt_patch* patch
     wt::AdjScanArgs args;
     cudaError_t e = wt::adjoint_scan_args(sums != nullptr, L, &args);
     if (e != cudaSuccess) return cuda_fail(e, "adjoint set-up");
-    const uint32_t mma_waves = wt::adjoint_mma_waves(host_patches, n_patches, n_waves, sums != nullptr);
+    const wt::MmaRule rule = wt::adjoint_mma_rule(host_patches, n_patches, n_waves, sums != nullptr);
     e = wt::launch_prep(patches, n_patches, waves, n_waves, P.hm, out_capacity, 256u, workspace, L.f, s,
-                        wt::MmaRule{mma_waves, 1u}, &args);
+                        rule, &args);
     if (e != cudaSuccess) return cuda_fail(e, "prep launch");
     uint32_t maxw = 0;
     for (uint32_t i = 0; i < n_patches; ++i) maxw = host_patches[i].wave_count > maxw ? host_patches[i].wave_count : maxw;
-    e = wt::launch_adjoint(patches, n_patches, waves, n_waves, maxw > 0 ? maxw : 1, mma_waves > 0, P.hm, d_pos, d_nrm, flags, grad_out,
+    e = wt::launch_adjoint(patches, n_patches, waves, n_waves, maxw > 0 ? maxw : 1, rule.max_waves > 0, P.hm, d_pos, d_nrm, flags, grad_out,
                            workspace, L, sums, s);
     if (e != cudaSuccess) return cuda_fail(e, "adjoint launch");
     return WT_OK;

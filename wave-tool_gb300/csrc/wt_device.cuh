@@ -146,6 +146,19 @@ __host__ __device__ __forceinline__ bool mma_patch(const wt_patch& P, uint32_t m
            same_sum(P.tr[0], P.bl[0], P.tl[0], P.br[0]) && same_sum(P.tr[1], P.bl[1], P.tl[1], P.br[1]);
 }
 
+// The same by a rule: waves enough and full column blocks, except for a patch of
+// many tiles, whose records the recurrence's adjoint would add up for longer than
+// the products take.
+__host__ __device__ __forceinline__ bool mma_fills(const wt_patch& P, const MmaRule& rule) {
+    const uint32_t blocks = (P.cols + 127u) / 128u;
+    return (P.wave_count >= rule.min_waves &&
+            (uint64_t)P.cols * (P.wave_count + rule.more) >= (uint64_t)rule.fill * blocks) ||
+           (uint64_t)P.rows * tiles_per_row(P.cols, 8) > 3000u;
+}
+__host__ __device__ __forceinline__ bool mma_patch(const wt_patch& P, const MmaRule& rule) {
+    return mma_patch(P, rule.max_waves) && mma_fills(P, rule);
+}
+
 // A wave whose sum coefficients leave room for the products' scales (finite, and
 // far from FP32's limits): amplitude, Q times it, and both times the wave number
 // at most 1e12.
