@@ -61,3 +61,19 @@ def test_part_filled_blocks_are_not_slower(wt, gpu, saved):
         g = torch.empty((surf.n_waves, 8), device="cuda")
         us.append(_graph_us(lambda: surf.adjoint(gp, gn, grad=g, sums=sums), n=5))
     assert us[0] <= 1.2 * us[1], us
+
+
+def test_a_mixed_table_is_one_kernel_s(wt, gpu):
+    """30 patches of 8 waves and 10 of 64: at most what the two kinds take as two
+    calls (split between recurrence and products in one call they took a tenth
+    more)."""
+    import torch
+
+    def us(w):
+        surf = wt.Surface(w.patches, w.waves)
+        gp, gn = (u.cuda() for u in _upstream(w.n_vertices, 5))
+        g = torch.empty((surf.n_waves, 8), device="cuda")
+        return _graph_us(lambda: surf.adjoint(gp, gn, grad=g), n=5)
+
+    few, many = _table(30, 520, 200, 8), _table(10, 520, 200, 64, seed=4)
+    assert us(_join(few, many)) <= us(few) + us(many)

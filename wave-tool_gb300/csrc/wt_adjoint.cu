@@ -550,42 +550,53 @@ uint64_t adjoint_records(const wt_patch& p) {
 // 33.2, 4 of 64^2 with 32 31.7 / 30.6, one of 192^2 with 32 31.7 / 42.3.  Patches
 // of fewer columns leave most of an item's 128 empty (16 of 32^2 with 32 waves
 // 38.1 / 34.2): they run as products only in a table that has them anyway.
-// The products take about as long for a row of a column block of one column and 8
-// waves as for one of 128 and 64 (2.6 ns, 3 to 4 where few items share the SMs), the
-// recurrence 8.4 + 1.57 waves ps a vertex (from saved sums 10.8 + 1.06 waves), so
-// patches of few waves, and in small tables those of part-filled column blocks,
-// stay with it, if they are tiles enough to keep its warps at work.  Measured,
-// recurrence / products, us: 40 of 129 x 200, 8 waves 57 / 91, 32 105 / 102; of 256 x
-// 200, 12 waves 78 / 95, 24 115 / 101; of 520 x 200 (80000 vertices more than fill
-// the SMs once), 8 waves 115 / 132, 12 145 / 134; 10 of 1000 x 600, 8 waves 149 /
-// 163, 12 181 / 168; from saved sums 40 of 520 x 200, 16 waves 135 / 151, 24 177 /
-// 153, of 129 x 200, 32 waves 84 / 93, 48 111 / 100.  (64 patches of 64-1024 side
-// with 8-64 waves with their poor patches left out 442, with them 427, so only from
-// kFewTiles tiles on; one of 3000 x 2000, 8 waves, 224 / 137: mma_fills.)
-MmaRule adjoint_mma_rule(const wt_patch* host_patches, uint32_t n_patches, uint32_t n_waves, bool saved) {
-    constexpr uint64_t kFewTiles = 6000, kManyBlocks = 20000;  // (blocks: rows times column blocks)
-    const MmaRule any{kMmaMinWaves, kMmaAdjMaxWaves, 1u, 0u, 0u};
-    if (n_waves < kMmaMinWaves) return MmaRule{};
-    const auto qualifies = [&](const wt_patch& p, const MmaRule& rule) { return p.cols >= 64 && dev::mma_patch(p, rule); };
-    uint64_t blocks = 0, poor = 0;
-    for (uint32_t i = 0; i < n_patches; ++i)
-        if (qualifies(host_patches[i], any)) blocks += (uint64_t)host_patches[i].rows * ((host_patches[i].cols + 127u) / 128u);
-    MmaRule rule = blocks >= kManyBlocks ? MmaRule{saved ? 20u : 11u, kMmaAdjMaxWaves, 1u, 0u, 0u}
-                                         : MmaRule{kMmaMinWaves, kMmaAdjMaxWaves, 1u, saved ? 10u : 5u, saved ? 3400u : 2450u};
-    for (uint32_t i = 0; i < n_patches; ++i) {
-        const wt_patch& p = host_patches[i];
-        if (qualifies(p, any) && !dev::mma_fills(p, rule)) poor += (uint64_t)p.rows * dev::tiles_per_row(p.cols, 8);
+// The products take as long for a row of a column block of one column and 8 waves as
+// for one of 128 and 64, so tables of few waves or part-filled blocks are left to the
+// recurrence, as a whole (a table split between the two waits for each in turn: 30
+// patches of 520 x 200 with 8 waves and 10 with 64, 149 us by products, 182 split),
+// if they are tiles enough to keep its warps at work and no patch has so many that
+// adding up its records takes longer (one of 3000 x 2000, 8 waves: 224 by recurrence,
+// 137).  Both sides by what they measured: 0.37 us a row on the fullest SM (from
+// saved sums 0.41), 8.4 + 1.57 waves ps (10.8 + 1.06 waves) a vertex, columns rounded
+// up to 32.  Measured, recurrence / products, us: 40 of 129 x 200, 8 waves 60 / 94, 32
+// 108 / 106; of 256 x 200, 12 waves 83 / 100, 24 115 / 104; of 520 x 200, 8 waves 129 /
+// 137, 12 145 / 140; 64 of 200 x 150, 16 waves 104 / 100; 30 of 300 x 160, 16 waves 83 /
+// 72; 10 of 1000 x 600, 8 waves 153 / 170, 12 181 / 175; from saved sums 40 of 520 x
+// 200, 16 waves 135 / 151, 24 177 / 153, of 129 x 200, 32 waves 87 / 96, 48 111 / 100; 64
+// of 200 x 150, 16 waves 96 / 111.
+MmaRule adjoint_mma_rule(const wt_patch* host_patches, uint32_t n_patches, uint32_t n_waves, uint32_t sms, bool saved) {
+    constexpr uint64_t kFewTiles = 6000, kLongPatch = 3000;
+    const MmaRule rule{kMmaAdjMaxWaves, 1u};
+    uint64_t rowct = 0, terms = 0, tiles = 0, longest = 0;
+    double recurrence = 0.0;  // us
+    const auto each = [&](auto f) {
+        for (uint32_t i = 0; n_waves >= kMmaMinWaves && i < n_patches; ++i)
+            if (host_patches[i].cols >= 64 && dev::mma_patch(host_patches[i], kMmaAdjMaxWaves)) f(host_patches[i]);
+    };
+    each([&](const wt_patch& p) {
+        const uint64_t t = (uint64_t)p.rows * dev::tiles_per_row(p.cols, 8);
+        tiles += t;
+        longest = t > longest ? t : longest;
+        rowct += (uint64_t)p.rows * ((p.cols + 127u) / 128u);
+        terms += (uint64_t)p.cols * p.rows * p.wave_count;
+        recurrence += 1e-6 * (double)p.rows * ((p.cols + 31u) & ~31u) *
+                      (saved ? 10.8 + 1.06 * p.wave_count : 8.4 + 1.57 * p.wave_count);
+    });
+    if (terms < (saved ? 9ull << 16 : 6ull << 16)) return MmaRule{};
+    if (tiles < kFewTiles || longest > kLongPatch) return rule;
+    // the items, as the prep finds them
+    uint32_t items[dev::kItemChoices] = {};
+    const auto count = [&](uint32_t k) {
+        const uint32_t h = dev::mma_item_rows(rowct, sms, k);
+        each([&](const wt_patch& p) { items[k] += (p.cols + 127u) / 128u * ((p.rows + h - 1u) / h); });
+    };
+    count(0);
+    uint32_t k = 0;
+    if (dev::mma_compares(rule, rowct, items[0], sms)) {
+        for (k = 1; k < dev::kItemChoices; ++k) count(k);
+        k = dev::mma_item_choice(rowct, sms, items);
     }
-    if (poor < kFewTiles) rule = any;
-    uint64_t left = saved ? 9ull << 16 : 6ull << 16;
-    for (uint32_t i = 0; i < n_patches; ++i) {
-        const wt_patch& p = host_patches[i];
-        if (!qualifies(p, rule)) continue;
-        const uint64_t terms = (uint64_t)p.cols * p.rows * p.wave_count;
-        if (terms >= left) return rule;
-        left -= terms;
-    }
-    return MmaRule{};
+    return recurrence < (saved ? 0.41 : 0.37) * dev::mma_item_cost(rowct, sms, items[k]) ? MmaRule{} : rule;
 }
 
 cudaError_t launch_adjoint(const wt_patch* patches, uint32_t n_patches, const wt_wave* waves, uint32_t n_waves,

@@ -333,7 +333,7 @@ static wt_status run_adjoint(const wt_patch* host_patches, const wt_patch* patch
     wt::AdjScanArgs args;
     cudaError_t e = wt::adjoint_scan_args(sums != nullptr, L, &args);
     if (e != cudaSuccess) return cuda_fail(e, "adjoint set-up");
-    const wt::MmaRule rule = wt::adjoint_mma_rule(host_patches, n_patches, n_waves, sums != nullptr);
+    const wt::MmaRule rule = wt::adjoint_mma_rule(host_patches, n_patches, n_waves, (uint32_t)wt::sm_count(), sums != nullptr);
     e = wt::launch_prep(patches, n_patches, waves, n_waves, P.hm, out_capacity, 256u, workspace, L.f, s,
                         rule, &args);
     if (e != cudaSuccess) return cuda_fail(e, "prep launch");

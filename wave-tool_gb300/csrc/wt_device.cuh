@@ -146,19 +146,6 @@ __host__ __device__ __forceinline__ bool mma_patch(const wt_patch& P, uint32_t m
            same_sum(P.tr[0], P.bl[0], P.tl[0], P.br[0]) && same_sum(P.tr[1], P.bl[1], P.tl[1], P.br[1]);
 }
 
-// The same by a rule: waves enough and full column blocks, except for a patch of
-// many tiles, whose records the recurrence's adjoint would add up for longer than
-// the products take.
-__host__ __device__ __forceinline__ bool mma_fills(const wt_patch& P, const MmaRule& rule) {
-    const uint32_t blocks = (P.cols + 127u) / 128u;
-    return (P.wave_count >= rule.min_waves &&
-            (uint64_t)P.cols * (P.wave_count + rule.more) >= (uint64_t)rule.fill * blocks) ||
-           (uint64_t)P.rows * tiles_per_row(P.cols, 8) > 3000u;
-}
-__host__ __device__ __forceinline__ bool mma_patch(const wt_patch& P, const MmaRule& rule) {
-    return mma_patch(P, rule.max_waves) && mma_fills(P, rule);
-}
-
 // A wave whose sum coefficients leave room for the products' scales (finite, and
 // far from FP32's limits): amplitude, Q times it, and both times the wave number
 // at most 1e12.
@@ -171,7 +158,7 @@ __device__ __forceinline__ bool mma_wave(const wt_wave& w) {
 // patches' 128-column blocks): a whole number of items per SM, as few as make
 // them at most 128 rows (operand A, formed once per item, is then a tenth of its
 // work), and k more.
-__device__ __forceinline__ uint32_t mma_item_rows(uint64_t rowct, uint32_t sms, uint32_t k) {
+__host__ __device__ __forceinline__ uint32_t mma_item_rows(uint64_t rowct, uint32_t sms, uint32_t k) {
     const uint32_t r = (uint32_t)min(rowct, (uint64_t)0xf0000000u);  // (beyond, 128 rows either way)
     const uint32_t w = (r + 128u * sms - 1u) / (128u * sms) + k;
     return max((r + sms * w - 1u) / (sms * w), 4u);
@@ -188,18 +175,22 @@ __device__ __forceinline__ uint32_t mma_item_rows(uint64_t rowct, uint32_t sms, 
 // if compared, plain 19.6 -> 23.1.)
 constexpr uint32_t kItemChoices = 4;
 constexpr float kItemRows = 6.0f;  // what an item costs besides its rows, in rows
-__device__ __forceinline__ bool mma_compares(const MmaRule& rule, uint64_t rowct, uint32_t items, uint32_t sms) {
+__host__ __device__ __forceinline__ bool mma_compares(const MmaRule& rule, uint64_t rowct, uint32_t items, uint32_t sms) {
     return rule.spread > 0 && rowct >= (uint64_t)rule.spread * sms &&
            (uint64_t)((items + sms - 1u) / sms) * sms * 6u > (uint64_t)items * 7u;
 }
-// The choice with the least work on the fullest SM, for items of average rows
-// (items: their count for each k).
-__device__ __forceinline__ uint32_t mma_item_choice(uint64_t rowct, uint32_t sms, const uint32_t* items) {
+// The work on the fullest SM, in rows, for items of average rows, and the choice
+// with the least of it (items: their count for each k).
+__host__ __device__ __forceinline__ float mma_item_cost(uint64_t rowct, uint32_t sms, uint32_t items) {
+    const float n = (float)items;
+    return (float)((items + sms - 1u) / sms) * fmaf(kItemRows, n, (float)rowct) / n;
+}
+__host__ __device__ __forceinline__ uint32_t mma_item_choice(uint64_t rowct, uint32_t sms, const uint32_t* items) {
     uint32_t best = 0;
     float least = INFINITY;
 #pragma unroll 1
     for (uint32_t k = 0; k < kItemChoices; ++k) {
-        const float n = (float)items[k], cost = (float)((items[k] + sms - 1u) / sms) * fmaf(kItemRows, n, (float)rowct) / n;
+        const float cost = mma_item_cost(rowct, sms, items[k]);
         if (cost < least) {
             least = cost;
             best = k;

@@ -180,7 +180,7 @@ __device__ void prep_small(const wt_patch* __restrict__ patches, uint32_t n, con
             ok = patch_ok(P, n_waves, out_capacity);
             wc = ok ? P.wave_count : 0u;
             tiles_p = ok ? P.rows * tiles_per_row(P.cols, tile_cols / 32) : 0u;
-            mma_p = ok && mma_patch(P, rule);
+            mma_p = ok && mma_patch(P, rule.max_waves);
         }
         uint32_t x = wc;  // inclusive prefix of the pair counts
         for (int o = 1; o < 32; o <<= 1) {
@@ -468,7 +468,7 @@ __device__ void prep_medium(const wt_patch* __restrict__ patches, uint32_t n, co
     if (p < n) {
         const wt_patch P = patches[p];
         ok = patch_ok(P, n_waves, out_capacity);
-        mma = ok && mma_patch(P, rule);
+        mma = ok && mma_patch(P, rule.max_waves);
         count = ok ? P.wave_count : 0u;
         tl = ok ? P.rows * tiles_per_row(P.cols, tile_cols / 32) : 0u;
         rows = P.rows;
@@ -673,7 +673,7 @@ __global__ void __launch_bounds__(1024) k_prep_scan(const wt_patch* __restrict__
         unsigned long long rowct = 0;
         for (uint32_t p = threadIdx.x; p < n; p += blockDim.x) {
             const wt_patch P = patches[p];
-            const bool ok = patch_ok(P, n_waves, out_capacity), mma = ok && mma_patch(P, rule);
+            const bool ok = patch_ok(P, n_waves, out_capacity), mma = ok && mma_patch(P, rule.max_waves);
             if (!ok) flag_error(hdr, WT_ERR_INVALID_ARG, p);
             pair_off[p] = ok ? P.wave_count : 0u;
             tiles[p] = ok ? P.rows * tiles_per_row(P.cols, tile_cols / 32) | (mma ? kMmaFlag : 0u) : 0u;
@@ -1196,7 +1196,7 @@ cudaError_t launch_displace(const FwdConfig& cfg, const wt_patch* patches, uint3
     // with fewer waves than mma_patch asks for, no patch can qualify
     const bool mma = !naive && n_waves >= kMmaMinWaves;
     cudaError_t e = launch_prep(patches, n_patches, waves, n_waves, hm, out_capacity, 32u * cfg.s, ws, L, s,
-                                MmaRule{kMmaMinWaves, mma ? kMmaMaxWaves : 0u, x.sums ? 64u : 0u, 0u, 0u});
+                                MmaRule{mma ? kMmaMaxWaves : 0u, x.sums ? 64u : 0u});
     if (e != cudaSuccess) return e;
     if (naive) return launch_forward_naive(patches, n_patches, waves, hm, pos, nrm, flags, ws, L, out_capacity, s);
     if (mma) {

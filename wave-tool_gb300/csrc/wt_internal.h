@@ -160,13 +160,11 @@ inline int hm_kind(const HmDev& hm) {
 // Waves of a patch that runs as matrix products (mma_patch).
 constexpr uint32_t kMmaMinWaves = 8, kMmaMaxWaves = 128, kMmaAdjMaxWaves = 64;
 
-// What the prep queues as matrix products: the patches that mma_patch admits with
-// min_waves to max_waves waves (max_waves 0: none) and that fill their 128-column
-// blocks (mma_fills: a block's columns on average times waves + more, at least
-// fill), in items of rows whose number is compared with others (mma_compares) from
-// `spread` rows an SM on (0: never).
+// What the prep queues as matrix products: the patches that mma_patch admits with at
+// most max_waves waves (0: none), in items of rows whose number is compared with
+// others (mma_compares) from `spread` rows an SM on (0: never).
 struct MmaRule {
-    uint32_t min_waves, max_waves, spread, more, fill;
+    uint32_t max_waves, spread;
 };
 
 // Limit of every wait inside the matrix-product kernels, in nanoseconds, and the
@@ -222,7 +220,7 @@ cudaError_t launch_single(const FwdConfig& cfg, const wt_patch* patches, const w
 uint64_t adjoint_records(const wt_patch& p);
 // The patches of the matrix-product kernel for an adjoint over this table (saved:
 // from saved sums); max_waves 0: it does not run.
-MmaRule adjoint_mma_rule(const wt_patch* host_patches, uint32_t n_patches, uint32_t n_waves, bool saved);
+MmaRule adjoint_mma_rule(const wt_patch* host_patches, uint32_t n_patches, uint32_t n_waves, uint32_t sms, bool saved);
 // The scan arguments of an adjoint over layout L (saved: from saved sums).
 cudaError_t adjoint_scan_args(bool saved, const AdjLayout& L, AdjScanArgs* out);
 // The patches the prep queued as matrix products (wt_adjoint_mma.cu); exits at
