@@ -58,3 +58,27 @@ def test_an_uneven_table_is_not_much_slower(wt, gpu):
         sums = torch.empty((surf.n_vertices, 8), device="cuda")
         us.append(_graph_us(lambda: surf.displace(pos, nrm, sums=sums), n=5))
     assert us[0] <= 1.25 * us[1], us
+
+
+@pytest.mark.parametrize("sizes", [[(503, 503, 9), (40, 40, 50), (123, 123, 25), (130, 131, 14), (114, 114, 36)],
+                                   [(700, 100, 8)] * 12])
+def test_patches_of_different_sizes(wt, oracle, gpu, sizes):
+    """Gradients where the number of items per SM is chosen for patches unlike one
+    another, and where the choices come out alike."""
+    parts = [_table(1, c, r, k, seed=5 + i) for i, (c, r, k) in enumerate(sizes)]
+    patches, waves, v = [], [], 0
+    for t in parts:
+        p = t.patches.copy()
+        p["wave_offset"], p["out_offset"] = len(waves), v
+        patches.append(p)
+        waves.extend(t.waves)
+        v += t.n_vertices
+    w = SimpleNamespace(patches=np.concatenate(patches), waves=np.array(waves, dtype=parts[0].waves.dtype), heightmap=None,
+                        n_vertices=v)
+    gp, gn = _upstream(v, 6)
+    g64 = oracle.adjoint_f64(w.patches, w.waves, gp.numpy(), gn.numpy())
+    for saved in (False, True):
+        g, _ = run_adjoint(wt, w, gp, gn, saved=saved)
+        for p in w.patches:
+            at = slice(int(p["wave_offset"]), int(p["wave_offset"]) + int(p["wave_count"]))
+            _check(g[at], g64[at])

@@ -174,22 +174,24 @@ __host__ __device__ __forceinline__ uint32_t mma_item_rows(uint64_t rowct, uint3
 // 57.3 and 35.5 -> 28.2.  (Saving forward of 64 columns, 53 rows an SM: 20.9 -> 25.4
 // if compared, plain 19.6 -> 23.1.)
 constexpr uint32_t kItemChoices = 4;
-constexpr float kItemRows = 6.0f;  // what an item costs besides its rows, in rows
+constexpr float kItemRows = 8.0f;  // what an item costs besides its rows, in rows
 __host__ __device__ __forceinline__ bool mma_compares(const MmaRule& rule, uint64_t rowct, uint32_t items, uint32_t sms) {
     return rule.spread > 0 && rowct >= (uint64_t)rule.spread * sms &&
            (uint64_t)((items + sms - 1u) / sms) * sms * 6u > (uint64_t)items * 7u;
 }
 // The work on the fullest SM, in rows, for items of average rows, and the choice
-// with the least of it (items: their count for each k).
+// with the least of it, where that is a twentieth less than the first's (items: their
+// count for each k; 12 patches of 700 x 300, 16 waves, 204 against 203 rows: adjoint
+// 98.5 -> 103.6 us without that margin).
 __host__ __device__ __forceinline__ float mma_item_cost(uint64_t rowct, uint32_t sms, uint32_t items) {
     const float n = (float)items;
     return (float)((items + sms - 1u) / sms) * fmaf(kItemRows, n, (float)rowct) / n;
 }
 __host__ __device__ __forceinline__ uint32_t mma_item_choice(uint64_t rowct, uint32_t sms, const uint32_t* items) {
     uint32_t best = 0;
-    float least = INFINITY;
+    float least = 0.95f * mma_item_cost(rowct, sms, items[0]);
 #pragma unroll 1
-    for (uint32_t k = 0; k < kItemChoices; ++k) {
+    for (uint32_t k = 1; k < kItemChoices; ++k) {
         const float cost = mma_item_cost(rowct, sms, items[k]);
         if (cost < least) {
             least = cost;
