@@ -7,8 +7,8 @@
 // the caller, :1073).
 //
 // Three launches (two when the scan kernel forms the constants: small tables), and
-// before the last one the matrix products of parallelogram patches (wt_mma.cu)
-// when the call has 8 waves or more; one launch for one patch (wt_single.cu).  All
+// before or after the last one (launch_displace) the matrix products of parallelogram
+// patches (wt_mma.cu) when the call has 8 waves or more; one launch for one patch (wt_single.cu).  All
 // stream-ordered and graph-capturable:
 //   k_prep_scan              validate patches and waves, prefix sums, LPT sort
 //                            of patches by wave count, tile queue reset (one
@@ -1199,11 +1199,21 @@ cudaError_t launch_displace(const FwdConfig& cfg, const wt_patch* patches, uint3
                                 MmaRule{mma ? kMmaMaxWaves : 0u, x.sums ? 64u : 0u});
     if (e != cudaSuccess) return e;
     if (naive) return launch_forward_naive(patches, n_patches, waves, hm, pos, nrm, flags, ws, L, out_capacity, s);
-    if (mma) {
-        e = launch_forward_mma(patches, hm, pos, nrm, flags, ws, L, x, s);
-        if (e != cudaSuccess) return e;
-    }
-    return launch_forward(cfg, patches, n_patches, hm, pos, nrm, flags, ws, L, x, s);
+    const auto recurrence = [&] { return launch_forward(cfg, patches, n_patches, hm, pos, nrm, flags, ws, L, x, s); };
+    const auto products = [&] {
+        return mma ? launch_forward_mma(patches, hm, pos, nrm, flags, ws, L, x, s) : cudaSuccess;
+    };
+    // The products' kernel takes nearly all of an SM's shared memory, also for a table
+    // without a patch of theirs, and what follows it starts later and with less cache.
+    // Tables too large for the recurrence kernel's table in shared memory look their
+    // tiles up through that cache: recurrence first (5000 skewed patches of 24 x 24, 9
+    // waves, 231.8 -> 225.5 us, saving 252.6 -> 240.2; 1200 of 16 x 16 55.5 -> 53.5).  The
+    // others the other way round (200 parallelograms of 200 x 100, 8 waves, saving, 63.1
+    // against 67.5; 64 of 64-128 side 25.7 against 27.2; 700 skewed 43.4 and 43.3).
+    const bool first = n_patches <= kTabPatches;
+    e = first ? products() : recurrence();
+    if (e != cudaSuccess) return e;
+    return first ? recurrence() : products();
 }
 
 cudaError_t launch_forward_naive(const wt_patch* patches, uint32_t n_patches, const wt_wave* waves,
