@@ -182,3 +182,28 @@ def test_saved_sums_off_a_sector(wt, gpu, alone):
     assert surf.status()[0] == 0
     assert torch.equal(off, want) and torch.equal(p1, p0) and torch.equal(n1, n0)
     assert bool((buf[:4] == 0).all()) and bool((buf[-4:] == 0).all())
+
+
+# A normal from the saved sums: 1 - sum, two products and their rounding, the inverse
+# root (2 ulp) and the product with it, at most 8 x 2^-24 in all, twice that where the
+# cross product's terms add up.
+@pytest.mark.parametrize("cols", [32, 33, 64, 65, 95, 96, 97, 128, 129, 160, 223])
+@pytest.mark.parametrize("alone", [True, False])
+def test_saved_sums_at_every_width(wt, gpu, cols, alone):
+    """All eight sums of each vertex in their places, where warps of the epilogue have
+    all, some or none of their 32 columns: the displacement's three are the outputs,
+    the slopes' five give the normals."""
+    import torch
+    patches, waves, _ = patch_table([(cols, 21, 9), (cols, 4, 60)], 11, 0, None)
+    patches["y_offset"] = 0.0
+    if alone:
+        patches = patches[:1].copy()
+    surf = wt.Surface(patches, waves)
+    sums = torch.full((surf.n_vertices + 1, 8), 7.0, device="cuda")
+    pos, nrm = surf.displace(flags=1, sums=sums[:-1])
+    assert surf.status()[0] == 0
+    assert torch.equal(sums[:-1, :3], pos[:, :3]) and bool((sums[-1] == 7.0).all())
+    jx, jz, sxx, sxz, szz = (sums[:-1, i].double() for i in (3, 4, 5, 6, 7))
+    n = torch.linalg.cross(torch.stack([-sxz, jz, 1 - szz], 1), torch.stack([1 - sxx, jx, -sxz], 1))
+    n = n / n.norm(dim=1, keepdim=True)
+    assert float((nrm[:, :3].double() - n).abs().max()) <= 2.0**-20

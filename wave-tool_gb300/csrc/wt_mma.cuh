@@ -366,24 +366,34 @@ struct Output {
 
 // One vertex from its sums and texels (world: the position in the world, else the
 // displacement alone, whatever the grid point: a patch may span more than FP32's
-// largest number).  Roundings spelt out where
-// a multiply-add could be fused one way in one output mode and another way in
+// largest number; whole: every lane of the warp has a vertex).  Roundings spelt out
+// where a multiply-add could be fused one way in one output mode and another way in
 // the next: every mode writes the same bits.
 template <int MODE, int HM>
 __device__ __forceinline__ void finish(const VertexSums& s, float xl, float zl, bool world, const PatchAux& a,
-                                       const HmDev& hm, const HmTexels& T, uint64_t v, const Output& o) {
+                                       const HmDev& hm, const HmTexels& T, uint64_t v, const Output& o, bool whole) {
     if (MODE == kModeSave) {
-        // On a 32-byte boundary (16 is asked for) a vertex's eight sums are one store, a
-        // whole sector, instead of two half ones: 40 patches of 129 x 200 x 8 36.1 ->
-        // 32.4 us, of 520 x 200 x 8 69.5 -> 65.9.
+        // 16 bytes a lane; where the warp's 32 columns all exist, two lanes exchange
+        // halves first, so that each store writes whole 32-byte sectors (a vertex's eight
+        // sums) instead of half ones.  Half sectors / one 32-byte store a lane / exchanged,
+        // us: 64 patches of 64-1024 side 230 / 215 / 204, 40 of 520 x 200, 8 waves, 71 / 66 /
+        // 64, 1100 of 128 x 100, 8 waves, 158 / 171 / 158, 24 waves 189 / 192 / 180.  Not in
+        // patches of up to 64 columns, where half of the epilogue's warps have no column and
+        // the others' instructions count: 1500 of 64 x 64, 16 waves, 107 / 117 / 117.
         float4* const at = o.sums + 2 * v;
-        if ((reinterpret_cast<uintptr_t>(o.sums) & 31u) == 0) {
-            asm volatile("st.global.cs.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(at), "f"(s.dx), "f"(s.dy),
-                         "f"(s.dz), "f"(s.jx), "f"(s.jz), "f"(s.sxx), "f"(s.sxz), "f"(s.szz)
-                         : "memory");
+        const float4 a4 = make_float4(s.dx, s.dy, s.dz, s.jx), b4 = make_float4(s.jz, s.sxx, s.sxz, s.szz);
+        if (whole) {
+            const bool odd = threadIdx.x & 1u;
+            float4 other = odd ? a4 : b4;
+            other.x = __shfl_xor_sync(0xffffffffu, other.x, 1);
+            other.y = __shfl_xor_sync(0xffffffffu, other.y, 1);
+            other.z = __shfl_xor_sync(0xffffffffu, other.z, 1);
+            other.w = __shfl_xor_sync(0xffffffffu, other.w, 1);
+            __stcs(odd ? at - 1 : at, odd ? other : a4);
+            __stcs(odd ? at + 1 : at + 2, odd ? b4 : other);
         } else {
-            __stcs(at, make_float4(s.dx, s.dy, s.dz, s.jx));
-            __stcs(at + 1, make_float4(s.jz, s.sxx, s.sxz, s.szz));
+            __stcs(at, a4);
+            __stcs(at + 1, b4);
         }
     }
     const float px0 = 1.0f - s.sxx, px2 = -s.sxz, pz0 = -s.sxz, pz2 = 1.0f - s.szz;
@@ -435,6 +445,7 @@ __device__ __forceinline__ void tile_epilogue(const Tile& t, const PatchAux& a, 
     const uint32_t at = t.acc + ((32u * quad) << 16);
     const uint64_t v0 = t.out0 + col;
     const bool in = col < t.cols;
+    const bool whole = MODE == kModeSave && t.cols > 64u && t.c0 + 32u * quad + 32u <= t.cols;  // the warp's columns
     const float4 i0 = t.inv[0], i1 = t.inv[1];
     float rowf = (float)(t.row0 + first);
     // two rows at a time: their texel loads are issued before the first is used
@@ -473,8 +484,8 @@ __device__ __forceinline__ void tile_epilogue(const Tile& t, const PatchAux& a, 
             else T[u] = HmTexels{};
         }
         if (in) {
-            finish<MODE, HM>(v[0], xl[0], zl[0], world, a, hm, T[0], v0 + r * t.cols, o);
-            if (second) finish<MODE, HM>(v[1], xl[1], zl[1], world, a, hm, T[1], v0 + (r + step) * t.cols, o);
+            finish<MODE, HM>(v[0], xl[0], zl[0], world, a, hm, T[0], v0 + r * t.cols, o, whole);
+            if (second) finish<MODE, HM>(v[1], xl[1], zl[1], world, a, hm, T[1], v0 + (r + step) * t.cols, o, whole);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
