@@ -561,7 +561,8 @@ wt_status wt_get_tuning(wt_tuning* tuning);
  * for the workload's shape bucket (the bit lengths of n_patches and n_waves, and
  * of out_capacity with one patch): later wt_gerstner_displace calls in that
  * bucket use it.  A workload none of whose patches depends on the shape (all
- * matrix products, see wt_tuning) is not timed and caches nothing.  Returns the
+ * matrix products, see wt_tuning) is not timed and caches nothing; with one
+ * patch the built-in shape's kernel and another shape's are timed against one another.  Returns the
  * shape in *best (may be NULL).  Arguments as wt_gerstner_displace; the outputs
  * are overwritten. */
 wt_status wt_autotune_displace(const wt_patch* patches, uint32_t n_patches,

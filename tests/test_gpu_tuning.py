@@ -113,3 +113,38 @@ def test_a_large_patch_does_not_tune_a_small_one(wt, gpu, default_tuning):
     assert (best["max_vertices_per_lane"], best["warps_per_block"], best["epilogue_in_shared"]) in SHAPES
     torch.cuda.synchronize()
     assert _one_launch(wt, wt.Surface(small.patches, small.waves))
+
+
+def test_one_patch_of_products_is_tuned_by_route(wt, gpu, default_tuning):
+    """A large patch of many waves is faster in the general path's launches than in the
+    one-patch kernel: the tuned call takes the faster of the two."""
+    import torch
+    from wave_tool_gb300 import workloads
+    w = workloads.config5(time_s=100.0)
+    surf = wt.Surface(w.patches, w.waves)
+    pos, nrm = surf.alloc_outputs(0)
+
+    def us():
+        best = 1e9
+        for _ in range(20):
+            pos.zero_()
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            surf.displace(pos, nrm, flags=0)
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b) * 1e3)
+        return best
+
+    default = wt.get_tuning()
+    one = us()
+    wt.set_tuning(16, 0, 32, 8, 0)
+    three = us()
+    wt.set_tuning(*[default[k] for k in ("warps_per_block", "blocks_per_sm", "wave_chunk", "max_vertices_per_lane",
+                                         "epilogue_in_shared")])
+    p0, n0 = surf.displace(flags=0)
+    surf.autotune(pos, nrm, reps=3)
+    tuned = us()
+    assert tuned <= 1.04 * min(one, three), (tuned, one, three)
+    p1, n1 = surf.displace(flags=0)
+    assert torch.equal(p0, p1) and torch.equal(n0, n1)

@@ -509,7 +509,9 @@ namespace {
 // noise, and later tables of the bucket would be given the winner.  For the same
 // reason a candidate has to be faster than `start` by 1 % and 1.5 us (the best of six
 // batches of one shape, repeated twelve times: 20.7 to 21.3 us, 35.8 to 36.9, 43.6
-// to 45.5).
+// to 45.5).  One patch that runs as matrix products has two routes, the one-patch
+// kernel of the built-in shape and the three launches of any other: those two are
+// timed (2048^2, 128 waves: 82 against 74 us; 1024^2, 32 waves, 19 against 21).
 constexpr float kTuneFactor = 0.99f, kTuneMs = 0.0015f;
 
 template <typename Run, typename Clear>
@@ -547,13 +549,16 @@ wt_status autotune(Run run, Clear clear, uint32_t bucket, uint32_t n_patches, ui
     // candidate's best of three batches over two passes: one batch per
     // candidate was enough for clock ramps and noise to reorder close shapes
     for (uint32_t r = 0; r < 4 * reps && st == WT_OK; ++r) st = run(start);
-    bool shaped = false;
+    bool shaped = false, routed = false;
     if (st == WT_OK && n_patches > 0) {
         wt::WsHeader h;
         e = cudaMemcpyAsync(&h, ws, sizeof(h), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) st = cuda_fail(e, "autotune: reading the workspace header");
-        else shaped = !(flags & WT_PHASE_FP32_NAIVE) && h.total_tiles > h.mma_items;
+        else if (!(flags & WT_PHASE_FP32_NAIVE)) {
+            shaped = h.total_tiles > h.mma_items;
+            routed = !shaped && n_patches == 1 && h.total_tiles > 0;
+        }
     }
     float start_ms = 1e30f;
     const auto timed_best = [&](const wt::FwdConfig& c, float* least) -> wt_status {
@@ -565,10 +570,11 @@ wt_status autotune(Run run, Clear clear, uint32_t bucket, uint32_t n_patches, ui
         }
         return st2;
     };
-    for (int pass = 0; pass < 2 && st == WT_OK && shaped; ++pass) {
+    for (int pass = 0; pass < 2 && st == WT_OK && (shaped || routed); ++pass) {
         st = timed_best(start, &start_ms);
         for (const auto& sh : shapes) {
             for (int ch : chunks) {
+                if (!shaped && !(sh[0] == 8 && sh[1] == 16 && ch == 32)) continue;  // (a route each)
                 const wt::FwdConfig c = {sh[0], ch, sh[1], 0, sh[2]};
                 float ms = best_ms;
                 if (st == WT_OK) st = timed_best(c, &ms);
@@ -580,7 +586,7 @@ wt_status autotune(Run run, Clear clear, uint32_t bucket, uint32_t n_patches, ui
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (st != WT_OK) return st;
-    if (shaped) {
+    if (shaped || (routed && (best_cfg.epi != start.epi || best_cfg.warps != start.warps || best_cfg.s != start.s))) {
         std::lock_guard<std::mutex> g(g_tune_mu);
         cache[bucket] = best_cfg;
     }
