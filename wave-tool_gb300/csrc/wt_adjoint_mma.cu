@@ -28,7 +28,7 @@
 // (about 400 instructions per 32 vertices: the normal's adjoint, the scales, 16
 // values split into hi and lo); the products take 30 % of the tensor pipe,
 // DRAM 19 % (dL/dpos and dL/dnrm once).  Measured, 64 patches of 64-1024 side
-// with 8-64 waves, 16 M vertices, the whole call: 432 us against 1054 with the
+// with 8-64 waves, 16 M vertices, the whole call: 433 us against 1056 with the
 // recurrence.  On the way: 8 vertex warps and 6 for operands 587 us; 16 and 2 of
 // them, gradients loaded a half tile ahead 490; the next tile's operand B before
 // this tile's sines 466; the sines in the queue's warp 445.  One scale for the

@@ -2,11 +2,14 @@
 // outputs that follow the displacement.
 //
 // The projected grid restates src/render-engine.cpp:797-1042 in FP64 as a
-// set of steps: wt_projected_grid runs them one after another on the host,
-// wt_projected_grid_async spreads them over the lanes of two warps of a kernel
-// that reads the camera from device memory, so that camera ->
-// corners -> displaced vertices is one stream of kernels a CUDA graph can
-// replay with a new camera every frame.
+// set of steps, twice: wt_projected_grid runs projected_grid() on the host,
+// wt_projected_grid_async a kernel that orders the same steps by the lanes of two
+// warps (k_projected_grid).  The two share the vectors, the bases, the camera's
+// checks and the frustum's edges; they round differently in FP64, and
+// test_async_projected_grid_matches_host holds the kernel to the host's results.
+// The kernel reads the camera from device memory, so that camera -> corners ->
+// displaced vertices is one stream of kernels a CUDA graph can replay with a new
+// camera every frame.
 //
 // k_vertex_stage computes the rest of water-grid.vert's outputs
 // (:150-158, :190-193) from the displaced positions and exact normals: a
@@ -48,14 +51,14 @@ struct M4 {
     double m[4][4];
 };
 
-WT_HD M4 identity() {
+inline M4 identity() {
     M4 r;
     for (int c = 0; c < 4; ++c)
         for (int k = 0; k < 4; ++k) r.m[c][k] = (c == k) ? 1.0 : 0.0;
     return r;
 }
 
-WT_HD M4 mul(const M4& a, const M4& b) {
+inline M4 mul(const M4& a, const M4& b) {
     M4 r;
     for (int c = 0; c < 4; ++c)
         for (int k = 0; k < 4; ++k) {
@@ -93,7 +96,7 @@ WT_HD Basis camera_basis(D3 pos, double cy, double sy, double sp, double cp) {
 
 // Right-handed look-at along the basis' forward vector (glm::lookAt, whose
 // side vector normalize(cross(forward, up)) is the basis' right vector).
-WT_HD M4 view_matrix(const Basis& b) {
+inline M4 view_matrix(const Basis& b) {
     const D3 s = b.right, u = b.up;
     M4 v = identity();
     v.m[0][0] = s.x; v.m[1][0] = s.y; v.m[2][0] = s.z; v.m[3][0] = -dot(s, b.pos);
@@ -103,7 +106,7 @@ WT_HD M4 view_matrix(const Basis& b) {
 }
 
 // OpenGL perspective, depth mapped to [-1, 1] (glm::perspective).
-WT_HD M4 perspective(double tan_half_fov, double aspect, double zn, double zf) {
+inline M4 perspective(double tan_half_fov, double aspect, double zn, double zf) {
     const double f = 1.0 / tan_half_fov;
     M4 p;
     for (int c = 0; c < 4; ++c)
@@ -151,7 +154,7 @@ struct Frame {
 // pos + d * (X*tx*right + Y*ty*up + fwd), tx = tan(fov/2) * aspect,
 // ty = tan(fov/2): the view-projection inverses the reference forms with
 // glm::inverse are used in this closed form.
-WT_HD void frame_setup(const wt_camera& c, double sy, double cy, double sp, double cp, double sf, double cf,
+inline void frame_setup(const wt_camera& c, double sy, double cy, double sp, double cp, double sf, double cf,
                        Frame* f) {
     f->amp = c.displaceable_amplitude;
     f->z_near = c.z_near;
@@ -192,7 +195,7 @@ WT_HD void frame_setup(const wt_camera& c, double sy, double cy, double sp, doub
 
 // Frustum corner i with NDC x and y widened (:815-838); bit 2 = right,
 // bit 1 = top, bit 0 = far.
-WT_HD D3 frustum_corner(const Frame& f, int i) {
+inline D3 frustum_corner(const Frame& f, int i) {
     const double depth = (i & 1) ? f.z_far : f.z_near;
     const double X = ((i & 4) ? kFrustumPad : -kFrustumPad) * f.tx * depth;
     const double Y = ((i & 2) ? kFrustumPad : -kFrustumPad) * f.ty * depth;
@@ -207,7 +210,7 @@ WT_HD int edge_end(int e, int which) {
 }
 
 // Where edge (e0, e1) crosses the planes y = +-amp (:857-883): 0 to 2 points.
-WT_HD int edge_points(const Frame& f, D3 e0, D3 e1, double px[2], double pz[2]) {
+inline int edge_points(const Frame& f, D3 e0, D3 e1, double px[2], double pz[2]) {
     if (e0.y == e1.y) return 0;  // parallel to the planes: no single crossing
     const double lo = fmin(e0.y, e1.y), hi = fmax(e0.y, e1.y);
     int n = 0;
@@ -224,7 +227,7 @@ WT_HD int edge_points(const Frame& f, D3 e0, D3 e1, double px[2], double pz[2]) 
 }
 
 // NDC of the base-plane point (px, 0, pz) in the projector (:993-1005).
-WT_HD void projector_ndc(const Frame& f, double px, double pz, double* X, double* Y) {
+inline void projector_ndc(const Frame& f, double px, double pz, double* X, double* Y) {
     const D3 q = D3{px, 0.0, pz} - f.pj.pos;
     const double iw = 1.0 / dot(f.pj.fwd, q);
     *X = dot(f.pj.right, q) * f.itx * iw;
@@ -232,7 +235,7 @@ WT_HD void projector_ndc(const Frame& f, double px, double pz, double* X, double
 }
 
 // The projector's ray through NDC (X, Y) cast onto y = 0 (:1007-1036).
-WT_HD bool corner_ray(const Frame& f, double X, double Y, double* cx, double* cz) {
+inline bool corner_ray(const Frame& f, double X, double Y, double* cx, double* cz) {
     const D3 dir = (X * f.tx) * f.pj.right + (Y * f.ty) * f.pj.up + f.pj.fwd;
     if (dir.y == 0.0) return false;
     const double t = -f.pj.pos.y / dir.y;
@@ -241,12 +244,12 @@ WT_HD bool corner_ray(const Frame& f, double X, double Y, double* cx, double* cz
     return isfinite(*cx) && isfinite(*cz);
 }
 
-WT_HD void view_matrices(const wt_camera& c, const Frame& f, double sy, double cy, M4* vp, M4* yaw) {
+inline void view_matrices(const wt_camera& c, const Frame& f, double sy, double cy, M4* vp, M4* yaw) {
     *vp = mul(perspective(f.ty, c.aspect, c.z_near, c.z_far), view_matrix(f.cam));
     *yaw = view_matrix(Basis{f.cam.pos, D3{cy, 0.0, sy}, D3{-sy, 0.0, cy}, D3{0.0, 1.0, 0.0}});
 }
 
-WT_HD void camera_trig(const wt_camera& c, int which, double* s, double* co) {
+inline void camera_trig(const wt_camera& c, int which, double* s, double* co) {
     if (which == 0) sincos_pi((c.yaw_deg - 360.0 * floor(c.yaw_deg / 360.0)) / 180.0, s, co);
     else if (which == 1) sincos_pi(fmin(fmax(c.pitch_deg, -kPitchLimit), kPitchLimit) / 180.0, s, co);
     else sincos_pi(c.fov_deg / 360.0, s, co);
@@ -289,7 +292,7 @@ inline void projected_grid(const wt_camera& c, Grid* g) {
     g->visible = true;
 }
 
-WT_HD void store_result(const wt_camera& c, const Grid& g, wt_patch* patch, wt_view* view) {
+inline void store_result(const wt_camera& c, const Grid& g, wt_patch* patch, wt_view* view) {
     if (view) {
         for (int col = 0; col < 4; ++col)
             for (int r = 0; r < 4; ++r) {

@@ -69,8 +69,8 @@ __device__ __forceinline__ float unordered(uint32_t k) {
 // tiles, normalise), 10.0 us this way; what is left is launches and latency
 // (33 MFMA, 2 MB).
 // A tile is 16 x 16 threads of M x M texels: M = 2 for layers that fill the GPU
-// only so, 4 where there are tiles enough (a quarter of the factors and half
-// the shared-memory reads per texel: 1024^2 x 64 terms 22.6 against 26.2 us,
+// only so, 4 where there are tiles enough (half of the factors and of the
+// shared-memory reads per texel: 1024^2 x 64 terms 22.6 against 26.2 us,
 // 2048^2 x 128 105 against 143 us).
 constexpr uint32_t kNoiseBlocks = 608; // resident blocks at most (4 per SM)
 __host__ __device__ constexpr uint32_t noise_tile(int m) { return 16u * (uint32_t)m; }

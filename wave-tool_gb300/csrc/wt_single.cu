@@ -12,9 +12,12 @@
 // operands (all warps form the first tile's) and the last issuing.  The same
 // device functions as the general path (wt_prep.cuh, wt_forward.cuh,
 // wt_mma.cuh), so the same bits.
-// Measured back to back (before: prep + forward kernels): 128^2 x 4 waves
-// 14.3 -> 8.0 us, 1024^2 x 32 34.8 -> 22.5 us, projected grid + vertex stage
-// 513^2 x 4 50.4 -> 32.8 us and 1024^2 x 32 with the noise layer 69.6 -> 56.5 us.
+// Measured back to back (before: prep + forward kernels): 128^2 x 4 waves 14.3 -> 8.4
+// us, 1024^2 x 32 34.8 -> 13.5 as products (22.5 by recurrence), 2048^2 x 128 244 ->
+// 75; projected grid + vertex stage (10 us of it the grid's kernel) 513^2 x 4 49 ->
+// 24.6 us and 1024^2 x 32 with the noise layer 69.7 -> 49.0.  From 64 waves on two
+// million vertices the general path's launches, with six warps for the operands,
+// take less (2048^2 x 128 72): the autotuner finds that.
 #include <cuda_runtime.h>
 
 #include <atomic>

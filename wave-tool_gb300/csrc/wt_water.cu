@@ -889,7 +889,8 @@ extern "C" wt_status wt_water_raster(const float* clip, uint64_t n_vertices, con
     e = launch_dependent(k_water_raster, dim3((unsigned)rb), s, static_cast<const int4*>(win), n_vertices, indices,
                          n_triangles, width, height, own_pixels(n_triangles), frag, queue_count, queue);
     if (e != cudaSuccess) return cuda_fail(e, "wt_water_raster launch");
-    // the queue: a resident grid, at most one warp per triangle
+    // the queue, whose length only the device knows: a resident grid, smaller for a
+    // mesh of fewer triangles than that has warps
     e = launch_dependent(k_water_raster_deferred,
                          dim3(resident_grid(k_water_raster_deferred, g_occ_deferred, sms, 32 * n_triangles)), s,
                          reinterpret_cast<const float4*>(clip), static_cast<const int4*>(win), width, height, frag,
